@@ -26,6 +26,7 @@ UNITS = {
     "tube.cu": ["-fmad=false"],
     "dense.cu": ["-fmad=false"],
     "sweep_f64.cu": [],
+    "sweep_split.cu": [],
     "sweep_f32.cu": ["-ftz=true"],
     "sweep_multi.cu": ["-ftz=true"],
     "sweep_combo32.cu": ["-ftz=true"],

@@ -96,6 +96,7 @@ Rec64 rec64(hz_operator *op)
     r.pos = op->pos64.as<double4_32a>();
     r.nrm = op->nrm64.as<double4_32a>();
     r.posk = op->posk64.ptr ? op->posk64.as<double4_32a>() : nullptr;
+    r.split = op->use_split ? &op->split : nullptr;
     return r;
 }
 
@@ -409,6 +410,7 @@ static int build_combo(hz_operator *op, int64_t *n_out)
                       op->delta.as<double>(), op->jac.as<double>(), op->reg.as<double>(), op->w.as<double>(),
                       op->adist.as<double>(), op->pos64.as<double4_32a>(), op->nrm64.as<double4_32a>(), s));
     HZ_CHECK_CUDA(cudaMemsetAsync(op->dreg.ptr, 0, nn * sizeof(double), s));
+    op->use_split = false;
     HZ_TRY(check_device_error(op, "hz_build (Combo)"));
     // FP32 records as the classic operator's (reg scaled by 4 pi: the Combo
     // kernel's c4 = 1/(4 pi) is folded into the densities), |d| in nrm32.w
@@ -472,7 +474,7 @@ int hz_set_wait_limit(long long polls)
 {
     if (polls < 0) polls = kWaitLimit;
     if (set_wait_limit_f32(polls) || set_wait_limit_combo32(polls) || set_wait_limit_f64(polls) ||
-        set_wait_limit_multi(polls)) {
+        set_wait_limit_multi(polls) || set_wait_limit_split(polls)) {
         set_error("hz_set_wait_limit: cudaMemcpyToSymbol failed");
         cudaGetLastError();
         return HZ_ERR_CUDA;
@@ -631,6 +633,16 @@ int hz_build(hz_operator *op, int64_t *n_out)
         op->posk64.release();
     }
     HZ_TRY(build_records32(op, sweep32_reg_scale(op->p.interior)));
+    const SweepConst sc = sweep_const(op);
+    op->use_split = split_serves(n, sc.wave, op->H, sc.extent);
+    if (op->use_split) {
+        HZ_TRY(op->split64.ensure(split_record_bytes(op->r32.npad)));
+        op->split = split_record_views(op->split64.ptr, op->r32);
+        HZ_TRY(build_split_records(sc, op->split, op->r32, op->pos64.as<double4_32a>(), op->nrm64.as<double4_32a>(),
+                                   s));
+    } else {
+        op->split64.release();
+    }
     // scratch for the FP64 sweep densities (double4_32a per point) and staging
     HZ_TRY(op->scratch.ensure(nn * sizeof(double4_32a) + 256));
     HZ_TRY(op->io.ensure(nn * sizeof(double) * 8));

@@ -70,11 +70,26 @@ struct DevBuf {
 };
 
 // ------------------------------------------------------------ sweep types
+// Records of the split FP64 sweep (sweep_split.cu), in the blocked sweep order.
+struct RecSplit {
+    int64_t npad = 0;
+    float4 *rec = nullptr;        // fixed source records
+    float4 *dens = nullptr;       // [2][npad] split densities of the product in hand
+    double4_32a *tile = nullptr;  // per tile: origin and radius times k
+    float2 *table = nullptr;      // cosines
+    int *expo = nullptr;          // density scales and their block maxima
+    const int *perm = nullptr;
+    const double4_32a *tpos = nullptr;
+    double4_32a *partial = nullptr;
+    size_t partial_bytes = 0;
+};
+
 // Source/target record of the FP64 sweep (lexicographic tube order).
 struct Rec64 {
     double4_32a *pos;  // x*, y*, z*, reg
     double4_32a *nrm;  // nx, ny, nz, w
     const double4_32a *posk = nullptr;  // k x*, k y*, k z*, reg (optional: the scaled FP64 sweep)
+    const RecSplit *split = nullptr;    // records of the split sweep, where it serves
 };
 
 // Tile geometry of the FP32 sweep.
@@ -205,11 +220,21 @@ int set_wait_limit_f32(long long polls);
 int set_wait_limit_combo32(long long polls);
 int set_wait_limit_f64(long long polls);
 int set_wait_limit_multi(long long polls);
+int set_wait_limit_split(long long polls);
 
 int sweep_f64(const SweepConst &c, const Rec64 &r, int mode, const double *p_re, const double *p_im,
               const double *pt_re, const double *pt_im, double *q_re, double *q_im, double *qt_re,
               double *qt_im, double2 *scratch, cudaStream_t s, cudaEvent_t ev0 = nullptr,
               cudaEvent_t ev1 = nullptr);
+// sweep_split.cu
+size_t split_record_bytes(int64_t npad);
+RecSplit split_record_views(void *mem, const Rec32 &r);
+bool split_serves(int64_t n, double wave, double H, double extent);
+int build_split_records(const SweepConst &c, const RecSplit &v, const Rec32 &r, const double4_32a *pos,
+                        const double4_32a *nrm, cudaStream_t s);
+int sweep_split(const SweepConst &c, const RecSplit &v, const double4_32a *nrm, int mode, const double *p_re,
+                const double *p_im, const double *pt_re, const double *pt_im, double *q_re, double *q_im,
+                double *qt_re, double *qt_im, cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1);
 // posk[i] = (k x, k y, k z, reg) of pos[i]: the FP64 sweep's scaled records.
 int scale_records64(int64_t n, double k, const double4_32a *pos, double4_32a *posk, cudaStream_t s);
 // sweep_f32.cu
@@ -272,6 +297,9 @@ struct hz_operator {
     hz::DevBuf idx, xs, nrm, delta, jac, reg, w, dreg;
     hz::DevBuf pos64, nrm64;
     hz::DevBuf posk64;  // pos64 with the coordinates scaled by k (FP64 sweep)
+    hz::DevBuf split64;  // records of the split FP64 sweep
+    hz::RecSplit split{};
+    bool use_split = false;
     // FP32 sweep records
     hz::Rec32 r32{};
     hz::DevBuf perm, pos32, nrm32, origin32, tpos32, split32, nearmask32, partial32;

@@ -263,6 +263,8 @@ int sweep_f64(const SweepConst &c, const Rec64 &r, int mode, const double *p_re,
                   c.wave * c.extent, kMaxPhase64);
         return HZ_ERR_ARG;
     }
+    if (r.split)
+        return sweep_split(c, *r.split, r.nrm, mode, p_re, p_im, pt_re, pt_im, q_re, q_im, qt_re, qt_im, s, ev0, ev1);
     double4_32a *dens = reinterpret_cast<double4_32a *>(scratch);
     const bool useA = (mode & SWEEP_A) != 0, useH = (mode & SWEEP_AH) != 0;
     // Coordinates scaled by k (records built by scale_records64) save three

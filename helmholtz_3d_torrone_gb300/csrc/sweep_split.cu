@@ -1,0 +1,702 @@
+// sweep_split.cu -- the FP64 products q = A p, qt = A^H pt (sweep_f64.cu) with
+// every pair evaluated as pairs of FP32 numbers (pair_split.cuh).
+//
+// Bound by the FP32 pipe: about 215 of its slots a pair (A p), against the 38.5
+// FP64 instructions (about 2,600 slots) of sweep64_kernel.
+//
+// One thread owns one target of the blocked sweep order (Rec32::perm); a CTA
+// of 256 threads walks a contiguous range of (target tile, half source tile)
+// units, as sweep32_kernel does, so the chip is full from a few thousand
+// points on.  Half tiles of 128 sources (96 bytes of fixed record and 16 of
+// density each) come by TMA bulk copies, double-buffered on mbarriers with
+// bounded waits; the cosine table takes 64 KB of shared memory, which leaves
+// room for two CTAs an SM.  Per target and source tile about 50 FP64
+// instructions set up the offsets and the phase of the tile's origin; they and
+// the FP64 sums (the 48-bit sums of 16 sources are added in FP64) run on the
+// otherwise idle FP64 pipe.
+#include "hz_internal.cuh"
+#include "bulk_copy.cuh"
+#include "pair_split.cuh"
+
+namespace hz {
+namespace {
+
+constexpr double kPiS = 3.14159265358979323846264338328;
+constexpr int kHalf = 128;       // sources per staged half tile
+constexpr int kRun = 16;         // sources per 48-bit sum
+constexpr int kRecs = 6;         // float4 of fixed record per source
+constexpr int kExpBlocks = 152;  // blocks of the density maximum
+
+struct ArgsSplit {
+    int64_t npad, units;
+    int64_t nctas;
+    float tau2, ktau;
+    double wave, tau;
+    const float4 *rec;          // [kRecs][npad]
+    const float4 *densA, *densH;
+    const double4_32a *tile;    // scaled origin, scaled radius (at least k tau)
+    const float2 *table;
+    const double4_32a *tpos;    // unscaled position and weight per slot
+    const double4_32a *nrm;     // tube order: (n, w)
+    const int *perm;
+    const int *expo;            // exponents of the density scales (A, A^H)
+    const double *p_re, *p_im, *pt_re, *pt_im;
+    double *q_re, *q_im, *qt_re, *qt_im;
+    double4_32a *partial;       // [nctas][2][256]
+    unsigned *err;
+};
+
+// float 2^e, -126 <= e <= 127
+__device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }
+__device__ __forceinline__ double pow2d(int e) { return __hiloint2double((e + 1023) << 20, 0); }
+// smallest e with v < 2^e
+__device__ __forceinline__ int exponent_above(float v) { return ((__float_as_int(v) >> 23) & 255) - 126; }
+
+__global__ void split_table_kernel(float2 *tab)
+{
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < kSplitTable; j += gridDim.x * blockDim.x) {
+        const double c = cospi((double)j / (kSplitTable / 2));
+        const double h = rint(c * 8388608.0) / 8388608.0;  // the head on the grid 2^-23
+        tab[j] = make_float2((float)h, (float)(c - h));
+    }
+}
+
+__global__ void split_tile_kernel(int64_t ntiles, const double4_32a *__restrict__ origin, double wave, double ktau,
+                                  double4_32a *__restrict__ tile)
+{
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t >= ntiles) return;
+    const double4_32a o = origin[t];
+    tile[t] = make_double4_32a(wave * o.x, wave * o.y, wave * o.z, fmax(wave * o.w * (1.0 + 1e-9), ktau));
+}
+
+__device__ __forceinline__ void split_coord(double v, double unit, double inv_unit, int &h, float &f, float &l)
+{
+    const double r = rint(v * inv_unit);
+    h = (int)r;
+    f = (float)v;
+    l = (float)fma(-r, unit, v);
+}
+
+// Fixed source records (see the packing in load_source); reg2 = 2 reg / scale.
+__global__ void __launch_bounds__(256) split_records_kernel(int64_t npad, const int *__restrict__ perm,
+                                                            const double4_32a *__restrict__ tpos,
+                                                            const double4_32a *__restrict__ pos,
+                                                            const double4_32a *__restrict__ nrm,
+                                                            const double4_32a *__restrict__ tile, double wave,
+                                                            double reg_scale, float4 *__restrict__ rec)
+{
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= npad) return;
+    const int c = perm[i];
+    const double4_32a o = tile[i / kTile32];
+    const int eS = exponent_above((float)(o.w * (1.0 + 1e-6)));
+    const double uS = pow2d(eS - 30), iS = pow2d(30 - eS);
+    double s[3] = {0, 0, 0}, n[3] = {0, 0, 0}, reg = 0;
+    if (c >= 0) {
+        const double4_32a x = tpos[i], m = nrm[c];
+        s[0] = wave * x.x - o.x;
+        s[1] = wave * x.y - o.y;
+        s[2] = wave * x.z - o.z;
+        n[0] = m.x;
+        n[1] = m.y;
+        n[2] = m.z;
+        reg = pos[c].w * reg_scale;
+    }
+    int sh[3], nh[3];
+    float sf[3], sl[3], nf[3], nl[3];
+    for (int a = 0; a < 3; a++) {
+        split_coord(s[a], uS, iS, sh[a], sf[a], sl[a]);
+        split_coord(n[a], pow2d(-30), pow2d(30), nh[a], nf[a], nl[a]);
+    }
+    const double s2 = fma(s[2], s[2], fma(s[1], s[1], s[0] * s[0]));
+    const double sn = fma(s[2], n[2], fma(s[1], n[1], s[0] * n[0]));
+    const long long S2 = __double2ll_rn(s2 * iS * iS), SN = __double2ll_rn(2.0 * sn * iS * pow2d(30));
+    const FF rg = ff_of_double(reg);
+    auto f = [](int v) { return __int_as_float(v); };
+    rec[0 * npad + i] = make_float4(f(sh[0]), f(sh[1]), f(sh[2]), f(nh[0]));
+    rec[1 * npad + i] = make_float4(f(nh[1]), f(nh[2]), f((int)S2), f((int)(S2 >> 32)));
+    rec[2 * npad + i] = make_float4(f((int)SN), f((int)(SN >> 32)), sf[0], sf[1]);
+    rec[3 * npad + i] = make_float4(sf[2], sl[0], sl[1], sl[2]);
+    rec[4 * npad + i] = make_float4(nf[0], nf[1], nf[2], nl[0]);
+    rec[5 * npad + i] = make_float4(nl[1], nl[2], rg.h, rg.l);
+}
+
+// Largest exponent field of |w p| and |pt| per block (high words of doubles
+// order like their values).
+__global__ void __launch_bounds__(256) split_max_kernel(int64_t n, const double4_32a *__restrict__ nrm,
+                                                        const double *__restrict__ p_re,
+                                                        const double *__restrict__ p_im,
+                                                        const double *__restrict__ pt_re,
+                                                        const double *__restrict__ pt_im, int *__restrict__ part)
+{
+    int a = 0, b = 0;
+    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n; s += (int64_t)gridDim.x * blockDim.x) {
+        if (p_re) {
+            const double w = nrm[s].w;
+            a = max(a, max(__double2hiint(w * p_re[s]) & 0x7fffffff, __double2hiint(w * p_im[s]) & 0x7fffffff));
+        }
+        if (pt_re) b = max(b, max(__double2hiint(pt_re[s]) & 0x7fffffff, __double2hiint(pt_im[s]) & 0x7fffffff));
+    }
+    a = __reduce_max_sync(0xffffffffu, a);
+    b = __reduce_max_sync(0xffffffffu, b);
+    __shared__ int sh[2][8];
+    if ((threadIdx.x & 31) == 0) {
+        sh[0][threadIdx.x >> 5] = a;
+        sh[1][threadIdx.x >> 5] = b;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        int v = 0;
+        for (int w = 0; w < 8; w++) v = max(v, sh[threadIdx.x][w]);
+        part[threadIdx.x * kExpBlocks + blockIdx.x] = v;
+    }
+}
+
+// Densities scaled to at most 1 and split: -k^2 sg/(8 pi) w p for A (the
+// entries carry -2 (x_t - x_s).n), +k^2 sg/(8 pi) pt for A^H; the scale's
+// exponents go to expo.
+__global__ void __launch_bounds__(256) split_dens_kernel(int64_t npad, const int *__restrict__ perm,
+                                                         const double4_32a *__restrict__ tpos,
+                                                         const double *__restrict__ p_re,
+                                                         const double *__restrict__ p_im,
+                                                         const double *__restrict__ pt_re,
+                                                         const double *__restrict__ pt_im, double scale,
+                                                         const int *__restrict__ part, int *__restrict__ expo,
+                                                         float4 *__restrict__ densA, float4 *__restrict__ densH)
+{
+    __shared__ int ex[2];
+    if (threadIdx.x < 64) {
+        const int m = threadIdx.x >> 5;
+        int v = 0;
+        for (int b = threadIdx.x & 31; b < kExpBlocks; b += 32) v = max(v, part[m * kExpBlocks + b]);
+        v = __reduce_max_sync(0xffffffffu, v);
+        // values below 2^(e + 1); clamped so that 2^e and 2^-e are normal
+        int e = (v >> 20) - 1022;
+        e = max(-1000, min(1000, e));
+        if ((threadIdx.x & 31) == 0) {
+            ex[m] = e;
+            if (blockIdx.x == 0) expo[m] = e;
+        }
+    }
+    __syncthreads();
+    const double fa = pow2d(-ex[0]), fh = pow2d(-ex[1]);
+    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < npad; s += (int64_t)gridDim.x * blockDim.x) {
+        const int c = perm[s];
+        if (p_re) {
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (c >= 0) {
+                const double w = tpos[s].w;
+                const FF r = ff_of_double(-scale * ((w * p_re[c]) * fa)), i = ff_of_double(-scale * ((w * p_im[c]) * fa));
+                v = make_float4(r.h, i.h, r.l, i.l);
+            }
+            densA[s] = v;
+        }
+        if (pt_re) {
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (c >= 0) {
+                const FF r = ff_of_double(scale * (pt_re[c] * fh)), i = ff_of_double(scale * (pt_im[c] * fh));
+                v = make_float4(r.h, i.h, r.l, i.l);
+            }
+            densH[s] = v;
+        }
+    }
+}
+
+// What a thread holds of its target for one source tile.
+struct Offsets {
+    int h[3];           // A / 2^(eL - 30)
+    float f[3], l[3];   // A and its tail
+    FF a2, rc;          // |a|^2 and |a| (far tiles)
+    long long a2i;      // |a|^2 in the close tiles' unit
+    long long an;       // A.n_t in the unit 2^(eL - 60)
+};
+
+struct TargetNormal {
+    int h[3];
+    float f[3], l[3];  // 2 n and twice its tail
+};
+
+// Uniform constants of one (target tile, source tile) pair.
+struct TileUnits {
+    int shS;             // eL - eS: from the sources' unit to the pair's
+    int shT;             // eL - eS - 1 (at least 0)
+    int x;               // close tiles: extra shift that keeps r^2 below 2^62
+    float w32, w8;       // 2^32 and 2^8 units of W
+    float r32, r8;       // the same after the extra shift
+    float n32, n8;       // 2^32 and 2^8 units of A.n
+};
+
+template <int MODE, bool DIR, bool CLOSE>
+__device__ __forceinline__ void split_pair(const ArgsSplit &a, const float4 (*st)[kHalf], int j, const float2 *tab,
+                                           const Offsets &t, const TargetNormal &tn, FF treg, const TileUnits &u,
+                                           int64_t tslot, int64_t sslot, FF (&accA)[2], FF (&accH)[2])
+{
+    constexpr bool A = (MODE & SWEEP_A) != 0, H = (MODE & SWEEP_AH) != 0;
+    constexpr bool SRC = (A && DIR) || (H && !DIR);  // (x_t - x_s).n_s wanted
+    constexpr bool TGT = (A && !DIR) || (H && DIR);  // (x_t - x_s).n_t wanted
+    const float4 r0 = st[0][j], r1 = st[1][j], r2_ = st[2][j], r3 = st[3][j];
+    const int s0 = __float_as_int(r0.x), s1 = __float_as_int(r0.y), s2 = __float_as_int(r0.z);
+    long long W = ((((long long)__float_as_int(r1.w) << 32) | (unsigned)__float_as_int(r1.z)) >> u.shS) + 128;
+    W += (long long)t.h[0] * s0;
+    W += (long long)t.h[1] * s1;
+    W += (long long)t.h[2] * s2;
+    float e = fmul(t.f[0], r3.y);
+    e = ffma(t.f[1], r3.z, e);
+    e = ffma(t.f[2], r3.w, e);
+    e = ffma(t.l[0], r2_.z, e);
+    e = ffma(t.l[1], r2_.w, e);
+    e = ffma(t.l[2], r3.x, e);
+    FF r2, w;
+    bool far = true;
+    if (CLOSE) {
+        r2 = ff_of_int((W >> u.x) + t.a2i, u.r32, u.r8, e);
+        far = r2.h > a.tau2;
+        if (fabsf(fsub(r2.h, a.tau2)) <= 1e-6f * a.tau2) {
+            // decided as the reference does: rho^2 without fused operations
+            const double4_32a p = a.tpos[tslot], q = a.tpos[sslot];
+            const double dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+            far = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz))) > a.tau;
+        }
+    } else {
+        w = ff_of_int(W, u.w32, u.w8, e);
+        const FF q = fast_two_sum(t.a2.h, w.h);
+        r2 = {q.h, fadd(q.l, fadd(t.a2.l, w.l))};
+    }
+    FF rho, y, th, c, s, ur, ui;
+    split_root(r2, rho, y);
+    th = CLOSE ? rho : split_phase_offset(w, rho, t.rc);
+    split_sincos(th, tab, c, s);
+    split_kernel(y, c, s, ur, ui);
+    const FF y2 = ff_mul(y, y);
+    FF vsr, vsi, vtr, vti;
+    if (SRC) {
+        const float4 r4 = st[4][j], r5 = st[5][j];
+        long long N = ((((long long)__float_as_int(r2_.y) << 32) | (unsigned)__float_as_int(r2_.x)) >> u.shS) + 128;
+        N += (long long)t.h[0] * __float_as_int(r0.w);
+        N += (long long)t.h[1] * __float_as_int(r1.x);
+        N += (long long)t.h[2] * __float_as_int(r1.y);
+        float g = fmul(t.f[0], r4.w);
+        g = ffma(t.f[1], r5.x, g);
+        g = ffma(t.f[2], r5.y, g);
+        g = ffma(t.l[0], r4.x, g);
+        g = ffma(t.l[1], r4.y, g);
+        g = ffma(t.l[2], r4.z, g);
+        const FF f = ff_mul(y2, ff_of_int(N, u.n32, u.n8, g));
+        vsr = ff_mul(ur, f);
+        vsi = ff_mul(ui, f);
+    }
+    if (TGT) {
+        long long D = (long long)tn.h[0] * s0;
+        D += (long long)tn.h[1] * s1;
+        D += (long long)tn.h[2] * s2;
+        float g = fmul(tn.f[0], r3.y);
+        g = ffma(tn.f[1], r3.z, g);
+        g = ffma(tn.f[2], r3.w, g);
+        g = ffma(tn.l[0], r2_.z, g);
+        g = ffma(tn.l[1], r2_.w, g);
+        g = ffma(tn.l[2], r3.x, g);
+        const FF f = ff_mul(y2, ff_of_int(t.an + (D >> u.shT), u.n32, u.n8, g));
+        vtr = ff_mul(ur, f);
+        vti = ff_mul(ui, f);
+    }
+    FF ar = DIR ? vsr : vtr, ai = DIR ? vsi : vti, hr = DIR ? vtr : vsr, hi = DIR ? vti : vsi;
+    if (CLOSE && !far) {
+        const float4 r5 = st[5][j];
+        const FF srg = {r5.z, r5.w};
+        ar = ff_neg(DIR ? srg : treg);
+        hr = DIR ? treg : srg;
+        ai = hi = {0.f, 0.f};
+    }
+    if (A) {
+        const float4 d = st[kRecs][j];
+        const FF dr = {d.x, d.z}, di = {d.y, d.w};
+        split_dot2<-1>(accA[0], ar, dr, ai, di);
+        split_dot2<1>(accA[1], ar, di, ai, dr);
+    }
+    if (H) {
+        const float4 d = st[kRecs + (A ? 1 : 0)][j];
+        const FF dr = {d.x, d.z}, di = {d.y, d.w};
+        split_dot2<1>(accH[0], hr, dr, hi, di);
+        split_dot2<-1>(accH[1], hr, di, hi, dr);
+    }
+}
+
+template <int MODE, bool DIR, bool CLOSE>
+__device__ __forceinline__ void split_half(const ArgsSplit &a, const float4 (*st)[kHalf], const float2 *tab,
+                                           const Offsets &t, const TargetNormal &tn, FF treg, const TileUnits &u,
+                                           int64_t tslot, int64_t sslot0, double (&dA)[2], double (&dH)[2])
+{
+#pragma unroll 1
+    for (int j0 = 0; j0 < kHalf; j0 += kRun) {
+        FF accA[2] = {{0.f, 0.f}, {0.f, 0.f}}, accH[2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll 1
+        for (int j = j0; j < j0 + kRun; j++)
+            split_pair<MODE, DIR, CLOSE>(a, st, j, tab, t, tn, treg, u, tslot, sslot0 + j, accA, accH);
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            if (MODE & SWEEP_A) dA[q] += (double)accA[q].h + (double)accA[q].l;
+            if (MODE & SWEEP_AH) dH[q] += (double)accH[q].h + (double)accH[q].l;
+        }
+    }
+}
+
+// e^{i x}, 0 <= x < 4000, from the split table
+__device__ __forceinline__ void split_phase64(double x, const float2 *tab, double &cr, double &sr)
+{
+    const int m = __double2int_rn(x * (kSplitTable / (2.0 * kPiS)));
+    double r = fma(-(double)m, 0.003067961575652589 / 4, x);  // the step to 31 bits, and the rest
+    r = fma(-(double)m, 1.1869336926769907e-13 / 4, r);
+    const float2 c = tab[m & (kSplitTable - 1)], s = tab[(m - kSplitTable / 4) & (kSplitTable - 1)];
+    const double tc = (double)c.x + (double)c.y, ts = (double)s.x + (double)s.y;
+    const double z = r * r, sn = fma(r * z, -1.0 / 6.0, r), cm = z * fma(z, -1.0 / 24.0, 0.5);
+    cr = tc - fma(ts, sn, tc * cm);
+    sr = ts + fma(tc, sn, -(ts * cm));
+}
+
+template <int MODE>
+__device__ __forceinline__ void split_write(const ArgsSplit &a, int64_t s, double ar, double ai, double hr, double hi)
+{
+    const int c = a.perm[s];
+    if (c < 0) return;
+    if (MODE & SWEEP_A) {
+        const double f = pow2d(a.expo[0]), r = f * ar, i = f * ai;
+        if (!isfinite(r) || !isfinite(i)) atomicOr(a.err, DEV_ERR_NONFINITE);
+        a.q_re[c] = r + 0.5 * a.p_re[c];
+        a.q_im[c] = i + 0.5 * a.p_im[c];
+    }
+    if (MODE & SWEEP_AH) {
+        const double f = pow2d(a.expo[1]), w = a.tpos[s].w, r = f * (w * hr), i = f * (w * hi);
+        if (!isfinite(r) || !isfinite(i)) atomicOr(a.err, DEV_ERR_NONFINITE);
+        a.qt_re[c] = r + 0.5 * a.pt_re[c];
+        a.qt_im[c] = i + 0.5 * a.pt_im[c];
+    }
+}
+
+// float4 arrays of a staged half tile
+template <int MODE>
+constexpr int kSplitArrays = kRecs + (MODE == SWEEP_PAIR ? 2 : 1);
+
+template <int MODE, bool DIR>
+__global__ void __launch_bounds__(kTile32, 2) sweep_split_kernel(ArgsSplit a)
+{
+    constexpr int NA = kSplitArrays<MODE>;
+    constexpr bool TGT = ((MODE & SWEEP_A) && !DIR) || ((MODE & SWEEP_AH) && DIR);
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ alignas(8) uint64_t bar[2];
+    float2 *tab = reinterpret_cast<float2 *>(smem);
+    float4(*stage)[kHalf] = reinterpret_cast<float4(*)[kHalf]>(smem + kSplitTable * sizeof(float2));
+    const int64_t halves = a.npad / kHalf;
+    const int64_t u_begin = (int64_t)blockIdx.x * a.units / a.nctas;
+    const int64_t u_end = ((int64_t)blockIdx.x + 1) * a.units / a.nctas;
+    if (threadIdx.x == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        fence_barrier_init();
+    }
+    for (int i = threadIdx.x; i < kSplitTable / 2; i += kTile32)
+        reinterpret_cast<float4 *>(tab)[i] = __ldg(reinterpret_cast<const float4 *>(a.table) + i);
+    __syncthreads();
+    if (u_begin >= u_end) return;
+    auto issue = [&](int64_t u, int buf) {
+        const int64_t base = (u % halves) * kHalf;
+        const uint32_t bytes = kHalf * sizeof(float4);
+        mbar_arrive_expect_tx(&bar[buf], NA * bytes);
+#pragma unroll
+        for (int r = 0; r < kRecs; r++) bulk_g2s(&stage[buf * NA + r][0], a.rec + r * a.npad + base, bytes, &bar[buf]);
+        if (MODE & SWEEP_A) bulk_g2s(&stage[buf * NA + kRecs][0], a.densA + base, bytes, &bar[buf]);
+        if (MODE & SWEEP_AH) bulk_g2s(&stage[buf * NA + NA - 1][0], a.densH + base, bytes, &bar[buf]);
+    };
+    if (threadIdx.x == 0) issue(u_begin, 0);
+    int seg = 0;
+    for (int64_t u = u_begin; u < u_end;) {
+        const int64_t blk = u / halves;
+        const int64_t seg_end = (u_end < (blk + 1) * halves) ? u_end : (blk + 1) * halves;
+        const bool whole = (u == blk * halves) && (seg_end == (blk + 1) * halves);
+        const int64_t slot = blk * kTile32 + threadIdx.x;
+        const double4_32a tp = a.tpos[slot];
+        const double X = a.wave * tp.x, Y = a.wave * tp.y, Z = a.wave * tp.z;
+        const double4_32a to = a.tile[blk];
+        const float ox = (float)to.x, oy = (float)to.y, oz = (float)to.z, Rt = (float)to.w;
+        FF treg = {0.f, 0.f};
+        TargetNormal tn = {};
+        double nx = 0, ny = 0, nz = 0;
+        {
+            const float4 r5 = a.rec[5 * a.npad + slot];
+            treg = {r5.z, r5.w};
+            if (TGT) {
+                const int c = a.perm[slot];
+                if (c >= 0) {
+                    const double4_32a m = a.nrm[c];
+                    nx = m.x;
+                    ny = m.y;
+                    nz = m.z;
+                }
+                const float4 r0 = a.rec[slot], r1 = a.rec[a.npad + slot], r4 = a.rec[4 * a.npad + slot];
+                tn.h[0] = __float_as_int(r0.w);
+                tn.h[1] = __float_as_int(r1.x);
+                tn.h[2] = __float_as_int(r1.y);
+                tn.f[0] = 2.f * r4.x;
+                tn.f[1] = 2.f * r4.y;
+                tn.f[2] = 2.f * r4.z;
+                tn.l[0] = 2.f * r4.w;
+                tn.l[1] = 2.f * r5.x;
+                tn.l[2] = 2.f * r5.y;
+            }
+        }
+        double q[4] = {0, 0, 0, 0};
+        double dA[2] = {0, 0}, dH[2] = {0, 0};
+        Offsets t = {};
+        TileUnits un = {};
+        bool close = false, fresh = true;
+        double phr = 1.0, phi = 0.0;
+        for (; u < seg_end; u++) {
+            const int64_t it = u - u_begin;
+            const int buf = (int)(it & 1);
+            if (threadIdx.x == 0 && u + 1 < u_end) issue(u + 1, buf ^ 1);
+            const int64_t half = u - blk * halves, tile = half >> 1;
+            if (fresh || !(half & 1)) {
+                // offsets of this thread's target from the source tile's origin
+                fresh = false;
+                const double4_32a o = a.tile[tile];
+                const float Rs = (float)o.w;
+                const float cx = ox - (float)o.x, cy = oy - (float)o.y, cz = oz - (float)o.z;
+                const float ct = sqrtf(fmaf(cx, cx, fmaf(cy, cy, cz * cz)));
+                close = ct - Rt < 2.5f * Rs + a.ktau + 1e-4f * (ct + Rt + fabsf(ox) + fabsf(oy) + fabsf(oz));
+                const int eS = exponent_above((float)(o.w * (1.0 + 1e-6)));
+                const int eL = max(eS + 1, exponent_above(2.0002f * (ct + Rt)));
+                un.shS = eL - eS;
+                un.shT = eL - eS - 1;
+                un.x = max(0, eL - eS - 3);
+                un.w32 = pow2f(eL + eS - 28);
+                un.w8 = pow2f(eL + eS - 52);
+                un.r32 = un.w32 * pow2f(un.x);
+                un.r8 = un.w8 * pow2f(un.x);
+                un.n32 = pow2f(eL - 28);
+                un.n8 = pow2f(eL - 52);
+                const double uL = pow2d(eL - 30), iL = pow2d(30 - eL);
+                const double ax = -2.0 * (X - o.x), ay = -2.0 * (Y - o.y), az = -2.0 * (Z - o.z);
+                const double A[3] = {ax, ay, az};
+#pragma unroll
+                for (int i = 0; i < 3; i++) {
+                    const double m = fma(A[i], iL, 6755399441055744.0);  // nearest integer in the low word
+                    t.h[i] = __double2loint(m);
+                    t.f[i] = (float)A[i];
+                    t.l[i] = (float)fma(-uL, m - 6755399441055744.0, A[i]);
+                }
+                const double a2 = 0.25 * fma(az, az, fma(ay, ay, ax * ax));
+                if (close) {
+                    t.a2i = __double2ll_rn(a2 * pow2d(60 - eL - eS - un.x));
+                } else {
+                    const double y0 = (double)rsqrt_seed((float)a2);
+                    const double e = fma(-(a2 * y0), y0, 1.0);
+                    const double y = fma(y0 * e, fma(e, 0.375, 0.5), y0);
+                    const double g = a2 * y;
+                    const double rc = fma(fma(-g, g, a2), 0.5 * y, g);
+                    t.a2 = ff_of_double(a2);
+                    t.rc = ff_of_double(rc);
+                    split_phase64(rc, tab, phr, phi);
+                }
+                if (TGT) t.an = __double2ll_rn(fma(az, nz, fma(ay, ny, ax * nx)) * pow2d(60 - eL)) + 128;
+            }
+            const bool ok = mbar_wait_bounded(&bar[buf], (uint32_t)((it >> 1) & 1), g_data_wait_limit);
+            if (__syncthreads_or(!ok)) {
+                if (threadIdx.x == 0) {
+                    atomicOr(a.err, DEV_ERR_WAIT);
+                    mbar_drain(&bar[buf], (uint32_t)((it >> 1) & 1), &bar[buf ^ 1], (uint32_t)(((it + 1) >> 1) & 1),
+                               u + 1 < u_end);
+                }
+                return;
+            }
+            if (close)
+                split_half<MODE, DIR, true>(a, stage + buf * NA, tab, t, tn, treg, un, slot, half * kHalf, dA, dH);
+            else
+                split_half<MODE, DIR, false>(a, stage + buf * NA, tab, t, tn, treg, un, slot, half * kHalf, dA, dH);
+            if ((half & 1) || u + 1 == seg_end) {
+                if (close) {
+                    q[0] += dA[0];
+                    q[1] += dA[1];
+                    q[2] += dH[0];
+                    q[3] += dH[1];
+                } else {
+                    if (MODE & SWEEP_A) {
+                        q[0] += fma(phr, dA[0], -(phi * dA[1]));
+                        q[1] += fma(phr, dA[1], phi * dA[0]);
+                    }
+                    if (MODE & SWEEP_AH) {
+                        q[2] += fma(phr, dH[0], phi * dH[1]);
+                        q[3] += fma(phr, dH[1], -(phi * dH[0]));
+                    }
+                }
+                dA[0] = dA[1] = dH[0] = dH[1] = 0.0;
+            }
+            __syncthreads();
+        }
+        if (whole)
+            split_write<MODE>(a, slot, q[0], q[1], q[2], q[3]);
+        else
+            a.partial[((int64_t)blockIdx.x * 2 + seg) * kTile32 + threadIdx.x] =
+                make_double4_32a(q[0], q[1], q[2], q[3]);
+        seg = 1;
+    }
+}
+
+// Adds up, in CTA order, the pieces of target tiles split between CTAs.
+template <int MODE>
+__global__ void __launch_bounds__(kTile32) split_fixup_kernel(ArgsSplit a)
+{
+    const int64_t blk = blockIdx.x, halves = a.npad / kHalf;
+    auto cta_of = [&](int64_t u) { return ((u + 1) * a.nctas - 1) / a.units; };
+    const int64_t c_lo = cta_of(blk * halves), c_hi = cta_of((blk + 1) * halves - 1);
+    if (c_lo == c_hi) return;
+    double q[4] = {0, 0, 0, 0};
+    for (int64_t c = c_lo; c <= c_hi; c++) {
+        const int64_t first = (c * a.units / a.nctas) / halves;
+        const double4_32a v = a.partial[(c * 2 + (first == blk ? 0 : 1)) * kTile32 + threadIdx.x];
+        q[0] += v.x;
+        q[1] += v.y;
+        q[2] += v.z;
+        q[3] += v.w;
+    }
+    split_write<MODE>(a, blk * kTile32 + threadIdx.x, q[0], q[1], q[2], q[3]);
+}
+
+int sm_count()
+{
+    int dev = 0, sms = 152;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
+template <int MODE, bool DIR>
+int launch_split(ArgsSplit a, size_t partial_bytes, cudaStream_t s)
+{
+    constexpr size_t smem = kSplitTable * sizeof(float2) + 2 * kSplitArrays<MODE> * kHalf * sizeof(float4);
+    HZ_CHECK_CUDA(cudaFuncSetAttribute(sweep_split_kernel<MODE, DIR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)smem));
+    const int64_t tiles = a.npad / kTile32;
+    a.units = tiles * (a.npad / kHalf);
+    int64_t p = 2 * (int64_t)sm_count();
+    const int64_t room = (int64_t)(partial_bytes / (2 * kTile32 * sizeof(double4_32a)));
+    if (p > room) p = room;
+    if (p > a.units) p = a.units;
+    if (p < 1) {
+        set_error("split FP64 sweep: partial buffer too small");
+        return HZ_ERR_STATE;
+    }
+    a.nctas = p;
+    sweep_split_kernel<MODE, DIR><<<(unsigned)p, kTile32, smem, s>>>(a);
+    HZ_CHECK_LAUNCH();
+    split_fixup_kernel<MODE><<<(unsigned)tiles, kTile32, 0, s>>>(a);
+    HZ_CHECK_LAUNCH();
+    return HZ_OK;
+}
+
+}  // namespace
+
+size_t split_record_bytes(int64_t npad)
+{
+    // records, densities, tiles, table, maxima and exponents
+    return (size_t)npad * (kRecs + 2) * sizeof(float4) + (size_t)(npad / kTile32) * sizeof(double4_32a) +
+           kSplitTable * sizeof(float2) + (2 * kExpBlocks + 8) * sizeof(int);
+}
+
+RecSplit split_record_views(void *mem, const Rec32 &r)
+{
+    RecSplit v;
+    v.npad = r.npad;
+    v.rec = static_cast<float4 *>(mem);
+    v.dens = v.rec + kRecs * r.npad;
+    v.tile = reinterpret_cast<double4_32a *>(v.dens + 2 * r.npad);
+    v.table = reinterpret_cast<float2 *>(v.tile + r.npad / kTile32);
+    v.expo = reinterpret_cast<int *>(v.table + kSplitTable);
+    v.perm = r.perm;
+    v.tpos = r.tpos;
+    v.partial = r.partial;
+    v.partial_bytes = r.partial_bytes;
+    return v;
+}
+
+// Where the split sweep serves: the table reduction of the origin phases ends
+// at k rho = 4000 (as the FP64 sweep's); k h <= 0.8 (eight points a
+// wavelength) keeps the phases within a tile small, so the error stays at or
+// below the FP64 sweep's (at k h = 1, 4.5e-15 against 4.2e-15); k >= 1/64
+// keeps 1/(k rho)^3 far inside the FP32 range; below 2048 points the FP64
+// sweep's error (2e-15 and less) is the smaller one.
+bool split_serves(int64_t n, double wave, double H, double extent)
+{
+    return n >= 2048 && wave >= 1.0 / 64 && wave * H <= 0.8 && wave * extent < 4000.0;
+}
+
+int build_split_records(const SweepConst &c, const RecSplit &v, const Rec32 &r, const double4_32a *pos,
+                        const double4_32a *nrm, cudaStream_t s)
+{
+    const int64_t tiles = r.npad / kTile32;
+    split_table_kernel<<<32, 256, 0, s>>>(v.table);
+    HZ_CHECK_LAUNCH();
+    split_tile_kernel<<<(unsigned)((tiles + 255) / 256), 256, 0, s>>>(tiles, r.origin, c.wave, c.wave * c.tau, v.tile);
+    HZ_CHECK_LAUNCH();
+    const double sg = (c.interior == 1) ? -1.0 : 1.0;
+    split_records_kernel<<<(unsigned)((r.npad + 255) / 256), 256, 0, s>>>(
+        r.npad, r.perm, r.tpos, pos, nrm, v.tile, c.wave, 2.0 * sg * (4.0 * kPiS) / (c.wave * c.wave), v.rec);
+    HZ_CHECK_LAUNCH();
+    return HZ_OK;
+}
+
+int sweep_split(const SweepConst &c, const RecSplit &v, const double4_32a *nrm, int mode, const double *p_re,
+                const double *p_im, const double *pt_re, const double *pt_im, double *q_re, double *q_im,
+                double *qt_re, double *qt_im, cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1)
+{
+    const bool useA = (mode & SWEEP_A) != 0, useH = (mode & SWEEP_AH) != 0;
+    const double sg = (c.interior == 1) ? -1.0 : 1.0;
+    const double *pr = useA ? p_re : nullptr, *pi = useA ? p_im : nullptr;
+    const double *tr = useH ? pt_re : nullptr, *ti = useH ? pt_im : nullptr;
+    int *part = v.expo + 8;
+    split_max_kernel<<<kExpBlocks, 256, 0, s>>>(c.n, nrm, pr, pi, tr, ti, part);
+    HZ_CHECK_LAUNCH();
+    int64_t b = (v.npad + 255) / 256;
+    const int64_t cap = 8 * (int64_t)sm_count();
+    if (b > cap) b = cap;
+    split_dens_kernel<<<(unsigned)b, 256, 0, s>>>(v.npad, v.perm, v.tpos, pr, pi, tr, ti,
+                                                  sg * c.wave * c.wave / (8.0 * kPiS), part, v.expo, v.dens,
+                                                  v.dens + v.npad);
+    HZ_CHECK_LAUNCH();
+    ArgsSplit a;
+    a.npad = v.npad;
+    a.units = 0;
+    a.nctas = 0;
+    a.wave = c.wave;
+    a.tau = c.tau;
+    a.ktau = (float)(c.wave * c.tau);
+    a.tau2 = (float)((c.wave * c.tau) * (c.wave * c.tau));
+    a.rec = v.rec;
+    a.densA = v.dens;
+    a.densH = v.dens + v.npad;
+    a.tile = v.tile;
+    a.table = v.table;
+    a.tpos = v.tpos;
+    a.nrm = nrm;
+    a.perm = v.perm;
+    a.expo = v.expo;
+    a.p_re = p_re; a.p_im = p_im; a.pt_re = pt_re; a.pt_im = pt_im;
+    a.q_re = q_re; a.q_im = q_im; a.qt_re = qt_re; a.qt_im = qt_im;
+    a.partial = v.partial;
+    a.err = c.err;
+    if (ev0) HZ_CHECK_CUDA(record_timing_event(ev0, s));
+    const bool dir = c.dirichlet != 0;
+    int rc;
+    if (mode == SWEEP_PAIR)
+        rc = dir ? launch_split<SWEEP_PAIR, true>(a, v.partial_bytes, s) : launch_split<SWEEP_PAIR, false>(a, v.partial_bytes, s);
+    else if (mode == SWEEP_A)
+        rc = dir ? launch_split<SWEEP_A, true>(a, v.partial_bytes, s) : launch_split<SWEEP_A, false>(a, v.partial_bytes, s);
+    else
+        rc = dir ? launch_split<SWEEP_AH, true>(a, v.partial_bytes, s) : launch_split<SWEEP_AH, false>(a, v.partial_bytes, s);
+    HZ_TRY(rc);
+    if (ev1) HZ_CHECK_CUDA(record_timing_event(ev1, s));
+    return HZ_OK;
+}
+
+HZ_DEFINE_WAIT_LIMIT_SETTER(set_wait_limit_split)
+
+}  // namespace hz
