@@ -239,7 +239,7 @@ int hz_batch_create(hz_operator *const *ops, int count, hz_batch **out)
         items[r].c = sweep_const(op);
         items[r].r = op->r32;
         items[r].pos64 = op->pos64.as<double4_32a>();
-        items[r].dens = op->dens32.as<float4>();
+        items[r].dens = op->dens32.as<float>();
     }
     for (int k = 0; k < kBatchShapes && rc == HZ_OK; k++)
         rc = batch32_describe(items.data(), count, k, b->desc.as<char>() + (size_t)k * db, b->units[k], b->blocks[k],

@@ -85,7 +85,6 @@ SweepConst sweep_const(const hz_operator *op)
     c.dirichlet = op->p.dirichlet;
     c.interior = op->p.interior;
     c.err = op->err.as<unsigned>();
-    c.phase_split = op->phase_mode == HZ_PHASE_SPLIT;
     c.extent = 1.7320508075688772 * (op->p.int_u - op->p.int_l);
     return c;
 }
@@ -146,7 +145,7 @@ struct MatrixFreeOp final : LinOp {
                              op->scratch.as<double2>(), s, e0, e1);
         const int cfg = (mode == SWEEP_PAIR || op->sweep_cfg_a < 0) ? op->sweep_cfg : op->sweep_cfg_a;
         return sweep_f32(c, op->r32, op->pos64.as<double4_32a>(), mode, p_re, p_im, pt_re, pt_im, q_re, q_im, qt_re,
-                         qt_im, op->dens32.as<float4>(), s, e0, e1, cfg);
+                         qt_im, op->dens32.as<float>(), s, e0, e1, cfg);
     }
     void capture_begin() override { op->timer.next = 0; }
     void capture_end() override
@@ -166,7 +165,7 @@ struct MatrixFreeOp final : LinOp {
     uint64_t key() const override
     {
         return ((uint64_t)(uintptr_t)op << 8) ^ (uint64_t)(precision * 16 + op->sweep_cfg) ^
-               ((uint64_t)op->phase_mode << 6) ^ ((uint64_t)(op->sweep_cfg_a + 1) << 32) ^ 1ull;
+               ((uint64_t)(op->sweep_cfg_a + 1) << 32) ^ 1ull;
     }
 };
 
@@ -342,7 +341,7 @@ int need_built(hz_operator *op)
 }  // namespace
 
 // FP32 sweep records of the tube (or annulus) points in blocked order.
-static int build_records32(hz_operator *op, double reg_scale)
+static int build_records32(hz_operator *op, double lambda, double reg_scale)
 {
     cudaStream_t s = op->stream;
     const int N = op->p.N;
@@ -350,6 +349,7 @@ static int build_records32(hz_operator *op, double reg_scale)
     const int64_t unit = (int64_t)kThreads32 * kTgt32;  // multiple of kTile32
     const int64_t npad = ((n + unit - 1) / unit) * unit;
     op->r32.npad = npad;
+    op->r32.lambda = lambda;
     if (npad > 0) {
         HZ_TRY(op->perm.ensure(npad * sizeof(int)));
         HZ_TRY(op->pos32.ensure(npad * sizeof(float4)));
@@ -360,12 +360,14 @@ static int build_records32(hz_operator *op, double reg_scale)
         HZ_TRY(op->origin32.ensure(ntiles * sizeof(double4_32a)));
         HZ_TRY(op->split32.ensure((2 * npad + 2 * ntiles) * sizeof(float4)));
         HZ_TRY(op->nearmask32.ensure(ntiles * op->r32.mwords * sizeof(uint32_t)));
-        HZ_TRY(op->dens32.ensure(npad * sizeof(float4)));
+        HZ_TRY(op->soa32.ensure(npad * kFixed32 * sizeof(float)));
+        HZ_TRY(op->dens32.ensure(npad * 6 * sizeof(float)));  // split re, im, -im of both densities
         HZ_TRY(sweep_order(N, n, op->idx.as<int64_t>(), op->perm.as<int>(), npad, op->scratch, s));
     }
     op->r32.perm = op->perm.as<int>();
     op->r32.pos = op->pos32.as<float4>();
     op->r32.nrm = op->nrm32.as<float4>();
+    op->r32.soa = op->combo ? nullptr : op->soa32.as<float>();
     op->r32.origin = op->origin32.as<double4_32a>();
     op->r32.tpos = op->tpos32.as<double4_32a>();
     {
@@ -414,7 +416,7 @@ static int build_combo(hz_operator *op, int64_t *n_out)
     HZ_TRY(check_device_error(op, "hz_build (Combo)"));
     // FP32 records as the classic operator's (reg scaled by 4 pi: the Combo
     // kernel's c4 = 1/(4 pi) is folded into the densities), |d| in nrm32.w
-    HZ_TRY(build_records32(op, 4.0 * 3.14159265358979323846264338328));
+    HZ_TRY(build_records32(op, 1.0, 4.0 * 3.14159265358979323846264338328));
     HZ_TRY(combo32_set_distances(op->r32, op->adist.as<double>(), s));
     HZ_TRY(op->scratch.ensure(nn * sizeof(double4_32a) + 256));
     HZ_TRY(op->io.ensure(nn * sizeof(double) * 8));
@@ -448,8 +450,7 @@ int hz_set_phase_mode(hz_operator *op, int mode)
         set_error("hz_set_phase_mode: need an operator and HZ_PHASE_DIRECT or HZ_PHASE_SPLIT");
         return HZ_ERR_ARG;
     }
-    op->phase_mode = mode;
-    return HZ_OK;
+    return HZ_OK;  // both modes run the phase centred on the source tile (pair32.cuh)
 }
 
 int hz_set_combo(hz_operator *op, const hz_dense_opts *o)
@@ -632,7 +633,8 @@ int hz_build(hz_operator *op, int64_t *n_out)
     } else {
         op->posk64.release();
     }
-    HZ_TRY(build_records32(op, sweep32_reg_scale(op->p.interior)));
+    const double lambda = lambda32(op->p.wave);
+    HZ_TRY(build_records32(op, lambda, sweep32_reg_scale(op->p.interior, lambda)));
     const SweepConst sc = sweep_const(op);
     op->use_split = split_serves(n, sc.wave, op->H, sc.extent);
     if (op->use_split) {
@@ -687,7 +689,7 @@ int hz_autotune(hz_operator *op, int *chosen, double *ms_per_sweep)
             float ms_min = 1e30f;
             for (int rep = 0; rep < 2 && rc == HZ_OK; rep++) {
                 rc = sweep_f32(c, op->r32, op->pos64.as<double4_32a>(), mode, io, io + n, io + 2 * n, io + 3 * n,
-                               io + 4 * n, io + 5 * n, io + 6 * n, io + 7 * n, op->dens32.as<float4>(), s, e0, e1,
+                               io + 4 * n, io + 5 * n, io + 6 * n, io + 7 * n, op->dens32.as<float>(), s, e0, e1,
                                cfg);
                 if (rc == HZ_OK && cudaEventSynchronize(e1) == cudaSuccess) {
                     float ms = 0.f;

@@ -94,6 +94,7 @@ struct Rec64 {
 
 // Tile geometry of the FP32 sweep.
 constexpr int kTile32 = 256;  // sources per shared-memory tile
+constexpr int kFixed32 = 7;   // floats per source of Rec32::soa
 constexpr int kThreads32 = 256;
 constexpr int kTgt32 = 2;     // targets per thread
 constexpr int kTile64 = 128;
@@ -114,13 +115,16 @@ inline cudaError_t record_timing_event(cudaEvent_t ev, cudaStream_t s)
 
 struct Rec32 {
     int64_t npad;        // multiple of kTile32 and of kThreads32*kTgt32
+    double lambda = 1.0; // factor of every FP32 coordinate: k where the centred pair
+                         // arithmetic serves (lambda32), else 1
     int *perm;           // npad entries, -1 for padding
-    float4 *pos;         // x-o, y-o, z-o relative to the slot's tile origin; .w = reg
+    float4 *pos;         // lambda (x-o, y-o, z-o) relative to the slot's tile origin; .w = reg
     float4 *nrm;         // nx, ny, nz, w
+    float *soa = nullptr;    // per tile [kFixed32][kTile32]: minus the position, normal, reg (may be NULL)
     double4_32a *origin;     // per tile: origin (x, y, z) and bounding radius .w
     double4_32a *tpos;       // per slot FP64 position (x, y, z), .w = w (targets)
-    float4 *thi, *tlo;       // per slot position split into FP32 head + tail (x = hi + lo)
-    float4 *ohi, *olo;       // per tile origin split into FP32 head + tail
+    float4 *thi, *tlo;       // per slot position times lambda, split into FP32 head + tail
+    float4 *ohi, *olo;       // per tile origin times lambda, split likewise; ohi.w = radius times lambda
     uint32_t *nearmask;      // [target tile][mwords]: bit s set unless source tile s is
                              // farther than tau from every point of the target tile
     int64_t mwords;          // 32-bit words per mask row: ceil(tiles / 32)
@@ -135,7 +139,6 @@ struct SweepConst {
     int dirichlet;
     int interior;
     unsigned *err;  // device error word
-    int phase_split = 0;  // FP32 sweep: phase reduced with a split k/(2 pi) (HZ_PHASE_SPLIT)
     double extent = 0.0;  // largest point distance: the domain's diagonal sqrt(3) (int_u - int_l)
 };
 
@@ -208,7 +211,7 @@ int tube_init(const hz_params &p, const double *d, const double *gx, const doubl
 int sweep_order(int N, int64_t n, const int64_t *idx, int *perm, int64_t npad, DevBuf &scratch,
                 cudaStream_t s);
 // reg_scale multiplies the regularisation factor stored in pos32.w (the
-// FP32 sweep folds sg/(4 pi) into its densities and divides it out here).
+// FP32 sweep folds lambda^2 sg/(4 pi) into its densities and divides it out here).
 // Fill every array of r (npad, perm and the pointers set by the caller):
 // FP32 records, tile origins, split positions and the near-tile mask for
 // the regularisation radius tau.
@@ -240,10 +243,17 @@ int scale_records64(int64_t n, double k, const double4_32a *pos, double4_32a *po
 // sweep_f32.cu
 int sweep_f32(const SweepConst &c, const Rec32 &r, const double4_32a *pos64, int mode,
               const double *p_re, const double *p_im, const double *pt_re, const double *pt_im,
-              double *q_re, double *q_im, double *qt_re, double *qt_im, float4 *dens,
+              double *q_re, double *q_im, double *qt_re, double *qt_im, float *dens,
               cudaStream_t s, cudaEvent_t ev0 = nullptr, cudaEvent_t ev1 = nullptr, int cfg = 0);
-// 1 / (sg / 4 pi): the factor applied to regularisation factors in pos32.w
-double sweep32_reg_scale(int interior);
+// The factor of the FP32 coordinates for wave number k, and the factor of the
+// regularisation factors in pos32.w (the inverse of the densities').
+double lambda32(double wave);
+struct Const32 {
+    int scaled;
+    float k, kh, kl, tau2, guard_lo, guard_hi;
+};
+Const32 constants32(const SweepConst &c, double lambda);
+double sweep32_reg_scale(int interior, double lambda);
 // number of compiled FP32 sweep variants (block shape x targets per thread)
 int sweep32_num_configs();
 // Batched FP32 products (sweep_f32.cu): Q[r] = A_r P[r] for the described
@@ -253,7 +263,7 @@ struct Batch32Item {
     SweepConst c;
     Rec32 r;
     const double4_32a *pos64;
-    float4 *dens;
+    float *dens;
 };
 size_t batch32_desc_bytes(int R);
 // Describes nops operators: items[cols[i]] owning column cols[i] (cols NULL:
@@ -302,7 +312,7 @@ struct hz_operator {
     bool use_split = false;
     // FP32 sweep records
     hz::Rec32 r32{};
-    hz::DevBuf perm, pos32, nrm32, origin32, tpos32, split32, nearmask32, partial32;
+    hz::DevBuf perm, pos32, nrm32, soa32, origin32, tpos32, split32, nearmask32, partial32;
     // scratch and error word
     hz::DevBuf scratch, err;
     hz::DevBuf io;  // staging for host <-> device vectors
@@ -311,7 +321,6 @@ struct hz_operator {
     hz::SweepTimer timer;
     int sweep_cfg = 0;  // FP32 sweep variant of the fused A p + A^H pt pass (hz_autotune)
     int sweep_cfg_a = -1;  // variant of the single-product passes (A p or A^H p); -1: sweep_cfg
-    int phase_mode = HZ_PHASE_SPLIT; // HZ_PHASE_SPLIT (default) or HZ_PHASE_DIRECT (hz_set_phase_mode)
     // Combo formulation (hz_set_combo): annulus points, FP64 products only
     int combo = 0;
     hz_dense_opts combo_opts{};

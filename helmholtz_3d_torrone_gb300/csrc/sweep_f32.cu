@@ -10,35 +10,43 @@
 //    x_t - o = (t_hi - o_hi) + (t_lo - o_lo): the head difference is rounded
 //    to half an ulp of itself, so the offset of close pairs keeps FP32
 //    relative precision with no FP64 instruction in the tile loop.
-//  * The phase k*rho is reduced in revolutions with k/(2 pi) split into an
-//    FP32 head and tail before the SFU's sin/cos (the MODE bit
-//    SWEEP_PHASE_SPLIT, the operator's default), or passed to the SFU as one
-//    FP32 product (hz_set_phase_mode(op, HZ_PHASE_DIRECT)).  rho itself
-//    carries an FP32 rounding, so some phase error remains either way; the
-//    FP32 product stays within 1e-7 of the FP64 product (2.9e-8 split,
-//    4.6e-8 direct on the 256^3 torus at k = 20), and the split reduction
-//    costs about 6 % of the throughput.
+//  * Coordinates are stored times k, and away from near tiles the phase is
+//    taken about the source tile's origin (pair32.cuh): |k rho - k rho_c| is
+//    small, goes to the SFU's sin/cos without a range reduction, and the
+//    tile's sum is turned by e^{i k rho_c} once.  Against the phase reduced per
+//    pair the error to the FP64 product fell, 3.2e-7 -> 2.6e-7 of |K p| on the
+//    64^3 torus (k = 15) and 3.4e-7 -> 3.1e-7 at 128^3 (k = 20).
 //  * The near-field test rho <= tau is decided in FP64 (with the FP64
 //    sweep's own arithmetic) whenever the FP32 rho^2 lies within 1e-4 of
 //    tau^2, so FP32 and FP64 operators classify every pair alike.
 //  * Per tile the contributions are summed in FP32; across tiles into FP32
 //    head + tail pairs by TwoSum (about 48 significant bits).
 //
-// Throughput design: the kernel is bound by instruction issue on the FP32
-// pipe, and GB300 runs FP64 at 1/64 of the FP32 rate, so the tile loop
-// holds no FP64 instruction at all.  A source tile whose bounding sphere is
-// farther than tau (with a 1e-3 margin) from the bounding spheres of all of
-// the block's target tiles holds no near pair; a bit mask built once per
-// tube in FP64 says which, and such tiles run a loop without near-field
-// tests or selects.  The factor sg/(4 pi) is folded into the densities (and
+// Throughput design: the kernel is bound by the FP32 and SFU pipes (22 FP32
+// operations and three SFU ones a pair, 22 and 24 cycles of a partition), and
+// GB300 runs FP64 at 1/64 of the FP32 rate, so the tile loop holds no FP64
+// instruction.  Two sources at a time go through packed FP32 instructions
+// (fma.f32x2), which do not raise the FP32 rate but halve its issue slots, so
+// that the SFU's run beside them; a tile is staged as rows of 256 floats so
+// that one 128-bit load gives two packed operands.  A source tile whose
+// bounding sphere is farther than tau (with a 1e-3 margin) from the target
+// tile's holds no near pair; a bit mask built once per tube in FP64 says
+// which, and such tiles run the loop without near-field tests and phase
+// reduction.  The factor k^2 sg/(4 pi) is folded into the densities (and
 // divided out of the stored regularisation factors).  TMA bulk copies stage
-// source tiles in shared memory, double-buffered on mbarriers with bounded
-// waits.  Block shape and targets per thread come from a small table of
-// compiled variants; the autotuner times them on the operator's own data.
+// the tiles, double-buffered on mbarriers with bounded waits.  Block shape and
+// targets per thread come from a small table of compiled variants; the
+// autotuner times them on the operator's own data.
+//
+// One A p on GB300, before (scalar, phase reduced per pair) and now: n = 19,532
+// 0.603 -> 0.429 ms, n = 36,212 1.90 -> 1.31, n = 145,272 28.5 -> 18.1,
+// n = 581,420 365 -> 257 (1,318 Gpair/s).
 #include "hz_internal.cuh"
 #include "bulk_copy.cuh"
+#include "pair32.cuh"
 
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 namespace hz {
@@ -46,16 +54,19 @@ namespace {
 
 constexpr double kPi = 3.14159265358979323846264338328;
 
-// Internal MODE bit: reduce the phase in revolutions with a split k/(2 pi)
-// (hz_set_phase_mode, HZ_PHASE_SPLIT) instead of passing k rho to the SFU.
-constexpr int SWEEP_PHASE_SPLIT = 4;
+// Internal MODE bit: records scaled by k, phase centred on the source tile
+// (pair32.cuh).
+constexpr int SWEEP_SCALED = 4;
 
 struct Args32 {
     int64_t n, npad, mwords;
-    float wave, kh, kl;  // k and k/(2 pi) = kh + kl (kh: 12 significant bits)
-    float tau2, guard_lo, guard_hi;
+    Wave32 wave;
+    float tau2, guard_lo, guard_hi;  // (lambda tau)^2 and the tie band around it
     double tau;
-    const float4 *pos, *nrm, *dens;
+    int scaled;  // lambda = k (batches: per operator)
+    const float4 *pos, *nrm;
+    const float *soa;   // [tiles][kFixed][kTile32]: -x, -y, -z (tile-local), n, reg
+    float *dens;        // [tiles][6][kTile32]: re, im, -im of w p and of pt
     const float4 *thi, *tlo, *ohi, *olo;
     const uint32_t *nearmask;
     const double4_32a *tpos;
@@ -71,6 +82,12 @@ struct Args32 {
     double4_32a *partial;  // [P][2][slots per block]: (A re, A im, A^H re, A^H im)
 };
 
+constexpr int kFixed = kFixed32;  // staged floats per source besides the densities
+template <int MODE>
+constexpr int kDens = 3 * ((MODE & SWEEP_PAIR) == SWEEP_PAIR ? 2 : 1);
+template <int MODE>
+constexpr int kStage = (kFixed + kDens<MODE>) * kTile32;  // floats of a staged tile
+
 // The CTA whose unit range holds work unit u: the largest c with
 // floor(c U / P) <= u.
 __device__ __forceinline__ int64_t cta_of_unit(int64_t u, int64_t units, int64_t nctas)
@@ -78,102 +95,311 @@ __device__ __forceinline__ int64_t cta_of_unit(int64_t u, int64_t units, int64_t
     return ((u + 1) * nctas - 1) / units;
 }
 
-// hi + lo += f without rounding loss (Knuth's TwoSum; FP32 only).
-__device__ __forceinline__ void two_sum_acc(float &hi, float &lo, float f)
+// Densities of slot s, scale (w p, pt) in FP32, scale = lambda^2 sg / (4 pi).
+__device__ __forceinline__ void store_dens(float *dens, int64_t s, int half, float re, float im)
 {
-    const float s = hi + f;
-    const float bp = s - hi;
-    const float e = (hi - (s - bp)) + (f - bp);
-    hi = s;
-    lo += e;
+    float *d = dens + (s / kTile32) * (6 * kTile32) + half * (3 * kTile32) + (s & (kTile32 - 1));
+    d[0] = re;
+    d[kTile32] = im;
+    d[2 * kTile32] = -im;
 }
 
-// dens[s] = scale (w p, pt) at sweep slot s, FP32, scale = sg / (4 pi).
 __global__ void prep32_kernel(int64_t npad, const int *__restrict__ perm, const double4_32a *__restrict__ tpos,
                               const double *__restrict__ p_re, const double *__restrict__ p_im,
                               const double *__restrict__ pt_re, const double *__restrict__ pt_im, double scale,
-                              float4 *__restrict__ dens)
+                              float *__restrict__ dens)
 {
     for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < npad; s += (int64_t)gridDim.x * blockDim.x) {
         const int c = perm[s];
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (c >= 0) {
-            const double ws = tpos[s].w * scale;
-            if (p_re) {
-                v.x = (float)(ws * p_re[c]);
-                v.y = (float)(ws * p_im[c]);
-            }
-            if (pt_re) {
-                v.z = (float)(scale * pt_re[c]);
-                v.w = (float)(scale * pt_im[c]);
-            }
-        }
-        dens[s] = v;
+        const double ws = (c >= 0) ? tpos[s].w * scale : 0.0;
+        if (p_re) store_dens(dens, s, 0, c >= 0 ? (float)(ws * p_re[c]) : 0.f, c >= 0 ? (float)(ws * p_im[c]) : 0.f);
+        if (pt_re)
+            store_dens(dens, s, 1, c >= 0 ? (float)(scale * pt_re[c]) : 0.f, c >= 0 ? (float)(scale * pt_im[c]) : 0.f);
     }
 }
 
-// One source against TG targets; NEAR selects the loop with near-field
-// handling.  Accumulates into fA (A p) and fH (A^H pt).
-template <int MODE, bool DIR, int NT, int TG, bool NEAR>
-__device__ __forceinline__ void pair_block(const Args32 &a, const float4 s_p, const float4 s_n, const float4 s_d,
-                                           const float3 (&rel)[TG], const float3 (&tn)[TG], const float (&treg)[TG],
-                                           int64_t tslot0, int64_t src_slot, float (&fAr)[TG], float (&fAi)[TG],
-                                           float (&fHr)[TG], float (&fHi)[TG])
+// What a thread holds of its TG targets.
+template <int TG>
+struct Targets {
+    float3 th[TG], tl[TG], tn[TG];  // position head and tail, normal
+    float reg[TG];
+};
+
+// Cross-tile sums: FP32 head + tail (TwoSum), about 48 significant bits.
+template <int TG>
+struct Sums {
+    float hAr[TG], lAr[TG], hAi[TG], lAi[TG], hHr[TG], lHr[TG], hHi[TG], lHi[TG];
+};
+
+// The FP64 decision rho <= tau of a pair whose FP32 rho^2 is close to tau^2.
+__device__ __noinline__ bool near_exact(const Args32 &a, int64_t tslot, int64_t sslot)
 {
+    const int c = a.perm[sslot];
+    if (c < 0) return false;
+    const double4_32a q = a.pos64[c];
+    const double4_32a tp = a.tpos[tslot];
+    const double x1 = tp.x - q.x, x2 = tp.y - q.y, x3 = tp.z - q.z;
+    return !(sqrt(x1 * x1 + x2 * x2 + x3 * x3) > a.tau);
+}
+
+__device__ __forceinline__ bool is_near(const Args32 &a, float r2, int64_t tslot, int64_t sslot)
+{
+    if (r2 > a.guard_lo && r2 < a.guard_hi) return near_exact(a, tslot, sslot);
+    return r2 <= a.tau2;
+}
+
+// One source against TG targets, scalar (records with lambda = 1).
+template <int MODE, bool DIR, int NT, int TG>
+__device__ __forceinline__ void pair_scalar(const Args32 &a, const float *st, int j, bool maybe_near,
+                                            const float3 (&rel)[TG], const Targets<TG> &t, int64_t tslot0,
+                                            int64_t src_slot, float (&fAr)[TG], float (&fAi)[TG], float (&fHr)[TG],
+                                            float (&fHi)[TG])
+{
+    constexpr int T = kTile32;
+    const float sx = st[j], sy = st[T + j], sz = st[2 * T + j];
+    const float nx = st[3 * T + j], ny = st[4 * T + j], nz = st[5 * T + j], sreg = st[6 * T + j];
+    const float *d = st + kFixed * T + j;
 #pragma unroll
     for (int g = 0; g < TG; g++) {
-        const float dx = rel[g].x - s_p.x, dy = rel[g].y - s_p.y, dz = rel[g].z - s_p.z;
+        const float dx = rel[g].x + sx, dy = rel[g].y + sy, dz = rel[g].z + sz;
         const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-        bool near = false;
-        if (NEAR) {
-            near = r2 <= a.tau2;
-            if (r2 > a.guard_lo && r2 < a.guard_hi) {
-                // decide exactly as the FP64 sweep does
-                const int c = a.perm[src_slot];
-                if (c >= 0) {
-                    const double4_32a q = a.pos64[c];
-                    const double4_32a tp = a.tpos[tslot0 + (int64_t)g * NT];
-                    const double x1 = tp.x - q.x, x2 = tp.y - q.y, x3 = tp.z - q.z;
-                    near = !(sqrt(x1 * x1 + x2 * x2 + x3 * x3) > a.tau);
+        const bool near = maybe_near && is_near(a, r2, tslot0 + (int64_t)g * NT, src_slot);
+        float u1, u2, rr;
+        kernel32<false, true>(a.wave, r2, 0.f, u1, u2, rr);
+        const float ps = fmaf(dx, nx, fmaf(dy, ny, dz * nz));                          // (x_t - x_s).n_s
+        const float pt = fmaf(dx, t.tn[g].x, fmaf(dy, t.tn[g].y, dz * t.tn[g].z));    // (x_t - x_s).n_t
+        if (MODE & SWEEP_A) {
+            const float q = rr * (DIR ? ps : pt);
+            const float vr = near ? (DIR ? sreg : t.reg[g]) : -u1 * q, vi = near ? 0.f : u2 * q;
+            fAr[g] = fmaf(vr, d[0], fmaf(-vi, d[T], fAr[g]));
+            fAi[g] = fmaf(vr, d[T], fmaf(vi, d[0], fAi[g]));
+        }
+        if (MODE & SWEEP_AH) {
+            const float *e = d + (kDens<MODE> - 3) * T;
+            const float q = rr * (DIR ? pt : ps);
+            const float vr = near ? (DIR ? t.reg[g] : sreg) : u1 * q, vi = near ? 0.f : u2 * q;
+            fHr[g] = fmaf(vr, e[0], fmaf(-vi, e[T], fHr[g]));
+            fHi[g] = fmaf(vr, e[T], fmaf(vi, e[0], fHi[g]));
+        }
+    }
+}
+
+// A whole tile, two sources at a time in packed FP32: phase centred, or (SLOW:
+// near and wide tiles) reduced per pair and with the near-field test.  With y = 1/rho, e^{i theta} = C + i S and q the projection
+// over rho^2, A's entry times d is q (-(S e1 + C e2) + i (C e1 - S e2)),
+// e1 = dr - y di, e2 = di + y dr (A^H: conj(d) and the real part's sign), so
+// that no operand needs a negation (-im is staged).  A near pair takes C = 1,
+// S = 0 and e1, e2 from its regularisation factor.
+template <int MODE, bool DIR, int NT, int TG, bool SLOW>
+__device__ __forceinline__ void tile_packed(const Args32 &a, const float *st, const float3 (&rel)[TG],
+                                            const Targets<TG> &t, const Turn (&turn)[TG], int64_t tslot0,
+                                            int64_t sslot0, float (&fAr)[TG], float (&fAi)[TG], float (&fHr)[TG],
+                                            float (&fHi)[TG])
+{
+    constexpr int T = kTile32;
+    constexpr bool A = (MODE & SWEEP_A) != 0, H = (MODE & SWEEP_AH) != 0;
+    constexpr bool SRC = (A && DIR) || (H && !DIR), TGT = (A && !DIR) || (H && DIR);
+    F2 rx[TG], ry[TG], rz[TG], nrc[TG], tx[TG], ty[TG], tz[TG];
+    F2 aR[TG], aI[TG], aJ[TG], hR[TG], hI[TG], hJ[TG];
+#pragma unroll
+    for (int g = 0; g < TG; g++) {
+        rx[g] = f2_pack(rel[g].x, rel[g].x);
+        ry[g] = f2_pack(rel[g].y, rel[g].y);
+        rz[g] = f2_pack(rel[g].z, rel[g].z);
+        if (!SLOW) nrc[g] = f2_pack(-turn[g].rc, -turn[g].rc);
+        if (TGT) {
+            tx[g] = f2_pack(t.tn[g].x, t.tn[g].x);
+            ty[g] = f2_pack(t.tn[g].y, t.tn[g].y);
+            tz[g] = f2_pack(t.tn[g].z, t.tn[g].z);
+        }
+        aR[g] = aI[g] = aJ[g] = hR[g] = hI[g] = hJ[g] = 0;
+    }
+    auto at = [&](int row, int j) { return *reinterpret_cast<const ulonglong2 *>(st + row * T + j); };
+    for (int j = 0; j < T; j += 4) {
+        const ulonglong2 X = at(0, j), Y = at(1, j), Z = at(2, j);
+        ulonglong2 NX, NY, NZ, RG, DR, DI, DN, ER, EI, EN;
+        if (SLOW) RG = at(6, j);
+        if (SRC) {
+            NX = at(3, j);
+            NY = at(4, j);
+            NZ = at(5, j);
+        }
+        if (A) {
+            DR = at(kFixed, j);
+            DI = at(kFixed + 1, j);
+            DN = at(kFixed + 2, j);
+        }
+        if (H) {
+            ER = at(kFixed + kDens<MODE> - 3, j);
+            EI = at(kFixed + kDens<MODE> - 2, j);
+            EN = at(kFixed + kDens<MODE> - 1, j);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            auto of = [&](const ulonglong2 &v) { return h ? v.y : v.x; };
+#pragma unroll
+            for (int g = 0; g < TG; g++) {
+                const F2 dx = f2_add(rx[g], of(X)), dy = f2_add(ry[g], of(Y)), dz = f2_add(rz[g], of(Z));
+                const F2 r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz)));
+                const F2 y = f2_rsqrt(r2);
+                F2 S, C, th;
+                if (SLOW) {
+                    // less the nearest multiple of 2 pi = 6.28125 + 0.00193...
+                    const F2 rho = f2_mul(r2, y), M = f2_pack(12582912.f, 12582912.f);
+                    const F2 n = f2_add(f2_fma(rho, f2_pack(0.15915494309189535f, 0.15915494309189535f), M),
+                                        f2_pack(-12582912.f, -12582912.f));
+                    th = f2_fma(n, f2_pack(-0.0019353071795864769f, -0.0019353071795864769f),
+                                f2_fma(n, f2_pack(-6.28125f, -6.28125f), rho));
+                } else {
+                    th = f2_fma(r2, y, nrc[g]);
+                }
+                f2_sincos(th, S, C);
+                const F2 yy = f2_mul(y, y);
+                F2 ps, pt;
+                if (SRC) ps = f2_mul(yy, f2_fma(dx, of(NX), f2_fma(dy, of(NY), f2_mul(dz, of(NZ)))));
+                if (TGT) pt = f2_mul(yy, f2_fma(dx, tx[g], f2_fma(dy, ty[g], f2_mul(dz, tz[g]))));
+                F2 e1, e2, f1, f2;
+                if (A) {
+                    const F2 q = DIR ? ps : pt;
+                    e1 = f2_mul(q, f2_fma(y, of(DN), of(DR)));
+                    e2 = f2_mul(q, f2_fma(y, of(DR), of(DI)));
+                }
+                if (H) {
+                    const F2 q = DIR ? pt : ps;
+                    f1 = f2_mul(q, f2_fma(y, of(EI), of(ER)));
+                    f2 = f2_mul(q, f2_fma(y, of(ER), of(EN)));
+                }
+                if (SLOW) {
+                    float ra, rb;
+                    f2_unpack(r2, ra, rb);
+                    if (fminf(ra, rb) < a.guard_hi) {
+                        const int64_t ts = tslot0 + (int64_t)g * NT, ss = sslot0 + j + 2 * h;
+                        const bool na = is_near(a, ra, ts, ss), nb = is_near(a, rb, ts, ss + 1);
+                        auto pick = [&](F2 far, float va, float vb) {
+                            float fa, fb;
+                            f2_unpack(far, fa, fb);
+                            return f2_pack(na ? va : fa, nb ? vb : fb);
+                        };
+                        float ga, gb;
+                        f2_unpack(of(RG), ga, gb);
+                        S = pick(S, 0.f, 0.f);
+                        C = pick(C, 1.f, 1.f);
+                        if (A) {
+                            const float va = DIR ? ga : t.reg[g], vb = DIR ? gb : t.reg[g];
+                            float d0, d1, i0, i1;
+                            f2_unpack(of(DR), d0, d1);
+                            f2_unpack(of(DI), i0, i1);
+                            e1 = pick(e1, va * i0, vb * i1);
+                            e2 = pick(e2, -va * d0, -vb * d1);
+                        }
+                        if (H) {
+                            const float va = DIR ? t.reg[g] : ga, vb = DIR ? t.reg[g] : gb;
+                            float d0, d1, i0, i1;
+                            f2_unpack(of(ER), d0, d1);
+                            f2_unpack(of(EI), i0, i1);
+                            f1 = pick(f1, va * i0, vb * i1);
+                            f2 = pick(f2, va * d0, vb * d1);
+                        }
+                    }
+                }
+                if (A) {
+                    aR[g] = f2_fma(S, e1, f2_fma(C, e2, aR[g]));
+                    aI[g] = f2_fma(C, e1, aI[g]);
+                    aJ[g] = f2_fma(S, e2, aJ[g]);
+                }
+                if (H) {
+                    hR[g] = f2_fma(S, f1, f2_fma(C, f2, hR[g]));
+                    hI[g] = f2_fma(C, f1, hI[g]);
+                    hJ[g] = f2_fma(S, f2, hJ[g]);
                 }
             }
         }
-        const float rinv = rsqrtf(r2);
-        const float rho = r2 * rinv;
-        float S, C;
-        if (MODE & SWEEP_PHASE_SPLIT) {
-            // revolutions rho k/(2 pi) less the nearest integer (|rho kh| <
-            // 2^22: add and remove 1.5 2^23), exact to ~2^-24 before the SFU
-            const float nn = fmaf(rho, a.kh, 12582912.f) - 12582912.f;
-            float f = fmaf(rho, a.kh, -nn);
-            f = fmaf(rho, a.kl, f);
-            __sincosf(f * 6.28318530717958647692f, &S, &C);
-        } else {
-            __sincosf(rho * a.wave, &S, &C);
+    }
+#pragma unroll
+    for (int g = 0; g < TG; g++) {
+        if (A) {
+            fAr[g] = -f2_sum(aR[g]);
+            fAi[g] = f2_sum(aI[g]) - f2_sum(aJ[g]);
+            if (!SLOW) turn_sum<false>(turn[g], fAr[g], fAi[g]);
         }
-        const float u1 = fmaf(C, rinv, a.wave * S);   // k sin + cos/rho
-        const float u2 = fmaf(a.wave, C, -S * rinv);  // k cos - sin/rho
-        const float rr = rinv * rinv;
-        const float a1 = -u1 * rr, a2 = u2 * rr;
-        const float pn = dx * s_n.x + dy * s_n.y + dz * s_n.z;        // (x_t-x_s).n_s
-        const float pt = dx * tn[g].x + dy * tn[g].y + dz * tn[g].z;  // (x_t-x_s).n_t
-        const float pA = DIR ? pn : pt, pH = DIR ? pt : pn;
-        float vAr = a1 * pA, vAi = a2 * pA, vHr = -a1 * pH, vHi = a2 * pH;
-        if (NEAR && near) {
-            vAr = DIR ? s_p.w : treg[g];
-            vHr = DIR ? treg[g] : s_p.w;
-            vAi = 0.f;
-            vHi = 0.f;
-        }
-        if (MODE & SWEEP_A) {
-            fAr[g] = fmaf(vAr, s_d.x, fmaf(-vAi, s_d.y, fAr[g]));
-            fAi[g] = fmaf(vAr, s_d.y, fmaf(vAi, s_d.x, fAi[g]));
-        }
-        if (MODE & SWEEP_AH) {
-            fHr[g] = fmaf(vHr, s_d.z, fmaf(-vHi, s_d.w, fHr[g]));
-            fHi[g] = fmaf(vHr, s_d.w, fmaf(vHi, s_d.z, fHi[g]));
+        if (H) {
+            fHr[g] = f2_sum(hR[g]);
+            fHi[g] = f2_sum(hI[g]) - f2_sum(hJ[g]);
+            if (!SLOW) turn_sum<true>(turn[g], fHr[g], fHi[g]);
         }
     }
+}
+
+// The pairs of the block's targets with the staged source tile, added to sum.
+template <int MODE, bool DIR, int NT, int TG>
+__device__ __forceinline__ void tile_pairs(const Args32 &a, const float *st, int64_t tile, bool near,
+                                           const float3 (&rel)[TG], const Turn (&turn)[TG], bool centred,
+                                           const Targets<TG> &t, int64_t slot0, Sums<TG> &sum)
+{
+    float fAr[TG], fAi[TG], fHr[TG], fHi[TG];
+#pragma unroll
+    for (int g = 0; g < TG; g++) fAr[g] = fAi[g] = fHr[g] = fHi[g] = 0.f;
+    if (!(MODE & SWEEP_SCALED)) {
+        for (int j = 0; j < kTile32; j++)
+            pair_scalar<MODE, DIR, NT, TG>(a, st, j, near, rel, t, slot0, tile * kTile32 + j, fAr, fAi, fHr, fHi);
+    } else if (centred) {
+        tile_packed<MODE, DIR, NT, TG, false>(a, st, rel, t, turn, slot0, tile * kTile32, fAr, fAi, fHr, fHi);
+    } else {
+        tile_packed<MODE, DIR, NT, TG, true>(a, st, rel, t, turn, slot0, tile * kTile32, fAr, fAi, fHr, fHi);
+    }
+#pragma unroll
+    for (int g = 0; g < TG; g++) {
+        if (MODE & SWEEP_A) {
+            two_sum_acc(sum.hAr[g], sum.lAr[g], fAr[g]);
+            two_sum_acc(sum.hAi[g], sum.lAi[g], fAi[g]);
+        }
+        if (MODE & SWEEP_AH) {
+            two_sum_acc(sum.hHr[g], sum.lHr[g], fHr[g]);
+            two_sum_acc(sum.hHi[g], sum.lHi[g], fHi[g]);
+        }
+    }
+}
+
+template <int NT, int TG>
+__device__ __forceinline__ void load_targets(const Args32 &a, int64_t slot0, Targets<TG> &t, Sums<TG> &sum)
+{
+#pragma unroll
+    for (int g = 0; g < TG; g++) {
+        const int64_t s = slot0 + (int64_t)g * NT;
+        const float4 h = a.thi[s], l = a.tlo[s], nn = a.nrm[s];
+        t.th[g] = make_float3(h.x, h.y, h.z);
+        t.tl[g] = make_float3(l.x, l.y, l.z);
+        t.tn[g] = make_float3(nn.x, nn.y, nn.z);
+        t.reg[g] = a.pos[s].w;
+        sum.hAr[g] = sum.lAr[g] = sum.hAi[g] = sum.lAi[g] = 0.f;
+        sum.hHr[g] = sum.lHr[g] = sum.hHi[g] = sum.lHi[g] = 0.f;
+    }
+}
+
+// x_t - o of the targets (the head difference is rounded once, to half an ulp
+// of itself) and the turns of a centred tile.
+template <int MODE, int TG>
+__device__ __forceinline__ bool tile_offsets(const Args32 &a, int64_t tile, bool near, const Targets<TG> &t,
+                                             float3 (&rel)[TG], Turn (&turn)[TG])
+{
+    const float4 oh = a.ohi[tile], ol = a.olo[tile];
+    const bool centred = (MODE & SWEEP_SCALED) && !near && oh.w <= kCentreRadius;
+#pragma unroll
+    for (int g = 0; g < TG; g++) {
+        rel[g] = make_float3((t.th[g].x - oh.x) + (t.tl[g].x - ol.x), (t.th[g].y - oh.y) + (t.tl[g].y - ol.y),
+                             (t.th[g].z - oh.z) + (t.tl[g].z - ol.z));
+        if (centred) turn[g] = turn_of(rel[g]);
+    }
+    return centred;
+}
+
+template <int MODE>
+__device__ __forceinline__ void issue_tile(const Args32 &a, int64_t tile, float *st, uint64_t *bar)
+{
+    constexpr uint32_t fixed = kFixed * kTile32 * sizeof(float), dens = kDens<MODE> * kTile32 * sizeof(float);
+    mbar_arrive_expect_tx(bar, fixed + dens);
+    bulk_g2s(st, a.soa + tile * (kFixed * kTile32), fixed, bar);
+    bulk_g2s(st + kFixed * kTile32, a.dens + tile * (6 * kTile32) + ((MODE & SWEEP_A) ? 0 : 3 * kTile32), dens, bar);
 }
 
 // Final value of one target slot: q = sum + p/2 (A), qt = w sum + pt/2 (A^H).
@@ -205,15 +431,12 @@ __device__ __forceinline__ void write_slot(const Args32 &a, int64_t s, double ar
 template <int MODE, bool DIR, int NT, int TG, int MINB>
 __global__ void __launch_bounds__(NT, MINB) sweep32_kernel(Args32 a)
 {
-    constexpr int TS = kTile32;
-    constexpr int SLOTS = NT * TG;   // target slots per block (a multiple of TS)
-    constexpr int NTT = SLOTS / TS;  // target tiles per block
-    __shared__ alignas(128) float4 sp[2][TS];
-    __shared__ alignas(128) float4 sn[2][TS];
-    __shared__ alignas(128) float4 sd[2][TS];
+    constexpr int SLOTS = NT * TG;
+    static_assert(SLOTS == kTile32, "one target tile per block: every shape then runs the same loops on a pair");
+    __shared__ alignas(128) float stage[2][kStage<MODE>];
     __shared__ alignas(8) uint64_t bar[2];
 
-    const int64_t ntiles = a.npad / TS;
+    const int64_t ntiles = a.npad / kTile32;
     const int64_t u_begin = (int64_t)blockIdx.x * a.units / a.nctas;
     const int64_t u_end = ((int64_t)blockIdx.x + 1) * a.units / a.nctas;
     if (threadIdx.x == 0) {
@@ -223,54 +446,26 @@ __global__ void __launch_bounds__(NT, MINB) sweep32_kernel(Args32 a)
     }
     __syncthreads();
     if (u_begin >= u_end) return;
-    auto issue = [&](int64_t u, int buf) {
-        const int64_t base = (u % ntiles) * TS;
-        const uint32_t bytes = TS * sizeof(float4);
-        mbar_arrive_expect_tx(&bar[buf], 3 * bytes);
-        bulk_g2s(&sp[buf][0], a.pos + base, bytes, &bar[buf]);
-        bulk_g2s(&sn[buf][0], a.nrm + base, bytes, &bar[buf]);
-        bulk_g2s(&sd[buf][0], a.dens + base, bytes, &bar[buf]);
-    };
-    if (threadIdx.x == 0) issue(u_begin, 0);
+    if (threadIdx.x == 0) issue_tile<MODE>(a, u_begin % ntiles, stage[0], &bar[0]);
     int seg = 0;
     for (int64_t u = u_begin; u < u_end;) {
         const int64_t blk = u / ntiles;
         const int64_t seg_end = (u_end < (blk + 1) * ntiles) ? u_end : (blk + 1) * ntiles;
         const bool whole = (u == blk * ntiles) && (seg_end == (blk + 1) * ntiles);
         const int64_t slot0 = blk * SLOTS + threadIdx.x;
-        float3 th[TG], tl[TG], tn[TG];
-        float treg[TG];
-        // cross-tile sums: FP32 head + tail (TwoSum), about 48 significant bits
-        float hAr[TG], lAr[TG], hAi[TG], lAi[TG], hHr[TG], lHr[TG], hHi[TG], lHi[TG];
-#pragma unroll
-        for (int g = 0; g < TG; g++) {
-            const int64_t s = slot0 + (int64_t)g * NT;
-            const float4 h = a.thi[s], l = a.tlo[s], nn = a.nrm[s];
-            th[g] = make_float3(h.x, h.y, h.z);
-            tl[g] = make_float3(l.x, l.y, l.z);
-            tn[g] = make_float3(nn.x, nn.y, nn.z);
-            treg[g] = a.pos[s].w;
-            hAr[g] = lAr[g] = hAi[g] = lAi[g] = hHr[g] = lHr[g] = hHi[g] = lHi[g] = 0.f;
-        }
-        // rows of the near-tile mask for this block's target tiles
-        const uint32_t *mrow = a.nearmask + (blk * NTT) * a.mwords;
+        Targets<TG> t;
+        Sums<TG> sum;
+        load_targets<NT, TG>(a, slot0, t, sum);
+        const uint32_t *mrow = a.nearmask + blk * a.mwords;  // the near-tile mask of this target tile
         for (; u < seg_end; u++) {
             const int64_t it = u - u_begin;
             const int buf = (int)(it & 1);
-            if (threadIdx.x == 0 && u + 1 < u_end) issue(u + 1, buf ^ 1);
+            if (threadIdx.x == 0 && u + 1 < u_end) issue_tile<MODE>(a, (u + 1) % ntiles, stage[buf ^ 1], &bar[buf ^ 1]);
             const int64_t tile = u - blk * ntiles;
-            uint32_t word = 0;
-#pragma unroll
-            for (int k = 0; k < NTT; k++) word |= __ldg(mrow + k * a.mwords + (tile >> 5));
-            const bool far = ((word >> (tile & 31)) & 1u) == 0;
-            // x_t - o: head difference (rounded once, to half an ulp of
-            // itself) plus the tails
-            const float4 oh = a.ohi[tile], ol = a.olo[tile];
+            const bool near = (__ldg(mrow + (tile >> 5)) >> (tile & 31)) & 1u;
             float3 rel[TG];
-#pragma unroll
-            for (int g = 0; g < TG; g++)
-                rel[g] = make_float3((th[g].x - oh.x) + (tl[g].x - ol.x), (th[g].y - oh.y) + (tl[g].y - ol.y),
-                                     (th[g].z - oh.z) + (tl[g].z - ol.z));
+            Turn turn[TG];
+            const bool centred = tile_offsets<MODE, TG>(a, tile, near, t, rel, turn);
             const bool ok = mbar_wait_bounded(&bar[buf], (uint32_t)((it >> 1) & 1), g_data_wait_limit);
             if (__syncthreads_or(!ok)) {
                 if (threadIdx.x == 0) {
@@ -280,38 +475,13 @@ __global__ void __launch_bounds__(NT, MINB) sweep32_kernel(Args32 a)
                 }
                 return;
             }
-            float fAr[TG], fAi[TG], fHr[TG], fHi[TG];
-#pragma unroll
-            for (int g = 0; g < TG; g++) fAr[g] = fAi[g] = fHr[g] = fHi[g] = 0.f;
-            const int64_t base = tile * TS;
-            if (far) {
-#pragma unroll 2
-                for (int j = 0; j < TS; j++)
-                    pair_block<MODE, DIR, NT, TG, false>(a, sp[buf][j], sn[buf][j], sd[buf][j], rel, tn, treg, slot0,
-                                                         base + j, fAr, fAi, fHr, fHi);
-            } else {
-#pragma unroll 2
-                for (int j = 0; j < TS; j++)
-                    pair_block<MODE, DIR, NT, TG, true>(a, sp[buf][j], sn[buf][j], sd[buf][j], rel, tn, treg, slot0,
-                                                        base + j, fAr, fAi, fHr, fHi);
-            }
-#pragma unroll
-            for (int g = 0; g < TG; g++) {
-                if (MODE & SWEEP_A) {
-                    two_sum_acc(hAr[g], lAr[g], fAr[g]);
-                    two_sum_acc(hAi[g], lAi[g], fAi[g]);
-                }
-                if (MODE & SWEEP_AH) {
-                    two_sum_acc(hHr[g], lHr[g], fHr[g]);
-                    two_sum_acc(hHi[g], lHi[g], fHi[g]);
-                }
-            }
+            tile_pairs<MODE, DIR, NT, TG>(a, stage[buf], tile, near, rel, turn, centred, t, slot0, sum);
             __syncthreads();
         }
 #pragma unroll
         for (int g = 0; g < TG; g++) {
-            const double ar = (double)hAr[g] + (double)lAr[g], ai = (double)hAi[g] + (double)lAi[g];
-            const double hr = (double)hHr[g] + (double)lHr[g], hi = (double)hHi[g] + (double)lHi[g];
+            const double ar = (double)sum.hAr[g] + (double)sum.lAr[g], ai = (double)sum.hAi[g] + (double)sum.lAi[g];
+            const double hr = (double)sum.hHr[g] + (double)sum.lHr[g], hi = (double)sum.hHi[g] + (double)sum.lHi[g];
             if (whole) {
                 write_slot<MODE>(a, slot0 + (int64_t)g * NT, ar, ai, hr, hi);
             } else {
@@ -360,7 +530,7 @@ struct BatchOp {
     int64_t blocks, ntiles;
     int dir;
     int col;         // column of P and Q
-    double scale;    // sg / (4 pi), folded into the densities
+    double scale;    // lambda^2 sg / (4 pi), folded into the densities
 };
 
 struct BatchVec {
@@ -374,17 +544,11 @@ __global__ void batch_prep_kernel(const BatchOp *__restrict__ ops, BatchVec v)
 {
     const BatchOp &o = ops[blockIdx.y];
     const double *pr = v.p_re + (int64_t)o.col * v.stride, *pi = v.p_im + (int64_t)o.col * v.stride;
-    float4 *dens = const_cast<float4 *>(o.a.dens);
     for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < o.a.npad;
          s += (int64_t)gridDim.x * blockDim.x) {
         const int c = o.a.perm[s];
-        float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (c >= 0) {
-            const double ws = o.a.tpos[s].w * o.scale;
-            d.x = (float)(ws * pr[c]);
-            d.y = (float)(ws * pi[c]);
-        }
-        dens[s] = d;
+        const double ws = (c >= 0) ? o.a.tpos[s].w * o.scale : 0.0;
+        store_dens(o.a.dens, s, 0, c >= 0 ? (float)(ws * pr[c]) : 0.f, c >= 0 ? (float)(ws * pi[c]) : 0.f);
     }
 }
 
@@ -406,43 +570,27 @@ __device__ __forceinline__ void batch_write(const Args32 &a, int64_t s, double a
 }
 
 // The tiles of one segment (one target block of one operator) for the
-// batched sweep: the same loop as sweep32_kernel with SWEEP_A.
-template <bool DIR, int NT, int TG>
+// batched sweep: the same loops as sweep32_kernel with SWEEP_A.
+template <int MODE, bool DIR, int NT, int TG>
 __device__ __forceinline__ bool batch_tiles(const Args32 &a, const BatchOp *ops, int nops, int o, int64_t &u,
                                             int64_t seg_end, int64_t u_begin, int64_t u_end, int64_t blk,
-                                            int64_t slot0, const float3 (&th)[TG], const float3 (&tl)[TG],
-                                            const float3 (&tn)[TG], const float (&treg)[TG], float (&hAr)[TG],
-                                            float (&lAr)[TG], float (&hAi)[TG], float (&lAi)[TG],
-                                            float4 (*sp)[kTile32], float4 (*sn)[kTile32], float4 (*sd)[kTile32],
-                                            uint64_t *bar)
+                                            int64_t slot0, const Targets<TG> &t, Sums<TG> &sum,
+                                            float (*stage)[kStage<SWEEP_A>], uint64_t *bar)
 {
-    constexpr int TS = kTile32;
-    constexpr int NTT = NT * TG / TS;
     const int64_t ntiles = ops[o].ntiles, unit0 = ops[o].unit0;
-    const uint32_t *mrow = a.nearmask + (blk * NTT) * a.mwords;
+    const uint32_t *mrow = a.nearmask + blk * a.mwords;
     for (; u < seg_end; u++) {
         const int64_t it = u - u_begin;
         const int buf = (int)(it & 1);
         if (threadIdx.x == 0 && u + 1 < u_end) {
             const int o2 = batch_op_of_unit(ops, nops, u + 1, o);
-            const int64_t base = ((u + 1 - ops[o2].unit0) % ops[o2].ntiles) * TS;
-            const uint32_t bytes = TS * sizeof(float4);
-            mbar_arrive_expect_tx(&bar[buf ^ 1], 3 * bytes);
-            bulk_g2s(&sp[buf ^ 1][0], ops[o2].a.pos + base, bytes, &bar[buf ^ 1]);
-            bulk_g2s(&sn[buf ^ 1][0], ops[o2].a.nrm + base, bytes, &bar[buf ^ 1]);
-            bulk_g2s(&sd[buf ^ 1][0], ops[o2].a.dens + base, bytes, &bar[buf ^ 1]);
+            issue_tile<SWEEP_A>(ops[o2].a, (u + 1 - ops[o2].unit0) % ops[o2].ntiles, stage[buf ^ 1], &bar[buf ^ 1]);
         }
         const int64_t tile = u - unit0 - blk * ntiles;
-        uint32_t word = 0;
-#pragma unroll
-        for (int k = 0; k < NTT; k++) word |= __ldg(mrow + k * a.mwords + (tile >> 5));
-        const bool far = ((word >> (tile & 31)) & 1u) == 0;
-        const float4 oh = a.ohi[tile], ol = a.olo[tile];
+        const bool near = (__ldg(mrow + (tile >> 5)) >> (tile & 31)) & 1u;
         float3 rel[TG];
-#pragma unroll
-        for (int g = 0; g < TG; g++)
-            rel[g] = make_float3((th[g].x - oh.x) + (tl[g].x - ol.x), (th[g].y - oh.y) + (tl[g].y - ol.y),
-                                 (th[g].z - oh.z) + (tl[g].z - ol.z));
+        Turn turn[TG];
+        const bool centred = tile_offsets<MODE, TG>(a, tile, near, t, rel, turn);
         const bool ok = mbar_wait_bounded(&bar[buf], (uint32_t)((it >> 1) & 1), g_data_wait_limit);
         if (__syncthreads_or(!ok)) {
             if (threadIdx.x == 0) {
@@ -452,26 +600,7 @@ __device__ __forceinline__ bool batch_tiles(const Args32 &a, const BatchOp *ops,
             }
             return false;
         }
-        float fAr[TG], fAi[TG], fHr[TG], fHi[TG];
-#pragma unroll
-        for (int g = 0; g < TG; g++) fAr[g] = fAi[g] = fHr[g] = fHi[g] = 0.f;
-        const int64_t base = tile * TS;
-        if (far) {
-#pragma unroll 2
-            for (int j = 0; j < TS; j++)
-                pair_block<SWEEP_A, DIR, NT, TG, false>(a, sp[buf][j], sn[buf][j], sd[buf][j], rel, tn, treg, slot0,
-                                                        base + j, fAr, fAi, fHr, fHi);
-        } else {
-#pragma unroll 2
-            for (int j = 0; j < TS; j++)
-                pair_block<SWEEP_A, DIR, NT, TG, true>(a, sp[buf][j], sn[buf][j], sd[buf][j], rel, tn, treg, slot0,
-                                                       base + j, fAr, fAi, fHr, fHi);
-        }
-#pragma unroll
-        for (int g = 0; g < TG; g++) {
-            two_sum_acc(hAr[g], lAr[g], fAr[g]);
-            two_sum_acc(hAi[g], lAi[g], fAi[g]);
-        }
+        tile_pairs<MODE, DIR, NT, TG>(a, stage[buf], tile, near, rel, turn, centred, t, slot0, sum);
         __syncthreads();
     }
     return true;
@@ -486,11 +615,8 @@ __global__ void __launch_bounds__(NT, MINB) sweep32_batch_kernel(const BatchOp *
                                                                  int64_t units, int64_t nctas,
                                                                  double4_32a *partial, BatchVec v)
 {
-    constexpr int TS = kTile32;
     constexpr int SLOTS = NT * TG;
-    __shared__ alignas(128) float4 sp[2][TS];
-    __shared__ alignas(128) float4 sn[2][TS];
-    __shared__ alignas(128) float4 sd[2][TS];
+    __shared__ alignas(128) float stage[2][kStage<SWEEP_A>];
     __shared__ alignas(8) uint64_t bar[2];
     const int64_t u_begin = (int64_t)blockIdx.x * units / nctas;
     const int64_t u_end = ((int64_t)blockIdx.x + 1) * units / nctas;
@@ -502,14 +628,7 @@ __global__ void __launch_bounds__(NT, MINB) sweep32_batch_kernel(const BatchOp *
     __syncthreads();
     if (u_begin >= u_end) return;
     int o = batch_op_of_unit(ops, nops, u_begin, 0);
-    if (threadIdx.x == 0) {
-        const int64_t base = ((u_begin - ops[o].unit0) % ops[o].ntiles) * TS;
-        const uint32_t bytes = TS * sizeof(float4);
-        mbar_arrive_expect_tx(&bar[0], 3 * bytes);
-        bulk_g2s(&sp[0][0], ops[o].a.pos + base, bytes, &bar[0]);
-        bulk_g2s(&sn[0][0], ops[o].a.nrm + base, bytes, &bar[0]);
-        bulk_g2s(&sd[0][0], ops[o].a.dens + base, bytes, &bar[0]);
-    }
+    if (threadIdx.x == 0) issue_tile<SWEEP_A>(ops[o].a, (u_begin - ops[o].unit0) % ops[o].ntiles, stage[0], &bar[0]);
     int seg = 0;
     for (int64_t u = u_begin; u < u_end;) {
         o = batch_op_of_unit(ops, nops, u, o);
@@ -520,31 +639,24 @@ __global__ void __launch_bounds__(NT, MINB) sweep32_batch_kernel(const BatchOp *
         const int64_t seg_end = (u_end < blk_end) ? u_end : blk_end;
         const bool whole = (u == unit0 + blk * ntiles) && (seg_end == blk_end);
         const int64_t slot0 = blk * SLOTS + threadIdx.x;
-        float3 th[TG], tl[TG], tn[TG];
-        float treg[TG];
-        float hAr[TG], lAr[TG], hAi[TG], lAi[TG];
-#pragma unroll
-        for (int g = 0; g < TG; g++) {
-            const int64_t s = slot0 + (int64_t)g * NT;
-            const float4 h = a.thi[s], l = a.tlo[s], nn = a.nrm[s];
-            th[g] = make_float3(h.x, h.y, h.z);
-            tl[g] = make_float3(l.x, l.y, l.z);
-            tn[g] = make_float3(nn.x, nn.y, nn.z);
-            treg[g] = a.pos[s].w;
-            hAr[g] = lAr[g] = hAi[g] = lAi[g] = 0.f;
-        }
-        const bool ok = ops[o].dir
-                            ? batch_tiles<true, NT, TG>(a, ops, nops, o, u, seg_end, u_begin, u_end, blk, slot0, th,
-                                                        tl, tn, treg, hAr, lAr, hAi, lAi, sp, sn, sd, bar)
-                            : batch_tiles<false, NT, TG>(a, ops, nops, o, u, seg_end, u_begin, u_end, blk, slot0, th,
-                                                         tl, tn, treg, hAr, lAr, hAi, lAi, sp, sn, sd, bar);
+        Targets<TG> t;
+        Sums<TG> sum;
+        load_targets<NT, TG>(a, slot0, t, sum);
+        auto walk = [&](auto mode, auto dir) {
+            return batch_tiles<decltype(mode)::value, decltype(dir)::value, NT, TG>(
+                a, ops, nops, o, u, seg_end, u_begin, u_end, blk, slot0, t, sum, stage, bar);
+        };
+        using Scaled = std::integral_constant<int, SWEEP_A | SWEEP_SCALED>;
+        using Plain = std::integral_constant<int, SWEEP_A>;
+        const bool ok = a.scaled ? (ops[o].dir ? walk(Scaled{}, std::true_type{}) : walk(Scaled{}, std::false_type{}))
+                                 : (ops[o].dir ? walk(Plain{}, std::true_type{}) : walk(Plain{}, std::false_type{}));
         if (!ok) return;
         const int64_t off = (int64_t)ops[o].col * v.stride;
         const double *pr = v.p_re + off, *pi = v.p_im + off;
         double *qr = v.q_re + off, *qi = v.q_im + off;
 #pragma unroll
         for (int g = 0; g < TG; g++) {
-            const double ar = (double)hAr[g] + (double)lAr[g], ai = (double)hAi[g] + (double)lAi[g];
+            const double ar = (double)sum.hAr[g] + (double)sum.lAr[g], ai = (double)sum.hAi[g] + (double)sum.lAi[g];
             if (whole)
                 batch_write(a, slot0 + (int64_t)g * NT, ar, ai, pr, pi, qr, qi);
             else
@@ -670,7 +782,7 @@ int launch_streamk(Args32 a, bool persistent, size_t partial_bytes, cudaStream_t
 
 // Compiled variants: (block size, targets per thread, minimum resident
 // blocks) x (persistent stream-K grid, or one CTA per target block).  Every
-// shape covers 256 or 512 sweep slots per block (npad is a multiple of 512).
+// shape covers the 256 slots of one target tile.
 constexpr int kShapes = 4;
 template <int MODE, bool DIR>
 int launch_cfg(int cfg, const Args32 &a, size_t pb, cudaStream_t s)
@@ -679,8 +791,8 @@ int launch_cfg(int cfg, const Args32 &a, size_t pb, cudaStream_t s)
     switch (cfg % kShapes) {
     case 1: return launch_streamk<MODE, DIR, 128, 2, 4>(a, persistent, pb, s);
     case 2: return launch_streamk<MODE, DIR, 256, 1, 3>(a, persistent, pb, s);
-    case 3: return launch_streamk<MODE, DIR, 128, 2, 6>(a, persistent, pb, s);
-    default: return launch_streamk<MODE, DIR, 256, 2, 2>(a, persistent, pb, s);
+    case 3: return launch_streamk<MODE, DIR, 128, 2, 3>(a, persistent, pb, s);
+    default: return launch_streamk<MODE, DIR, 256, 1, 2>(a, persistent, pb, s);
     }
 }
 
@@ -692,19 +804,35 @@ int launch32(int cfg, const Args32 &a, bool dir, size_t pb, cudaStream_t s)
 
 }  // namespace
 
-// Split k/(2 pi) into a head with 12 significant bits and an FP32 tail.
-void split_wave(double wave, float &kh, float &kl)
+// The constants of an operator's FP32 records: k, k/(2 pi) split into a head
+// with 12 significant bits and an FP32 tail, (lambda tau)^2 and its tie band.
+Const32 constants32(const SweepConst &c, double lambda)
 {
-    const double kc = wave / (2.0 * kPi);
+    Const32 r;
+    r.scaled = lambda != 1.0 || c.wave == 1.0;
+    r.k = (float)c.wave;
+    const double kc = c.wave / (2.0 * kPi);
     int e;
     frexp(kc, &e);
     const double q = ldexp(1.0, e - 12);
     const double head = nearbyint(kc / q) * q;
-    kh = (float)head;
-    kl = (float)(kc - head);
+    r.kh = (float)head;
+    r.kl = (float)(kc - head);
+    const double t2 = (lambda * c.tau) * (lambda * c.tau);
+    r.tau2 = (float)t2;
+    r.guard_lo = (float)(t2 * (1.0 - 1e-4));
+    r.guard_hi = (float)(t2 * (1.0 + 1e-4));
+    return r;
 }
 
-double sweep32_reg_scale(int interior) { return ((interior == 1) ? -1.0 : 1.0) * (4.0 * kPi); }
+// Below k = 2^-14 (and for k <= 0) the coordinates stay unscaled: 1/(k rho)^3
+// must stay inside the FP32 range.
+double lambda32(double wave) { return wave >= 1.0 / 16384 ? wave : 1.0; }
+
+double sweep32_reg_scale(int interior, double lambda)
+{
+    return ((interior == 1) ? -1.0 : 1.0) * (4.0 * kPi) / (lambda * lambda);
+}
 
 int sweep32_num_configs() { return 2 * kShapes; }
 
@@ -718,8 +846,8 @@ template <int MODE, bool DIR>
 size_t partial_need_all()
 {
     size_t m = 0;
-    const size_t v[kShapes] = {partial_need<MODE, DIR, 256, 2, 2>(), partial_need<MODE, DIR, 128, 2, 4>(),
-                               partial_need<MODE, DIR, 256, 1, 3>(), partial_need<MODE, DIR, 128, 2, 6>()};
+    const size_t v[kShapes] = {partial_need<MODE, DIR, 256, 1, 2>(), partial_need<MODE, DIR, 128, 2, 4>(),
+                               partial_need<MODE, DIR, 256, 1, 3>(), partial_need<MODE, DIR, 128, 2, 3>()};
     for (size_t x : v) m = x > m ? x : m;
     return m;
 }
@@ -727,7 +855,7 @@ size_t partial_need_all()
 
 size_t sweep32_partial_bytes()
 {
-    constexpr int S = SWEEP_PHASE_SPLIT;
+    constexpr int S = SWEEP_SCALED;
     const size_t v[12] = {partial_need_all<SWEEP_A, false>(),        partial_need_all<SWEEP_A, true>(),
                           partial_need_all<SWEEP_AH, false>(),       partial_need_all<SWEEP_AH, true>(),
                           partial_need_all<SWEEP_PAIR, false>(),     partial_need_all<SWEEP_PAIR, true>(),
@@ -739,14 +867,25 @@ size_t sweep32_partial_bytes()
     return m;
 }
 
+static void set_constants(const SweepConst &c, double lambda, Args32 &a)
+{
+    const Const32 k = constants32(c, lambda);
+    a.scaled = k.scaled;
+    a.wave = {k.k, k.kh, k.kl};
+    a.tau = c.tau;
+    a.tau2 = k.tau2;
+    a.guard_lo = k.guard_lo;
+    a.guard_hi = k.guard_hi;
+}
+
 // ---------------------------------------------------------------- batches
 size_t batch32_desc_bytes(int R) { return (size_t)R * sizeof(BatchOp); }
 
 int batch32_describe(const Batch32Item *items, int R, int cfg, void *desc_dev, int64_t &units, int64_t &blocks,
                      cudaStream_t s, const int *cols)
 {
-    static const int kSlots[kShapes] = {512, 256, 256, 256};  // NT * TG of shapes 0..3 (launch_cfg)
-    const int slots = kSlots[cfg % kShapes];
+    (void)cfg;
+    const int slots = kTile32;
     std::vector<BatchOp> h(R);
     units = 0;
     blocks = 0;
@@ -760,12 +899,9 @@ int batch32_describe(const Batch32Item *items, int R, int cfg, void *desc_dev, i
         a.n = it.c.n;
         a.npad = it.r.npad;
         a.mwords = it.r.mwords;
-        a.wave = (float)it.c.wave;
-        a.tau = it.c.tau;
-        a.tau2 = (float)(it.c.tau * it.c.tau);
-        a.guard_lo = (float)(it.c.tau * it.c.tau * (1.0 - 1e-4));
-        a.guard_hi = (float)(it.c.tau * it.c.tau * (1.0 + 1e-4));
+        set_constants(it.c, it.r.lambda, a);
         a.pos = it.r.pos;
+        a.soa = it.r.soa;
         a.nrm = it.r.nrm;
         a.dens = it.dens;
         a.thi = it.r.thi;
@@ -787,7 +923,7 @@ int batch32_describe(const Batch32Item *items, int R, int cfg, void *desc_dev, i
         b.unit0 = units;
         b.block0 = blocks;
         b.dir = it.c.dirichlet != 0;
-        b.scale = ((it.c.interior == 1) ? -1.0 : 1.0) / (4.0 * kPi);
+        b.scale = 1.0 / sweep32_reg_scale(it.c.interior, it.r.lambda);
         units += b.blocks * b.ntiles;
         blocks += b.blocks;
     }
@@ -799,10 +935,10 @@ int batch32_describe(const Batch32Item *items, int R, int cfg, void *desc_dev, i
 size_t batch32_partial_bytes()
 {
     const size_t v[kShapes] = {
-        (size_t)batch_resident_ctas<256, 2, 2>() * 2 * 512 * sizeof(double4_32a),
+        (size_t)batch_resident_ctas<256, 1, 2>() * 2 * 256 * sizeof(double4_32a),
         (size_t)batch_resident_ctas<128, 2, 4>() * 2 * 256 * sizeof(double4_32a),
         (size_t)batch_resident_ctas<256, 1, 3>() * 2 * 256 * sizeof(double4_32a),
-        (size_t)batch_resident_ctas<128, 2, 6>() * 2 * 256 * sizeof(double4_32a)};
+        (size_t)batch_resident_ctas<128, 2, 3>() * 2 * 256 * sizeof(double4_32a)};
     size_t m = 0;
     for (size_t x : v) m = x > m ? x : m;
     return m;
@@ -827,8 +963,8 @@ int sweep_f32_batch(int cfg, const void *desc_dev, int R, int ncols, int64_t uni
     switch (cfg % kShapes) {
     case 1: HZ_TRY((launch_batch<128, 2, 4>(ops, R, units, blocks, partial, partial_bytes, v, s))); break;
     case 2: HZ_TRY((launch_batch<256, 1, 3>(ops, R, units, blocks, partial, partial_bytes, v, s))); break;
-    case 3: HZ_TRY((launch_batch<128, 2, 6>(ops, R, units, blocks, partial, partial_bytes, v, s))); break;
-    default: HZ_TRY((launch_batch<256, 2, 2>(ops, R, units, blocks, partial, partial_bytes, v, s))); break;
+    case 3: HZ_TRY((launch_batch<128, 2, 3>(ops, R, units, blocks, partial, partial_bytes, v, s))); break;
+    default: HZ_TRY((launch_batch<256, 1, 2>(ops, R, units, blocks, partial, partial_bytes, v, s))); break;
     }
     if (ev1) HZ_CHECK_CUDA(record_timing_event(ev1, s));
     return HZ_OK;
@@ -836,12 +972,12 @@ int sweep_f32_batch(int cfg, const void *desc_dev, int R, int ncols, int64_t uni
 
 int sweep_f32(const SweepConst &c, const Rec32 &r, const double4_32a *pos64, int mode, const double *p_re,
               const double *p_im, const double *pt_re, const double *pt_im, double *q_re, double *q_im,
-              double *qt_re, double *qt_im, float4 *dens, cudaStream_t s, cudaEvent_t ev0,
+              double *qt_re, double *qt_im, float *dens, cudaStream_t s, cudaEvent_t ev0,
               cudaEvent_t ev1, int cfg)
 {
     if (c.n <= 0) return HZ_OK;
     const bool useA = (mode & SWEEP_A) != 0, useH = (mode & SWEEP_AH) != 0;
-    const double scale = ((c.interior == 1) ? -1.0 : 1.0) / (4.0 * kPi);
+    const double scale = 1.0 / sweep32_reg_scale(c.interior, r.lambda);
     {
         int dev = 0, sms = 152;
         cudaGetDevice(&dev);
@@ -856,18 +992,15 @@ int sweep_f32(const SweepConst &c, const Rec32 &r, const double4_32a *pos64, int
     Args32 a;
     a.n = c.n;
     a.npad = r.npad;
-    a.wave = (float)c.wave;
-    a.tau = c.tau;
+    set_constants(c, r.lambda, a);
     a.mwords = r.mwords;
     a.thi = r.thi;
     a.tlo = r.tlo;
     a.ohi = r.ohi;
     a.olo = r.olo;
     a.nearmask = r.nearmask;
-    a.tau2 = (float)(c.tau * c.tau);
-    a.guard_lo = (float)(c.tau * c.tau * (1.0 - 1e-4));
-    a.guard_hi = (float)(c.tau * c.tau * (1.0 + 1e-4));
     a.pos = r.pos;
+    a.soa = r.soa;
     a.nrm = r.nrm;
     a.dens = dens;
     a.tpos = r.tpos;
@@ -878,10 +1011,9 @@ int sweep_f32(const SweepConst &c, const Rec32 &r, const double4_32a *pos64, int
     a.err = c.err;
     if (ev0) HZ_CHECK_CUDA(record_timing_event(ev0, s));
     a.partial = r.partial;
-    split_wave(c.wave, a.kh, a.kl);
     const bool dir = c.dirichlet != 0;
-    constexpr int S = SWEEP_PHASE_SPLIT;
-    if (c.phase_split) {
+    constexpr int S = SWEEP_SCALED;
+    if (a.scaled) {
         if (mode == SWEEP_PAIR) HZ_TRY(launch32<SWEEP_PAIR | S>(cfg, a, dir, r.partial_bytes, s));
         else if (mode == SWEEP_A) HZ_TRY(launch32<SWEEP_A | S>(cfg, a, dir, r.partial_bytes, s));
         else HZ_TRY(launch32<SWEEP_AH | S>(cfg, a, dir, r.partial_bytes, s));

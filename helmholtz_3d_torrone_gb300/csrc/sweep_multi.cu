@@ -11,6 +11,7 @@
 // densities of a tile are staged as RB/2 rows of two complex values each.
 #include "hz_internal.cuh"
 #include "pair64.cuh"
+#include "pair32.cuh"
 #include "bulk_copy.cuh"
 #include "krylov_multi.cuh"
 
@@ -27,7 +28,8 @@ constexpr int kRBMax64 = 16;
 struct ArgsM32 {
     int64_t n, npad, mwords;
     int nr;  // right-hand sides in this pass (<= RB)
-    float wave, tau2, guard_lo, guard_hi;
+    Wave32 wave;
+    float tau2, guard_lo, guard_hi;
     double tau;
     const float4 *pos, *nrm;
     const float4 *dens;  // [RB/2][npad]: (p'_{2q} re, im, p'_{2q+1} re, im)
@@ -39,16 +41,6 @@ struct ArgsM32 {
     double *q_re, *q_im;        // [nr][n]
     unsigned *err;
 };
-
-// hi + lo += f without rounding loss (TwoSum, FP32 only)
-__device__ __forceinline__ void two_sum_m(float &hi, float &lo, float f)
-{
-    const float s = hi + f;
-    const float bp = s - hi;
-    const float e = (hi - (s - bp)) + (f - bp);
-    hi = s;
-    lo += e;
-}
 
 template <int RB>
 __global__ void prepm32_kernel(int64_t n, int64_t npad, int nr, const int *__restrict__ perm,
@@ -77,15 +69,15 @@ __global__ void prepm32_kernel(int64_t n, int64_t npad, int nr, const int *__res
     }
 }
 
-template <int RB, bool DIR, bool NEAR>
+template <int RB, bool DIR, bool SCALED, bool SLOW>
 __device__ __forceinline__ void pairm32(const ArgsM32 &a, const float4 s_p, const float4 s_n, const float3 rel,
-                                        const float3 tn, float treg, int64_t tslot, int64_t src_slot,
+                                        const float3 tn, float treg, float rc, int64_t tslot, int64_t src_slot,
                                         const float4 *sd, int j, float (&acc)[2 * RB])
 {
     const float dx = rel.x - s_p.x, dy = rel.y - s_p.y, dz = rel.z - s_p.z;
     const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
     bool near = false;
-    if (NEAR) {
+    if (SLOW) {
         near = r2 <= a.tau2;
         if (r2 > a.guard_lo && r2 < a.guard_hi) {
             const int c = a.perm[src_slot];
@@ -98,16 +90,12 @@ __device__ __forceinline__ void pairm32(const ArgsM32 &a, const float4 s_p, cons
             }
         }
     }
-    const float rinv = rsqrtf(r2);
-    const float rho = r2 * rinv;
-    float S, C;
-    __sincosf(rho * a.wave, &S, &C);
-    const float u1 = fmaf(C, rinv, a.wave * S);
-    const float u2 = fmaf(a.wave, C, -S * rinv);
-    const float rr = rinv * rinv;
-    const float pA = DIR ? (dx * s_n.x + dy * s_n.y + dz * s_n.z) : (dx * tn.x + dy * tn.y + dz * tn.z);
-    float vr = -u1 * rr * pA, vi = u2 * rr * pA;
-    if (NEAR && near) {
+    float u1, u2, rr;
+    kernel32<SCALED, SLOW>(a.wave, r2, rc, u1, u2, rr);
+    const float pA = DIR ? fmaf(dx, s_n.x, fmaf(dy, s_n.y, dz * s_n.z)) : fmaf(dx, tn.x, fmaf(dy, tn.y, dz * tn.z));
+    const float f = rr * pA;
+    float vr = -u1 * f, vi = u2 * f;
+    if (SLOW && near) {
         vr = DIR ? s_p.w : treg;
         vi = 0.f;
     }
@@ -125,7 +113,7 @@ constexpr int kNT32m = 256;
 template <int RB>
 constexpr size_t smem_m32() { return 2 * (2 + RB / 2) * kTile32 * sizeof(float4); }
 
-template <int RB, bool DIR>
+template <int RB, bool DIR, bool SCALED>
 __global__ void __launch_bounds__(kNT32m, RB <= 8 ? 2 : 1) sweepm32_kernel(ArgsM32 a)
 {
     constexpr int TS = kTile32;
@@ -163,10 +151,13 @@ __global__ void __launch_bounds__(kNT32m, RB <= 8 ? 2 : 1) sweepm32_kernel(ArgsM
     for (int64_t tile = 0; tile < ntiles; tile++) {
         const int buf = (int)(tile & 1);
         if (threadIdx.x == 0 && tile + 1 < ntiles) issue(tile + 1, buf ^ 1);
-        const bool far = ((__ldg(mrow + (tile >> 5)) >> (tile & 31)) & 1u) == 0;
         const float4 oh = a.ohi[tile], ol = a.olo[tile];
+        const bool slow =
+            ((__ldg(mrow + (tile >> 5)) >> (tile & 31)) & 1u) || (SCALED && oh.w > kCentreRadius);
         const float3 rel = make_float3((th.x - oh.x) + (tl.x - ol.x), (th.y - oh.y) + (tl.y - ol.y),
                                        (th.z - oh.z) + (tl.z - ol.z));
+        Turn turn = {};
+        if (SCALED && !slow) turn = turn_of(rel);
         const bool ok = mbar_wait_bounded(&bar[buf], (uint32_t)((tile >> 1) & 1), g_data_wait_limit);
         if (__syncthreads_or(!ok)) {
             if (threadIdx.x == 0) {
@@ -181,15 +172,19 @@ __global__ void __launch_bounds__(kNT32m, RB <= 8 ? 2 : 1) sweepm32_kernel(ArgsM
 #pragma unroll
         for (int i = 0; i < 2 * RB; i++) acc[i] = 0.f;
         const int64_t base = tile * TS;
-        if (far) {
+        if (slow) {
             for (int j = 0; j < TS; j++)
-                pairm32<RB, DIR, false>(a, P[j], Nn[j], rel, tn, treg, slot, base + j, D, j, acc);
+                pairm32<RB, DIR, SCALED, true>(a, P[j], Nn[j], rel, tn, treg, 0.f, slot, base + j, D, j, acc);
         } else {
             for (int j = 0; j < TS; j++)
-                pairm32<RB, DIR, true>(a, P[j], Nn[j], rel, tn, treg, slot, base + j, D, j, acc);
+                pairm32<RB, DIR, SCALED, false>(a, P[j], Nn[j], rel, tn, treg, turn.rc, slot, base + j, D, j, acc);
+            if (SCALED) {
+#pragma unroll
+                for (int r = 0; r < RB; r++) turn_sum<false>(turn, acc[2 * r], acc[2 * r + 1]);
+            }
         }
 #pragma unroll
-        for (int i = 0; i < 2 * RB; i++) two_sum_m(acch[i], accl[i], acc[i]);
+        for (int i = 0; i < 2 * RB; i++) two_sum_acc(acch[i], accl[i], acc[i]);
         __syncthreads();
     }
     const int c = a.perm[slot];
@@ -412,10 +407,12 @@ int launch_m32(const SweepConst &c, const Rec32 &r32, const Rec64 &r64, int nr, 
                double *qr, double *qi, void *scratch, cudaStream_t s)
 {
     constexpr int smem = (int)smem_m32<RB>();
-    HZ_CHECK_CUDA(cudaFuncSetAttribute(sweepm32_kernel<RB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    HZ_CHECK_CUDA(cudaFuncSetAttribute(sweepm32_kernel<RB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    const Const32 k32 = constants32(c, r32.lambda);
+    auto kernel = k32.scaled ? (c.dirichlet ? sweepm32_kernel<RB, true, true> : sweepm32_kernel<RB, false, true>)
+                             : (c.dirichlet ? sweepm32_kernel<RB, true, false> : sweepm32_kernel<RB, false, false>);
+    HZ_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     float4 *dens = static_cast<float4 *>(scratch);
-    const double scale = ((c.interior == 1) ? -1.0 : 1.0) / (4.0 * kPi);
+    const double scale = 1.0 / sweep32_reg_scale(c.interior, r32.lambda);
     prepm32_kernel<RB><<<blocks_for(r32.npad), 256, 0, s>>>(c.n, r32.npad, nr, r32.perm, r32.tpos, pr, pi, scale,
                                                             dens);
     HZ_CHECK_LAUNCH();
@@ -423,12 +420,12 @@ int launch_m32(const SweepConst &c, const Rec32 &r32, const Rec64 &r64, int nr, 
     a.n = c.n;
     a.npad = r32.npad;
     a.nr = nr;
-    a.wave = (float)c.wave;
+    a.wave = {k32.k, k32.kh, k32.kl};
     a.tau = c.tau;
     a.mwords = r32.mwords;
-    a.tau2 = (float)(c.tau * c.tau);
-    a.guard_lo = (float)(c.tau * c.tau * (1.0 - 1e-4));
-    a.guard_hi = (float)(c.tau * c.tau * (1.0 + 1e-4));
+    a.tau2 = k32.tau2;
+    a.guard_lo = k32.guard_lo;
+    a.guard_hi = k32.guard_hi;
     a.pos = r32.pos;
     a.nrm = r32.nrm;
     a.dens = dens;
@@ -446,8 +443,7 @@ int launch_m32(const SweepConst &c, const Rec32 &r32, const Rec64 &r64, int nr, 
     a.q_im = qi;
     a.err = c.err;
     const unsigned blocks = (unsigned)(r32.npad / kNT32m);
-    if (c.dirichlet) sweepm32_kernel<RB, true><<<blocks, kNT32m, smem, s>>>(a);
-    else sweepm32_kernel<RB, false><<<blocks, kNT32m, smem, s>>>(a);
+    kernel<<<blocks, kNT32m, smem, s>>>(a);
     HZ_CHECK_LAUNCH();
     return HZ_OK;
 }

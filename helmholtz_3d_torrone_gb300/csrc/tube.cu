@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(kTile32) rec32_kernel(const int *__restrict__ 
                                                         float4 *__restrict__ pos32, float4 *__restrict__ nrm32,
                                                         double4_32a *__restrict__ origin, double4_32a *__restrict__ tpos,
                                                         float4 *__restrict__ thi, float4 *__restrict__ tlo,
-                                                        double reg_scale)
+                                                        double reg_scale, double lambda, float *__restrict__ soa)
 {
     const int64_t s = (int64_t)blockIdx.x * kTile32 + threadIdx.x;
     const int c = perm[s];
@@ -310,8 +310,8 @@ __global__ void __launch_bounds__(kTile32) rec32_kernel(const int *__restrict__ 
         origin[blockIdx.x] = make_double4_32a(org[0], org[1], org[2],
                                               sqrt(ext[0] * ext[0] + ext[1] * ext[1] + ext[2] * ext[2]) * (1.0 + 1e-12));
     if (c >= 0) {
-        pos32[s] = make_float4((float)(p.x - org[0]), (float)(p.y - org[1]), (float)(p.z - org[2]),
-                               (float)(p.w * reg_scale));
+        pos32[s] = make_float4((float)(lambda * (p.x - org[0])), (float)(lambda * (p.y - org[1])),
+                               (float)(lambda * (p.z - org[2])), (float)(p.w * reg_scale));
         nrm32[s] = make_float4((float)q.x, (float)q.y, (float)q.z, (float)q.w);
         tpos[s] = make_double4_32a(p.x, p.y, p.z, q.w);
     } else {
@@ -320,20 +320,36 @@ __global__ void __launch_bounds__(kTile32) rec32_kernel(const int *__restrict__ 
         tpos[s] = make_double4_32a(org[0], org[1], org[2], 0.0);
         p = make_double4_32a(org[0], org[1], org[2], 0.0);
     }
-    const float hx = (float)p.x, hy = (float)p.y, hz = (float)p.z;
+    if (soa) {
+        const float4 a = pos32[s], b = nrm32[s];
+        float *t = soa + (int64_t)blockIdx.x * (kFixed32 * kTile32) + threadIdx.x;
+        t[0] = -a.x;
+        t[kTile32] = -a.y;
+        t[2 * kTile32] = -a.z;
+        t[3 * kTile32] = b.x;
+        t[4 * kTile32] = b.y;
+        t[5 * kTile32] = b.z;
+        t[6 * kTile32] = a.w;
+    }
+    const double lx = lambda * p.x, ly = lambda * p.y, lz = lambda * p.z;
+    const float hx = (float)lx, hy = (float)ly, hz = (float)lz;
     thi[s] = make_float4(hx, hy, hz, 0.f);
-    tlo[s] = make_float4((float)(p.x - (double)hx), (float)(p.y - (double)hy), (float)(p.z - (double)hz), 0.f);
+    tlo[s] = make_float4((float)(lx - (double)hx), (float)(ly - (double)hy), (float)(lz - (double)hz), 0.f);
 }
 
-// Tile origins split into FP32 head + tail (x = hi + lo to about 2^-48 |x|).
+// Tile origins times lambda split into FP32 head + tail (x = hi + lo to about
+// 2^-48 |x|); ohi.w = the tile's radius times lambda, rounded up.
 __global__ void split_origin_kernel(int64_t ntiles, const double4_32a *__restrict__ origin, float4 *__restrict__ ohi,
-                                    float4 *__restrict__ olo)
+                                    float4 *__restrict__ olo, double lambda)
 {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= ntiles) return;
-    const double4_32a o = origin[t];
+    double4_32a o = origin[t];
+    o.x *= lambda;
+    o.y *= lambda;
+    o.z *= lambda;
     const float hx = (float)o.x, hy = (float)o.y, hz = (float)o.z;
-    ohi[t] = make_float4(hx, hy, hz, 0.f);
+    ohi[t] = make_float4(hx, hy, hz, __double2float_ru(lambda * o.w));
     olo[t] = make_float4((float)(o.x - (double)hx), (float)(o.y - (double)hy), (float)(o.z - (double)hz), 0.f);
 }
 
@@ -437,9 +453,9 @@ int build_rec32(const Rec32 &r, const double4_32a *pos64, const double4_32a *nrm
     const int64_t ntiles = r.npad / kTile32;
     if (ntiles == 0) return HZ_OK;
     rec32_kernel<<<(unsigned)ntiles, kTile32, 0, s>>>(r.perm, pos64, nrm64, r.pos, r.nrm, r.origin, r.tpos, r.thi,
-                                                      r.tlo, reg_scale);
+                                                      r.tlo, reg_scale, r.lambda, r.soa);
     HZ_CHECK_LAUNCH();
-    split_origin_kernel<<<(unsigned)((ntiles + 255) / 256), 256, 0, s>>>(ntiles, r.origin, r.ohi, r.olo);
+    split_origin_kernel<<<(unsigned)((ntiles + 255) / 256), 256, 0, s>>>(ntiles, r.origin, r.ohi, r.olo, r.lambda);
     HZ_CHECK_LAUNCH();
     const int64_t cells = ntiles * r.mwords;
     nearmask_kernel<<<(unsigned)((cells + 255) / 256), 256, 0, s>>>(ntiles, r.mwords, r.origin, tau * (1.0 + 1e-3),
