@@ -25,7 +25,15 @@ void set_error(const char *fmt, ...)
     va_end(ap);
 }
 
-void note_launch(int count) { g_launches.fetch_add(count, std::memory_order_relaxed); }
+static thread_local long long g_noted = 0;
+
+void note_launch(int count)
+{
+    g_launches.fetch_add(count, std::memory_order_relaxed);
+    g_noted += count;
+}
+
+long long launches_noted() { return g_noted; }
 
 int DevBuf::ensure(size_t nbytes)
 {

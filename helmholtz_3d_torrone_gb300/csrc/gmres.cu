@@ -17,83 +17,118 @@
 namespace hz {
 namespace {
 
-constexpr int kGB = 128;  // partial-sum blocks
 constexpr int kGT = 256;
+constexpr int kChunk = 256;     // vector elements of a block of the products
 constexpr int kMaxRestart = 128;
 
-// h[j] = sum_i conj(V_j[i]) w[i] for j < k (partials per block)
+// partial[blk][j] = sum over the block's chunk of conj(V_j) w, j < k.  A warp
+// takes every eighth j, two at a time, so a block needs no barrier between
+// them (one j after another with two barriers each took 108 us at n = 36,311
+// and k about 60; the FP64 operations alone take 17 us).
 __global__ void __launch_bounds__(kGT) vh_kernel(int64_t n, int k, const double *__restrict__ vr,
                                                  const double *__restrict__ vi, const double *__restrict__ wr,
-                                                 const double *__restrict__ wi, double *partial)
+                                                 const double *__restrict__ wi, double2 *__restrict__ partial)
 {
-    __shared__ double sh[kGT / 32][2];
-    for (int j = 0; j < k; j++) {
+    const int64_t base = blockIdx.x * (int64_t)kChunk;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double y0[kChunk / 32], y1[kChunk / 32];
+#pragma unroll
+    for (int e = 0; e < kChunk / 32; e++) {
+        const int64_t i = base + lane + 32 * e;
+        y0[e] = i < n ? wr[i] : 0.0;
+        y1[e] = i < n ? wi[i] : 0.0;
+    }
+    for (int j = 2 * warp; j < k; j += 16) {
+        const bool two = j + 1 < k;
         const double *a0 = vr + (int64_t)j * n, *a1 = vi + (int64_t)j * n;
-        double s0 = 0.0, s1 = 0.0;
-        for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-            const double x0 = a0[i], x1 = a1[i], y0 = wr[i], y1 = wi[i];
-            s0 += x0 * y0 + x1 * y1;  // conj(v) w
-            s1 += x0 * y1 - x1 * y0;
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            s0 += __shfl_down_sync(0xffffffffu, s0, o);
-            s1 += __shfl_down_sync(0xffffffffu, s1, o);
-        }
-        if ((threadIdx.x & 31) == 0) {
-            sh[threadIdx.x >> 5][0] = s0;
-            sh[threadIdx.x >> 5][1] = s1;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double a = 0, b = 0;
-            for (int w = 0; w < kGT / 32; w++) {
-                a += sh[w][0];
-                b += sh[w][1];
+        double s0 = 0.0, s1 = 0.0, t0 = 0.0, t1 = 0.0;
+#pragma unroll
+        for (int e = 0; e < kChunk / 32; e++) {
+            const int64_t i = base + lane + 32 * e;
+            if (i < n) {
+                const double x0 = a0[i], x1 = a1[i];
+                s0 += x0 * y0[e] + x1 * y1[e];  // conj(v) w
+                s1 += x0 * y1[e] - x1 * y0[e];
+                if (two) {
+                    const double u0 = a0[n + i], u1 = a1[n + i];
+                    t0 += u0 * y0[e] + u1 * y1[e];
+                    t1 += u0 * y1[e] - u1 * y0[e];
+                }
             }
-            partial[((int64_t)blockIdx.x * kMaxRestart + j) * 2] = a;
-            partial[((int64_t)blockIdx.x * kMaxRestart + j) * 2 + 1] = b;
         }
-        __syncthreads();
+        // fold the four sums over the lanes: halves first, so that the tree
+        // costs 12 additions a lane instead of 20
+        const bool up = lane & 16;
+        double p = up ? t0 : s0, q = up ? t1 : s1;
+        p += __shfl_xor_sync(0xffffffffu, up ? s0 : t0, 16);
+        q += __shfl_xor_sync(0xffffffffu, up ? s1 : t1, 16);
+        const bool up2 = lane & 8;
+        double r = up2 ? q : p;
+        r += __shfl_xor_sync(0xffffffffu, up2 ? p : q, 8);
+        for (int o = 4; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+        // lane 0: Re s, 8: Im s, 16: Re t, 24: Im t
+        if ((lane & 7) == 0 && (two || !up))
+            reinterpret_cast<double *>(partial + (int64_t)blockIdx.x * kMaxRestart + j + (up ? 1 : 0))[up2 ? 1 : 0] = r;
     }
 }
 
-// h (k complex) from the partials, summed in block order, into hdev; also
+// h[j] = sum of the blocks' partials, one warp per j, in a fixed order; also
 // stored into (accumulate = 0) or added to (accumulate = 1) hsum if given.
-__global__ void vh_reduce_kernel(int k, const double *partial, double *hdev, double *hsum, int accumulate)
+__global__ void __launch_bounds__(128) vh_reduce_kernel(int k, int nb, const double2 *__restrict__ partial,
+                                                        double2 *hdev, double2 *hsum, int accumulate)
 {
-    const int j = threadIdx.x;
+    const int j = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (j >= k) return;
     double a = 0, b = 0;
-    for (int q = 0; q < kGB; q++) {
-        a += partial[((int64_t)q * kMaxRestart + j) * 2];
-        b += partial[((int64_t)q * kMaxRestart + j) * 2 + 1];
+    for (int q = lane; q < nb; q += 32) {
+        const double2 v = partial[(int64_t)q * kMaxRestart + j];
+        a += v.x;
+        b += v.y;
     }
-    hdev[2 * j] = a;
-    hdev[2 * j + 1] = b;
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    if (lane) return;
+    hdev[j] = make_double2(a, b);
     if (!hsum) return;
     if (accumulate) {
-        hsum[2 * j] += a;
-        hsum[2 * j + 1] += b;
-    } else {
-        hsum[2 * j] = a;
-        hsum[2 * j + 1] = b;
+        a += hsum[j].x;
+        b += hsum[j].y;
     }
+    hsum[j] = make_double2(a, b);
 }
 
-// w -= sum_j V_j h_j
-__global__ void vupdate_kernel(int64_t n, int k, const double *__restrict__ vr, const double *__restrict__ vi,
-                               const double *__restrict__ h, double *wr, double *wi)
+// w -= sum_j V_j h_j; with npart also the block's sum of |w|^2
+__global__ void __launch_bounds__(kGT) vupdate_kernel(int64_t n, int k, const double *__restrict__ vr,
+                                                      const double *__restrict__ vi, const double2 *__restrict__ h,
+                                                      double *wr, double *wi, double2 *npart)
 {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double a = wr[i], b = wi[i];
+    const int64_t i = blockIdx.x * (int64_t)kGT + threadIdx.x;
+    double a = 0, b = 0;
+    if (i < n) {
+        a = wr[i];
+        b = wi[i];
+#pragma unroll 4
         for (int j = 0; j < k; j++) {
             const double x0 = vr[(int64_t)j * n + i], x1 = vi[(int64_t)j * n + i];
-            const double h0 = h[2 * j], h1 = h[2 * j + 1];
+            const double h0 = h[j].x, h1 = h[j].y;
             a -= x0 * h0 - x1 * h1;
             b -= x0 * h1 + x1 * h0;
         }
         wr[i] = a;
         wi[i] = b;
+    }
+    if (!npart) return;
+    __shared__ double sh[kGT / 32];
+    double s = a * a + b * b;
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s = 0.0;
+        for (int w = 0; w < kGT / 32; w++) s += sh[w];
+        npart[(int64_t)blockIdx.x * kMaxRestart] = make_double2(s, 0.0);
     }
 }
 
@@ -150,21 +185,24 @@ int gmres_solve(LinOp &A, int64_t n, int m, const double *b_re, const double *b_
     if (m > kMaxRestart - 1) m = kMaxRestart - 1;
     // V: (m+1) basis vectors; w; Ax scratch
     HZ_TRY(work.ensure(((size_t)(m + 1) + 2) * 2 * (size_t)n * sizeof(double)));
-    HZ_TRY(small.ensure((size_t)kGB * kMaxRestart * 2 * sizeof(double) + 8 * kMaxRestart * sizeof(double) + 64));
+    // products in chunks of kChunk elements: partial sums [blocks][kMaxRestart]
+    const int nb = (int)((n + kChunk - 1) / kChunk);
+    static_assert(kChunk == kGT, "the update's blocks write the partial sums of the norm");
+    HZ_TRY(small.ensure(((size_t)nb * kMaxRestart + 3 * kMaxRestart) * sizeof(double2)));
     double *V = work.as<double>();
     double *vr = V, *vi = V + (size_t)(m + 1) * n;
     double *wr = V + 2 * (size_t)(m + 1) * n, *wi = wr + n;
     double *tr = wi + n, *ti = tr + n;
-    double *partial = small.as<double>();
-    double *hdev = partial + (size_t)kGB * kMaxRestart * 2;
-    double *hsum = hdev + 2 * kMaxRestart;
-    double *ydev = hsum + 2 * kMaxRestart;
+    double2 *partial = small.as<double2>();
+    double2 *hdev = partial + (size_t)nb * kMaxRestart;
+    double2 *hsum = hdev + kMaxRestart;
+    double *ydev = reinterpret_cast<double *>(hsum + kMaxRestart);
     const int vb = vblocks(n);
-    std::vector<double> hh(2 * kMaxRestart);
+    std::vector<double> hh(4 * kMaxRestart);
     auto norm2 = [&](const double *ar, const double *ai, double &out) -> int {
-        vh_kernel<<<kGB, kGT, 0, s>>>(n, 1, ar, ai, ar, ai, partial);
+        vh_kernel<<<nb, kGT, 0, s>>>(n, 1, ar, ai, ar, ai, partial);
         HZ_CHECK_LAUNCH();
-        vh_reduce_kernel<<<1, kMaxRestart, 0, s>>>(1, partial, hdev, nullptr, 0);
+        vh_reduce_kernel<<<1, 128, 0, s>>>(1, nb, partial, hdev, nullptr, 0);
         HZ_CHECK_LAUNCH();
         HZ_CHECK_CUDA(cudaMemcpyAsync(hh.data(), hdev, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
         HZ_CHECK_CUDA(cudaStreamSynchronize(s));
@@ -201,17 +239,19 @@ int gmres_solve(LinOp &A, int64_t n, int m, const double *b_re, const double *b_
                            s));
             // CGS2 against V_0..V_k
             for (int pass = 0; pass < 2; pass++) {
-                vh_kernel<<<kGB, kGT, 0, s>>>(n, k + 1, vr, vi, wr, wi, partial);
+                vh_kernel<<<nb, kGT, 0, s>>>(n, k + 1, vr, vi, wr, wi, partial);
                 HZ_CHECK_LAUNCH();
-                vh_reduce_kernel<<<1, kMaxRestart, 0, s>>>(k + 1, partial, hdev, hsum, pass);
+                vh_reduce_kernel<<<(k + 4) / 4, 128, 0, s>>>(k + 1, nb, partial, hdev, hsum, pass);
                 HZ_CHECK_LAUNCH();
-                vupdate_kernel<<<vb, 256, 0, s>>>(n, k + 1, vr, vi, hdev, wr, wi);
+                vupdate_kernel<<<nb, kGT, 0, s>>>(n, k + 1, vr, vi, hdev, wr, wi, pass ? partial : nullptr);
                 HZ_CHECK_LAUNCH();
             }
-            double hn = 0;
-            HZ_TRY(norm2(wr, wi, hn));
-            HZ_CHECK_CUDA(cudaMemcpyAsync(hh.data(), hsum, 2 * (k + 1) * sizeof(double), cudaMemcpyDeviceToHost, s));
+            // ||w||^2 (the update's partial sums) beside the coefficients: one copy
+            vh_reduce_kernel<<<1, 128, 0, s>>>(1, nb, partial, hsum + kMaxRestart - 1, nullptr, 0);
+            HZ_CHECK_LAUNCH();
+            HZ_CHECK_CUDA(cudaMemcpyAsync(hh.data(), hsum, kMaxRestart * sizeof(double2), cudaMemcpyDeviceToHost, s));
             HZ_CHECK_CUDA(cudaStreamSynchronize(s));
+            const double hn = sqrt(fabs(hh[2 * (kMaxRestart - 1)]));
             A.iteration_done(false);
             for (int j = 0; j <= k; j++) H[(size_t)j * m + k] = cplx(hh[2 * j], hh[2 * j + 1]);
             H[(size_t)(k + 1) * m + k] = hn;

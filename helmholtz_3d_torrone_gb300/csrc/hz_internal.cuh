@@ -19,6 +19,7 @@ int stage_in(double *dst, const double *src, size_t count, int where, cudaStream
 int stage_out(double *dst, const double *src, size_t count, int where, cudaStream_t s);
 int where_ok(int where);
 void note_launch(int count = 1);
+long long launches_noted();  // by the calling thread
 
 #define HZ_CHECK_CUDA(call)                                                                      \
     do {                                                                                         \

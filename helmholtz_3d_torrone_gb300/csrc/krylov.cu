@@ -47,13 +47,26 @@ __device__ void block_reduce_store(double (&v)[ND], double *partial)
     }
 }
 
-__device__ void sum_partials(const double *partial, int nd, double *out)
+// Sums of the kDotBlocks partials, one thread each (kernels of one block of
+// kDotBlocks threads; a single thread's serial loop took 20 to 40 us, most of
+// the time between two products of a small system): a fixed tree, and the
+// result in every thread.
+template <int ND>
+__device__ void sum_partials(const double *partial, double (&out)[ND])
 {
-    for (int d = 0; d < nd; d++) {
-        double s = 0.0;
-        for (int b = 0; b < kDotBlocks; b++) s += partial[b * kMaxDots + d];
-        out[d] = s;
+    static_assert(kDotBlocks == 256, "eight warps");
+    __shared__ double sh[8][ND];
+#pragma unroll
+    for (int d = 0; d < ND; d++) {
+        double x = partial[threadIdx.x * kMaxDots + d];
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5][d] = x;
     }
+    __syncthreads();
+#pragma unroll
+    for (int d = 0; d < ND; d++)
+        out[d] = ((sh[0][d] + sh[1][d]) + (sh[2][d] + sh[3][d])) + ((sh[4][d] + sh[5][d]) + (sh[6][d] + sh[7][d]));
+    __syncthreads();
 }
 
 // <a, b> = sum a conj(b): (sum ar br + ai bi, sum ai br - ar bi); optionally
@@ -97,7 +110,8 @@ __global__ void bicg_init_kernel(int64_t n, const double *__restrict__ b_re, con
 __global__ void bicg_start_kernel(const double *partial, KrylovScalars *sc)
 {
     double s[3];
-    sum_partials(partial, 3, s);
+    sum_partials(partial, s);
+    if (threadIdx.x) return;
     sc->rho_re = s[0];
     sc->rho_im = s[1];
     sc->normb = sqrt(s[2]);
@@ -106,25 +120,20 @@ __global__ void bicg_start_kernel(const double *partial, KrylovScalars *sc)
     sc->status = (s[2] > 0.0) ? 0 : 1;
 }
 
-// alpha = <r,rt> / <q,pt>
-__global__ void bicg_alpha_kernel(const double *partial, KrylovScalars *sc)
-{
-    double s[3];
-    sum_partials(partial, 3, s);
-    const double ca = sc->rho_re, cb = sc->rho_im, cc = s[0], cd = s[1];
-    const double num = ca * cc + cb * cd, numi = cb * cc - ca * cd, den = cc * cc + cd * cd;
-    sc->alpha_re = num / den;
-    sc->alpha_im = numi / den;
-    if (den == 0.0) sc->status = 2;
-}
-
+// alpha = <r,rt> / <q,pt>, summed by every block in the same order (one
+// launch fewer), then the vector updates and the new partial sums.
 __global__ void __launch_bounds__(kDotThreads) bicg_update_kernel(
-    int64_t n, const KrylovScalars *__restrict__ sc, double *x_re, double *x_im, double *r_re, double *r_im,
+    int64_t n, KrylovScalars *sc, const double *qpt, double *x_re, double *x_im, double *r_re, double *r_im,
     double *rt_re, double *rt_im, const double *__restrict__ p_re, const double *__restrict__ p_im,
     const double *__restrict__ q_re, const double *__restrict__ q_im, const double *__restrict__ qt_re,
     const double *__restrict__ qt_im, double *partial)
 {
-    const double al = sc->alpha_re, ali = sc->alpha_im;
+    double s[2];
+    sum_partials(qpt, s);
+    const double ca = sc->rho_re, cb = sc->rho_im, cc = s[0], cd = s[1];
+    const double den = cc * cc + cd * cd;
+    const double al = (ca * cc + cb * cd) / den, ali = (cb * cc - ca * cd) / den;
+    if (den == 0.0 && blockIdx.x == 0 && threadIdx.x == 0) sc->status = 2;
     double v[3] = {0.0, 0.0, 0.0};
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
         const double pr = p_re[j], pi = p_im[j], qr = q_re[j], qi = q_im[j], tr = qt_re[j], ti = qt_im[j];
@@ -148,7 +157,8 @@ __global__ void __launch_bounds__(kDotThreads) bicg_update_kernel(
 __global__ void bicg_beta_kernel(const double *partial, KrylovScalars *sc, double *host_err)
 {
     double s[3];
-    sum_partials(partial, 3, s);
+    sum_partials(partial, s);
+    if (threadIdx.x) return;
     const double cc = sc->rho_re, cd = sc->rho_im, ca = s[0], cb = s[1];
     const double num = ca * cc + cb * cd, numi = cb * cc - ca * cd, den = cc * cc + cd * cd;
     sc->beta_re = num / den;
@@ -196,7 +206,8 @@ __global__ void stab_init_kernel(int64_t n, const double *__restrict__ b_re, con
 __global__ void stab_start_kernel(const double *partial, KrylovScalars *sc)
 {
     double s[3];
-    sum_partials(partial, 3, s);
+    sum_partials(partial, s);
+    if (threadIdx.x) return;
     sc->normb = sqrt(s[2]);
     sc->rho_re = 1.0;  // rho_0 = alpha = omega = 1
     sc->rho_im = 0.0;
@@ -220,7 +231,8 @@ __device__ void cdiv(double ar, double ai, double br, double bi, double &cr, dou
 __global__ void stab_beta_kernel(const double *partial, KrylovScalars *sc)
 {
     double s[3];
-    sum_partials(partial, 3, s);
+    sum_partials(partial, s);
+    if (threadIdx.x) return;
     double q1r, q1i, q2r, q2i;
     cdiv(s[0], s[1], sc->rho_re, sc->rho_im, q1r, q1i);
     cdiv(sc->alpha_re, sc->alpha_im, sc->omega_re, sc->omega_im, q2r, q2i);
@@ -248,7 +260,8 @@ __global__ void stab_p_kernel(int64_t n, const KrylovScalars *__restrict__ sc, c
 __global__ void stab_alpha_kernel(const double *partial, KrylovScalars *sc)
 {
     double s[3];
-    sum_partials(partial, 3, s);
+    sum_partials(partial, s);
+    if (threadIdx.x) return;
     if (s[0] == 0.0 && s[1] == 0.0) sc->status = 2;
     cdiv(sc->rho_re, sc->rho_im, s[0], s[1], sc->alpha_re, sc->alpha_im);
 }
@@ -269,8 +282,9 @@ __global__ void stab_s_kernel(int64_t n, const KrylovScalars *__restrict__ sc, d
 __global__ void stab_omega_kernel(const double *partial_st, const double *partial_tt, KrylovScalars *sc)
 {
     double a[3], b[3];
-    sum_partials(partial_st, 3, a);
-    sum_partials(partial_tt, 3, b);
+    sum_partials(partial_st, a);
+    sum_partials(partial_tt, b);
+    if (threadIdx.x) return;
     // omega = t^H s / t^H t, and t^H s = sum conj(t) s = cdot(s, t)
     const double tt = b[2];
     sc->omega_re = a[0] / tt;
@@ -305,7 +319,8 @@ __global__ void __launch_bounds__(kDotThreads) stab_update_kernel(
 __global__ void stab_err_kernel(const double *partial, KrylovScalars *sc, double *host_err)
 {
     double s[3];
-    sum_partials(partial, 3, s);
+    sum_partials(partial, s);
+    if (threadIdx.x) return;
     sc->preerr = sc->err;
     sc->err = sqrt(s[2]) / sc->normb;
     host_err[0] = sc->err;
@@ -344,7 +359,8 @@ __global__ void scale_kernel(int64_t n, double a, const double *x_re, const doub
 __global__ void norm_kernel(const double *partial, double *out)
 {
     double s[3];
-    sum_partials(partial, 3, s);
+    sum_partials(partial, s);
+    if (threadIdx.x) return;
     out[0] = sqrt(s[2]);
 }
 
@@ -391,18 +407,16 @@ double *Krylov::im(int v) { return vecs.as<double>() + (size_t)(2 * v + 1) * n; 
 
 int Krylov::bicg_iteration(LinOp &A, cudaStream_t s)
 {
-    double *pp = partial.as<double>();
+    double *pp = partial.as<double>(), *pp2 = pp + kDotBlocks * kMaxDots;
     KrylovScalars *sc = scal.as<KrylovScalars>();
     const int vb = vec_blocks(n);
     HZ_TRY(A.apply(SWEEP_PAIR, re(P), im(P), re(PT), im(PT), re(Q), im(Q), re(QT), im(QT), s));
     cdot_kernel<<<kDotBlocks, kDotThreads, 0, s>>>(n, re(Q), im(Q), re(PT), im(PT), pp);
     HZ_CHECK_LAUNCH();
-    bicg_alpha_kernel<<<1, 1, 0, s>>>(pp, sc);
+    bicg_update_kernel<<<kDotBlocks, kDotThreads, 0, s>>>(n, sc, pp, re(X), im(X), re(R), im(R), re(RT), im(RT),
+                                                          re(P), im(P), re(Q), im(Q), re(QT), im(QT), pp2);
     HZ_CHECK_LAUNCH();
-    bicg_update_kernel<<<kDotBlocks, kDotThreads, 0, s>>>(n, sc, re(X), im(X), re(R), im(R), re(RT), im(RT),
-                                                          re(P), im(P), re(Q), im(Q), re(QT), im(QT), pp);
-    HZ_CHECK_LAUNCH();
-    bicg_beta_kernel<<<1, 1, 0, s>>>(pp, sc, host_err);
+    bicg_beta_kernel<<<1, kDotBlocks, 0, s>>>(pp2, sc, host_err);
     HZ_CHECK_LAUNCH();
     bicg_p_kernel<<<vb, 256, 0, s>>>(n, sc, re(R), im(R), re(RT), im(RT), re(P), im(P), re(PT), im(PT));
     HZ_CHECK_LAUNCH();
@@ -418,14 +432,14 @@ int Krylov::stab_iteration(LinOp &A, cudaStream_t s)
     // rho_new = <r, rh>, beta, p = r + beta (p - omega v)
     cdot_kernel<<<kDotBlocks, kDotThreads, 0, s>>>(n, re(R), im(R), re(RH), im(RH), pp);
     HZ_CHECK_LAUNCH();
-    stab_beta_kernel<<<1, 1, 0, s>>>(pp, sc);
+    stab_beta_kernel<<<1, kDotBlocks, 0, s>>>(pp, sc);
     HZ_CHECK_LAUNCH();
     stab_p_kernel<<<vb, 256, 0, s>>>(n, sc, re(R), im(R), re(P), im(P), re(V), im(V));
     HZ_CHECK_LAUNCH();
     HZ_TRY(A.apply(SWEEP_A, re(P), im(P), nullptr, nullptr, re(V), im(V), nullptr, nullptr, s));
     cdot_kernel<<<kDotBlocks, kDotThreads, 0, s>>>(n, re(V), im(V), re(RH), im(RH), pp);
     HZ_CHECK_LAUNCH();
-    stab_alpha_kernel<<<1, 1, 0, s>>>(pp, sc);
+    stab_alpha_kernel<<<1, kDotBlocks, 0, s>>>(pp, sc);
     HZ_CHECK_LAUNCH();
     stab_s_kernel<<<vb, 256, 0, s>>>(n, sc, re(R), im(R), re(V), im(V));
     HZ_CHECK_LAUNCH();
@@ -434,12 +448,12 @@ int Krylov::stab_iteration(LinOp &A, cudaStream_t s)
     HZ_CHECK_LAUNCH();
     cdot_kernel<<<kDotBlocks, kDotThreads, 0, s>>>(n, re(Q), im(Q), re(Q), im(Q), pp2);
     HZ_CHECK_LAUNCH();
-    stab_omega_kernel<<<1, 1, 0, s>>>(pp, pp2, sc);
+    stab_omega_kernel<<<1, kDotBlocks, 0, s>>>(pp, pp2, sc);
     HZ_CHECK_LAUNCH();
     stab_update_kernel<<<kDotBlocks, kDotThreads, 0, s>>>(n, sc, re(X), im(X), re(R), im(R), re(P), im(P),
                                                           re(Q), im(Q), re(RH), im(RH), pp);
     HZ_CHECK_LAUNCH();
-    stab_err_kernel<<<1, 1, 0, s>>>(pp, sc, host_err);
+    stab_err_kernel<<<1, kDotBlocks, 0, s>>>(pp, sc, host_err);
     HZ_CHECK_LAUNCH();
     return HZ_OK;
 }
@@ -459,7 +473,7 @@ int Krylov::solve(LinOp &A, int method, const double *b_re, const double *b_im, 
         HZ_CHECK_LAUNCH();
         cdot_kernel<<<kDotBlocks, kDotThreads, 0, s>>>(n, re(R), im(R), re(RT), im(RT), pp);
         HZ_CHECK_LAUNCH();
-        bicg_start_kernel<<<1, 1, 0, s>>>(pp, sc);
+        bicg_start_kernel<<<1, kDotBlocks, 0, s>>>(pp, sc);
         HZ_CHECK_LAUNCH();
     } else {
         stab_init_kernel<<<vb, 256, 0, s>>>(n, b_re, b_im, re(X), im(X), re(R), im(R), re(RH), im(RH), re(P),
@@ -467,7 +481,7 @@ int Krylov::solve(LinOp &A, int method, const double *b_re, const double *b_im, 
         HZ_CHECK_LAUNCH();
         cdot_kernel<<<kDotBlocks, kDotThreads, 0, s>>>(n, re(R), im(R), re(R), im(R), pp);
         HZ_CHECK_LAUNCH();
-        stab_start_kernel<<<1, 1, 0, s>>>(pp, sc);
+        stab_start_kernel<<<1, kDotBlocks, 0, s>>>(pp, sc);
         HZ_CHECK_LAUNCH();
     }
     KrylovScalars h{};
@@ -494,9 +508,11 @@ int Krylov::solve(LinOp &A, int method, const double *b_re, const double *b_im, 
             bool captured = false;
             if (cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
                 A.capture_begin();
+                const long long before = launches_noted();
                 int rc = (method == HZ_BICG) ? bicg_iteration(A, cs) : stab_iteration(A, cs);
                 cudaError_t e = cudaStreamEndCapture(cs, &g);
                 A.capture_end();
+                graph_launches = (int)(launches_noted() - before);
                 if (rc == HZ_OK && e == cudaSuccess && g) {
                     if (cudaGraphInstantiate(&graph_exec, g, 0) == cudaSuccess) captured = true;
                 }
@@ -518,7 +534,7 @@ int Krylov::solve(LinOp &A, int method, const double *b_re, const double *b_im, 
     for (int it = 1; it <= maxit; it++) {
         if (exec) {
             HZ_CHECK_CUDA(cudaGraphLaunch(exec, s));
-            note_launch(method == HZ_BICG ? 7 : 14);
+            note_launch(graph_launches);
         } else {
             HZ_TRY(method == HZ_BICG ? bicg_iteration(A, s) : stab_iteration(A, s));
         }
@@ -589,7 +605,7 @@ int vec_norm(int64_t n, const double *x_re, const double *x_im, double *dev_part
 {
     cdot_kernel<<<kDotBlocks, kDotThreads, 0, s>>>(n, x_re, x_im, x_re, x_im, dev_partial);
     HZ_CHECK_LAUNCH();
-    norm_kernel<<<1, 1, 0, s>>>(dev_partial, dev_out);
+    norm_kernel<<<1, kDotBlocks, 0, s>>>(dev_partial, dev_out);
     HZ_CHECK_LAUNCH();
     HZ_CHECK_CUDA(cudaMemcpyAsync(&host_out, dev_out, sizeof(double), cudaMemcpyDeviceToHost, s));
     HZ_CHECK_CUDA(cudaStreamSynchronize(s));

@@ -79,6 +79,7 @@ class Krylov {
     DevBuf vecs, partial, scal;
     double *host_err = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
+    int graph_launches = 0;  // kernels of the captured iteration
     uint64_t graph_key = 0;
     int graph_key_method = -1;
     cudaStream_t graph_stream = nullptr;
