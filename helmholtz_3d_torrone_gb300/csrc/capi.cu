@@ -225,9 +225,9 @@ struct MultiMatrixFreeOp final : MultiOp {
         : op(o), precision(prec), scratch(sc), pack(pk) {}
     int apply(int R, const double *p_re, const double *p_im, double *q_re, double *q_im, cudaStream_t s) override
     {
-        HZ_TRY(scratch->ensure(multi_rhs_scratch_bytes(op->n, op->r32.npad)));
         const int64_t n = op->n;
         const int m = cols.empty() ? R : (int)cols.size();
+        HZ_TRY(scratch->ensure(multi_rhs_scratch_bytes(precision, m, n, op->r32, rec64(op))));
         pairs += (long long)n * n * multi_rhs_passes(precision, m);
         if (m == R)
             return sweep_multi(sweep_const(op), op->r32, rec64(op), precision, R, p_re, p_im, q_re, q_im,

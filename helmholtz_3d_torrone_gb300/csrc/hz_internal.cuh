@@ -239,6 +239,9 @@ int build_split_records(const SweepConst &c, const RecSplit &v, const Rec32 &r, 
 int sweep_split(const SweepConst &c, const RecSplit &v, const double4_32a *nrm, int mode, const double *p_re,
                 const double *p_im, const double *pt_re, const double *pt_im, double *q_re, double *q_im,
                 double *qt_re, double *qt_im, cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1);
+size_t split_cols_scratch_bytes(int64_t npad, int nr);
+int sweep_split_cols(const SweepConst &c, const RecSplit &v, const double4_32a *nrm, int nr, const double *p_re,
+                     const double *p_im, double *q_re, double *q_im, void *scratch, cudaStream_t s);
 // posk[i] = (k x, k y, k z, reg) of pos[i]: the FP64 sweep's scaled records.
 int scale_records64(int64_t n, double k, const double4_32a *pos, double4_32a *posk, cudaStream_t s);
 // sweep_f32.cu

@@ -67,7 +67,8 @@ int gmres_multi_solve(MultiOp &A, int64_t n, int R, int m, const double *b_re, c
 // sweep_multi.cu
 // kernel passes (one evaluation of every pair each) for nrhs columns
 long long multi_rhs_passes(int precision, int nrhs);
-size_t multi_rhs_scratch_bytes(int64_t n, int64_t npad);
+// scratch of sweep_multi for these columns and records
+size_t multi_rhs_scratch_bytes(int precision, int nrhs, int64_t n, const Rec32 &r32, const Rec64 &r64);
 int sweep_multi(const SweepConst &c, const Rec32 &r32, const Rec64 &r64, int precision, int nrhs,
                 const double *p_re, const double *p_im, double *q_re, double *q_im, void *scratch,
                 cudaStream_t s);

@@ -2,13 +2,17 @@
 // RB density vectors with one kernel evaluation per point pair.
 //
 // Every pair's kernel value (distance, phase, sin/cos, projection) is
-// computed once and multiplied into RB densities, so the per-RHS cost falls
-// from a full pair evaluation to four fused multiply-adds.  Both precisions
-// follow the single-vector sweeps (sweep_f32.cu, sweep_f64.cu) for the
-// kernel arithmetic, tiling, TMA staging and the near-field rules (the FP32
-// pass uses the same near-tile mask, head/tail target offsets and TwoSum
-// cross-tile sums, with no FP64 instruction in its tile loop); the
-// densities of a tile are staged as RB/2 rows of two complex values each.
+// computed once and multiplied into RB densities.  The FP32 pass follows
+// sweep_f32.cu (pair32.cuh, the near-tile mask, head/tail target offsets and
+// TwoSum cross-tile sums, no FP64 instruction in the tile loop); its densities
+// lie in rows of two columns, (re, re, im, im), so that a column pair costs
+// four packed FMAs.  The FP64 pass is sweep_split.cu's where that serves, else
+// the kernel below with the arithmetic of pair64.cuh.
+//
+// A pass on GB300 (torus), before and now: FP32, 16 columns, n = 27,508 5.76 ->
+// 3.20 ms, n = 145,272 102 -> 74; 8 columns 3.94 -> 1.89 and 56.6 -> 44; 32
+// columns 9.33 -> 5.80 and 177 -> 147.  FP64, 16 columns, 259 -> 38.8 and
+// 5,455 -> 1,036; 8 columns 169 -> 21.9 and 3,558 -> 589.
 #include "hz_internal.cuh"
 #include "pair64.cuh"
 #include "pair32.cuh"
@@ -25,20 +29,23 @@ constexpr int kRBMax32 = 32;
 constexpr int kRBMax64 = 16;
 
 // ------------------------------------------------------------------ FP32
+constexpr int kHalf32 = 128;  // sources per staged half tile
+
 struct ArgsM32 {
-    int64_t n, npad, mwords;
+    int64_t n, npad, mwords, splits;
     int nr;  // right-hand sides in this pass (<= RB)
     Wave32 wave;
     float tau2, guard_lo, guard_hi;
     double tau;
     const float4 *pos, *nrm;
-    const float4 *dens;  // [RB/2][npad]: (p'_{2q} re, im, p'_{2q+1} re, im)
+    const float4 *dens;  // [RB/2][npad]: (re_{2q}, re_{2q+1}, im_{2q}, im_{2q+1})
     const float4 *thi, *tlo, *ohi, *olo;
     const uint32_t *nearmask;
     const double4_32a *tpos, *pos64;
     const int *perm;
     const double *p_re, *p_im;  // [nr][n] (diagonal term)
     double *q_re, *q_im;        // [nr][n]
+    float4 *sums;               // [splits][RB][npad]: re and im, head + tail each
     unsigned *err;
 };
 
@@ -47,157 +54,217 @@ __global__ void prepm32_kernel(int64_t n, int64_t npad, int nr, const int *__res
                                const double4_32a *__restrict__ tpos, const double *__restrict__ p_re,
                                const double *__restrict__ p_im, double scale, float4 *__restrict__ dens)
 {
+    const int q = blockIdx.y, r0 = 2 * q, r1 = 2 * q + 1;
     for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < npad; s += (int64_t)gridDim.x * blockDim.x) {
         const int c = perm[s];
-        const double ws = (c >= 0) ? tpos[s].w * scale : 0.0;
-#pragma unroll
-        for (int q = 0; q < RB / 2; q++) {
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (c >= 0) {
-                const int r0 = 2 * q, r1 = 2 * q + 1;
-                if (r0 < nr) {
-                    v.x = (float)(ws * p_re[(int64_t)r0 * n + c]);
-                    v.y = (float)(ws * p_im[(int64_t)r0 * n + c]);
-                }
-                if (r1 < nr) {
-                    v.z = (float)(ws * p_re[(int64_t)r1 * n + c]);
-                    v.w = (float)(ws * p_im[(int64_t)r1 * n + c]);
-                }
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (c >= 0) {
+            const double ws = tpos[s].w * scale;
+            if (r0 < nr) {
+                v.x = (float)(ws * p_re[(int64_t)r0 * n + c]);
+                v.z = (float)(ws * p_im[(int64_t)r0 * n + c]);
             }
-            dens[(int64_t)q * npad + s] = v;
+            if (r1 < nr) {
+                v.y = (float)(ws * p_re[(int64_t)r1 * n + c]);
+                v.w = (float)(ws * p_im[(int64_t)r1 * n + c]);
+            }
         }
+        dens[(int64_t)q * npad + s] = v;
     }
 }
 
+// One source: its entries for the thread's kTgM targets, multiplied into RB
+// columns two at a time.
+constexpr int kTgM = 2;
+constexpr int kNT32m = kTile32 / kTgM;  // threads of a CTA, which owns one target tile
+
 template <int RB, bool DIR, bool SCALED, bool SLOW>
-__device__ __forceinline__ void pairm32(const ArgsM32 &a, const float4 s_p, const float4 s_n, const float3 rel,
-                                        const float3 tn, float treg, float rc, int64_t tslot, int64_t src_slot,
-                                        const float4 *sd, int j, float (&acc)[2 * RB])
+__device__ __forceinline__ void pairm32(const ArgsM32 &a, const float4 *st, int j, const float3 (&rel)[kTgM],
+                                        const float3 (&tn)[kTgM], const float (&treg)[kTgM], const Turn (&turn)[kTgM],
+                                        int64_t tslot, int64_t src_slot, F2 (&accR)[kTgM][RB / 2],
+                                        F2 (&accI)[kTgM][RB / 2])
 {
-    const float dx = rel.x - s_p.x, dy = rel.y - s_p.y, dz = rel.z - s_p.z;
-    const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-    bool near = false;
-    if (SLOW) {
-        near = r2 <= a.tau2;
-        if (r2 > a.guard_lo && r2 < a.guard_hi) {
-            const int c = a.perm[src_slot];
-            if (c >= 0) {
-                const double4_32a q = a.pos64[c];
-                const double4_32a tp = a.tpos[tslot];
-                const double x1 = tp.x - q.x, x2 = tp.y - q.y, x3 = tp.z - q.z;
-                const double rr2 = x1 * x1 + x2 * x2 + x3 * x3;
-                near = !(sqrt(rr2) > a.tau);
+    const float4 s_p = st[j], s_n = st[kHalf32 + j];
+    F2 VR[kTgM], VI[kTgM], NV[kTgM];
+#pragma unroll
+    for (int g = 0; g < kTgM; g++) {
+        const float dx = rel[g].x - s_p.x, dy = rel[g].y - s_p.y, dz = rel[g].z - s_p.z;
+        const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+        bool near = false;
+        if (SLOW) {
+            near = r2 <= a.tau2;
+            if (r2 > a.guard_lo && r2 < a.guard_hi) {
+                const int c = a.perm[src_slot];
+                if (c >= 0) {
+                    const double4_32a q = a.pos64[c];
+                    const double4_32a tp = a.tpos[tslot + g * kNT32m];
+                    const double x1 = tp.x - q.x, x2 = tp.y - q.y, x3 = tp.z - q.z;
+                    near = !(sqrt(x1 * x1 + x2 * x2 + x3 * x3) > a.tau);
+                }
             }
         }
-    }
-    float u1, u2, rr;
-    kernel32<SCALED, SLOW>(a.wave, r2, rc, u1, u2, rr);
-    const float pA = DIR ? fmaf(dx, s_n.x, fmaf(dy, s_n.y, dz * s_n.z)) : fmaf(dx, tn.x, fmaf(dy, tn.y, dz * tn.z));
-    const float f = rr * pA;
-    float vr = -u1 * f, vi = u2 * f;
-    if (SLOW && near) {
-        vr = DIR ? s_p.w : treg;
-        vi = 0.f;
+        float u1, u2, rr;
+        kernel32<SCALED, SLOW>(a.wave, r2, SLOW ? 0.f : turn[g].rc, u1, u2, rr);
+        const float pA = DIR ? fmaf(dx, s_n.x, fmaf(dy, s_n.y, dz * s_n.z))
+                             : fmaf(dx, tn[g].x, fmaf(dy, tn[g].y, dz * tn[g].z));
+        const float f = rr * pA;
+        float vr = -u1 * f, vi = u2 * f;
+        if (SLOW && near) {
+            vr = DIR ? s_p.w : treg[g];
+            vi = 0.f;
+        }
+        VR[g] = f2_pack(vr, vr);
+        VI[g] = f2_pack(vi, vi);
+        NV[g] = f2_pack(-vi, -vi);
     }
 #pragma unroll
     for (int q = 0; q < RB / 2; q++) {
-        const float4 d = sd[q * kTile32 + j];
-        acc[4 * q + 0] = fmaf(vr, d.x, fmaf(-vi, d.y, acc[4 * q + 0]));
-        acc[4 * q + 1] = fmaf(vr, d.y, fmaf(vi, d.x, acc[4 * q + 1]));
-        acc[4 * q + 2] = fmaf(vr, d.z, fmaf(-vi, d.w, acc[4 * q + 2]));
-        acc[4 * q + 3] = fmaf(vr, d.w, fmaf(vi, d.z, acc[4 * q + 3]));
+        const ulonglong2 d = *reinterpret_cast<const ulonglong2 *>(st + (2 + q) * kHalf32 + j);
+#pragma unroll
+        for (int g = 0; g < kTgM; g++) {
+            accR[g][q] = f2_fma(VR[g], d.x, f2_fma(NV[g], d.y, accR[g][q]));
+            accI[g][q] = f2_fma(VR[g], d.y, f2_fma(VI[g], d.x, accI[g][q]));
+        }
     }
 }
 
-constexpr int kNT32m = 256;
+// Two targets a thread halve the loads of the staged densities (a 128-bit
+// broadcast load takes four of an SM's cycles, and one a pair for every two
+// columns bound the one-target form).  The cross-tile sums (FP32 head + tail)
+// live in global memory, read and written once a tile from L2: in registers
+// they left one CTA of eight warps an SM (16 columns, n = 27,750: 5.8 ms), in
+// shared memory two of four (3.7 ms).
 template <int RB>
-constexpr size_t smem_m32() { return 2 * (2 + RB / 2) * kTile32 * sizeof(float4); }
+constexpr size_t smem_m32 = 2 * (2 + RB / 2) * kHalf32 * sizeof(float4);
+template <int RB>
+constexpr int kCtas32m = RB <= 8 ? 4 : RB <= 16 ? 3 : 2;
 
 template <int RB, bool DIR, bool SCALED>
-__global__ void __launch_bounds__(kNT32m, RB <= 8 ? 2 : 1) sweepm32_kernel(ArgsM32 a)
+__global__ void __launch_bounds__(kNT32m, kCtas32m<RB>) sweepm32_kernel(ArgsM32 a)
 {
-    constexpr int TS = kTile32;
+    constexpr int NA = 2 + RB / 2;
     extern __shared__ __align__(128) float4 smem32[];
     __shared__ alignas(8) uint64_t bar[2];
-    float4 *sp[2] = {smem32, smem32 + (2 + RB / 2) * TS};
-    const int64_t slot = (int64_t)blockIdx.x * kNT32m + threadIdx.x;
-    const float4 th = a.thi[slot], tl = a.tlo[slot];
-    const float4 nn4 = a.nrm[slot];
-    const float3 tn = make_float3(nn4.x, nn4.y, nn4.z);
-    const float treg = a.pos[slot].w;
-    // near-tile mask row of this block's target tile (kNT32m == kTile32)
-    const uint32_t *mrow = a.nearmask + (slot / TS) * a.mwords;
-    // cross-tile sums: FP32 head + tail (TwoSum)
-    float acch[2 * RB], accl[2 * RB];
+    float4 *stage[2] = {smem32, smem32 + NA * kHalf32};
+    const int64_t blk = blockIdx.x, slot = blk * kTile32 + threadIdx.x;
+    float3 th[kTgM], tl[kTgM], tn[kTgM], rel[kTgM];
+    float treg[kTgM];
 #pragma unroll
-    for (int i = 0; i < 2 * RB; i++) acch[i] = accl[i] = 0.f;
-    const int64_t ntiles = a.npad / TS;
+    for (int g = 0; g < kTgM; g++) {
+        const float4 h = a.thi[slot + g * kNT32m], l = a.tlo[slot + g * kNT32m], m = a.nrm[slot + g * kNT32m];
+        th[g] = make_float3(h.x, h.y, h.z);
+        tl[g] = make_float3(l.x, l.y, l.z);
+        tn[g] = make_float3(m.x, m.y, m.z);
+        treg[g] = a.pos[slot + g * kNT32m].w;
+    }
+    const uint32_t *mrow = a.nearmask + blk * a.mwords;  // near-tile mask row
+    const int64_t tiles = a.npad / kTile32;
+    const int64_t h_begin = 2 * ((int64_t)blockIdx.y * tiles / a.splits);
+    const int64_t h_end = 2 * (((int64_t)blockIdx.y + 1) * tiles / a.splits);
+    float4 *sum = a.sums + (int64_t)blockIdx.y * RB * a.npad + slot;
+    bool first = true;
     if (threadIdx.x == 0) {
         mbar_init(&bar[0], 1);
         mbar_init(&bar[1], 1);
         fence_barrier_init();
     }
     __syncthreads();
-    auto issue = [&](int64_t tile, int buf) {
-        const int64_t base = tile * TS;
-        const uint32_t bytes = TS * sizeof(float4);
-        mbar_arrive_expect_tx(&bar[buf], (2 + RB / 2) * bytes);
-        bulk_g2s(sp[buf], a.pos + base, bytes, &bar[buf]);
-        bulk_g2s(sp[buf] + TS, a.nrm + base, bytes, &bar[buf]);
+    auto issue = [&](int64_t h, int buf) {
+        const int64_t base = h * kHalf32;
+        const uint32_t bytes = kHalf32 * sizeof(float4);
+        mbar_arrive_expect_tx(&bar[buf], NA * bytes);
+        bulk_g2s(stage[buf], a.pos + base, bytes, &bar[buf]);
+        bulk_g2s(stage[buf] + kHalf32, a.nrm + base, bytes, &bar[buf]);
 #pragma unroll
-        for (int q = 0; q < RB / 2; q++) bulk_g2s(sp[buf] + (2 + q) * TS, a.dens + q * a.npad + base, bytes, &bar[buf]);
+        for (int q = 0; q < RB / 2; q++)
+            bulk_g2s(stage[buf] + (2 + q) * kHalf32, a.dens + q * a.npad + base, bytes, &bar[buf]);
     };
-    if (threadIdx.x == 0) issue(0, 0);
-    for (int64_t tile = 0; tile < ntiles; tile++) {
-        const int buf = (int)(tile & 1);
-        if (threadIdx.x == 0 && tile + 1 < ntiles) issue(tile + 1, buf ^ 1);
-        const float4 oh = a.ohi[tile], ol = a.olo[tile];
-        const bool slow =
-            ((__ldg(mrow + (tile >> 5)) >> (tile & 31)) & 1u) || (SCALED && oh.w > kCentreRadius);
-        const float3 rel = make_float3((th.x - oh.x) + (tl.x - ol.x), (th.y - oh.y) + (tl.y - ol.y),
-                                       (th.z - oh.z) + (tl.z - ol.z));
-        Turn turn = {};
-        if (SCALED && !slow) turn = turn_of(rel);
-        const bool ok = mbar_wait_bounded(&bar[buf], (uint32_t)((tile >> 1) & 1), g_data_wait_limit);
+    if (threadIdx.x == 0 && h_begin < h_end) issue(h_begin, 0);
+    F2 accR[kTgM][RB / 2], accI[kTgM][RB / 2];
+    Turn turn[kTgM];
+#pragma unroll
+    for (int g = 0; g < kTgM; g++) {
+#pragma unroll
+        for (int q = 0; q < RB / 2; q++) accR[g][q] = accI[g][q] = 0;
+        rel[g] = make_float3(0.f, 0.f, 0.f);
+        turn[g] = {};
+    }
+    bool slow = false;
+    for (int64_t h = h_begin; h < h_end; h++) {
+        const int64_t it = h - h_begin, tile = h >> 1;
+        const int buf = (int)(it & 1);
+        if (threadIdx.x == 0 && h + 1 < h_end) issue(h + 1, buf ^ 1);
+        if (!(h & 1)) {
+            const float4 oh = a.ohi[tile], ol = a.olo[tile];
+            slow = ((__ldg(mrow + (tile >> 5)) >> (tile & 31)) & 1u) || (SCALED && oh.w > kCentreRadius);
+#pragma unroll
+            for (int g = 0; g < kTgM; g++) {
+                rel[g] = make_float3((th[g].x - oh.x) + (tl[g].x - ol.x), (th[g].y - oh.y) + (tl[g].y - ol.y),
+                                     (th[g].z - oh.z) + (tl[g].z - ol.z));
+                if (SCALED && !slow) turn[g] = turn_of(rel[g]);
+            }
+        }
+        const bool ok = mbar_wait_bounded(&bar[buf], (uint32_t)((it >> 1) & 1), g_data_wait_limit);
         if (__syncthreads_or(!ok)) {
             if (threadIdx.x == 0) {
                 atomicOr(a.err, DEV_ERR_WAIT);
-                mbar_drain(&bar[buf], (uint32_t)((tile >> 1) & 1), &bar[buf ^ 1], (uint32_t)(((tile + 1) >> 1) & 1),
-                           tile + 1 < ntiles);
+                mbar_drain(&bar[buf], (uint32_t)((it >> 1) & 1), &bar[buf ^ 1], (uint32_t)(((it + 1) >> 1) & 1),
+                           h + 1 < h_end);
             }
             return;
         }
-        const float4 *P = sp[buf], *Nn = sp[buf] + TS, *D = sp[buf] + 2 * TS;
-        float acc[2 * RB];
-#pragma unroll
-        for (int i = 0; i < 2 * RB; i++) acc[i] = 0.f;
-        const int64_t base = tile * TS;
+        const float4 *st = stage[buf];
+        const int64_t base = h * kHalf32;
         if (slow) {
-            for (int j = 0; j < TS; j++)
-                pairm32<RB, DIR, SCALED, true>(a, P[j], Nn[j], rel, tn, treg, 0.f, slot, base + j, D, j, acc);
+            for (int j = 0; j < kHalf32; j++)
+                pairm32<RB, DIR, SCALED, true>(a, st, j, rel, tn, treg, turn, slot, base + j, accR, accI);
         } else {
-            for (int j = 0; j < TS; j++)
-                pairm32<RB, DIR, SCALED, false>(a, P[j], Nn[j], rel, tn, treg, turn.rc, slot, base + j, D, j, acc);
-            if (SCALED) {
-#pragma unroll
-                for (int r = 0; r < RB; r++) turn_sum<false>(turn, acc[2 * r], acc[2 * r + 1]);
-            }
+            for (int j = 0; j < kHalf32; j++)
+                pairm32<RB, DIR, SCALED, false>(a, st, j, rel, tn, treg, turn, slot, base + j, accR, accI);
         }
+        if (h & 1) {
 #pragma unroll
-        for (int i = 0; i < 2 * RB; i++) two_sum_acc(acch[i], accl[i], acc[i]);
+            for (int g = 0; g < kTgM; g++)
+#pragma unroll
+                for (int q = 0; q < RB / 2; q++) {
+                    float re[2], im[2];
+                    f2_unpack(accR[g][q], re[0], re[1]);
+                    f2_unpack(accI[g][q], im[0], im[1]);
+                    accR[g][q] = accI[g][q] = 0;
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        if (SCALED && !slow) turn_sum<false>(turn[g], re[e], im[e]);
+                        float4 *at = sum + (int64_t)(2 * q + e) * a.npad + g * kNT32m;
+                        float4 x = first ? make_float4(0.f, 0.f, 0.f, 0.f) : *at;
+                        two_sum_acc(x.x, x.y, re[e]);
+                        two_sum_acc(x.z, x.w, im[e]);
+                        *at = x;
+                    }
+                }
+            first = false;
+        }
         __syncthreads();
     }
+}
+
+// Adds up the shares of the source tiles in order, and the diagonal term.
+template <int RB>
+__global__ void __launch_bounds__(256) reducem32_kernel(ArgsM32 a)
+{
+    const int r = blockIdx.y;
+    const int64_t slot = blockIdx.x * (int64_t)256 + threadIdx.x;
+    if (slot >= a.npad) return;
     const int c = a.perm[slot];
     if (c < 0) return;
-#pragma unroll
-    for (int r = 0; r < RB; r++) {
-        if (r >= a.nr) break;
-        const double vr = (double)acch[2 * r] + (double)accl[2 * r];
-        const double vi = (double)acch[2 * r + 1] + (double)accl[2 * r + 1];
-        if (!isfinite(vr) || !isfinite(vi)) atomicOr(a.err, DEV_ERR_NONFINITE);
-        a.q_re[(int64_t)r * a.n + c] = vr + 0.5 * a.p_re[(int64_t)r * a.n + c];
-        a.q_im[(int64_t)r * a.n + c] = vi + 0.5 * a.p_im[(int64_t)r * a.n + c];
+    double vr = 0, vi = 0;
+    for (int64_t s = 0; s < a.splits; s++) {
+        const float4 v = a.sums[(s * RB + r) * a.npad + slot];
+        vr += (double)v.x + (double)v.y;
+        vi += (double)v.z + (double)v.w;
     }
+    if (!isfinite(vr) || !isfinite(vi)) atomicOr(a.err, DEV_ERR_NONFINITE);
+    a.q_re[(int64_t)r * a.n + c] = vr + 0.5 * a.p_re[(int64_t)r * a.n + c];
+    a.q_im[(int64_t)r * a.n + c] = vi + 0.5 * a.p_im[(int64_t)r * a.n + c];
 }
 
 // ------------------------------------------------------------------ FP64
@@ -353,11 +420,12 @@ int blocks_for(int64_t work)
 }
 
 // Block of the next pass for `left` remaining columns: the smallest compiled
-// block that holds them all, else the largest (one pass over RB columns
-// costs about c0 + c1 RB, so a wider block beats two narrower passes).
+// block that holds them all, else the largest.  FP32, 17 to 24 columns: 16 and
+// then 8 (74 + 44 ms at n = 145,272, one pass of 32 147 ms).
 int pass_block(int precision, int left)
 {
     const int top = (precision == HZ_PREC_F64) ? kRBMax64 : kRBMax32;
+    if (top == kRBMax32 && left > 16 && left <= 24) return 16;
     for (int rb = 8; rb < top; rb *= 2)
         if (left <= rb) return rb;
     return top;
@@ -402,23 +470,47 @@ int launch_m64(const SweepConst &c, const Rec64 &r64, int nr, const double *pr, 
     return HZ_OK;
 }
 
+// Shares of the source tiles of the FP32 pass: one when the target tiles fill
+// the chip six times over, else enough for about four rounds of resident CTAs
+// (short last round), of at least two tiles each.
+template <int RB>
+int64_t splits_m32(int64_t npad)
+{
+    int dev = 0, sms = 152;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int64_t tiles = npad / kTile32, ctas = (int64_t)kCtas32m<RB> * sms;
+    if (tiles >= 6 * ctas) return 1;
+    int64_t s = (4 * ctas + tiles - 1) / tiles;
+    if (s > tiles / 2) s = tiles / 2;
+    return s < 1 ? 1 : s;
+}
+
+template <int RB>
+size_t bytes_m32(int64_t npad)
+{
+    const int64_t sp = splits_m32<RB>(npad);
+    return (size_t)npad * (RB / 2 + sp * RB) * sizeof(float4);
+}
+
 template <int RB>
 int launch_m32(const SweepConst &c, const Rec32 &r32, const Rec64 &r64, int nr, const double *pr, const double *pi,
                double *qr, double *qi, void *scratch, cudaStream_t s)
 {
-    constexpr int smem = (int)smem_m32<RB>();
     const Const32 k32 = constants32(c, r32.lambda);
     auto kernel = k32.scaled ? (c.dirichlet ? sweepm32_kernel<RB, true, true> : sweepm32_kernel<RB, false, true>)
                              : (c.dirichlet ? sweepm32_kernel<RB, true, false> : sweepm32_kernel<RB, false, false>);
-    HZ_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    HZ_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_m32<RB>));
     float4 *dens = static_cast<float4 *>(scratch);
     const double scale = 1.0 / sweep32_reg_scale(c.interior, r32.lambda);
-    prepm32_kernel<RB><<<blocks_for(r32.npad), 256, 0, s>>>(c.n, r32.npad, nr, r32.perm, r32.tpos, pr, pi, scale,
-                                                            dens);
+    prepm32_kernel<RB><<<dim3((unsigned)(r32.npad / 256), RB / 2), 256, 0, s>>>(c.n, r32.npad, nr, r32.perm, r32.tpos,
+                                                                               pr, pi, scale, dens);
     HZ_CHECK_LAUNCH();
     ArgsM32 a;
     a.n = c.n;
     a.npad = r32.npad;
+    a.splits = splits_m32<RB>(r32.npad);
+    a.sums = dens + (int64_t)(RB / 2) * r32.npad;
     a.nr = nr;
     a.wave = {k32.k, k32.kh, k32.kl};
     a.tau = c.tau;
@@ -442,8 +534,10 @@ int launch_m32(const SweepConst &c, const Rec32 &r32, const Rec64 &r64, int nr, 
     a.q_re = qr;
     a.q_im = qi;
     a.err = c.err;
-    const unsigned blocks = (unsigned)(r32.npad / kNT32m);
-    kernel<<<blocks, kNT32m, smem, s>>>(a);
+    const unsigned tiles = (unsigned)(r32.npad / kTile32);
+    kernel<<<dim3(tiles, (unsigned)a.splits), kNT32m, smem_m32<RB>, s>>>(a);
+    HZ_CHECK_LAUNCH();
+    reducem32_kernel<RB><<<dim3(tiles, (unsigned)nr), 256, 0, s>>>(a);
     HZ_CHECK_LAUNCH();
     return HZ_OK;
 }
@@ -457,11 +551,22 @@ long long multi_rhs_passes(int precision, int nrhs)
     return p;
 }
 
-size_t multi_rhs_scratch_bytes(int64_t n, int64_t npad)
+size_t multi_rhs_scratch_bytes(int precision, int nrhs, int64_t n, const Rec32 &r32, const Rec64 &r64)
 {
-    const size_t a = (size_t)(kRBMax32 / 2) * (size_t)npad * sizeof(float4);
-    const size_t b = (size_t)(kRBMax64 / 2) * (size_t)n * sizeof(double4_32a);
-    return a > b ? a : b;
+    size_t most = 0;
+    for (int r0 = 0; r0 < nrhs;) {
+        const int rb = pass_block(precision, nrhs - r0), nr = (nrhs - r0 < rb) ? (nrhs - r0) : rb;
+        size_t b;
+        if (precision != HZ_PREC_F64)
+            b = rb == 8 ? bytes_m32<8>(r32.npad) : rb == 16 ? bytes_m32<16>(r32.npad) : bytes_m32<32>(r32.npad);
+        else if (r64.split)
+            b = split_cols_scratch_bytes(r32.npad, nr);
+        else
+            b = (size_t)(rb / 2) * (size_t)n * sizeof(double4_32a);
+        if (b > most) most = b;
+        r0 += nr;
+    }
+    return most;
 }
 
 int sweep_multi(const SweepConst &c, const Rec32 &r32, const Rec64 &r64, int precision, int nrhs,
@@ -475,7 +580,8 @@ int sweep_multi(const SweepConst &c, const Rec32 &r32, const Rec64 &r64, int pre
         const double *pr = p_re + (int64_t)r0 * c.n, *pi = p_im + (int64_t)r0 * c.n;
         double *qr = q_re + (int64_t)r0 * c.n, *qi = q_im + (int64_t)r0 * c.n;
         if (precision == HZ_PREC_F64) {
-            if (rb == 8) HZ_TRY(launch_m64<8>(c, r64, nr, pr, pi, qr, qi, scratch, s));
+            if (r64.split) HZ_TRY(sweep_split_cols(c, *r64.split, r64.nrm, nr, pr, pi, qr, qi, scratch, s));
+            else if (rb == 8) HZ_TRY(launch_m64<8>(c, r64, nr, pr, pi, qr, qi, scratch, s));
             else HZ_TRY(launch_m64<16>(c, r64, nr, pr, pi, qr, qi, scratch, s));
         } else {
             if (rb == 8) HZ_TRY(launch_m32<8>(c, r32, r64, nr, pr, pi, qr, qi, scratch, s));

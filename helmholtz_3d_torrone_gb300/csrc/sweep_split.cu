@@ -227,10 +227,11 @@ struct TileUnits {
     float n32, n8;       // 2^32 and 2^8 units of A.n
 };
 
+// The entries of one pair: A's (ar, ai) and A^H's before conjugation (hr, hi).
 template <int MODE, bool DIR, bool CLOSE>
-__device__ __forceinline__ void split_pair(const ArgsSplit &a, const float4 (*st)[kHalf], int j, const float2 *tab,
-                                           const Offsets &t, const TargetNormal &tn, FF treg, const TileUnits &u,
-                                           int64_t tslot, int64_t sslot, FF (&accA)[2], FF (&accH)[2])
+__device__ __forceinline__ void split_entry(const ArgsSplit &a, const float4 (*st)[kHalf], int j, const float2 *tab,
+                                            const Offsets &t, const TargetNormal &tn, FF treg, const TileUnits &u,
+                                            int64_t tslot, int64_t sslot, FF &ar, FF &ai, FF &hr, FF &hi)
 {
     constexpr bool A = (MODE & SWEEP_A) != 0, H = (MODE & SWEEP_AH) != 0;
     constexpr bool SRC = (A && DIR) || (H && !DIR);  // (x_t - x_s).n_s wanted
@@ -300,7 +301,10 @@ __device__ __forceinline__ void split_pair(const ArgsSplit &a, const float4 (*st
         vtr = ff_mul(ur, f);
         vti = ff_mul(ui, f);
     }
-    FF ar = DIR ? vsr : vtr, ai = DIR ? vsi : vti, hr = DIR ? vtr : vsr, hi = DIR ? vti : vsi;
+    ar = DIR ? vsr : vtr;
+    ai = DIR ? vsi : vti;
+    hr = DIR ? vtr : vsr;
+    hi = DIR ? vti : vsi;
     if (CLOSE && !far) {
         const float4 r5 = st[5][j];
         const FF srg = {r5.z, r5.w};
@@ -308,6 +312,16 @@ __device__ __forceinline__ void split_pair(const ArgsSplit &a, const float4 (*st
         hr = DIR ? treg : srg;
         ai = hi = {0.f, 0.f};
     }
+}
+
+template <int MODE, bool DIR, bool CLOSE>
+__device__ __forceinline__ void split_pair(const ArgsSplit &a, const float4 (*st)[kHalf], int j, const float2 *tab,
+                                           const Offsets &t, const TargetNormal &tn, FF treg, const TileUnits &u,
+                                           int64_t tslot, int64_t sslot, FF (&accA)[2], FF (&accH)[2])
+{
+    constexpr bool A = (MODE & SWEEP_A) != 0, H = (MODE & SWEEP_AH) != 0;
+    FF ar, ai, hr, hi;
+    split_entry<MODE, DIR, CLOSE>(a, st, j, tab, t, tn, treg, u, tslot, sslot, ar, ai, hr, hi);
     if (A) {
         const float4 d = st[kRecs][j];
         const FF dr = {d.x, d.z}, di = {d.y, d.w};
@@ -352,6 +366,88 @@ __device__ __forceinline__ void split_phase64(double x, const float2 *tab, doubl
     const double z = r * r, sn = fma(r * z, -1.0 / 6.0, r), cm = z * fma(z, -1.0 / 24.0, 0.5);
     cr = tc - fma(ts, sn, tc * cm);
     sr = ts + fma(tc, sn, -(ts * cm));
+}
+
+// Offsets of a thread's target (scaled position X, Y, Z in the tile with
+// origin `to`) from source tile `tile`, the tile's units, and for a far tile
+// the phase of its origin.
+template <bool TGT>
+__device__ __forceinline__ void set_tile(const ArgsSplit &a, int64_t tile, const double4_32a &to, double X, double Y,
+                                         double Z, double nx, double ny, double nz, const float2 *tab, Offsets &t,
+                                         TileUnits &un, bool &close, double &phr, double &phi)
+{
+    const float ox = (float)to.x, oy = (float)to.y, oz = (float)to.z, Rt = (float)to.w;
+    const double4_32a o = a.tile[tile];
+    const float Rs = (float)o.w;
+    const float cx = ox - (float)o.x, cy = oy - (float)o.y, cz = oz - (float)o.z;
+    const float ct = sqrtf(fmaf(cx, cx, fmaf(cy, cy, cz * cz)));
+    close = ct - Rt < 2.5f * Rs + a.ktau + 1e-4f * (ct + Rt + fabsf(ox) + fabsf(oy) + fabsf(oz));
+    const int eS = exponent_above((float)(o.w * (1.0 + 1e-6)));
+    const int eL = max(eS + 1, exponent_above(2.0002f * (ct + Rt)));
+    un.shS = eL - eS;
+    un.shT = eL - eS - 1;
+    un.x = max(0, eL - eS - 3);
+    un.w32 = pow2f(eL + eS - 28);
+    un.w8 = pow2f(eL + eS - 52);
+    un.r32 = un.w32 * pow2f(un.x);
+    un.r8 = un.w8 * pow2f(un.x);
+    un.n32 = pow2f(eL - 28);
+    un.n8 = pow2f(eL - 52);
+    const double uL = pow2d(eL - 30), iL = pow2d(30 - eL);
+    const double ax = -2.0 * (X - o.x), ay = -2.0 * (Y - o.y), az = -2.0 * (Z - o.z);
+    const double A[3] = {ax, ay, az};
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const double m = fma(A[i], iL, 6755399441055744.0);  // nearest integer in the low word
+        t.h[i] = __double2loint(m);
+        t.f[i] = (float)A[i];
+        t.l[i] = (float)fma(-uL, m - 6755399441055744.0, A[i]);
+    }
+    const double a2 = 0.25 * fma(az, az, fma(ay, ay, ax * ax));
+    if (close) {
+        t.a2i = __double2ll_rn(a2 * pow2d(60 - eL - eS - un.x));
+    } else {
+        const double y0 = (double)rsqrt_seed((float)a2);
+        const double e = fma(-(a2 * y0), y0, 1.0);
+        const double y = fma(y0 * e, fma(e, 0.375, 0.5), y0);
+        const double g = a2 * y;
+        const double rc = fma(fma(-g, g, a2), 0.5 * y, g);
+        t.a2 = ff_of_double(a2);
+        t.rc = ff_of_double(rc);
+        split_phase64(rc, tab, phr, phi);
+    }
+    if (TGT) t.an = __double2ll_rn(fma(az, nz, fma(ay, ny, ax * nx)) * pow2d(60 - eL)) + 128;
+}
+
+template <bool TGT>
+__device__ __forceinline__ void load_target(const ArgsSplit &a, int64_t slot, double &X, double &Y, double &Z,
+                                            double &nx, double &ny, double &nz, FF &treg, TargetNormal &tn)
+{
+    const double4_32a tp = a.tpos[slot];
+    X = a.wave * tp.x;
+    Y = a.wave * tp.y;
+    Z = a.wave * tp.z;
+    const float4 r5 = a.rec[5 * a.npad + slot];
+    treg = {r5.z, r5.w};
+    nx = ny = nz = 0.0;
+    if (!TGT) return;
+    const int c = a.perm[slot];
+    if (c >= 0) {
+        const double4_32a m = a.nrm[c];
+        nx = m.x;
+        ny = m.y;
+        nz = m.z;
+    }
+    const float4 r0 = a.rec[slot], r1 = a.rec[a.npad + slot], r4 = a.rec[4 * a.npad + slot];
+    tn.h[0] = __float_as_int(r0.w);
+    tn.h[1] = __float_as_int(r1.x);
+    tn.h[2] = __float_as_int(r1.y);
+    tn.f[0] = 2.f * r4.x;
+    tn.f[1] = 2.f * r4.y;
+    tn.f[2] = 2.f * r4.z;
+    tn.l[0] = 2.f * r4.w;
+    tn.l[1] = 2.f * r5.x;
+    tn.l[2] = 2.f * r5.y;
 }
 
 template <int MODE>
@@ -414,36 +510,11 @@ __global__ void __launch_bounds__(kTile32, 2) sweep_split_kernel(ArgsSplit a)
         const int64_t seg_end = (u_end < (blk + 1) * halves) ? u_end : (blk + 1) * halves;
         const bool whole = (u == blk * halves) && (seg_end == (blk + 1) * halves);
         const int64_t slot = blk * kTile32 + threadIdx.x;
-        const double4_32a tp = a.tpos[slot];
-        const double X = a.wave * tp.x, Y = a.wave * tp.y, Z = a.wave * tp.z;
         const double4_32a to = a.tile[blk];
-        const float ox = (float)to.x, oy = (float)to.y, oz = (float)to.z, Rt = (float)to.w;
-        FF treg = {0.f, 0.f};
+        double X, Y, Z, nx, ny, nz;
+        FF treg;
         TargetNormal tn = {};
-        double nx = 0, ny = 0, nz = 0;
-        {
-            const float4 r5 = a.rec[5 * a.npad + slot];
-            treg = {r5.z, r5.w};
-            if (TGT) {
-                const int c = a.perm[slot];
-                if (c >= 0) {
-                    const double4_32a m = a.nrm[c];
-                    nx = m.x;
-                    ny = m.y;
-                    nz = m.z;
-                }
-                const float4 r0 = a.rec[slot], r1 = a.rec[a.npad + slot], r4 = a.rec[4 * a.npad + slot];
-                tn.h[0] = __float_as_int(r0.w);
-                tn.h[1] = __float_as_int(r1.x);
-                tn.h[2] = __float_as_int(r1.y);
-                tn.f[0] = 2.f * r4.x;
-                tn.f[1] = 2.f * r4.y;
-                tn.f[2] = 2.f * r4.z;
-                tn.l[0] = 2.f * r4.w;
-                tn.l[1] = 2.f * r5.x;
-                tn.l[2] = 2.f * r5.y;
-            }
-        }
+        load_target<TGT>(a, slot, X, Y, Z, nx, ny, nz, treg, tn);
         double q[4] = {0, 0, 0, 0};
         double dA[2] = {0, 0}, dH[2] = {0, 0};
         Offsets t = {};
@@ -456,48 +527,8 @@ __global__ void __launch_bounds__(kTile32, 2) sweep_split_kernel(ArgsSplit a)
             if (threadIdx.x == 0 && u + 1 < u_end) issue(u + 1, buf ^ 1);
             const int64_t half = u - blk * halves, tile = half >> 1;
             if (fresh || !(half & 1)) {
-                // offsets of this thread's target from the source tile's origin
                 fresh = false;
-                const double4_32a o = a.tile[tile];
-                const float Rs = (float)o.w;
-                const float cx = ox - (float)o.x, cy = oy - (float)o.y, cz = oz - (float)o.z;
-                const float ct = sqrtf(fmaf(cx, cx, fmaf(cy, cy, cz * cz)));
-                close = ct - Rt < 2.5f * Rs + a.ktau + 1e-4f * (ct + Rt + fabsf(ox) + fabsf(oy) + fabsf(oz));
-                const int eS = exponent_above((float)(o.w * (1.0 + 1e-6)));
-                const int eL = max(eS + 1, exponent_above(2.0002f * (ct + Rt)));
-                un.shS = eL - eS;
-                un.shT = eL - eS - 1;
-                un.x = max(0, eL - eS - 3);
-                un.w32 = pow2f(eL + eS - 28);
-                un.w8 = pow2f(eL + eS - 52);
-                un.r32 = un.w32 * pow2f(un.x);
-                un.r8 = un.w8 * pow2f(un.x);
-                un.n32 = pow2f(eL - 28);
-                un.n8 = pow2f(eL - 52);
-                const double uL = pow2d(eL - 30), iL = pow2d(30 - eL);
-                const double ax = -2.0 * (X - o.x), ay = -2.0 * (Y - o.y), az = -2.0 * (Z - o.z);
-                const double A[3] = {ax, ay, az};
-#pragma unroll
-                for (int i = 0; i < 3; i++) {
-                    const double m = fma(A[i], iL, 6755399441055744.0);  // nearest integer in the low word
-                    t.h[i] = __double2loint(m);
-                    t.f[i] = (float)A[i];
-                    t.l[i] = (float)fma(-uL, m - 6755399441055744.0, A[i]);
-                }
-                const double a2 = 0.25 * fma(az, az, fma(ay, ay, ax * ax));
-                if (close) {
-                    t.a2i = __double2ll_rn(a2 * pow2d(60 - eL - eS - un.x));
-                } else {
-                    const double y0 = (double)rsqrt_seed((float)a2);
-                    const double e = fma(-(a2 * y0), y0, 1.0);
-                    const double y = fma(y0 * e, fma(e, 0.375, 0.5), y0);
-                    const double g = a2 * y;
-                    const double rc = fma(fma(-g, g, a2), 0.5 * y, g);
-                    t.a2 = ff_of_double(a2);
-                    t.rc = ff_of_double(rc);
-                    split_phase64(rc, tab, phr, phi);
-                }
-                if (TGT) t.an = __double2ll_rn(fma(az, nz, fma(ay, ny, ax * nx)) * pow2d(60 - eL)) + 128;
+                set_tile<TGT>(a, tile, to, X, Y, Z, nx, ny, nz, tab, t, un, close, phr, phi);
             }
             const bool ok = mbar_wait_bounded(&bar[buf], (uint32_t)((it >> 1) & 1), g_data_wait_limit);
             if (__syncthreads_or(!ok)) {
@@ -561,12 +592,304 @@ __global__ void __launch_bounds__(kTile32) split_fixup_kernel(ArgsSplit a)
     split_write<MODE>(a, blk * kTile32 + threadIdx.x, q[0], q[1], q[2], q[3]);
 }
 
+// ------------------------------------------------- several right-hand sides
+// Q = A P for blocks of RB = 4, 8 or 16 columns: the entry of a pair is formed
+// once (about 165 slots) and each column adds 50.  Wider blocks hold 4 RB FP32
+// sums a thread and keep their FP64 sums in shared memory, which leaves one CTA
+// an SM; their columns' independent chains fill the pipe instead of warps.
+constexpr int kColsMax = 16;
+template <int RB>
+constexpr int kColsCtas = RB <= 4 ? 2 : 1;
+template <int RB>
+constexpr size_t kColsSmem = kSplitTable * sizeof(float2) + 2 * (kRecs + RB) * kHalf * sizeof(float4) +
+                             (RB <= 4 ? 0 : 2 * RB * kTile32 * sizeof(double));
+
+struct ColsArgs {
+    int nr;
+    int64_t n, splits;
+    const double *p_re, *p_im;  // [nr][n]
+    double *q_re, *q_im;
+    double2 *partial;           // [splits][RB][npad], splits > 1
+};
+
+// Exponents and split densities of column blockIdx.y (see split_max_kernel).
+__global__ void __launch_bounds__(256) cols_max_kernel(int64_t n, const double4_32a *__restrict__ nrm,
+                                                       const double *__restrict__ p_re,
+                                                       const double *__restrict__ p_im, int *__restrict__ part)
+{
+    const double *pr = p_re + blockIdx.y * n, *pi = p_im + blockIdx.y * n;
+    int a = 0;
+    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n; s += (int64_t)gridDim.x * blockDim.x) {
+        const double w = nrm[s].w;
+        a = max(a, max(__double2hiint(w * pr[s]) & 0x7fffffff, __double2hiint(w * pi[s]) & 0x7fffffff));
+    }
+    a = __reduce_max_sync(0xffffffffu, a);
+    __shared__ int sh[8];
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = a;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; w++) a = max(a, sh[w]);
+        part[blockIdx.y * kExpBlocks + blockIdx.x] = a;
+    }
+}
+
+__global__ void __launch_bounds__(256) cols_dens_kernel(int64_t n, int64_t npad, int nr,
+                                                        const int *__restrict__ perm,
+                                                        const double4_32a *__restrict__ tpos,
+                                                        const double *__restrict__ p_re,
+                                                        const double *__restrict__ p_im, double scale,
+                                                        const int *__restrict__ part, int *__restrict__ expo,
+                                                        float4 *__restrict__ dens)
+{
+    const int r = blockIdx.y;
+    __shared__ int ex;
+    if (threadIdx.x < 32) {
+        int v = 0;
+        if (r < nr)
+            for (int b = threadIdx.x; b < kExpBlocks; b += 32) v = max(v, part[r * kExpBlocks + b]);
+        v = __reduce_max_sync(0xffffffffu, v);
+        if (threadIdx.x == 0) {
+            ex = max(-1000, min(1000, (v >> 20) - 1022));
+            if (blockIdx.x == 0) expo[r] = ex;
+        }
+    }
+    __syncthreads();
+    const double f = pow2d(-ex);
+    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < npad; s += (int64_t)gridDim.x * blockDim.x) {
+        const int c = perm[s];
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (c >= 0 && r < nr) {
+            const double w = tpos[s].w;
+            const FF x = ff_of_double(-scale * ((w * p_re[r * n + c]) * f)), y = ff_of_double(-scale * ((w * p_im[r * n + c]) * f));
+            v = make_float4(x.h, y.h, x.l, y.l);
+        }
+        dens[r * npad + s] = v;
+    }
+}
+
+// q[i] is column sum i: q + i when it lies in registers, strided in shared
+// memory otherwise.
+template <int RB, bool DIR, bool CLOSE>
+__device__ __forceinline__ void cols_half(const ArgsSplit &a, const float4 (*st)[kHalf], const float2 *tab,
+                                          const Offsets &t, const TargetNormal &tn, FF treg, const TileUnits &u,
+                                          int64_t tslot, int64_t sslot0, double phr, double phi, double *q)
+{
+    constexpr int STEP = RB <= 4 ? 1 : kTile32;
+#pragma unroll 1
+    for (int j0 = 0; j0 < kHalf; j0 += kRun) {
+        FF acc[2 * RB];
+#pragma unroll
+        for (int r = 0; r < 2 * RB; r++) acc[r] = {0.f, 0.f};
+#pragma unroll 1
+        for (int j = j0; j < j0 + kRun; j++) {
+            FF ar, ai, hr, hi;
+            split_entry<SWEEP_A, DIR, CLOSE>(a, st, j, tab, t, tn, treg, u, tslot, sslot0 + j, ar, ai, hr, hi);
+#pragma unroll
+            for (int r = 0; r < RB; r++) {
+                const float4 d = st[kRecs + r][j];
+                const FF dr = {d.x, d.z}, di = {d.y, d.w};
+                split_dot2<-1>(acc[2 * r], ar, dr, ai, di);
+                split_dot2<1>(acc[2 * r + 1], ar, di, ai, dr);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < RB; r++) {
+            const double x = (double)acc[2 * r].h + (double)acc[2 * r].l;
+            const double y = (double)acc[2 * r + 1].h + (double)acc[2 * r + 1].l;
+            double &u0 = q[2 * r * STEP], &u1 = q[(2 * r + 1) * STEP];
+            if (CLOSE) {
+                u0 += x;
+                u1 += y;
+            } else {
+                u0 = fma(phr, x, fma(-phi, y, u0));
+                u1 = fma(phr, y, fma(phi, x, u1));
+            }
+        }
+    }
+}
+
+// CTA (target tile, share of the source tiles); with several shares the
+// sums go to partial and cols_reduce_kernel adds them up.
+template <int RB, bool DIR>
+__global__ void __launch_bounds__(kTile32, kColsCtas<RB>) cols_kernel(ArgsSplit a, ColsArgs m)
+{
+    constexpr int NA = kRecs + RB, STEP = RB <= 4 ? 1 : kTile32;
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ alignas(8) uint64_t bar[2];
+    float2 *tab = reinterpret_cast<float2 *>(smem);
+    float4(*stage)[kHalf] = reinterpret_cast<float4(*)[kHalf]>(smem + kSplitTable * sizeof(float2));
+    if (threadIdx.x == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        fence_barrier_init();
+    }
+    for (int i = threadIdx.x; i < kSplitTable / 2; i += kTile32)
+        reinterpret_cast<float4 *>(tab)[i] = __ldg(reinterpret_cast<const float4 *>(a.table) + i);
+    __syncthreads();
+    const int64_t tiles = a.npad / kTile32, blk = blockIdx.x, slot = blk * kTile32 + threadIdx.x;
+    const int64_t h_begin = 2 * ((int64_t)blockIdx.y * tiles / m.splits);
+    const int64_t h_end = 2 * (((int64_t)blockIdx.y + 1) * tiles / m.splits);
+    auto issue = [&](int64_t h, int buf) {
+        const uint32_t bytes = kHalf * sizeof(float4);
+        mbar_arrive_expect_tx(&bar[buf], NA * bytes);
+#pragma unroll
+        for (int r = 0; r < kRecs; r++) bulk_g2s(&stage[buf * NA + r][0], a.rec + r * a.npad + h * kHalf, bytes, &bar[buf]);
+#pragma unroll
+        for (int r = 0; r < RB; r++)
+            bulk_g2s(&stage[buf * NA + kRecs + r][0], a.densA + r * a.npad + h * kHalf, bytes, &bar[buf]);
+    };
+    if (threadIdx.x == 0 && h_begin < h_end) issue(h_begin, 0);
+    const double4_32a to = a.tile[blk];
+    double X, Y, Z, nx, ny, nz, phr = 1.0, phi = 0.0;
+    FF treg;
+    TargetNormal tn = {};
+    load_target<!DIR>(a, slot, X, Y, Z, nx, ny, nz, treg, tn);
+    double qr[RB <= 4 ? 2 * RB : 1];
+    double *q = RB <= 4 ? qr
+                        : reinterpret_cast<double *>(smem + kSplitTable * sizeof(float2) +
+                                                     2 * NA * kHalf * sizeof(float4)) + threadIdx.x;
+#pragma unroll
+    for (int r = 0; r < 2 * RB; r++) q[r * STEP] = 0.0;
+    Offsets t = {};
+    TileUnits un = {};
+    bool close = false;
+    for (int64_t h = h_begin; h < h_end; h++) {
+        const int64_t it = h - h_begin;
+        const int buf = (int)(it & 1);
+        if (threadIdx.x == 0 && h + 1 < h_end) issue(h + 1, buf ^ 1);
+        if (!(h & 1)) set_tile<!DIR>(a, h >> 1, to, X, Y, Z, nx, ny, nz, tab, t, un, close, phr, phi);
+        const bool ok = mbar_wait_bounded(&bar[buf], (uint32_t)((it >> 1) & 1), g_data_wait_limit);
+        if (__syncthreads_or(!ok)) {
+            if (threadIdx.x == 0) {
+                atomicOr(a.err, DEV_ERR_WAIT);
+                mbar_drain(&bar[buf], (uint32_t)((it >> 1) & 1), &bar[buf ^ 1], (uint32_t)(((it + 1) >> 1) & 1),
+                           h + 1 < h_end);
+            }
+            return;
+        }
+        if (close)
+            cols_half<RB, DIR, true>(a, stage + buf * NA, tab, t, tn, treg, un, slot, h * kHalf, phr, phi, q);
+        else
+            cols_half<RB, DIR, false>(a, stage + buf * NA, tab, t, tn, treg, un, slot, h * kHalf, phr, phi, q);
+        __syncthreads();
+    }
+    if (m.splits > 1) {
+#pragma unroll
+        for (int r = 0; r < RB; r++)
+            m.partial[((int64_t)blockIdx.y * RB + r) * a.npad + slot] =
+                make_double2(q[2 * r * STEP], q[(2 * r + 1) * STEP]);
+        return;
+    }
+    const int c = a.perm[slot];
+    if (c < 0) return;
+#pragma unroll
+    for (int r = 0; r < RB; r++) {
+        if (r >= m.nr) break;
+        const double f = pow2d(a.expo[r]), x = f * q[2 * r * STEP], y = f * q[(2 * r + 1) * STEP];
+        if (!isfinite(x) || !isfinite(y)) atomicOr(a.err, DEV_ERR_NONFINITE);
+        m.q_re[r * m.n + c] = x + 0.5 * m.p_re[r * m.n + c];
+        m.q_im[r * m.n + c] = y + 0.5 * m.p_im[r * m.n + c];
+    }
+}
+
+template <int RB>
+__global__ void __launch_bounds__(256) cols_reduce_kernel(ArgsSplit a, ColsArgs m)
+{
+    const int r = blockIdx.y;
+    const int64_t slot = blockIdx.x * (int64_t)256 + threadIdx.x;
+    if (slot >= a.npad) return;
+    const int c = a.perm[slot];
+    if (c < 0) return;
+    double x = 0, y = 0;
+    for (int64_t s = 0; s < m.splits; s++) {
+        const double2 v = m.partial[(s * RB + r) * a.npad + slot];
+        x += v.x;
+        y += v.y;
+    }
+    const double f = pow2d(a.expo[r]);
+    x *= f;
+    y *= f;
+    if (!isfinite(x) || !isfinite(y)) atomicOr(a.err, DEV_ERR_NONFINITE);
+    m.q_re[r * m.n + c] = x + 0.5 * m.p_re[r * m.n + c];
+    m.q_im[r * m.n + c] = y + 0.5 * m.p_im[r * m.n + c];
+}
+
 int sm_count()
 {
     int dev = 0, sms = 152;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     return sms;
+}
+
+// Shares of the source tiles: about three rounds of resident CTAs, so that the
+// last one is short, and at least four tiles each (the set-up of a CTA copies
+// the 64 KB table).
+int64_t cols_splits(int64_t tiles, int ctas)
+{
+    int64_t s = (3 * (int64_t)ctas + tiles - 1) / tiles;
+    if (s > tiles / 4) s = tiles / 4;
+    return s < 1 ? 1 : s;
+}
+
+template <int RB>
+size_t cols_bytes(int64_t npad, int64_t &splits)
+{
+    splits = cols_splits(npad / kTile32, kColsCtas<RB> * sm_count());
+    // densities, partial sums, block maxima and exponents
+    return (size_t)npad * RB * (sizeof(float4) + (size_t)(splits > 1 ? splits : 0) * sizeof(double2)) +
+           (RB * kExpBlocks + RB) * sizeof(int);
+}
+
+template <int RB>
+int launch_cols(const SweepConst &c, const RecSplit &v, const double4_32a *nrm, int nr, const double *p_re,
+                const double *p_im, double *q_re, double *q_im, void *scratch, cudaStream_t s)
+{
+    const int64_t tiles = v.npad / kTile32;
+    const int sms = sm_count();
+    ColsArgs m;
+    m.nr = nr;
+    m.n = c.n;
+    cols_bytes<RB>(v.npad, m.splits);
+    m.p_re = p_re;
+    m.p_im = p_im;
+    m.q_re = q_re;
+    m.q_im = q_im;
+    float4 *dens = static_cast<float4 *>(scratch);
+    m.partial = reinterpret_cast<double2 *>(dens + (int64_t)RB * v.npad);
+    int *expo = reinterpret_cast<int *>(m.partial + (m.splits > 1 ? m.splits : 0) * RB * v.npad), *part = expo + RB;
+    cols_max_kernel<<<dim3(kExpBlocks, (unsigned)nr), 256, 0, s>>>(c.n, nrm, p_re, p_im, part);
+    HZ_CHECK_LAUNCH();
+    int64_t b = (v.npad + 255) / 256;
+    if (b > 2 * sms) b = 2 * sms;
+    const double sg = (c.interior == 1) ? -1.0 : 1.0;
+    cols_dens_kernel<<<dim3((unsigned)b, RB), 256, 0, s>>>(c.n, v.npad, nr, v.perm, v.tpos, p_re, p_im,
+                                                           sg * c.wave * c.wave / (8.0 * kPiS), part, expo, dens);
+    HZ_CHECK_LAUNCH();
+    ArgsSplit a = {};
+    a.npad = v.npad;
+    a.wave = c.wave;
+    a.tau = c.tau;
+    a.ktau = (float)(c.wave * c.tau);
+    a.tau2 = (float)((c.wave * c.tau) * (c.wave * c.tau));
+    a.rec = v.rec;
+    a.densA = dens;
+    a.tile = v.tile;
+    a.table = v.table;
+    a.tpos = v.tpos;
+    a.nrm = nrm;
+    a.perm = v.perm;
+    a.expo = expo;
+    a.err = c.err;
+    auto kernel = c.dirichlet ? cols_kernel<RB, true> : cols_kernel<RB, false>;
+    HZ_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kColsSmem<RB>));
+    kernel<<<dim3((unsigned)tiles, (unsigned)m.splits), kTile32, kColsSmem<RB>, s>>>(a, m);
+    HZ_CHECK_LAUNCH();
+    if (m.splits > 1) {
+        cols_reduce_kernel<RB><<<dim3((unsigned)tiles, (unsigned)nr), 256, 0, s>>>(a, m);
+        HZ_CHECK_LAUNCH();
+    }
+    return HZ_OK;
 }
 
 template <int MODE, bool DIR>
@@ -695,6 +1018,22 @@ int sweep_split(const SweepConst &c, const RecSplit &v, const double4_32a *nrm, 
     HZ_TRY(rc);
     if (ev1) HZ_CHECK_CUDA(record_timing_event(ev1, s));
     return HZ_OK;
+}
+
+size_t split_cols_scratch_bytes(int64_t npad, int nr)
+{
+    int64_t splits;
+    return nr <= 4 ? cols_bytes<4>(npad, splits) : nr <= 8 ? cols_bytes<8>(npad, splits) : cols_bytes<16>(npad, splits);
+}
+
+// One pass over nr <= 16 columns ([nr][n]); scratch of split_cols_scratch_bytes.
+int sweep_split_cols(const SweepConst &c, const RecSplit &v, const double4_32a *nrm, int nr, const double *p_re,
+                     const double *p_im, double *q_re, double *q_im, void *scratch, cudaStream_t s)
+{
+    static_assert(kColsMax == 16, "the multi right-hand-side sweep's FP64 block");
+    if (nr <= 4) return launch_cols<4>(c, v, nrm, nr, p_re, p_im, q_re, q_im, scratch, s);
+    if (nr <= 8) return launch_cols<8>(c, v, nrm, nr, p_re, p_im, q_re, q_im, scratch, s);
+    return launch_cols<16>(c, v, nrm, nr, p_re, p_im, q_re, q_im, scratch, s);
 }
 
 HZ_DEFINE_WAIT_LIMIT_SETTER(set_wait_limit_split)

@@ -88,3 +88,23 @@ def test_nonfinite_density_and_short_waits(hz):
         finally:
             hz.set_wait_limit(-1)
         assert np.array_equal(op.matvec(v), want)
+
+
+@pytest.mark.parametrize("nrhs", [1, 4, 5, 8, 9, 16, 19])
+def test_columns_equal_single_products(hz, nrhs):
+    """Blocks of 4, 8 and 16 columns, their remainders and a zero column: the
+    same entries as the single product, summed in another order."""
+    from helmholtz_3d_torrone_gb300 import geometry as G
+    for dirichlet in (0, 1):
+        p = hz.params(24, 6.0, int_l=-1.0, int_u=1.0, factor=3.0, dirichlet=dirichlet)
+        with hz.Operator(p) as op:
+            op.set_distance(G.sphere(24, radius=0.5, center=(0.011, 0.017, 0.005)))
+            n = op.build()
+            rng = np.random.default_rng(nrhs)
+            V = rng.standard_normal((nrhs, n)) + 1j * rng.standard_normal((nrhs, n))
+            V *= 10.0 ** rng.integers(-20, 20, nrhs)[:, None]
+            V[nrhs // 2] = 0.0
+            Q = op.matvec_multi(V, precision=hz.PREC_F64)
+            for v, q in zip(V, Q):
+                # a row's sum |A_ts p_s| is below 4 max |p| on this sphere
+                assert np.max(np.abs(q - op.matvec(v))) <= BOUND * 4 * np.max(np.abs(v))
