@@ -1390,8 +1390,12 @@ int hz_misfit_gradient(hz_operator *op, const hz_solve_opts *opts_in, const doub
     // k-derivatives: (dE/dk) sigma at the receivers, (dA/dk) sigma over the tube
     HZ_TRY(launch_eval_dk(n, op->pos64.as<double4_32a>(), op->nrm64.as<double4_32a>(), sg0, sg1, m, R, op->p.wave,
                           op->tau, op->p.interior, layer, Q0, Q1, s));
-    HZ_TRY(launch_sweep_dk(n, op->pos64.as<double4_32a>(), op->nrm64.as<double4_32a>(), op->dreg.as<double>(), sg0,
-                           sg1, op->p.wave, op->tau, op->p.interior, op->p.dirichlet, d0, d1, s));
+    if (op->use_split)
+        HZ_TRY(sweep_split_dk(sweep_const(op), op->split, op->nrm64.as<double4_32a>(), op->dreg.as<double>(), sg0, sg1,
+                              d0, d1, s));
+    else
+        HZ_TRY(launch_sweep_dk(n, op->pos64.as<double4_32a>(), op->nrm64.as<double4_32a>(), op->dreg.as<double>(), sg0,
+                               sg1, op->p.wave, op->tau, op->p.interior, op->p.dirichlet, d0, d1, s));
     // host side of the small reductions
     std::vector<double> hr0(m), hr1(m), hq0(m), hq1(m);
     HZ_CHECK_CUDA(cudaMemcpyAsync(hr0.data(), E0, m * sizeof(double), cudaMemcpyDeviceToHost, s));

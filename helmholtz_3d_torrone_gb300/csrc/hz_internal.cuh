@@ -239,6 +239,17 @@ int build_split_records(const SweepConst &c, const RecSplit &v, const Rec32 &r, 
 int sweep_split(const SweepConst &c, const RecSplit &v, const double4_32a *nrm, int mode, const double *p_re,
                 const double *p_im, const double *pt_re, const double *pt_im, double *q_re, double *q_im,
                 double *qt_re, double *qt_im, cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1);
+inline int sm_count()
+{
+    int dev = 0, sms = 152;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
+// q = (dA/dk) p where the split sweep serves (dreg = d reg / dk per tube point).
+int sweep_split_dk(const SweepConst &c, const RecSplit &v, const double4_32a *nrm, const double *dreg,
+                   const double *p_re, const double *p_im, double *q_re, double *q_im, cudaStream_t s);
 size_t split_cols_scratch_bytes(int64_t npad, int nr);
 int sweep_split_cols(const SweepConst &c, const RecSplit &v, const double4_32a *nrm, int nr, const double *p_re,
                      const double *p_im, double *q_re, double *q_im, void *scratch, cudaStream_t s);

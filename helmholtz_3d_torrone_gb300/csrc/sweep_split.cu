@@ -27,6 +27,9 @@ constexpr int kRun = 16;         // sources per 48-bit sum
 constexpr int kRecs = 6;         // float4 of fixed record per source
 constexpr int kExpBlocks = 152;  // blocks of the density maximum
 
+// MODE bit beside SWEEP_A: the k-derivative of A's entries.
+constexpr int SPLIT_DK = 8;
+
 struct ArgsSplit {
     int64_t npad, units;
     int64_t nctas;
@@ -43,6 +46,8 @@ struct ArgsSplit {
     const double *p_re, *p_im, *pt_re, *pt_im;
     double *q_re, *q_im, *qt_re, *qt_im;
     double4_32a *partial;       // [nctas][2][256]
+    const double *dreg;         // SPLIT_DK: d reg / dk in tube order, times dreg_scale
+    double dreg_scale;
     unsigned *err;
 };
 
@@ -236,6 +241,7 @@ __device__ __forceinline__ void split_entry(const ArgsSplit &a, const float4 (*s
     constexpr bool A = (MODE & SWEEP_A) != 0, H = (MODE & SWEEP_AH) != 0;
     constexpr bool SRC = (A && DIR) || (H && !DIR);  // (x_t - x_s).n_s wanted
     constexpr bool TGT = (A && !DIR) || (H && DIR);  // (x_t - x_s).n_t wanted
+    constexpr bool DK = (MODE & SPLIT_DK) != 0;      // the factor is e^{i theta} y alone
     const float4 r0 = st[0][j], r1 = st[1][j], r2_ = st[2][j], r3 = st[3][j];
     const int s0 = __float_as_int(r0.x), s1 = __float_as_int(r0.y), s2 = __float_as_int(r0.z);
     long long W = ((((long long)__float_as_int(r1.w) << 32) | (unsigned)__float_as_int(r1.z)) >> u.shS) + 128;
@@ -268,8 +274,15 @@ __device__ __forceinline__ void split_entry(const ArgsSplit &a, const float4 (*s
     split_root(r2, rho, y);
     th = CLOSE ? rho : split_phase_offset(w, rho, t.rc);
     split_sincos(th, tab, c, s);
-    split_kernel(y, c, s, ur, ui);
-    const FF y2 = ff_mul(y, y);
+    FF y2;
+    if (DK) {
+        ur = c;
+        ui = s;
+        y2 = y;
+    } else {
+        split_kernel(y, c, s, ur, ui);
+        y2 = ff_mul(y, y);
+    }
     FF vsr, vsi, vtr, vti;
     if (SRC) {
         const float4 r4 = st[4][j], r5 = st[5][j];
@@ -306,6 +319,12 @@ __device__ __forceinline__ void split_entry(const ArgsSplit &a, const float4 (*s
     hr = DIR ? vtr : vsr;
     hi = DIR ? vti : vsi;
     if (CLOSE && !far) {
+        if (DK) {
+            const int q = a.perm[DIR ? sslot : tslot];
+            ar = ai = {0.f, 0.f};
+            if (q >= 0) ar = ff_of_double(a.dreg[q] * a.dreg_scale);
+            return;
+        }
         const float4 r5 = st[5][j];
         const FF srg = {r5.z, r5.w};
         ar = ff_neg(DIR ? srg : treg);
@@ -457,9 +476,9 @@ __device__ __forceinline__ void split_write(const ArgsSplit &a, int64_t s, doubl
     if (c < 0) return;
     if (MODE & SWEEP_A) {
         const double f = pow2d(a.expo[0]), r = f * ar, i = f * ai;
-        if (!isfinite(r) || !isfinite(i)) atomicOr(a.err, DEV_ERR_NONFINITE);
-        a.q_re[c] = r + 0.5 * a.p_re[c];
-        a.q_im[c] = i + 0.5 * a.p_im[c];
+        if (!(MODE & SPLIT_DK) && (!isfinite(r) || !isfinite(i))) atomicOr(a.err, DEV_ERR_NONFINITE);
+        a.q_re[c] = (MODE & SPLIT_DK) ? r : r + 0.5 * a.p_re[c];
+        a.q_im[c] = (MODE & SPLIT_DK) ? i : i + 0.5 * a.p_im[c];
     }
     if (MODE & SWEEP_AH) {
         const double f = pow2d(a.expo[1]), w = a.tpos[s].w, r = f * (w * hr), i = f * (w * hi);
@@ -814,14 +833,6 @@ __global__ void __launch_bounds__(256) cols_reduce_kernel(ArgsSplit a, ColsArgs 
     m.q_im[r * m.n + c] = y + 0.5 * m.p_im[r * m.n + c];
 }
 
-int sm_count()
-{
-    int dev = 0, sms = 152;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms;
-}
-
 // Shares of the source tiles: about three rounds of resident CTAs, so that the
 // last one is short, and at least four tiles each (the set-up of a CTA copies
 // the 64 KB table).
@@ -840,6 +851,8 @@ size_t cols_bytes(int64_t npad, int64_t &splits)
     return (size_t)npad * RB * (sizeof(float4) + (size_t)(splits > 1 ? splits : 0) * sizeof(double2)) +
            (RB * kExpBlocks + RB) * sizeof(int);
 }
+
+ArgsSplit split_args(const SweepConst &c, const RecSplit &v, const double4_32a *nrm);
 
 template <int RB>
 int launch_cols(const SweepConst &c, const RecSplit &v, const double4_32a *nrm, int nr, const double *p_re,
@@ -866,21 +879,9 @@ int launch_cols(const SweepConst &c, const RecSplit &v, const double4_32a *nrm, 
     cols_dens_kernel<<<dim3((unsigned)b, RB), 256, 0, s>>>(c.n, v.npad, nr, v.perm, v.tpos, p_re, p_im,
                                                            sg * c.wave * c.wave / (8.0 * kPiS), part, expo, dens);
     HZ_CHECK_LAUNCH();
-    ArgsSplit a = {};
-    a.npad = v.npad;
-    a.wave = c.wave;
-    a.tau = c.tau;
-    a.ktau = (float)(c.wave * c.tau);
-    a.tau2 = (float)((c.wave * c.tau) * (c.wave * c.tau));
-    a.rec = v.rec;
+    ArgsSplit a = split_args(c, v, nrm);
     a.densA = dens;
-    a.tile = v.tile;
-    a.table = v.table;
-    a.tpos = v.tpos;
-    a.nrm = nrm;
-    a.perm = v.perm;
     a.expo = expo;
-    a.err = c.err;
     auto kernel = c.dirichlet ? cols_kernel<RB, true> : cols_kernel<RB, false>;
     HZ_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kColsSmem<RB>));
     kernel<<<dim3((unsigned)tiles, (unsigned)m.splits), kTile32, kColsSmem<RB>, s>>>(a, m);
@@ -967,28 +968,28 @@ int build_split_records(const SweepConst &c, const RecSplit &v, const Rec32 &r, 
     return HZ_OK;
 }
 
-int sweep_split(const SweepConst &c, const RecSplit &v, const double4_32a *nrm, int mode, const double *p_re,
-                const double *p_im, const double *pt_re, const double *pt_im, double *q_re, double *q_im,
-                double *qt_re, double *qt_im, cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1)
+namespace {
+
+// Densities of one product: scale as in split_dens_kernel.
+int split_densities(const SweepConst &c, const RecSplit &v, const double4_32a *nrm, const double *pr, const double *pi,
+                    const double *tr, const double *ti, double scale, cudaStream_t s)
 {
-    const bool useA = (mode & SWEEP_A) != 0, useH = (mode & SWEEP_AH) != 0;
-    const double sg = (c.interior == 1) ? -1.0 : 1.0;
-    const double *pr = useA ? p_re : nullptr, *pi = useA ? p_im : nullptr;
-    const double *tr = useH ? pt_re : nullptr, *ti = useH ? pt_im : nullptr;
-    int *part = v.expo + 8;
+    int *part = v.expo + 8;  // kExpBlocks maxima each
     split_max_kernel<<<kExpBlocks, 256, 0, s>>>(c.n, nrm, pr, pi, tr, ti, part);
     HZ_CHECK_LAUNCH();
     int64_t b = (v.npad + 255) / 256;
     const int64_t cap = 8 * (int64_t)sm_count();
     if (b > cap) b = cap;
-    split_dens_kernel<<<(unsigned)b, 256, 0, s>>>(v.npad, v.perm, v.tpos, pr, pi, tr, ti,
-                                                  sg * c.wave * c.wave / (8.0 * kPiS), part, v.expo, v.dens,
+    split_dens_kernel<<<(unsigned)b, 256, 0, s>>>(v.npad, v.perm, v.tpos, pr, pi, tr, ti, scale, part, v.expo, v.dens,
                                                   v.dens + v.npad);
     HZ_CHECK_LAUNCH();
-    ArgsSplit a;
+    return HZ_OK;
+}
+
+ArgsSplit split_args(const SweepConst &c, const RecSplit &v, const double4_32a *nrm)
+{
+    ArgsSplit a = {};
     a.npad = v.npad;
-    a.units = 0;
-    a.nctas = 0;
     a.wave = c.wave;
     a.tau = c.tau;
     a.ktau = (float)(c.wave * c.tau);
@@ -1002,22 +1003,51 @@ int sweep_split(const SweepConst &c, const RecSplit &v, const double4_32a *nrm, 
     a.nrm = nrm;
     a.perm = v.perm;
     a.expo = v.expo;
-    a.p_re = p_re; a.p_im = p_im; a.pt_re = pt_re; a.pt_im = pt_im;
-    a.q_re = q_re; a.q_im = q_im; a.qt_re = qt_re; a.qt_im = qt_im;
     a.partial = v.partial;
     a.err = c.err;
+    return a;
+}
+
+}  // namespace
+
+int sweep_split(const SweepConst &c, const RecSplit &v, const double4_32a *nrm, int mode, const double *p_re,
+                const double *p_im, const double *pt_re, const double *pt_im, double *q_re, double *q_im,
+                double *qt_re, double *qt_im, cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1)
+{
+    const bool useA = (mode & SWEEP_A) != 0, useH = (mode & SWEEP_AH) != 0;
+    const double sg = (c.interior == 1) ? -1.0 : 1.0;
+    HZ_TRY(split_densities(c, v, nrm, useA ? p_re : nullptr, useA ? p_im : nullptr, useH ? pt_re : nullptr,
+                           useH ? pt_im : nullptr, sg * c.wave * c.wave / (8.0 * kPiS), s));
+    ArgsSplit a = split_args(c, v, nrm);
+    a.p_re = p_re; a.p_im = p_im; a.pt_re = pt_re; a.pt_im = pt_im;
+    a.q_re = q_re; a.q_im = q_im; a.qt_re = qt_re; a.qt_im = qt_im;
     if (ev0) HZ_CHECK_CUDA(record_timing_event(ev0, s));
     const bool dir = c.dirichlet != 0;
-    int rc;
+    const size_t pb = v.partial_bytes;
     if (mode == SWEEP_PAIR)
-        rc = dir ? launch_split<SWEEP_PAIR, true>(a, v.partial_bytes, s) : launch_split<SWEEP_PAIR, false>(a, v.partial_bytes, s);
+        HZ_TRY((dir ? launch_split<SWEEP_PAIR, true>(a, pb, s) : launch_split<SWEEP_PAIR, false>(a, pb, s)));
     else if (mode == SWEEP_A)
-        rc = dir ? launch_split<SWEEP_A, true>(a, v.partial_bytes, s) : launch_split<SWEEP_A, false>(a, v.partial_bytes, s);
+        HZ_TRY((dir ? launch_split<SWEEP_A, true>(a, pb, s) : launch_split<SWEEP_A, false>(a, pb, s)));
     else
-        rc = dir ? launch_split<SWEEP_AH, true>(a, v.partial_bytes, s) : launch_split<SWEEP_AH, false>(a, v.partial_bytes, s);
-    HZ_TRY(rc);
+        HZ_TRY((dir ? launch_split<SWEEP_AH, true>(a, pb, s) : launch_split<SWEEP_AH, false>(a, pb, s)));
     if (ev1) HZ_CHECK_CUDA(record_timing_event(ev1, s));
     return HZ_OK;
+}
+
+// q = (dA/dk) p: far entries -(k / 4 pi) e^{i k rho} (x_t - x_s).n / rho w_s sg,
+// near ones w_s dreg (FP64 sincos per pair, one target a thread: 26.2 ms at
+// n = 9,542; here 0.9).
+int sweep_split_dk(const SweepConst &c, const RecSplit &v, const double4_32a *nrm, const double *dreg,
+                   const double *p_re, const double *p_im, double *q_re, double *q_im, cudaStream_t s)
+{
+    const double sg = (c.interior == 1) ? -1.0 : 1.0;
+    HZ_TRY(split_densities(c, v, nrm, p_re, p_im, nullptr, nullptr, -sg * c.wave / (8.0 * kPiS), s));
+    ArgsSplit a = split_args(c, v, nrm);
+    a.dreg = dreg;
+    a.dreg_scale = sg * 8.0 * kPiS / c.wave;
+    a.p_re = p_re; a.p_im = p_im; a.q_re = q_re; a.q_im = q_im;
+    constexpr int M = SWEEP_A | SPLIT_DK;
+    return c.dirichlet ? launch_split<M, true>(a, v.partial_bytes, s) : launch_split<M, false>(a, v.partial_bytes, s);
 }
 
 size_t split_cols_scratch_bytes(int64_t npad, int nr)

@@ -108,3 +108,28 @@ def test_columns_equal_single_products(hz, nrhs):
             for v, q in zip(V, Q):
                 # a row's sum |A_ts p_s| is below 4 max |p| on this sphere
                 assert np.max(np.abs(q - op.matvec(v))) <= BOUND * 4 * np.max(np.abs(v))
+
+
+def test_wave_number_gradient(hz):
+    """dJ/dk where dA/dk runs in split arithmetic, against central differences
+    (their truncation and the solver's tolerance: 1e-5)."""
+    from helmholtz_3d_torrone_gb300 import geometry as G
+    k, N = 6.0, 24
+    rng = np.random.default_rng(5)
+    rx = G.random_sphere_points(7, 0.9, seed=6)
+    target = rng.standard_normal(7) + 1j * rng.standard_normal(7)
+
+    def misfit(kk, dirichlet):
+        p = hz.params(N, kk, int_l=-1.0, int_u=1.0, factor=3.0, dirichlet=dirichlet)
+        with hz.Operator(p) as op:
+            op.set_distance(G.sphere(N, radius=0.5, center=(0.011, 0.017, 0.005)))
+            n = op.build()
+            assert n >= 2048
+            b = np.exp(1j * np.arange(n) / n)
+            J, _, dk, _, _ = op.misfit_gradient(b, rx, target, method=hz.BICG, precision=hz.PREC_F64, tol=1e-13)
+            return J, dk
+
+    for dirichlet in (0, 1):
+        h = 1e-5
+        fd = (misfit(k + h, dirichlet)[0] - misfit(k - h, dirichlet)[0]) / (2 * h)
+        assert abs(misfit(k, dirichlet)[1] - fd) <= 1e-5 * abs(fd)
