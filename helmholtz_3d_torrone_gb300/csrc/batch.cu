@@ -34,12 +34,12 @@ struct hz_batch {
     cudaStream_t stream = nullptr;
     int shape = 1;  // FP32 batch sweep shape (hz_batch_autotune)
     DevBuf desc;    // kBatchShapes descriptor arrays
-    int64_t units[kBatchShapes] = {}, blocks[kBatchShapes] = {};
+    int64_t units[kBatchShapes] = {};
     std::vector<Batch32Item> items;
     // the FP32 launch over a subset of the operators (sub_n > 0)
     DevBuf desc_sub;
     int sub_n = 0, sub_shape = -1;
-    int64_t sub_units = 0, sub_blocks = 0;
+    int64_t sub_units = 0;
     uint64_t sub_gen = 0;
     DevBuf partial;
     size_t partial_bytes = 0;
@@ -67,12 +67,11 @@ struct BatchF32 final : MultiOp {
     {
         (void)R;
         if (sub && b->sub_shape == b->shape)
-            return sweep_f32_batch(b->shape, b->desc_sub.ptr, b->sub_n, b->R, b->sub_units, b->sub_blocks,
-                                   b->partial.as<double4_32a>(), b->partial_bytes, p_re, p_im, q_re, q_im, b->nmax,
+            return sweep_f32_batch(b->shape, b->desc_sub.ptr, b->sub_n, b->R, b->sub_units, b->partial.as<double4_32a>(), b->partial_bytes, p_re, p_im, q_re, q_im, b->nmax,
                                    b->max_npad, s, nullptr, nullptr);
         const size_t db = batch32_desc_bytes(b->R);
         return sweep_f32_batch(b->shape, b->desc.as<char>() + (size_t)b->shape * db, b->R, b->R, b->units[b->shape],
-                               b->blocks[b->shape], b->partial.as<double4_32a>(), b->partial_bytes, p_re, p_im, q_re,
+                               b->partial.as<double4_32a>(), b->partial_bytes, p_re, p_im, q_re,
                                q_im, b->nmax, b->max_npad, s, nullptr, nullptr);
     }
     uint64_t key() const override
@@ -89,8 +88,8 @@ struct BatchF32 final : MultiOp {
         sub = false;
         b->sub_n = 0;
         b->sub_shape = -1;
-        HZ_TRY(batch32_describe(b->items.data(), (int)cols.size(), b->shape, b->desc_sub.ptr, b->sub_units,
-                                b->sub_blocks, s, cols.data()));
+        HZ_TRY(batch32_describe(b->items.data(), (int)cols.size(), b->shape, b->desc_sub.ptr, b->sub_units, s,
+                                cols.data()));
         b->sub_n = (int)cols.size();
         b->sub_shape = b->shape;
         b->sub_gen++;
@@ -242,8 +241,7 @@ int hz_batch_create(hz_operator *const *ops, int count, hz_batch **out)
         items[r].dens = op->dens32.as<float>();
     }
     for (int k = 0; k < kBatchShapes && rc == HZ_OK; k++)
-        rc = batch32_describe(items.data(), count, k, b->desc.as<char>() + (size_t)k * db, b->units[k], b->blocks[k],
-                              b->stream);
+        rc = batch32_describe(items.data(), count, k, b->desc.as<char>() + (size_t)k * db, b->units[k], b->stream);
     if (rc == HZ_OK) {
         b->partial_bytes = batch32_partial_bytes();
         rc = b->partial.ensure(b->partial_bytes);
@@ -277,8 +275,7 @@ int hz_batch_autotune(hz_batch *b, int *chosen, double *ms_per_sweep)
     for (int k = 0; k < kBatchShapes && rc == HZ_OK; k++) {
         float ms_min = 1e30f;
         for (int rep = 0; rep < 2 && rc == HZ_OK; rep++) {
-            rc = sweep_f32_batch(k, b->desc.as<char>() + (size_t)k * db, b->R, b->R, b->units[k], b->blocks[k],
-                                 b->partial.as<double4_32a>(), b->partial_bytes, v, v + tot, v + 2 * tot, v + 3 * tot,
+            rc = sweep_f32_batch(k, b->desc.as<char>() + (size_t)k * db, b->R, b->R, b->units[k], b->partial.as<double4_32a>(), b->partial_bytes, v, v + tot, v + 2 * tot, v + 3 * tot,
                                  b->nmax, b->max_npad, s, e0, e1);
             if (rc == HZ_OK && cudaEventSynchronize(e1) == cudaSuccess) {
                 float ms = 0.f;

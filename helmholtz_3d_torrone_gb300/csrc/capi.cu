@@ -367,7 +367,8 @@ static int build_records32(hz_operator *op, double lambda, double reg_scale)
         op->r32.mwords = (ntiles + 31) / 32;
         HZ_TRY(op->origin32.ensure(ntiles * sizeof(double4_32a)));
         HZ_TRY(op->split32.ensure((2 * npad + 2 * ntiles) * sizeof(float4)));
-        HZ_TRY(op->nearmask32.ensure(ntiles * op->r32.mwords * sizeof(uint32_t)));
+        // the sweep's partition, and after it the near-tile mask
+        HZ_TRY(op->nearmask32.ensure(cuts32_bytes(ntiles) + ntiles * op->r32.mwords * sizeof(uint32_t)));
         HZ_TRY(op->soa32.ensure(npad * kFixed32 * sizeof(float)));
         HZ_TRY(op->dens32.ensure(npad * 6 * sizeof(float)));  // split re, im, -im of both densities
         HZ_TRY(sweep_order(N, n, op->idx.as<int64_t>(), op->perm.as<int>(), npad, op->scratch, s));
@@ -385,7 +386,8 @@ static int build_records32(hz_operator *op, double lambda, double reg_scale)
         op->r32.tlo = sp ? sp + npad : nullptr;
         op->r32.ohi = sp ? sp + 2 * npad : nullptr;
         op->r32.olo = sp ? sp + 2 * npad + ntiles : nullptr;
-        op->r32.nearmask = op->nearmask32.as<uint32_t>();
+        op->r32.nearmask =
+            sp ? reinterpret_cast<uint32_t *>(op->nearmask32.as<char>() + cuts32_bytes(ntiles)) : nullptr;
     }
     if (npad > 0) {
         const size_t pb = sweep32_partial_bytes();
@@ -396,6 +398,8 @@ static int build_records32(hz_operator *op, double lambda, double reg_scale)
     if (npad > 0)
         HZ_TRY(build_rec32(op->r32, op->pos64.as<double4_32a>(), op->nrm64.as<double4_32a>(),
                            reg_scale, op->tau, s));
+    op->r32.cuts = nullptr;
+    if (npad > 0 && !op->combo) HZ_TRY(build_cuts32(op->r32, op->nearmask32.ptr, s));
     return HZ_OK;
 }
 

@@ -129,6 +129,9 @@ struct Rec32 {
     uint32_t *nearmask;      // [target tile][mwords]: bit s set unless source tile s is
                              // farther than tau from every point of the target tile
     int64_t mwords;          // 32-bit words per mask row: ceil(tiles / 32)
+    int64_t *cuts = nullptr; // partition of the FP32 sweep at equal costs (build_cuts32), row costs,
+    int64_t *rows = nullptr; // and per target block the units summed so far
+    unsigned *done = nullptr;
     double4_32a *partial;    // stream-K scratch: pieces of target blocks split between CTAs
     size_t partial_bytes;
 };
@@ -283,15 +286,17 @@ struct Batch32Item {
 size_t batch32_desc_bytes(int R);
 // Describes nops operators: items[cols[i]] owning column cols[i] (cols NULL:
 // items[i], column i).
-int batch32_describe(const Batch32Item *items, int nops, int cfg, void *desc_dev, int64_t &units, int64_t &blocks,
-                     cudaStream_t s, const int *cols = nullptr);
+int batch32_describe(const Batch32Item *items, int nops, int cfg, void *desc_dev, int64_t &units, cudaStream_t s,
+                     const int *cols = nullptr);
 size_t batch32_partial_bytes();
 // Columns of described operators get their product; every column's padded
 // tail (and every column of an operator not described) is zeroed.
-int sweep_f32_batch(int cfg, const void *desc_dev, int nops, int ncols, int64_t units, int64_t blocks,
-                    double4_32a *partial, size_t partial_bytes, const double *p_re, const double *p_im,
+int sweep_f32_batch(int cfg, const void *desc_dev, int nops, int ncols, int64_t units, double4_32a *partial, size_t partial_bytes, const double *p_re, const double *p_im,
                     double *q_re, double *q_im, int64_t stride, int64_t max_npad, cudaStream_t s, cudaEvent_t ev0,
                     cudaEvent_t ev1);
+// Partition of the FP32 sweep, from the near-tile mask (sets r.cuts, rows, done).
+size_t cuts32_bytes(int64_t ntiles);
+int build_cuts32(Rec32 &r, void *mem, cudaStream_t s);
 // bytes of stream-K scratch that every FP32 sweep variant fits in
 size_t sweep32_partial_bytes();
 // FP32 products of the Combo formulation (sweep_combo32.cu) on the blocked

@@ -38,9 +38,11 @@
 // targets per thread come from a small table of compiled variants; the
 // autotuner times them on the operator's own data.
 //
-// One A p on GB300, before (scalar, phase reduced per pair) and now: n = 19,532
-// 0.603 -> 0.429 ms, n = 36,212 1.90 -> 1.31, n = 145,272 28.5 -> 18.1,
-// n = 581,420 365 -> 257 (1,318 Gpair/s).
+// One A p on GB300, first scalar with the phase reduced per pair, then packed
+// and centred, then with units of equal cost and near tiles centred as well:
+// n = 2,938 0.040 (packed) -> 0.037 ms, 9,765 0.149 -> 0.120, 19,532 0.603 ->
+// 0.429 -> 0.383, 36,212 1.90 -> 1.31 -> 1.18, 145,272 28.5 -> 18.1 -> 17.7,
+// 581,420 365 -> 257 -> 258 (1,307 Gpair/s).
 #include "hz_internal.cuh"
 #include "bulk_copy.cuh"
 #include "pair32.cuh"
@@ -64,6 +66,7 @@ struct Args32 {
     float tau2, guard_lo, guard_hi;  // (lambda tau)^2 and the tie band around it
     double tau;
     int scaled;  // lambda = k (batches: per operator)
+    int sub;     // units of a tile
     const float4 *pos, *nrm;
     const float *soa;   // [tiles][kFixed][kTile32]: -x, -y, -z (tile-local), n, reg
     float *dens;        // [tiles][6][kTile32]: re, im, -im of w p and of pt
@@ -75,10 +78,11 @@ struct Args32 {
     const double *p_re, *p_im, *pt_re, *pt_im;
     double *q_re, *q_im, *qt_re, *qt_im;
     unsigned *err;
-    // stream-K partition: CTA c takes work units [c U / P, (c+1) U / P) of
-    // the U = blocks x tiles (target block, source tile) units
-    int64_t units;
-    int64_t nctas;
+    // stream-K partition: CTA c takes the units [cta_begin(c), cta_begin(c + 1))
+    // of the blocks x tiles x sub (target block, part of a source tile) ones
+    const int64_t *cuts;   // units at equal costs (build_cuts32); NULL: a CTA takes a block
+    unsigned *done;        // per target block: units whose sums lie in partial
+    int nctas;
     double4_32a *partial;  // [P][2][slots per block]: (A re, A im, A^H re, A^H im)
 };
 
@@ -88,11 +92,39 @@ constexpr int kDens = 3 * ((MODE & SWEEP_PAIR) == SWEEP_PAIR ? 2 : 1);
 template <int MODE>
 constexpr int kStage = (kFixed + kDens<MODE>) * kTile32;  // floats of a staged tile
 
-// The CTA whose unit range holds work unit u: the largest c with
-// floor(c U / P) <= u.
-__device__ __forceinline__ int64_t cta_of_unit(int64_t u, int64_t units, int64_t nctas)
+// A tile counts `sub` units, and the FP32 sums over a unit are added to the
+// cross-tile sums one by one: a product does not depend on where the units are
+// cut.  Whole tiles are the cheapest (a unit's end costs 2 % of a half), but
+// small tubes need parts for every CTA to have its share: n = 2,938 0.042 ms
+// with tiles, 0.039 with halves, 0.037 with quarters; n = 9,765 0.123 and
+// 0.120 with halves; n = 145,272 17.5 with tiles, 17.9 with halves.
+constexpr int kRun32 = 64;  // sources of the smallest unit
+int sub_of(int64_t ntiles) { return ntiles < 24 ? 4 : ntiles < 80 ? 2 : 1; }
+
+// Relative cost of a tile: far, near tile (near-field test, its branch
+// taken now and then), the target tile itself (taken for most sources).
+constexpr int kCostFar = 16, kCostNear = 19, kCostSelf = 30;
+constexpr int kCuts = 16384;  // equal-cost cuts kept per tube: 27 or more a CTA
+
+// First unit of CTA c of P.  Cut by count, the CTAs with the near tiles set
+// the time: 0.149 ms at n = 9,765 and 1.30 at n = 36,212, of which 0.03 and
+// 0.2 were the others' waiting.
+__device__ __forceinline__ int64_t cta_begin(const Args32 &a, int c)
 {
-    return ((u + 1) * nctas - 1) / units;
+    if (!a.cuts) return (int64_t)c * (a.npad / kTile32) * a.sub;
+    return __ldg(a.cuts + (unsigned)c * (unsigned)kCuts / (unsigned)a.nctas);
+}
+
+// Largest c with cta_begin(c) <= u (all threads of a block take part).
+template <class Begin>
+__device__ __forceinline__ int cta_of_unit(int64_t u, int nctas, const Begin &begin)
+{
+    int count = 0;
+    for (int c0 = 0; c0 < nctas; c0 += blockDim.x) {
+        const int c = c0 + (int)threadIdx.x;
+        count += __syncthreads_count(c < nctas && begin(c) <= u);
+    }
+    return count - 1;
 }
 
 // Densities of slot s, scale (w p, pt) in FP32, scale = lambda^2 sg / (4 pi).
@@ -107,8 +139,10 @@ __device__ __forceinline__ void store_dens(float *dens, int64_t s, int half, flo
 __global__ void prep32_kernel(int64_t npad, const int *__restrict__ perm, const double4_32a *__restrict__ tpos,
                               const double *__restrict__ p_re, const double *__restrict__ p_im,
                               const double *__restrict__ pt_re, const double *__restrict__ pt_im, double scale,
-                              float *__restrict__ dens)
+                              float *__restrict__ dens, unsigned *__restrict__ done)
 {
+    if (blockIdx.x == 0)
+        for (int64_t b = threadIdx.x; b < npad / kTile32; b += blockDim.x) done[b] = 0;
     for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < npad; s += (int64_t)gridDim.x * blockDim.x) {
         const int c = perm[s];
         const double ws = (c >= 0) ? tpos[s].w * scale : 0.0;
@@ -184,14 +218,19 @@ __device__ __forceinline__ void pair_scalar(const Args32 &a, const float *st, in
     }
 }
 
-// A whole tile, two sources at a time in packed FP32: phase centred, or (SLOW:
-// near and wide tiles) reduced per pair and with the near-field test.  With y = 1/rho, e^{i theta} = C + i S and q the projection
-// over rho^2, A's entry times d is q (-(S e1 + C e2) + i (C e1 - S e2)),
-// e1 = dr - y di, e2 = di + y dr (A^H: conj(d) and the real part's sign), so
-// that no operand needs a negation (-im is staged).  A near pair takes C = 1,
-// S = 0 and e1, e2 from its regularisation factor.
-template <int MODE, bool DIR, int NT, int TG, bool SLOW>
-__device__ __forceinline__ void tile_packed(const Args32 &a, const float *st, const float3 (&rel)[TG],
+// How a tile is summed: phase centred, the same with the near-field test, or
+// (tiles wider than kCentreRadius) phase reduced per pair and the test.
+enum { TILE_FAR = 0, TILE_NEAR = 1, TILE_WIDE = 2 };
+
+// A unit of a tile, two sources at a time in packed FP32.  With y = 1/rho,
+// e^{i theta} = C + i S and q the projection over rho^2, A's entry times d is
+// q (-(S e1 + C e2) + i (C e1 - S e2)), e1 = dr - y di, e2 = di + y dr (A^H:
+// conj(d) and the real part's sign), so that no operand needs a negation (-im
+// is staged).  Near pairs add their regularisation factor times d to sums of
+// their own (they take no phase) and go on at rho^2 = 1e16, where the rest of
+// the loop adds 1e-16 of the entry's scale.
+template <int MODE, bool DIR, int NT, int TG, int KIND>
+__device__ __forceinline__ void unit_packed(const Args32 &a, const float *st, int j0, int j1, const float3 (&rel)[TG],
                                             const Targets<TG> &t, const Turn (&turn)[TG], int64_t tslot0,
                                             int64_t sslot0, float (&fAr)[TG], float (&fAi)[TG], float (&fHr)[TG],
                                             float (&fHi)[TG])
@@ -206,111 +245,139 @@ __device__ __forceinline__ void tile_packed(const Args32 &a, const float *st, co
         rx[g] = f2_pack(rel[g].x, rel[g].x);
         ry[g] = f2_pack(rel[g].y, rel[g].y);
         rz[g] = f2_pack(rel[g].z, rel[g].z);
-        if (!SLOW) nrc[g] = f2_pack(-turn[g].rc, -turn[g].rc);
+        if (KIND != TILE_WIDE) nrc[g] = f2_pack(-turn[g].rc, -turn[g].rc);
         if (TGT) {
             tx[g] = f2_pack(t.tn[g].x, t.tn[g].x);
             ty[g] = f2_pack(t.tn[g].y, t.tn[g].y);
             tz[g] = f2_pack(t.tn[g].z, t.tn[g].z);
         }
         aR[g] = aI[g] = aJ[g] = hR[g] = hI[g] = hJ[g] = 0;
+        if (A) fAr[g] = fAi[g] = 0.f;
+        if (H) fHr[g] = fHi[g] = 0.f;
     }
     auto at = [&](int row, int j) { return *reinterpret_cast<const ulonglong2 *>(st + row * T + j); };
-    for (int j = 0; j < T; j += 4) {
-        const ulonglong2 X = at(0, j), Y = at(1, j), Z = at(2, j);
-        ulonglong2 NX, NY, NZ, RG, DR, DI, DN, ER, EI, EN;
-        if (SLOW) RG = at(6, j);
-        if (SRC) {
-            NX = at(3, j);
-            NY = at(4, j);
-            NZ = at(5, j);
-        }
-        if (A) {
-            DR = at(kFixed, j);
-            DI = at(kFixed + 1, j);
-            DN = at(kFixed + 2, j);
-        }
-        if (H) {
-            ER = at(kFixed + kDens<MODE> - 3, j);
-            EI = at(kFixed + kDens<MODE> - 2, j);
-            EN = at(kFixed + kDens<MODE> - 1, j);
-        }
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            auto of = [&](const ulonglong2 &v) { return h ? v.y : v.x; };
+    // A fixed inner count lets the compiler unroll: with the unit's length as
+    // the bound the sweep was 3 % slower.
+#pragma unroll 1
+    for (int jb = j0; jb < j1; jb += kRun32) {
+#pragma unroll 8
+        for (int j = jb; j < jb + kRun32; j += 4) {
+            const ulonglong2 X = at(0, j), Y = at(1, j), Z = at(2, j);
+            ulonglong2 NX, NY, NZ, DR, DI, DN, ER, EI, EN;
+            if (SRC) {
+                NX = at(3, j);
+                NY = at(4, j);
+                NZ = at(5, j);
+            }
+            if (A) {
+                DR = at(kFixed, j);
+                DI = at(kFixed + 1, j);
+                DN = at(kFixed + 2, j);
+            }
+            if (H) {
+                ER = at(kFixed + kDens<MODE> - 3, j);
+                EI = at(kFixed + kDens<MODE> - 2, j);
+                EN = at(kFixed + kDens<MODE> - 1, j);
+            }
+            F2 DX[TG][2], DY[TG][2], DZ[TG][2], R2[TG][2];
+            auto offsets = [&](int g, int h) {
+                DX[g][h] = f2_add(rx[g], h ? X.y : X.x);
+                DY[g][h] = f2_add(ry[g], h ? Y.y : Y.x);
+                DZ[g][h] = f2_add(rz[g], h ? Z.y : Z.x);
+                R2[g][h] = f2_fma(DX[g][h], DX[g][h], f2_fma(DY[g][h], DY[g][h], f2_mul(DZ[g][h], DZ[g][h])));
+            };
 #pragma unroll
             for (int g = 0; g < TG; g++) {
-                const F2 dx = f2_add(rx[g], of(X)), dy = f2_add(ry[g], of(Y)), dz = f2_add(rz[g], of(Z));
-                const F2 r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz)));
-                const F2 y = f2_rsqrt(r2);
-                F2 S, C, th;
-                if (SLOW) {
-                    // less the nearest multiple of 2 pi = 6.28125 + 0.00193...
-                    const F2 rho = f2_mul(r2, y), M = f2_pack(12582912.f, 12582912.f);
-                    const F2 n = f2_add(f2_fma(rho, f2_pack(0.15915494309189535f, 0.15915494309189535f), M),
-                                        f2_pack(-12582912.f, -12582912.f));
-                    th = f2_fma(n, f2_pack(-0.0019353071795864769f, -0.0019353071795864769f),
-                                f2_fma(n, f2_pack(-6.28125f, -6.28125f), rho));
-                } else {
-                    th = f2_fma(r2, y, nrc[g]);
-                }
-                f2_sincos(th, S, C);
-                const F2 yy = f2_mul(y, y);
-                F2 ps, pt;
-                if (SRC) ps = f2_mul(yy, f2_fma(dx, of(NX), f2_fma(dy, of(NY), f2_mul(dz, of(NZ)))));
-                if (TGT) pt = f2_mul(yy, f2_fma(dx, tx[g], f2_fma(dy, ty[g], f2_mul(dz, tz[g]))));
-                F2 e1, e2, f1, f2;
-                if (A) {
-                    const F2 q = DIR ? ps : pt;
-                    e1 = f2_mul(q, f2_fma(y, of(DN), of(DR)));
-                    e2 = f2_mul(q, f2_fma(y, of(DR), of(DI)));
-                }
-                if (H) {
-                    const F2 q = DIR ? pt : ps;
-                    f1 = f2_mul(q, f2_fma(y, of(EI), of(ER)));
-                    f2 = f2_mul(q, f2_fma(y, of(ER), of(EN)));
-                }
-                if (SLOW) {
-                    float ra, rb;
-                    f2_unpack(r2, ra, rb);
-                    if (fminf(ra, rb) < a.guard_hi) {
-                        const int64_t ts = tslot0 + (int64_t)g * NT, ss = sslot0 + j + 2 * h;
-                        const bool na = is_near(a, ra, ts, ss), nb = is_near(a, rb, ts, ss + 1);
-                        auto pick = [&](F2 far, float va, float vb) {
-                            float fa, fb;
-                            f2_unpack(far, fa, fb);
-                            return f2_pack(na ? va : fa, nb ? vb : fb);
+                if (KIND != TILE_FAR) {
+                    offsets(g, 0);
+                    offsets(g, 1);
+                    float r[4];
+                    f2_unpack(R2[g][0], r[0], r[1]);
+                    f2_unpack(R2[g][1], r[2], r[3]);
+                    if (fminf(fminf(r[0], r[1]), fminf(r[2], r[3])) < a.guard_hi) {
+                        bool nr[4], tie = false;
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            nr[q] = r[q] <= a.tau2;
+                            tie |= r[q] > a.guard_lo && r[q] < a.guard_hi;
+                        }
+                        if (tie) {
+#pragma unroll
+                            for (int q = 0; q < 4; q++)
+                                nr[q] = is_near(a, r[q], tslot0 + (int64_t)g * NT, sslot0 + j + q);
+                        }
+                        const ulonglong2 RG = at(6, j);
+                        float w[4];
+                        f2_unpack(RG.x, w[0], w[1]);
+                        f2_unpack(RG.y, w[2], w[3]);
+                        auto add = [&](float own, bool src, const ulonglong2 &re, const ulonglong2 &im, float &fr,
+                                       float &fi) {
+                            float x[4], y[4];
+                            f2_unpack(re.x, x[0], x[1]);
+                            f2_unpack(re.y, x[2], x[3]);
+                            f2_unpack(im.x, y[0], y[1]);
+                            f2_unpack(im.y, y[2], y[3]);
+#pragma unroll
+                            for (int q = 0; q < 4; q++) {
+                                const float v = nr[q] ? (src ? w[q] : own) : 0.f;
+                                fr = fmaf(v, x[q], fr);
+                                fi = fmaf(v, y[q], fi);
+                            }
                         };
-                        float ga, gb;
-                        f2_unpack(of(RG), ga, gb);
-                        S = pick(S, 0.f, 0.f);
-                        C = pick(C, 1.f, 1.f);
-                        if (A) {
-                            const float va = DIR ? ga : t.reg[g], vb = DIR ? gb : t.reg[g];
-                            float d0, d1, i0, i1;
-                            f2_unpack(of(DR), d0, d1);
-                            f2_unpack(of(DI), i0, i1);
-                            e1 = pick(e1, va * i0, vb * i1);
-                            e2 = pick(e2, -va * d0, -vb * d1);
-                        }
-                        if (H) {
-                            const float va = DIR ? t.reg[g] : ga, vb = DIR ? t.reg[g] : gb;
-                            float d0, d1, i0, i1;
-                            f2_unpack(of(ER), d0, d1);
-                            f2_unpack(of(EI), i0, i1);
-                            f1 = pick(f1, va * i0, vb * i1);
-                            f2 = pick(f2, va * d0, vb * d1);
-                        }
+                        if (A) add(t.reg[g], DIR, DR, DI, fAr[g], fAi[g]);
+                        if (H) add(t.reg[g], !DIR, ER, EI, fHr[g], fHi[g]);
+#pragma unroll
+                        for (int q = 0; q < 4; q++) r[q] = nr[q] ? 1e16f : r[q];
+                        R2[g][0] = f2_pack(r[0], r[1]);
+                        R2[g][1] = f2_pack(r[2], r[3]);
                     }
                 }
-                if (A) {
-                    aR[g] = f2_fma(S, e1, f2_fma(C, e2, aR[g]));
-                    aI[g] = f2_fma(C, e1, aI[g]);
-                    aJ[g] = f2_fma(S, e2, aJ[g]);
-                }
-                if (H) {
-                    hR[g] = f2_fma(S, f1, f2_fma(C, f2, hR[g]));
-                    hI[g] = f2_fma(C, f1, hI[g]);
-                    hJ[g] = f2_fma(S, f2, hJ[g]);
+            }
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                auto of = [&](const ulonglong2 &v) { return h ? v.y : v.x; };
+#pragma unroll
+                for (int g = 0; g < TG; g++) {
+                    if (KIND == TILE_FAR) offsets(g, h);
+                    const F2 dx = DX[g][h], dy = DY[g][h], dz = DZ[g][h], r2 = R2[g][h];
+                    const F2 y = f2_rsqrt(r2);
+                    F2 S, C, th;
+                    if (KIND == TILE_WIDE) {
+                        // less the nearest multiple of 2 pi = 6.28125 + 0.00193...
+                        const F2 rho = f2_mul(r2, y), M = f2_pack(12582912.f, 12582912.f);
+                        const F2 n = f2_add(f2_fma(rho, f2_pack(0.15915494309189535f, 0.15915494309189535f), M),
+                                            f2_pack(-12582912.f, -12582912.f));
+                        th = f2_fma(n, f2_pack(-0.0019353071795864769f, -0.0019353071795864769f),
+                                    f2_fma(n, f2_pack(-6.28125f, -6.28125f), rho));
+                    } else {
+                        th = f2_fma(r2, y, nrc[g]);
+                    }
+                    f2_sincos(th, S, C);
+                    const F2 yy = f2_mul(y, y);
+                    F2 ps, pt;
+                    if (SRC) ps = f2_mul(yy, f2_fma(dx, of(NX), f2_fma(dy, of(NY), f2_mul(dz, of(NZ)))));
+                    if (TGT) pt = f2_mul(yy, f2_fma(dx, tx[g], f2_fma(dy, ty[g], f2_mul(dz, tz[g]))));
+                    F2 e1, e2, f1, f2;
+                    if (A) {
+                        const F2 q = DIR ? ps : pt;
+                        e1 = f2_mul(q, f2_fma(y, of(DN), of(DR)));
+                        e2 = f2_mul(q, f2_fma(y, of(DR), of(DI)));
+                    }
+                    if (H) {
+                        const F2 q = DIR ? pt : ps;
+                        f1 = f2_mul(q, f2_fma(y, of(EI), of(ER)));
+                        f2 = f2_mul(q, f2_fma(y, of(ER), of(EN)));
+                    }
+                    if (A) {
+                        aR[g] = f2_fma(S, e1, f2_fma(C, e2, aR[g]));
+                        aI[g] = f2_fma(C, e1, aI[g]);
+                        aJ[g] = f2_fma(S, e2, aJ[g]);
+                    }
+                    if (H) {
+                        hR[g] = f2_fma(S, f1, f2_fma(C, f2, hR[g]));
+                        hI[g] = f2_fma(C, f1, hI[g]);
+                        hJ[g] = f2_fma(S, f2, hJ[g]);
+                    }
                 }
             }
         }
@@ -318,45 +385,69 @@ __device__ __forceinline__ void tile_packed(const Args32 &a, const float *st, co
 #pragma unroll
     for (int g = 0; g < TG; g++) {
         if (A) {
-            fAr[g] = -f2_sum(aR[g]);
-            fAi[g] = f2_sum(aI[g]) - f2_sum(aJ[g]);
-            if (!SLOW) turn_sum<false>(turn[g], fAr[g], fAi[g]);
+            float re = -f2_sum(aR[g]), im = f2_sum(aI[g]) - f2_sum(aJ[g]);
+            if (KIND != TILE_WIDE) turn_sum<false>(turn[g], re, im);
+            fAr[g] += re;
+            fAi[g] += im;
         }
         if (H) {
-            fHr[g] = f2_sum(hR[g]);
-            fHi[g] = f2_sum(hI[g]) - f2_sum(hJ[g]);
-            if (!SLOW) turn_sum<true>(turn[g], fHr[g], fHi[g]);
+            float re = f2_sum(hR[g]), im = f2_sum(hI[g]) - f2_sum(hJ[g]);
+            if (KIND != TILE_WIDE) turn_sum<true>(turn[g], re, im);
+            fHr[g] += re;
+            fHi[g] += im;
         }
     }
 }
 
-// The pairs of the block's targets with the staged source tile, added to sum.
+// The pairs of the block's targets with the units [q0, q1) of the staged
+// source tile, added to sum.
 template <int MODE, bool DIR, int NT, int TG>
-__device__ __forceinline__ void tile_pairs(const Args32 &a, const float *st, int64_t tile, bool near,
+__device__ __forceinline__ void tile_pairs(const Args32 &a, const float *st, int64_t tile, int q0, int q1, bool near,
                                            const float3 (&rel)[TG], const Turn (&turn)[TG], bool centred,
                                            const Targets<TG> &t, int64_t slot0, Sums<TG> &sum)
 {
-    float fAr[TG], fAi[TG], fHr[TG], fHi[TG];
+    const int64_t sslot0 = tile * kTile32;
+    const int len = kTile32 / a.sub;
+    auto units = [&](auto unit) {
+#pragma unroll 1
+        for (int q = q0; q < q1; q++) {
+            float fAr[TG], fAi[TG], fHr[TG], fHi[TG];
+            unit(q * len, q * len + len, fAr, fAi, fHr, fHi);
 #pragma unroll
-    for (int g = 0; g < TG; g++) fAr[g] = fAi[g] = fHr[g] = fHi[g] = 0.f;
+            for (int g = 0; g < TG; g++) {
+                if (MODE & SWEEP_A) {
+                    two_sum_acc(sum.hAr[g], sum.lAr[g], fAr[g]);
+                    two_sum_acc(sum.hAi[g], sum.lAi[g], fAi[g]);
+                }
+                if (MODE & SWEEP_AH) {
+                    two_sum_acc(sum.hHr[g], sum.lHr[g], fHr[g]);
+                    two_sum_acc(sum.hHi[g], sum.lHi[g], fHi[g]);
+                }
+            }
+        }
+    };
     if (!(MODE & SWEEP_SCALED)) {
-        for (int j = 0; j < kTile32; j++)
-            pair_scalar<MODE, DIR, NT, TG>(a, st, j, near, rel, t, slot0, tile * kTile32 + j, fAr, fAi, fHr, fHi);
-    } else if (centred) {
-        tile_packed<MODE, DIR, NT, TG, false>(a, st, rel, t, turn, slot0, tile * kTile32, fAr, fAi, fHr, fHi);
-    } else {
-        tile_packed<MODE, DIR, NT, TG, true>(a, st, rel, t, turn, slot0, tile * kTile32, fAr, fAi, fHr, fHi);
-    }
+        units([&](int j0, int j1, float (&fAr)[TG], float (&fAi)[TG], float (&fHr)[TG], float (&fHi)[TG]) {
 #pragma unroll
-    for (int g = 0; g < TG; g++) {
-        if (MODE & SWEEP_A) {
-            two_sum_acc(sum.hAr[g], sum.lAr[g], fAr[g]);
-            two_sum_acc(sum.hAi[g], sum.lAi[g], fAi[g]);
-        }
-        if (MODE & SWEEP_AH) {
-            two_sum_acc(sum.hHr[g], sum.lHr[g], fHr[g]);
-            two_sum_acc(sum.hHi[g], sum.lHi[g], fHi[g]);
-        }
+            for (int g = 0; g < TG; g++) fAr[g] = fAi[g] = fHr[g] = fHi[g] = 0.f;
+            for (int j = j0; j < j1; j++)
+                pair_scalar<MODE, DIR, NT, TG>(a, st, j, near, rel, t, slot0, sslot0 + j, fAr, fAi, fHr, fHi);
+        });
+    } else if (!centred) {
+        units([&](int j0, int j1, float (&fAr)[TG], float (&fAi)[TG], float (&fHr)[TG], float (&fHi)[TG]) {
+            unit_packed<MODE, DIR, NT, TG, TILE_WIDE>(a, st, j0, j1, rel, t, turn, slot0, sslot0, fAr, fAi,
+                                                            fHr, fHi);
+        });
+    } else if (near) {
+        units([&](int j0, int j1, float (&fAr)[TG], float (&fAi)[TG], float (&fHr)[TG], float (&fHi)[TG]) {
+            unit_packed<MODE, DIR, NT, TG, TILE_NEAR>(a, st, j0, j1, rel, t, turn, slot0, sslot0, fAr, fAi,
+                                                            fHr, fHi);
+        });
+    } else {
+        units([&](int j0, int j1, float (&fAr)[TG], float (&fAi)[TG], float (&fHr)[TG], float (&fHi)[TG]) {
+            unit_packed<MODE, DIR, NT, TG, TILE_FAR>(a, st, j0, j1, rel, t, turn, slot0, sslot0, fAr, fAi,
+                                                            fHr, fHi);
+        });
     }
 }
 
@@ -379,11 +470,11 @@ __device__ __forceinline__ void load_targets(const Args32 &a, int64_t slot0, Tar
 // x_t - o of the targets (the head difference is rounded once, to half an ulp
 // of itself) and the turns of a centred tile.
 template <int MODE, int TG>
-__device__ __forceinline__ bool tile_offsets(const Args32 &a, int64_t tile, bool near, const Targets<TG> &t,
+__device__ __forceinline__ bool tile_offsets(const Args32 &a, int64_t tile, const Targets<TG> &t,
                                              float3 (&rel)[TG], Turn (&turn)[TG])
 {
     const float4 oh = a.ohi[tile], ol = a.olo[tile];
-    const bool centred = (MODE & SWEEP_SCALED) && !near && oh.w <= kCentreRadius;
+    const bool centred = (MODE & SWEEP_SCALED) && oh.w <= kCentreRadius;
 #pragma unroll
     for (int g = 0; g < TG; g++) {
         rel[g] = make_float3((t.th[g].x - oh.x) + (t.tl[g].x - ol.x), (t.th[g].y - oh.y) + (t.tl[g].y - ol.y),
@@ -422,12 +513,47 @@ __device__ __forceinline__ void write_slot(const Args32 &a, int64_t s, double ar
     }
 }
 
+// The pieces of a target block that the partition split between CTAs, summed
+// in CTA order by whichever CTA finishes last: the caller has written `units`
+// units' sums to partial; begin(c) is the partition, u0 the block's first unit,
+// total its units, and write(slot, sums) stores a slot.
+template <int SLOTS, class Begin, class Write>
+__device__ __forceinline__ void finish_block(unsigned *done, unsigned units, unsigned total, int64_t u0, int nctas,
+                                             const double4_32a *partial, const Begin &begin, const Write &write)
+{
+    __shared__ unsigned before;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) before = atomicAdd(done, units);
+    __syncthreads();
+    if (before + units != total) return;
+    __threadfence();
+    const int lo = cta_of_unit(u0, nctas, begin), hi = cta_of_unit(u0 + total - 1, nctas, begin);
+    for (int k = threadIdx.x; k < SLOTS; k += blockDim.x) {
+        double ar = 0.0, ai = 0.0, hr = 0.0, hi_ = 0.0;
+#pragma unroll 4
+        for (int c = lo; c <= hi; c++) {
+            const int64_t b = begin(c);
+            if (b == begin(c + 1)) continue;  // a CTA without units
+            // a CTA's first block is its slot 0, its last one slot 1
+            const double2 *v = reinterpret_cast<const double2 *>(partial + ((int64_t)c * 2 + (b < u0)) * SLOTS + k);
+            const double2 x = __ldcg(v), y = __ldcg(v + 1);
+            ar += x.x;
+            ai += x.y;
+            hr += y.x;
+            hi_ += y.y;
+        }
+        write(k, ar, ai, hr, hi_);
+    }
+}
+
 // Persistent stream-K sweep: every CTA walks its own contiguous range of
-// (target block, source tile) units, so all CTAs carry the same number of
-// tile pairs whatever the tube size.  A target block that lies wholly in
-// one CTA's range is written out directly; the pieces of a block split
-// between CTAs go to the partial buffer (slot 0: the CTA's first block,
-// slot 1: its last) and sweep32_fixup adds them up in CTA order.
+// (target block, part of a source tile) units, ranges of equal cost whatever
+// the tube size.  A target block that lies wholly in one CTA's range is written
+// out directly; the pieces of a block split between CTAs go to the partial
+// buffer (slot 0: the CTA's first block, slot 1: its last), and the CTA that
+// finishes a block adds them up (as a kernel of its own that took 10 us and a
+// launch, mostly 64-bit divisions).
 template <int MODE, bool DIR, int NT, int TG, int MINB>
 __global__ void __launch_bounds__(NT, MINB) sweep32_kernel(Args32 a)
 {
@@ -436,9 +562,8 @@ __global__ void __launch_bounds__(NT, MINB) sweep32_kernel(Args32 a)
     __shared__ alignas(128) float stage[2][kStage<MODE>];
     __shared__ alignas(8) uint64_t bar[2];
 
-    const int64_t ntiles = a.npad / kTile32;
-    const int64_t u_begin = (int64_t)blockIdx.x * a.units / a.nctas;
-    const int64_t u_end = ((int64_t)blockIdx.x + 1) * a.units / a.nctas;
+    const int64_t ntiles = a.npad / kTile32, bu = ntiles * a.sub;
+    const int64_t u_begin = cta_begin(a, blockIdx.x), u_end = cta_begin(a, blockIdx.x + 1);
     if (threadIdx.x == 0) {
         mbar_init(&bar[0], 1);
         mbar_init(&bar[1], 1);
@@ -446,38 +571,40 @@ __global__ void __launch_bounds__(NT, MINB) sweep32_kernel(Args32 a)
     }
     __syncthreads();
     if (u_begin >= u_end) return;
-    if (threadIdx.x == 0) issue_tile<MODE>(a, u_begin % ntiles, stage[0], &bar[0]);
+    if (threadIdx.x == 0) issue_tile<MODE>(a, (u_begin % bu) / a.sub, stage[0], &bar[0]);
     int seg = 0;
+    unsigned it = 0;
     for (int64_t u = u_begin; u < u_end;) {
-        const int64_t blk = u / ntiles;
-        const int64_t seg_end = (u_end < (blk + 1) * ntiles) ? u_end : (blk + 1) * ntiles;
-        const bool whole = (u == blk * ntiles) && (seg_end == (blk + 1) * ntiles);
+        const int64_t blk = u / bu, u0 = blk * bu, seg_begin = u;
+        const int64_t seg_end = (u_end < u0 + bu) ? u_end : u0 + bu;
         const int64_t slot0 = blk * SLOTS + threadIdx.x;
         Targets<TG> t;
         Sums<TG> sum;
         load_targets<NT, TG>(a, slot0, t, sum);
         const uint32_t *mrow = a.nearmask + blk * a.mwords;  // the near-tile mask of this target tile
-        for (; u < seg_end; u++) {
-            const int64_t it = u - u_begin;
+        for (; u < seg_end; it++) {
             const int buf = (int)(it & 1);
-            if (threadIdx.x == 0 && u + 1 < u_end) issue_tile<MODE>(a, (u + 1) % ntiles, stage[buf ^ 1], &bar[buf ^ 1]);
-            const int64_t tile = u - blk * ntiles;
+            const int64_t tile = (u - u0) / a.sub;
+            const int q0 = (int)((u - u0) % a.sub), q1 = (int)min((int64_t)a.sub, q0 + seg_end - u);
+            u += q1 - q0;
+            if (threadIdx.x == 0 && u < u_end)
+                issue_tile<MODE>(a, tile + 1 < ntiles ? tile + 1 : 0, stage[buf ^ 1], &bar[buf ^ 1]);
             const bool near = (__ldg(mrow + (tile >> 5)) >> (tile & 31)) & 1u;
             float3 rel[TG];
             Turn turn[TG];
-            const bool centred = tile_offsets<MODE, TG>(a, tile, near, t, rel, turn);
-            const bool ok = mbar_wait_bounded(&bar[buf], (uint32_t)((it >> 1) & 1), g_data_wait_limit);
+            const bool centred = tile_offsets<MODE, TG>(a, tile, t, rel, turn);
+            const bool ok = mbar_wait_bounded(&bar[buf], (it >> 1) & 1, g_data_wait_limit);
             if (__syncthreads_or(!ok)) {
                 if (threadIdx.x == 0) {
                     atomicOr(a.err, DEV_ERR_WAIT);
-                    mbar_drain(&bar[buf], (uint32_t)((it >> 1) & 1), &bar[buf ^ 1], (uint32_t)(((it + 1) >> 1) & 1),
-                               u + 1 < u_end);
+                    mbar_drain(&bar[buf], (it >> 1) & 1, &bar[buf ^ 1], ((it + 1) >> 1) & 1, u < u_end);
                 }
                 return;
             }
-            tile_pairs<MODE, DIR, NT, TG>(a, stage[buf], tile, near, rel, turn, centred, t, slot0, sum);
+            tile_pairs<MODE, DIR, NT, TG>(a, stage[buf], tile, q0, q1, near, rel, turn, centred, t, slot0, sum);
             __syncthreads();
         }
+        const bool whole = seg_end - seg_begin == bu;
 #pragma unroll
         for (int g = 0; g < TG; g++) {
             const double ar = (double)sum.hAr[g] + (double)sum.lAr[g], ai = (double)sum.hAi[g] + (double)sum.lAi[g];
@@ -489,33 +616,122 @@ __global__ void __launch_bounds__(NT, MINB) sweep32_kernel(Args32 a)
                     make_double4_32a(ar, ai, hr, hi);
             }
         }
+        if (!whole)
+            finish_block<SLOTS>(
+                a.done + blk, (unsigned)(seg_end - seg_begin), (unsigned)bu, u0, a.nctas, a.partial,
+                [&](int c) { return cta_begin(a, c); },
+                [&](int k, double ar, double ai, double hr, double hi) {
+                    write_slot<MODE>(a, blk * SLOTS + k, ar, ai, hr, hi);
+                });
         seg = 1;
     }
 }
 
-// Adds up, in CTA order, the pieces of every target block that the stream-K
-// partition split between CTAs (one CTA per target block; blocks that one
-// CTA covered whole return at once).
-template <int MODE, int SLOTS>
-__global__ void __launch_bounds__(256) sweep32_fixup(Args32 a)
+// Cost of 32 source tiles of a target tile's row.
+__device__ __forceinline__ int word_cost(const uint32_t *mrow, int64_t w, int64_t ntiles, int64_t self)
 {
-    const int64_t blk = blockIdx.x;
-    const int64_t ntiles = a.npad / kTile32;
-    const int64_t c_lo = cta_of_unit(blk * ntiles, a.units, a.nctas);
-    const int64_t c_hi = cta_of_unit((blk + 1) * ntiles - 1, a.units, a.nctas);
-    if (c_lo == c_hi) return;
-    for (int k = threadIdx.x; k < SLOTS; k += blockDim.x) {
-        double ar = 0.0, ai = 0.0, hr = 0.0, hi = 0.0;
-        for (int64_t c = c_lo; c <= c_hi; c++) {
-            const int64_t first = (c * a.units / a.nctas) / ntiles;  // first block of CTA c
-            const int sg = (first == blk) ? 0 : 1;
-            const double4_32a v = a.partial[(c * 2 + sg) * SLOTS + k];
-            ar += v.x;
-            ai += v.y;
-            hr += v.z;
-            hi += v.w;
+    const int tiles = (int)min((int64_t)32, ntiles - w * 32);
+    return tiles * kCostFar + __popc(mrow[w]) * (kCostNear - kCostFar) +
+           ((self >> 5) == w ? kCostSelf - kCostNear : 0);
+}
+
+// rows[t] = cost of target tile t's row
+__global__ void __launch_bounds__(256) row_cost_kernel(int64_t ntiles, int64_t mwords, const uint32_t *__restrict__ mask,
+                                                       int64_t *__restrict__ rows)
+{
+    const int64_t t = blockIdx.x * (int64_t)8 + (threadIdx.x >> 5);
+    if (t >= ntiles) return;
+    int64_t c = 0;
+    for (int64_t w = threadIdx.x & 31; w < mwords; w += 32) c += word_cost(mask + t * mwords, w, ntiles, t);
+    for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
+    if ((threadIdx.x & 31) == 0) rows[t] = c;
+}
+
+// rows: exclusive prefix sums, rows[ntiles] the total (one block)
+__global__ void __launch_bounds__(1024) row_scan_kernel(int64_t ntiles, int64_t *__restrict__ rows)
+{
+    __shared__ int64_t part[32], carry;
+    if (threadIdx.x == 0) carry = 0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int64_t b = 0; b <= ntiles; b += 1024) {
+        const int64_t t = b + threadIdx.x;
+        const int64_t v = t < ntiles ? rows[t] : 0;
+        int64_t x = v;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
         }
-        write_slot<MODE>(a, blk * SLOTS + k, ar, ai, hr, hi);
+        if (lane == 31) part[warp] = x;
+        __syncthreads();
+        if (warp == 0) {
+            int64_t p = part[lane];
+            for (int o = 1; o < 32; o <<= 1) {
+                const int64_t y = __shfl_up_sync(0xffffffffu, p, o);
+                if (lane >= o) p += y;
+            }
+            part[lane] = p;
+        }
+        __syncthreads();
+        const int64_t base = carry + (warp ? part[warp - 1] : 0);
+        if (t <= ntiles) rows[t] = base + x - v;
+        __syncthreads();
+        if (threadIdx.x == 0) carry += part[31];
+        __syncthreads();
+    }
+}
+
+// First lane whose inclusive sum of v exceeds r (the caller knows there is
+// one), r less the sums before it.
+__device__ __forceinline__ int lane_of(int v, int64_t &r)
+{
+    int x = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if ((int)(threadIdx.x & 31) >= o) x += y;
+    }
+    const int f = __ffs(__ballot_sync(0xffffffffu, x > r)) - 1;
+    r -= __shfl_sync(0xffffffffu, x - v, f);
+    return f;
+}
+
+// cuts[i]: the unit at cost i / kCuts of the total (one warp a cut)
+__global__ void __launch_bounds__(256) cuts_kernel(int64_t ntiles, int64_t mwords, int sub,
+                                                   const uint32_t *__restrict__ mask,
+                                                   const int64_t *__restrict__ rows, int64_t *__restrict__ cuts)
+{
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (i > kCuts) return;
+    const int64_t total = rows[ntiles], x = total / kCuts * i + total % kCuts * i / kCuts;
+    if (i == kCuts) {
+        if (lane == 0) cuts[i] = ntiles * ntiles * sub;
+        return;
+    }
+    int64_t lo = 0;  // the last row with rows[lo] <= x
+    for (int64_t len = ntiles; len > 1;) {
+        const int64_t step = (len + 31) / 32, at = lane * step;
+        const int k = __popc(__ballot_sync(0xffffffffu, at < len && rows[lo + (at < len ? at : 0)] <= x)) - 1;
+        lo += k * step;
+        len = min(step, len - k * step);
+    }
+    const uint32_t *mrow = mask + lo * mwords;
+    int64_t r = x - rows[lo], w = 0;
+    for (;; w += 32) {
+        const int c = w + lane < mwords ? word_cost(mrow, w + lane, ntiles, lo) : 0;
+        const int sum = __reduce_add_sync(0xffffffffu, c);
+        if (r < sum) {
+            w += lane_of(c, r);
+            break;
+        }
+        r -= sum;
+    }
+    const int64_t t = w * 32 + lane;
+    const int c = t >= ntiles ? 0 : t == lo ? kCostSelf : ((mrow[w] >> lane) & 1u) ? kCostNear : kCostFar;
+    const int f = lane_of(c, r);
+    if (lane == 0) {
+        const int64_t tile = w * 32 + f;
+        const int ct = tile == lo ? kCostSelf : ((mrow[w] >> f) & 1u) ? kCostNear : kCostFar;
+        cuts[i] = (lo * ntiles + tile) * sub + (int)(r * sub / ct);
     }
 }
 
@@ -525,9 +741,10 @@ __global__ void __launch_bounds__(256) sweep32_fixup(Args32 a)
 // product vectors are columns of [R][stride] arrays passed to the launch.
 struct BatchOp {
     Args32 a;
-    int64_t unit0;   // first global (target block, source tile) unit
-    int64_t block0;  // first global target block
-    int64_t blocks, ntiles;
+    int64_t unit0;   // first global unit
+    int64_t cost0, cost;  // costs of the operators before it, and its own
+    const int64_t *rows;  // its row costs (rows[ntiles]: the total)
+    int64_t ntiles;
     int dir;
     int col;         // column of P and Q
     double scale;    // lambda^2 sg / (4 pi), folded into the densities
@@ -544,6 +761,8 @@ __global__ void batch_prep_kernel(const BatchOp *__restrict__ ops, BatchVec v)
 {
     const BatchOp &o = ops[blockIdx.y];
     const double *pr = v.p_re + (int64_t)o.col * v.stride, *pi = v.p_im + (int64_t)o.col * v.stride;
+    if (blockIdx.x == 0)
+        for (int64_t b = threadIdx.x; b < o.ntiles; b += blockDim.x) o.a.done[b] = 0;
     for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < o.a.npad;
          s += (int64_t)gridDim.x * blockDim.x) {
         const int c = o.a.perm[s];
@@ -559,6 +778,28 @@ __device__ __forceinline__ int batch_op_of_unit(const BatchOp *ops, int nops, in
     return o;
 }
 
+// cost0 and cost of the described operators (one thread)
+__global__ void batch_cost_kernel(BatchOp *ops, int nops)
+{
+    int64_t c = 0;
+    for (int o = 0; o < nops; o++) {
+        ops[o].cost0 = c;
+        ops[o].cost = ops[o].rows[ops[o].ntiles];
+        c += ops[o].cost;
+    }
+}
+
+// First unit of CTA c: the operators' cuts laid end to end by their costs.
+__device__ __forceinline__ int64_t batch_begin(const BatchOp *ops, int nops, int nctas, int c)
+{
+    const int64_t total = ops[nops - 1].cost0 + ops[nops - 1].cost;
+    const int64_t x = total / nctas * c + total % nctas * c / nctas;
+    int o = 0;
+    while (o + 1 < nops && x >= ops[o + 1].cost0) o++;
+    const int64_t y = x - ops[o].cost0, n = ops[o].cost;
+    return ops[o].unit0 + __ldg(ops[o].a.cuts + (y / n * kCuts + y % n * kCuts / n));
+}
+
 __device__ __forceinline__ void batch_write(const Args32 &a, int64_t s, double ar, double ai, const double *p_re,
                                             const double *p_im, double *q_re, double *q_im)
 {
@@ -569,57 +810,55 @@ __device__ __forceinline__ void batch_write(const Args32 &a, int64_t s, double a
     q_im[c] = ai + 0.5 * p_im[c];
 }
 
-// The tiles of one segment (one target block of one operator) for the
+// The units of one segment (one target block of one operator) for the
 // batched sweep: the same loops as sweep32_kernel with SWEEP_A.
 template <int MODE, bool DIR, int NT, int TG>
 __device__ __forceinline__ bool batch_tiles(const Args32 &a, const BatchOp *ops, int nops, int o, int64_t &u,
-                                            int64_t seg_end, int64_t u_begin, int64_t u_end, int64_t blk,
+                                            int64_t u0, int64_t seg_end, int64_t u_end, unsigned &it, int64_t blk,
                                             int64_t slot0, const Targets<TG> &t, Sums<TG> &sum,
                                             float (*stage)[kStage<SWEEP_A>], uint64_t *bar)
 {
-    const int64_t ntiles = ops[o].ntiles, unit0 = ops[o].unit0;
     const uint32_t *mrow = a.nearmask + blk * a.mwords;
-    for (; u < seg_end; u++) {
-        const int64_t it = u - u_begin;
+    for (; u < seg_end; it++) {
         const int buf = (int)(it & 1);
-        if (threadIdx.x == 0 && u + 1 < u_end) {
-            const int o2 = batch_op_of_unit(ops, nops, u + 1, o);
-            issue_tile<SWEEP_A>(ops[o2].a, (u + 1 - ops[o2].unit0) % ops[o2].ntiles, stage[buf ^ 1], &bar[buf ^ 1]);
+        const int64_t tile = (u - u0) / a.sub;
+        const int q0 = (int)((u - u0) % a.sub), q1 = (int)min((int64_t)a.sub, q0 + seg_end - u);
+        u += q1 - q0;
+        if (threadIdx.x == 0 && u < u_end) {
+            const int o2 = batch_op_of_unit(ops, nops, u, o);
+            issue_tile<SWEEP_A>(ops[o2].a, (u - ops[o2].unit0) / ops[o2].a.sub % ops[o2].ntiles, stage[buf ^ 1], &bar[buf ^ 1]);
         }
-        const int64_t tile = u - unit0 - blk * ntiles;
         const bool near = (__ldg(mrow + (tile >> 5)) >> (tile & 31)) & 1u;
         float3 rel[TG];
         Turn turn[TG];
-        const bool centred = tile_offsets<MODE, TG>(a, tile, near, t, rel, turn);
-        const bool ok = mbar_wait_bounded(&bar[buf], (uint32_t)((it >> 1) & 1), g_data_wait_limit);
+        const bool centred = tile_offsets<MODE, TG>(a, tile, t, rel, turn);
+        const bool ok = mbar_wait_bounded(&bar[buf], (it >> 1) & 1, g_data_wait_limit);
         if (__syncthreads_or(!ok)) {
             if (threadIdx.x == 0) {
                 atomicOr(a.err, DEV_ERR_WAIT);
-                mbar_drain(&bar[buf], (uint32_t)((it >> 1) & 1), &bar[buf ^ 1], (uint32_t)(((it + 1) >> 1) & 1),
-                           u + 1 < u_end);
+                mbar_drain(&bar[buf], (it >> 1) & 1, &bar[buf ^ 1], ((it + 1) >> 1) & 1, u < u_end);
             }
             return false;
         }
-        tile_pairs<MODE, DIR, NT, TG>(a, stage[buf], tile, near, rel, turn, centred, t, slot0, sum);
+        tile_pairs<MODE, DIR, NT, TG>(a, stage[buf], tile, q0, q1, near, rel, turn, centred, t, slot0, sum);
         __syncthreads();
     }
     return true;
 }
 
 // Q[r] = A_r P[r] for every operator r of a batch in one persistent launch:
-// the stream-K partition of sweep32_kernel over the concatenated
-// (operator, target block, source tile) units, so operators of different
-// sizes share the GPU without a tail per operator.
+// the stream-K partition of sweep32_kernel over the concatenated units, so
+// operators of different sizes share the GPU without a tail per operator.
 template <int NT, int TG, int MINB>
 __global__ void __launch_bounds__(NT, MINB) sweep32_batch_kernel(const BatchOp *__restrict__ ops, int nops,
-                                                                 int64_t units, int64_t nctas,
-                                                                 double4_32a *partial, BatchVec v)
+                                                                 int64_t units, int nctas, double4_32a *partial,
+                                                                 BatchVec v)
 {
     constexpr int SLOTS = NT * TG;
     __shared__ alignas(128) float stage[2][kStage<SWEEP_A>];
     __shared__ alignas(8) uint64_t bar[2];
-    const int64_t u_begin = (int64_t)blockIdx.x * units / nctas;
-    const int64_t u_end = ((int64_t)blockIdx.x + 1) * units / nctas;
+    auto begin = [&](int c) { return c >= nctas ? units : batch_begin(ops, nops, nctas, c); };
+    const int64_t u_begin = begin(blockIdx.x), u_end = begin(blockIdx.x + 1);
     if (threadIdx.x == 0) {
         mbar_init(&bar[0], 1);
         mbar_init(&bar[1], 1);
@@ -628,23 +867,24 @@ __global__ void __launch_bounds__(NT, MINB) sweep32_batch_kernel(const BatchOp *
     __syncthreads();
     if (u_begin >= u_end) return;
     int o = batch_op_of_unit(ops, nops, u_begin, 0);
-    if (threadIdx.x == 0) issue_tile<SWEEP_A>(ops[o].a, (u_begin - ops[o].unit0) % ops[o].ntiles, stage[0], &bar[0]);
+    if (threadIdx.x == 0)
+        issue_tile<SWEEP_A>(ops[o].a, (u_begin - ops[o].unit0) / ops[o].a.sub % ops[o].ntiles, stage[0], &bar[0]);
     int seg = 0;
+    unsigned it = 0;
     for (int64_t u = u_begin; u < u_end;) {
         o = batch_op_of_unit(ops, nops, u, o);
         const Args32 a = ops[o].a;
-        const int64_t ntiles = ops[o].ntiles, unit0 = ops[o].unit0;
-        const int64_t blk = (u - unit0) / ntiles;
-        const int64_t blk_end = unit0 + (blk + 1) * ntiles;
-        const int64_t seg_end = (u_end < blk_end) ? u_end : blk_end;
-        const bool whole = (u == unit0 + blk * ntiles) && (seg_end == blk_end);
+        const int64_t ntiles = ops[o].ntiles, unit0 = ops[o].unit0, bu = ntiles * a.sub;
+        const int64_t blk = (u - unit0) / bu, u0 = unit0 + blk * bu, seg_begin = u;
+        const int64_t seg_end = (u_end < u0 + bu) ? u_end : u0 + bu;
+        const bool whole = seg_end - seg_begin == bu;
         const int64_t slot0 = blk * SLOTS + threadIdx.x;
         Targets<TG> t;
         Sums<TG> sum;
         load_targets<NT, TG>(a, slot0, t, sum);
         auto walk = [&](auto mode, auto dir) {
             return batch_tiles<decltype(mode)::value, decltype(dir)::value, NT, TG>(
-                a, ops, nops, o, u, seg_end, u_begin, u_end, blk, slot0, t, sum, stage, bar);
+                a, ops, nops, o, u, u0, seg_end, u_end, it, blk, slot0, t, sum, stage, bar);
         };
         using Scaled = std::integral_constant<int, SWEEP_A | SWEEP_SCALED>;
         using Plain = std::integral_constant<int, SWEEP_A>;
@@ -663,36 +903,12 @@ __global__ void __launch_bounds__(NT, MINB) sweep32_batch_kernel(const BatchOp *
                 partial[((int64_t)blockIdx.x * 2 + seg) * SLOTS + threadIdx.x + g * NT] =
                     make_double4_32a(ar, ai, 0.0, 0.0);
         }
+        if (!whole)
+            finish_block<SLOTS>(a.done + blk, (unsigned)(seg_end - seg_begin), (unsigned)bu, u0, nctas, partial, begin,
+                                [&](int k, double ar, double ai, double, double) {
+                                    batch_write(a, blk * SLOTS + k, ar, ai, pr, pi, qr, qi);
+                                });
         seg = 1;
-    }
-}
-
-// The batch's split blocks, summed in CTA order (one CTA per global block).
-template <int SLOTS>
-__global__ void __launch_bounds__(256) sweep32_batch_fixup(const BatchOp *__restrict__ ops, int nops, int64_t units,
-                                                           int64_t nctas, const double4_32a *partial, BatchVec v)
-{
-    const int64_t gb = blockIdx.x;
-    int o = 0;
-    while (o + 1 < nops && gb >= ops[o + 1].block0) o++;
-    const int64_t blk = gb - ops[o].block0, ntiles = ops[o].ntiles;
-    const int64_t u0 = ops[o].unit0 + blk * ntiles;
-    const int64_t c_lo = cta_of_unit(u0, units, nctas), c_hi = cta_of_unit(u0 + ntiles - 1, units, nctas);
-    if (c_lo == c_hi) return;
-    const Args32 &a = ops[o].a;
-    for (int k = threadIdx.x; k < SLOTS; k += blockDim.x) {
-        double ar = 0.0, ai = 0.0;
-        for (int64_t c = c_lo; c <= c_hi; c++) {
-            const int64_t ub = c * units / nctas;
-            const int oc = batch_op_of_unit(ops, nops, ub, 0);
-            const int64_t first = ops[oc].block0 + (ub - ops[oc].unit0) / ops[oc].ntiles;
-            const int sg = (first == gb) ? 0 : 1;
-            const double4_32a q = partial[(c * 2 + sg) * SLOTS + k];
-            ar += q.x;
-            ai += q.y;
-        }
-        const int64_t off = (int64_t)ops[o].col * v.stride;
-        batch_write(a, blk * SLOTS + k, ar, ai, v.p_re + off, v.p_im + off, v.q_re + off, v.q_im + off);
     }
 }
 
@@ -716,8 +932,8 @@ int64_t batch_resident_ctas()
 }
 
 template <int NT, int TG, int MINB>
-int launch_batch(const BatchOp *ops_dev, int nops, int64_t units, int64_t blocks, double4_32a *partial,
-                 size_t partial_bytes, const BatchVec &v, cudaStream_t s)
+int launch_batch(const BatchOp *ops_dev, int nops, int64_t units, double4_32a *partial, size_t partial_bytes,
+                 const BatchVec &v, cudaStream_t s)
 {
     constexpr int SLOTS = NT * TG;
     int64_t p = batch_resident_ctas<NT, TG, MINB>();
@@ -727,9 +943,7 @@ int launch_batch(const BatchOp *ops_dev, int nops, int64_t units, int64_t blocks
         set_error("batched FP32 sweep: partial buffer too small");
         return HZ_ERR_STATE;
     }
-    sweep32_batch_kernel<NT, TG, MINB><<<(unsigned)p, NT, 0, s>>>(ops_dev, nops, units, p, partial, v);
-    HZ_CHECK_LAUNCH();
-    sweep32_batch_fixup<SLOTS><<<(unsigned)blocks, 256, 0, s>>>(ops_dev, nops, units, p, partial, v);
+    sweep32_batch_kernel<NT, TG, MINB><<<(unsigned)p, NT, 0, s>>>(ops_dev, nops, units, (int)p, partial, v);
     HZ_CHECK_LAUNCH();
     return HZ_OK;
 }
@@ -761,22 +975,23 @@ int launch_streamk(Args32 a, bool persistent, size_t partial_bytes, cudaStream_t
 {
     constexpr int SLOTS = NT * TG;
     const int64_t blocks = a.npad / SLOTS;
-    a.units = blocks * (a.npad / kTile32);
-    int64_t p = persistent ? resident_ctas<MODE, DIR, NT, TG, MINB>() : blocks;
-    if (p > a.units) p = a.units;
-    if (persistent && (size_t)p * 2 * SLOTS * sizeof(double4_32a) > partial_bytes)
-        p = partial_bytes / (2 * SLOTS * sizeof(double4_32a));
+    int64_t p = blocks;
+    if (persistent) {
+        const int64_t units = blocks * (a.npad / kTile32) * a.sub;
+        p = resident_ctas<MODE, DIR, NT, TG, MINB>();
+        if (p > units) p = units;
+        if ((size_t)p * 2 * SLOTS * sizeof(double4_32a) > partial_bytes)
+            p = partial_bytes / (2 * SLOTS * sizeof(double4_32a));
+    } else {
+        a.cuts = nullptr;
+    }
     if (p < 1) {
         set_error("FP32 sweep: stream-K partial buffer too small");
         return HZ_ERR_STATE;
     }
-    a.nctas = p;
+    a.nctas = (int)p;
     sweep32_kernel<MODE, DIR, NT, TG, MINB><<<(unsigned)p, NT, 0, s>>>(a);
     HZ_CHECK_LAUNCH();
-    if (p != blocks) {
-        sweep32_fixup<MODE, SLOTS><<<(unsigned)blocks, 256, 0, s>>>(a);
-        HZ_CHECK_LAUNCH();
-    }
     return HZ_OK;
 }
 
@@ -878,17 +1093,36 @@ static void set_constants(const SweepConst &c, double lambda, Args32 &a)
     a.guard_hi = k.guard_hi;
 }
 
+size_t cuts32_bytes(int64_t ntiles)
+{
+    return (size_t)(kCuts + 1 + ntiles + 1) * sizeof(int64_t) + (size_t)ntiles * sizeof(unsigned);
+}
+
+int build_cuts32(Rec32 &r, void *mem, cudaStream_t s)
+{
+    const int64_t ntiles = r.npad / kTile32;
+    r.cuts = static_cast<int64_t *>(mem);
+    r.rows = r.cuts + kCuts + 1;
+    r.done = reinterpret_cast<unsigned *>(r.rows + ntiles + 1);
+    row_cost_kernel<<<(unsigned)((ntiles + 7) / 8), 256, 0, s>>>(ntiles, r.mwords, r.nearmask, r.rows);
+    HZ_CHECK_LAUNCH();
+    row_scan_kernel<<<1, 1024, 0, s>>>(ntiles, r.rows);
+    HZ_CHECK_LAUNCH();
+    cuts_kernel<<<kCuts / 8 + 1, 256, 0, s>>>(ntiles, r.mwords, sub_of(ntiles), r.nearmask, r.rows,
+                                                    r.cuts);
+    HZ_CHECK_LAUNCH();
+    return HZ_OK;
+}
+
 // ---------------------------------------------------------------- batches
 size_t batch32_desc_bytes(int R) { return (size_t)R * sizeof(BatchOp); }
 
-int batch32_describe(const Batch32Item *items, int R, int cfg, void *desc_dev, int64_t &units, int64_t &blocks,
-                     cudaStream_t s, const int *cols)
+int batch32_describe(const Batch32Item *items, int R, int cfg, void *desc_dev, int64_t &units, cudaStream_t s,
+                     const int *cols)
 {
     (void)cfg;
-    const int slots = kTile32;
     std::vector<BatchOp> h(R);
     units = 0;
-    blocks = 0;
     for (int r = 0; r < R; r++) {
         const int col = cols ? cols[r] : r;
         const Batch32Item &it = items[col];
@@ -913,21 +1147,25 @@ int batch32_describe(const Batch32Item *items, int R, int cfg, void *desc_dev, i
         a.perm = it.r.perm;
         a.pos64 = it.pos64;
         a.err = it.c.err;
-        if (it.r.npad % slots != 0) {
-            set_error("batched FP32 sweep: operator %d has %lld slots, not a multiple of %d", col,
-                      (long long)it.r.npad, slots);
+        if (it.r.npad % kTile32 != 0 || it.r.npad == 0 || !it.r.cuts) {
+            set_error("batched FP32 sweep: operator %d has %lld slots", col, (long long)it.r.npad);
             return HZ_ERR_STATE;
         }
         b.ntiles = it.r.npad / kTile32;
-        b.blocks = it.r.npad / slots;
         b.unit0 = units;
-        b.block0 = blocks;
+        b.rows = it.r.rows;
+        a.cuts = it.r.cuts;
+        a.done = it.r.done;
         b.dir = it.c.dirichlet != 0;
         b.scale = 1.0 / sweep32_reg_scale(it.c.interior, it.r.lambda);
-        units += b.blocks * b.ntiles;
-        blocks += b.blocks;
+        a.sub = sub_of(b.ntiles);
+        units += b.ntiles * b.ntiles * a.sub;
     }
     HZ_CHECK_CUDA(cudaMemcpyAsync(desc_dev, h.data(), R * sizeof(BatchOp), cudaMemcpyHostToDevice, s));
+    if (R > 0) {
+        batch_cost_kernel<<<1, 1, 0, s>>>(static_cast<BatchOp *>(desc_dev), R);
+        HZ_CHECK_LAUNCH();
+    }
     HZ_CHECK_CUDA(cudaStreamSynchronize(s));
     return HZ_OK;
 }
@@ -944,8 +1182,7 @@ size_t batch32_partial_bytes()
     return m;
 }
 
-int sweep_f32_batch(int cfg, const void *desc_dev, int R, int ncols, int64_t units, int64_t blocks,
-                    double4_32a *partial, size_t partial_bytes, const double *p_re, const double *p_im,
+int sweep_f32_batch(int cfg, const void *desc_dev, int R, int ncols, int64_t units, double4_32a *partial, size_t partial_bytes, const double *p_re, const double *p_im,
                     double *q_re, double *q_im, int64_t stride, int64_t max_npad, cudaStream_t s, cudaEvent_t ev0,
                     cudaEvent_t ev1)
 {
@@ -961,10 +1198,10 @@ int sweep_f32_batch(int cfg, const void *desc_dev, int R, int ncols, int64_t uni
     HZ_CHECK_LAUNCH();
     if (ev0) HZ_CHECK_CUDA(record_timing_event(ev0, s));
     switch (cfg % kShapes) {
-    case 1: HZ_TRY((launch_batch<128, 2, 4>(ops, R, units, blocks, partial, partial_bytes, v, s))); break;
-    case 2: HZ_TRY((launch_batch<256, 1, 3>(ops, R, units, blocks, partial, partial_bytes, v, s))); break;
-    case 3: HZ_TRY((launch_batch<128, 2, 3>(ops, R, units, blocks, partial, partial_bytes, v, s))); break;
-    default: HZ_TRY((launch_batch<256, 1, 2>(ops, R, units, blocks, partial, partial_bytes, v, s))); break;
+    case 1: HZ_TRY((launch_batch<128, 2, 4>(ops, R, units, partial, partial_bytes, v, s))); break;
+    case 2: HZ_TRY((launch_batch<256, 1, 3>(ops, R, units, partial, partial_bytes, v, s))); break;
+    case 3: HZ_TRY((launch_batch<128, 2, 3>(ops, R, units, partial, partial_bytes, v, s))); break;
+    default: HZ_TRY((launch_batch<256, 1, 2>(ops, R, units, partial, partial_bytes, v, s))); break;
     }
     if (ev1) HZ_CHECK_CUDA(record_timing_event(ev1, s));
     return HZ_OK;
@@ -986,7 +1223,7 @@ int sweep_f32(const SweepConst &c, const Rec32 &r, const double4_32a *pos64, int
         if (b > sms * 8) b = sms * 8;
         prep32_kernel<<<(unsigned)b, 256, 0, s>>>(r.npad, r.perm, r.tpos, useA ? p_re : nullptr,
                                                   useA ? p_im : nullptr, useH ? pt_re : nullptr,
-                                                  useH ? pt_im : nullptr, scale, dens);
+                                                  useH ? pt_im : nullptr, scale, dens, r.done);
         HZ_CHECK_LAUNCH();
     }
     Args32 a;
@@ -1011,6 +1248,9 @@ int sweep_f32(const SweepConst &c, const Rec32 &r, const double4_32a *pos64, int
     a.err = c.err;
     if (ev0) HZ_CHECK_CUDA(record_timing_event(ev0, s));
     a.partial = r.partial;
+    a.cuts = r.cuts;
+    a.done = r.done;
+    a.sub = sub_of(r.npad / kTile32);
     const bool dir = c.dirichlet != 0;
     constexpr int S = SWEEP_SCALED;
     if (a.scaled) {
