@@ -10,13 +10,17 @@
 // BothCurvs, MeanCurv, GaussianCurv at the end of this file, built with
 // -ffp-contract=off so the host arithmetic is unfused as well).
 //
-// On GB300 these kernels are bound by the FP64 pipe (about 1.2 TFLOP/s,
-// roughly 1/60 of FP32), not by HBM: a node costs ~750 FP64 operations
-// (WENO weights need six IEEE divisions per axis, the cross derivatives
-// nine candidates per plane) against 48 bytes of compulsory traffic.  One
-// thread per node with read-only cached loads is therefore enough; the
-// neighbourhood is served by L1/L2.
+// On GB300 these kernels are bound by the FP64 pipe (1.65 lanes a clock an SM,
+// 1/69 of FP32), not by HBM: a node costs 233 FP64 instructions an axis and
+// about 500 for the curvatures when the reference's expressions are compiled as
+// they stand (55 IEEE divisions a node), against 48 bytes of compulsory traffic.
+// hz_build's grids take a rewritten form with the same bits (grid_kernel
+// below): 4.57 -> 2.84 ms at 128^3, about 620 instructions a node.
 #include "hz_internal.cuh"
+
+#include <cstdint>
+#include <cstring>
+
 #include "../../include/helmholtz_ref_api.h"
 
 namespace hz {
@@ -147,14 +151,20 @@ struct Plane {
     __host__ __device__ double operator()(int u, int v) const { return a(base + (long long)u * sa + (long long)v * sb); }
 };
 
-// finite_difference3D.c:393-721 (secondpartialxy/xz/yz).
+// finite_difference3D.c:393-721 (secondpartialxy/xz/yz): on the boundary and
+// next to it, and everywhere.
+template <class P_>
+__host__ __device__ double cross_edge(const P_ &P, int ca, int cb, int N, double H)
+{
+    if ((ca == 0) || (ca == N) || (cb == 0) || (cb == N)) return 0.0;
+    return (P(1, 1) - P(-1, 1) - P(1, -1) + P(-1, -1)) / (4.0 * H * H);
+}
+
 template <class P_>
 __host__ __device__ double cross(const P_ &P, int ca, int cb, int N, double H)
 {
     const double coef[3] = {1.0, -4.0, 3.0};
-    if ((ca == 0) || (ca == N) || (cb == 0) || (cb == N)) return 0.0;
-    if ((ca < 2) || (ca > N - 2) || (cb < 2) || (cb > N - 2))
-        return (P(1, 1) - P(-1, 1) - P(1, -1) + P(-1, -1)) / (4.0 * H * H);
+    if ((ca < 2) || (ca > N - 2) || (cb < 2) || (cb > N - 2)) return cross_edge(P, ca, cb, N, H);
     double fin = 1000000.0;  // LARGENUM
 #pragma unroll
     for (int di = 0; di < 3; di++)
@@ -238,10 +248,289 @@ __host__ __device__ __forceinline__ void grid_node(const A &acc, int N, double H
     }
 }
 
-__global__ void __launch_bounds__(256) grid_kernel(int N, double H, const double *__restrict__ d,
+// ---- the grids of hz_build: the same bits in 60 % of the FP64 instructions ----
+//
+// Every rounding of grid_node above is kept; what falls away is work done
+// twice and the generality of the compiled division.  A division's quotient
+// is corrected once by Markstein's theorem (P. Markstein, IBM J. Res. Dev.
+// 34(1), 1990; also Brisebarre, Muller and Raina, IEEE Trans. Comput. 53(8),
+// 2004): with y = RN(1/b) and q within one unit in the last place of a/b, the
+// residual a - q b is exact in one FMA and RN(q + (a - q b) y) = RN(a/b).
+// Operands far from 1, zeros, infinities and NaN (and divisors whose
+// significand is all ones, which the theorem for 1/b excludes) go through the
+// plain division.
+
+// FP64 exponent within [lo, hi) (biased), whatever the sign
+__device__ __forceinline__ bool exponent_in(double v, unsigned lo, unsigned hi)
+{
+    return (((unsigned)__double2hiint(v) >> 20) & 0x7ffu) - lo < hi - lo;
+}
+
+// RN(1 / b) for b > 0
+__device__ __forceinline__ double recip_rn(double b)
+{
+    // FP32 range (2^-120 .. 2^120), significand not all ones
+    if (!exponent_in(b, 903, 1143) || __double2hiint(b) < 0 || __double2loint(b) == -1) return 1.0 / b;
+    const int hi = __double2hiint(b);
+    const float bf = __int_as_float(((hi - (896 << 20)) << 3) | (int)((unsigned)__double2loint(b) >> 29));
+    float yf;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(bf));
+    const int yb = __float_as_int(yf);
+    const double y0 = __hiloint2double((yb >> 3) + (896 << 20), yb << 29);
+    // relative error 2^-22 -> 2^-65 before rounding: within one last place
+    const double e = __fma_rn(-b, y0, 1.0);
+    const double y1 = __fma_rn(y0, __fma_rn(e, e, e), y0);
+    return __fma_rn(__fma_rn(-b, y1, 1.0), y1, y1);
+}
+
+// RN(a / b), y = RN(1 / b), for 1/4 < a < 8: the first correction brings the
+// quotient within one last place, the second one rounds.
+__device__ __forceinline__ double quotient_rn(double a, double b, double y)
+{
+    if (!exponent_in(b, 903, 1143)) return a / b;
+    double q = a * y;
+    q = __fma_rn(__fma_rn(-b, q, a), y, q);
+    return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+
+// RN(x / c) for c = 3, 6 or 12 and z = RN(1 / c): RN(1/3) is off by a third
+// of the half-unit bound, which keeps x z within one last place of x / c.
+__device__ __forceinline__ double by_const(double x, double c, double z)
+{
+    if (!exponent_in(x, 123, 1923)) return x / c;
+    const double q = x * z;
+    return __fma_rn(__fma_rn(-c, q, x), z, q);
+}
+#define HZ_BY(x, c) by_const((x), (c), 1.0 / (c))
+
+// H^2 and 4 H^2 as divisors, with their reciprocals.
+struct Divisor {
+    double b, y;
+    int fast;
+};
+__device__ __forceinline__ double divide(double x, const Divisor &v)
+{
+    if (!v.fast || !exponent_in(x, 623, 1423)) return x / v.b;
+    double q = x * v.y;
+    q = __fma_rn(__fma_rn(-v.b, q, x), v.y, q);
+    return __fma_rn(__fma_rn(-v.b, q, x), v.y, q);
+}
+
+// WENO5 between nodes q and q + 1 of a line, from the second differences
+// s0..s3 at q - 1 .. q + 2: the smoothness terms and the weights 6/(..)^2 serve
+// D+ at q and D- at q + 1 alike (their differences enter squared, so the sign
+// that the two sides give them falls out), p0, p2 are D+'s two corrections at
+// q, n0, n2 D-'s at q + 1.
+struct Interface {
+    double p0, p2, n0, n2;
+};
+__device__ __forceinline__ Interface weno_interface(double s0, double s1, double s2, double s3)
+{
+    const double eps = 1e-12;
+    const double xb = s3 - s2, yb = s3 - 3. * s2, xa = s0 - s1, ya = s0 - 3. * s1, xc = s2 - s1, yc = s2 + s1;
+    const double ISb = 13. * xb * xb + 3. * yb * yb;
+    const double ISc = 13. * xc * xc + 3. * yc * yc;
+    const double ISa = 13. * xa * xa + 3. * ya * ya;
+    const double db = eps + ISb, dc = eps + ISc, da = eps + ISa;
+    const double Db = db * db, Dc = dc * dc, Da = da * da;
+    const double rb = recip_rn(Db), rc = recip_rn(Dc), ra = recip_rn(Da);
+    const double a1 = quotient_rn(6., Dc, rc);
+    const double b3 = quotient_rn(3., Db, rb), a3 = quotient_rn(3., Da, ra);
+    const double wp = recip_rn(rb + a1 + a3), wn = recip_rn(ra + a1 + b3);
+    Interface f;
+    f.p0 = HZ_BY(rb * wp * (__fma_rn(-2., s2, s3) + s1), 3.);
+    f.p2 = HZ_BY((a3 * wp - .5) * (__fma_rn(-2., s1, s2) + s0), 6.);
+    f.n0 = HZ_BY(ra * wn * (__fma_rn(-2., s1, s0) + s2), 3.);
+    f.n2 = HZ_BY((b3 * wn - .5) * (__fma_rn(-2., s2, s1) + s3), 6.);
+    return f;
+}
+
+// The upwind choice of distance_application3D.c:56-140 between D+ and D-, on
+// integers where no value is NaN or infinite (a comparison is an FP64
+// instruction too): outside (at > 0) the larger of -min(D+, 0) and max(D-, 0),
+// inside of max(D+, 0) and -min(D-, 0).
+__device__ __forceinline__ double upwind(double at, double Dp, double Dn)
+{
+    if (!exponent_in(at, 0, 2047) || !exponent_in(Dp, 0, 2047) || !exponent_in(Dn, 0, 2047)) {
+        const double pp = rmax(0.0, Dp), pm = rmin(0.0, Dp), np = rmax(0.0, Dn), nm = rmin(0.0, Dn);
+        return at > 0.0 ? ((fabs(pm) > fabs(np)) ? pm : np) : ((fabs(pp) > fabs(nm)) ? pp : nm);
+    }
+    const long long sign = __double_as_longlong(at) > 0 ? 0 : 1ll << 63;
+    const long long p = __double_as_longlong(Dp) ^ sign, n = __double_as_longlong(Dn) ^ sign;
+    // now D+ counts where p < 0, D- where n > 0
+    const long long pm = p < 0 ? p & ~(1ll << 63) : 0, np = n > 0 ? n : 0;
+    return pm > np ? Dp : (np != 0 ? Dn : 0.0);
+}
+
+// Upwind WENO5 derivative along one axis on `len` nodes of a line.
+__device__ __forceinline__ void gradient_segment(int N, double H, const double *__restrict__ d, long long base,
+                                                 long long stride, int c0, int c1, double *__restrict__ out)
+{
+    const double ih = 1. / H;
+    auto val = [&](int m) { return __ldg(d + base + (long long)mirror(m, N) * stride); };
+    // D_m = (v(m + 1) - v(m)) / H around node c: b, c_, d_, e = D_{c-2} .. D_{c+1}
+    double v = val(c0 - 3), w = val(c0 - 2), at = 0, next = 0;
+    double a = (w - v) * ih;
+    v = val(c0 - 1);
+    double b = (v - w) * ih;
+    at = val(c0);
+    double cc = (at - v) * ih;
+    next = val(c0 + 1);
+    double dd = (next - at) * ih;
+    double last = val(c0 + 2);
+    double ee = (last - next) * ih;
+    double s0 = b - a, s1 = cc - b, s2 = dd - cc, s3 = ee - dd;  // at c0 - 2 .. c0 + 1
+    Interface f = weno_interface(s0, s1, s2, s3);
+#pragma unroll 1
+    for (int c = c0; c < c1; c++) {
+        const double v3 = val(c + 3);
+        const double ff = (v3 - last) * ih;
+        const double df = HZ_BY(-b + 7. * (cc + dd) - ee, 12.);
+        const double n0 = f.n0, n2 = f.n2;
+        s0 = s1;
+        s1 = s2;
+        s2 = s3;
+        s3 = ff - ee;
+        f = weno_interface(s0, s1, s2, s3);
+        const double Dp = df + f.p0 + f.p2, Dn = df - n0 - n2;
+        out[base + (long long)c * stride] = upwind(at, Dp, Dn);
+        at = next;
+        next = last;
+        last = v3;
+        b = cc;
+        cc = dd;
+        dd = ee;
+        ee = ff;
+    }
+}
+
+// |cross| of an inner node: only its square is used, so the candidates are
+// formed up to their sign; products with 1, 4 and 16 are exact and ride in
+// FMAs, those with 3, 9 and 12 are shared by the candidates.  Magnitudes
+// compare as integers (a NaN is never the smallest).
+template <class P_>
+__device__ __forceinline__ double cross_inner(const P_ &P, const Divisor &hh4)
+{
+    unsigned long long best = (unsigned long long)__double_as_longlong(1000000.0);  // LARGENUM
+    auto take = [&](double v) {
+        const unsigned long long m = (unsigned long long)__double_as_longlong(fabs(v));
+        best = m < best ? m : best;
+    };
+    const double nine = 9.0 * P(0, 0);
+    double u3[2], u12[2], v3[2], v12[2], du0, dv0;
+#pragma unroll
+    for (int s = 0; s < 2; s++) {
+        const int t = s ? 1 : -1;
+        u3[s] = 3.0 * P(2 * t, 0);
+        u12[s] = 12.0 * P(t, 0);
+        v3[s] = 3.0 * P(0, 2 * t);
+        v12[s] = 12.0 * P(0, t);
+    }
+    du0 = 3.0 * (P(1, 0) - P(-1, 0));
+    dv0 = 3.0 * (P(0, 1) - P(0, -1));
+#pragma unroll
+    for (int si = 0; si < 2; si++)
+#pragma unroll
+        for (int sj = 0; sj < 2; sj++) {
+            const int i = si ? 1 : -1, j = sj ? 1 : -1;
+            double v = __fma_rn(-4.0, P(2 * i, j), P(2 * i, 2 * j)) + u3[si];
+            v = __fma_rn(-4.0, P(i, 2 * j), v);
+            v = __fma_rn(16.0, P(i, j), v) - u12[si];
+            take(((v + v3[sj]) - v12[sj]) + nine);
+        }
+#pragma unroll
+    for (int s = 0; s < 2; s++) {
+        const int t = s ? 1 : -1;
+        take(__fma_rn(-4.0, P(1, t) - P(-1, t), P(1, 2 * t) - P(-1, 2 * t)) + du0);
+        take(__fma_rn(-4.0, P(t, 1) - P(t, -1), P(2 * t, 1) - P(2 * t, -1)) + dv0);
+    }
+    take(P(1, 1) - P(-1, 1) - P(1, -1) + P(-1, -1));
+    return divide(__longlong_as_double((long long)best), hh4);
+}
+
+// der2 of an inner node: only the chosen difference is divided where one of
+// the conditions says which (the smooth case: the central one).
+template <class L_>
+__device__ __forceinline__ double der2_inner(const L_ &L, const Divisor &hh, bool xorder)
+{
+    const double l0 = L(0), p1 = L(1), n1 = L(-1), p2 = L(2), n2 = L(-2);
+    const double Dpp = p2 - p1, Dp = p1 - l0, Dn = l0 - n1, Dnn = n1 - n2;
+    const double DDc = divide(__fma_rn(-2.0, l0, p1) + n1, hh);
+    const bool up = Dp * Dnn <= 0.0, down = Dpp * Dn <= 0.0;
+    if (!up && !down) return DDc;
+    const double DDp = divide(__fma_rn(4.0, p2, 2.0 * l0 - 5.0 * p1) - L(3), hh);
+    const double DDn = divide(__fma_rn(4.0, n2, 2.0 * l0 - 5.0 * n1) - L(-3), hh);
+    if (up && down) {
+        const double a = DDp, b = xorder ? DDc : DDn, c3 = xorder ? DDn : DDc;
+        const double q = (fabs(a) < fabs(b)) ? a : b;
+        return (fabs(q) < fabs(c3)) ? q : c3;
+    }
+    const double q = up ? DDp : DDn;
+    return (fabs(q) < fabs(DDc)) ? q : DDc;
+}
+
+__device__ __forceinline__ void curvature_node(const double *__restrict__ d, int N, double H, const Divisor &hh,
+                                               const Divisor &hh4, int i, int j, int k, long long o,
+                                               double *__restrict__ mc, double *__restrict__ gc)
+{
+    const long long S = N + 1;
+    const GridAcc acc{d};
+    // The boundary's forms axis by axis: a node's other derivatives stay in step
+    // with its warp (a fourth of the warps hold a boundary node).
+    auto second = [&](const Line<GridAcc> &L, int c, bool xorder) {
+        return c >= 3 && c <= N - 3 ? der2_inner(L, hh, xorder) : der2(L, c, N, H, xorder);
+    };
+    auto mixed = [&](const Plane<GridAcc> &P, int ca, int cb) {
+        return ca >= 2 && ca <= N - 2 && cb >= 2 && cb <= N - 2 ? cross_inner(P, hh4) : cross_edge(P, ca, cb, N, H);
+    };
+    const double dxx = second(Line<GridAcc>{acc, o, S}, j, true);
+    const double dyy = second(Line<GridAcc>{acc, o, S * S}, i, false);
+    const double dzz = second(Line<GridAcc>{acc, o, 1}, k, false);
+    const double dxy = mixed(Plane<GridAcc>{acc, o, S * S, S}, i, j);
+    const double dxz = mixed(Plane<GridAcc>{acc, o, S, 1}, j, k);
+    const double dyz = mixed(Plane<GridAcc>{acc, o, S * S, 1}, i, k);
+    const double diag = dxx * dyy + dyy * dzz + dxx * dzz;
+    const double crs = dxy * dxy + dyz * dyz + dxz * dxz;
+    mc[o] = -0.5 * (dxx + dyy + dzz);
+    gc[o] = diag - crs;
+}
+
+// Blocks [0, 3 grad_blocks): a segment of a line a thread, the axes x, y, z in
+// turn (neighbouring threads take neighbouring lines); the rest: a node's
+// curvatures a thread.  Bound by the FP64 pipe: 116 instructions a node and
+// axis (233 in grid_node) and about 260 for the curvatures.
+__global__ void __launch_bounds__(128) grid_kernel(int N, double H, const double *__restrict__ d,
                                                    double *__restrict__ gx, double *__restrict__ gy,
                                                    double *__restrict__ gz, double *__restrict__ mc,
-                                                   double *__restrict__ gc, int order)
+                                                   double *__restrict__ gc, Divisor hh, Divisor hh4, int segs,
+                                                   long long grad_blocks)
+{
+    const long long S = N + 1;
+    if (blockIdx.x < 3 * grad_blocks) {
+        const int axis = (int)(blockIdx.x / grad_blocks);
+        const long long t = (blockIdx.x - axis * grad_blocks) * 128 + threadIdx.x;
+        if (t >= S * S * segs) return;
+        const int seg = (int)(t / (S * S));
+        const long long line = t - seg * (S * S), u = line / S, v = line - u * S;
+        const int c0 = (int)(seg * S / segs), c1 = (int)((seg + 1) * S / segs);
+        if (axis == 0)
+            gradient_segment(N, H, d, u * S * S + v, S, c0, c1, gx);
+        else if (axis == 1)
+            gradient_segment(N, H, d, u * S + v, S * S, c0, c1, gy);
+        else
+            gradient_segment(N, H, d, (u * S + v) * S, 1, c0, c1, gz);
+        return;
+    }
+    const long long o = (blockIdx.x - 3 * grad_blocks) * 128 + threadIdx.x;
+    if (o >= S * S * S) return;
+    const int k = (int)(o % S), j = (int)((o / S) % S), i = (int)(o / (S * S));
+    curvature_node(d, N, H, hh, hh4, i, j, k, o, mc, gc);
+}
+
+// The gradient by WENO3 (grid_node for every node).
+__global__ void __launch_bounds__(256) gradient3_kernel(int N, double H, const double *__restrict__ d,
+                                                        double *__restrict__ gx, double *__restrict__ gy,
+                                                        double *__restrict__ gz)
 {
     const long long S = N + 1;
     const long long total = S * S * S;
@@ -252,16 +541,10 @@ __global__ void __launch_bounds__(256) grid_kernel(int N, double H, const double
         const int j = (int)((o / S) % S);
         const int i = (int)(o / (S * S));
         double out[5];
-        grid_node(acc, N, H, i, j, k, o, order, gx != nullptr, mc != nullptr, out);
-        if (gx) {
-            gx[o] = out[0];
-            gy[o] = out[1];
-            gz[o] = out[2];
-        }
-        if (mc) {
-            mc[o] = out[3];
-            gc[o] = out[4];
-        }
+        grid_node(acc, N, H, i, j, k, o, 3, true, false, out);
+        gx[o] = out[0];
+        gy[o] = out[1];
+        gz[o] = out[2];
     }
 }
 
@@ -407,10 +690,29 @@ int launch_grid_stencils(int N, double H, const double *d, double *gx, double *g
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    long long blocks = (total + 255) / 256;
-    const long long cap = (long long)sms * 16;
-    if (blocks > cap) blocks = cap;
-    grid_kernel<<<(unsigned)blocks, 256, 0, s>>>(N, H, d, gx, gy, gz, mc, gc, order);
+    if (gx && order != 5) {
+        long long blocks = (total + 255) / 256;
+        const long long cap = (long long)sms * 16;
+        if (blocks > cap) blocks = cap;
+        gradient3_kernel<<<(unsigned)blocks, 256, 0, s>>>(N, H, d, gx, gy, gz);
+        HZ_CHECK_LAUNCH();
+        gx = nullptr;
+    }
+    if (!gx && !mc) return HZ_OK;
+    // Segments of about 16 nodes (a segment computes one interface more than it
+    // has nodes), shorter ones where those would leave the GPU short of threads.
+    long long segs = (S + 15) / 16;
+    while (segs < S && 3 * S * S * segs < 512LL * sms) segs++;
+    auto divisor = [](double b) {
+        uint64_t u;
+        memcpy(&u, &b, sizeof(u));
+        const unsigned e = (unsigned)(u >> 52);
+        return Divisor{b, 1.0 / b, e > 623 && e < 1423 && (u << 12) >> 12 != (1ull << 52) - 1};
+    };
+    const long long grad_blocks = gx ? (S * S * segs + 127) / 128 : 0;
+    const long long blocks = 3 * grad_blocks + (mc ? (total + 127) / 128 : 0);
+    grid_kernel<<<(unsigned)blocks, 128, 0, s>>>(N, H, d, gx, gy, gz, mc, gc, divisor(H * H), divisor(4.0 * H * H),
+                                                 (int)segs, grad_blocks);
     HZ_CHECK_LAUNCH();
     return HZ_OK;
 }
