@@ -15,6 +15,7 @@
 #include "hz_internal.cuh"
 #include "krylov_multi.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <complex>
 #include <vector>
@@ -22,74 +23,96 @@
 namespace hz {
 namespace {
 
-constexpr int kMB = 64;   // partial-sum blocks per column
+constexpr int kMB = 128;  // partial-sum blocks per column, at most
+constexpr int kMChunk = 256;  // vector elements of a block at a time
 constexpr int kMT = 256;
 constexpr int kMaxM = 128;
 
 // partial[(c * kMB + blk) * kMaxM + j] (complex) = block sum of
-// conj(V_j[col]) w[col] for the c-th active column col = cols[c], j < k.
-// Launched with exactly kMB blocks in x, so every partial slot is written.
+// conj(V_j[cols[c]]) w[cols[c]], j < k.  A warp takes every eighth pair of
+// vectors and keeps their sums in shared memory from chunk to chunk, so a block
+// needs no barrier between vectors (one vector after another with two barriers
+// each: 390 us at 16 columns of n = 27,700 and k about 50; the FP64 operations
+// alone take 170).
 __global__ void __launch_bounds__(kMT) mvh_kernel(int64_t n, int R, int k, const int *__restrict__ cols,
                                                   const double *__restrict__ vr, const double *__restrict__ vi,
                                                   const double *__restrict__ wr, const double *__restrict__ wi,
                                                   double *partial)
 {
-    __shared__ double sh[kMT / 32][2];
-    const int c = blockIdx.y, col = cols[c];
+    constexpr int E = kMChunk / 32;
+    __shared__ double acc[kMaxM * 2];
+    const int c = blockIdx.y, col = cols[c], warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t chunks = (n + kMChunk - 1) / kMChunk;
     const double *w0 = wr + (int64_t)col * n, *w1 = wi + (int64_t)col * n;
-    for (int j = 0; j < k; j++) {
-        const double *a0 = vr + ((int64_t)j * R + col) * n, *a1 = vi + ((int64_t)j * R + col) * n;
-        double s0 = 0.0, s1 = 0.0;
-        for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-            const double x0 = a0[i], x1 = a1[i], y0 = w0[i], y1 = w1[i];
-            s0 += x0 * y0 + x1 * y1;
-            s1 += x0 * y1 - x1 * y0;
+    const int64_t ch0 = blockIdx.x * chunks / gridDim.x, ch1 = (blockIdx.x + 1) * chunks / gridDim.x;
+    for (int64_t ch = ch0; ch < ch1; ch++) {
+        const int64_t base = ch * kMChunk + lane;
+        double y0[E], y1[E];
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const bool in = base + 32 * e < n;
+            y0[e] = in ? w0[base + 32 * e] : 0.0;
+            y1[e] = in ? w1[base + 32 * e] : 0.0;
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            s0 += __shfl_down_sync(0xffffffffu, s0, o);
-            s1 += __shfl_down_sync(0xffffffffu, s1, o);
-        }
-        if ((threadIdx.x & 31) == 0) {
-            sh[threadIdx.x >> 5][0] = s0;
-            sh[threadIdx.x >> 5][1] = s1;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double a = 0, b = 0;
-            for (int q = 0; q < kMT / 32; q++) {
-                a += sh[q][0];
-                b += sh[q][1];
+        for (int j = 2 * warp; j < k; j += 2 * (kMT / 32)) {
+            const bool two = j + 1 < k;
+            const double *a0 = vr + ((int64_t)j * R + col) * n, *a1 = vi + ((int64_t)j * R + col) * n;
+            const int64_t next = two ? (int64_t)R * n : 0;
+            double s0 = 0.0, s1 = 0.0, t0 = 0.0, t1 = 0.0;
+#pragma unroll
+            for (int e = 0; e < E; e++) {
+                const int64_t i = base + 32 * e;
+                if (i < n) {
+                    const double x0 = a0[i], x1 = a1[i], u0 = a0[next + i], u1 = a1[next + i];
+                    s0 += x0 * y0[e] + x1 * y1[e];  // conj(v) w
+                    s1 += x0 * y1[e] - x1 * y0[e];
+                    t0 += u0 * y0[e] + u1 * y1[e];
+                    t1 += u0 * y1[e] - u1 * y0[e];
+                }
             }
-            double *p = partial + (((int64_t)c * kMB + blockIdx.x) * kMaxM + j) * 2;
-            p[0] = a;
-            p[1] = b;
+            // fold the four sums over the lanes, halves first (as gmres.cu)
+            const bool up = lane & 16, up2 = lane & 8;
+            double p = up ? t0 : s0, q = up ? t1 : s1;
+            p += __shfl_xor_sync(0xffffffffu, up ? s0 : t0, 16);
+            q += __shfl_xor_sync(0xffffffffu, up ? s1 : t1, 16);
+            double r = up2 ? q : p;
+            r += __shfl_xor_sync(0xffffffffu, up2 ? p : q, 8);
+            for (int o = 4; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+            // lane 0: Re s, 8: Im s, 16: Re t, 24: Im t; always this warp's slots
+            if ((lane & 7) == 0 && (two || !up)) {
+                double *o = acc + 2 * (j + (up ? 1 : 0)) + (up2 ? 1 : 0);
+                *o = ch == ch0 ? r : *o + r;
+            }
         }
-        __syncthreads();
     }
+    __syncthreads();
+    double *p = partial + ((int64_t)c * kMB + blockIdx.x) * kMaxM * 2;
+    for (int q = threadIdx.x; q < 2 * k; q += kMT) p[q] = acc[q];
 }
 
-// h[c][j] from the partials in block order; also into (pass 0) or added to
+// h[c][j] from the partials (one warp each, a fixed order); also into (pass 0) or added to
 // (pass 1) hsum[c][j].
-__global__ void mvh_reduce_kernel(int k, const double *partial, double *h, double *hsum, int pass)
+__global__ void __launch_bounds__(128) mvh_reduce_kernel(int k, int nb, const double *__restrict__ partial, double *h,
+                                                         double *hsum, int pass)
 {
-    const int c = blockIdx.x, j = threadIdx.x;
+    const int c = blockIdx.y, j = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (j >= k) return;
     double a = 0, b = 0;
-    for (int q = 0; q < kMB; q++) {
+    for (int q = lane; q < nb; q += 32) {
         const double *p = partial + (((int64_t)c * kMB + q) * kMaxM + j) * 2;
         a += p[0];
         b += p[1];
     }
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    if (lane) return;
     double *o = h + ((int64_t)c * kMaxM + j) * 2, *t = hsum + ((int64_t)c * kMaxM + j) * 2;
     o[0] = a;
     o[1] = b;
-    if (pass) {
-        t[0] += a;
-        t[1] += b;
-    } else {
-        t[0] = a;
-        t[1] = b;
-    }
+    t[0] = pass ? t[0] + a : a;
+    t[1] = pass ? t[1] + b : b;
 }
 
 // w[col] -= sum_j V_j[col] h[c][j]
@@ -101,6 +124,7 @@ __global__ void mvupdate_kernel(int64_t n, int R, int k, const int *__restrict__
     double *w0 = wr + (int64_t)col * n, *w1 = wi + (int64_t)col * n;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         double a = w0[i], b = w1[i];
+#pragma unroll 4
         for (int j = 0; j < k; j++) {
             const double x0 = vr[((int64_t)j * R + col) * n + i], x1 = vi[((int64_t)j * R + col) * n + i];
             const double h0 = hc[2 * j], h1 = hc[2 * j + 1];
@@ -137,6 +161,7 @@ __global__ void mxupdate_kernel(int64_t n, int R, int k, const int *__restrict__
     double *x0 = xr + (int64_t)col * n, *x1 = xi + (int64_t)col * n;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         double a = x0[i], b = x1[i];
+#pragma unroll 4
         for (int j = 0; j < k; j++) {
             const double v0 = vr[((int64_t)j * R + col) * n + i], v1 = vi[((int64_t)j * R + col) * n + i];
             a += v0 * yc[2 * j] - v1 * yc[2 * j + 1];
@@ -201,6 +226,7 @@ int gmres_multi_solve(MultiOp &A, int64_t n, int R, int m, const double *b_re, c
     double *ndev = ydev + hsz;
     int *cdev = reinterpret_cast<int *>(ndev + 2 * R);
     const int gx = mblocks(n);
+    const int nb = (int)std::max<int64_t>(1, std::min<int64_t>(kMB, (n + kMChunk - 1) / kMChunk));
     std::vector<double> hh(hsz), hn_host(hsz), nrm(R);
     std::vector<Col> C(R);
     std::vector<int> act;  // active columns (device list order)
@@ -217,9 +243,9 @@ int gmres_multi_solve(MultiOp &A, int64_t n, int R, int m, const double *b_re, c
         const int a = (int)cl.size();
         HZ_CHECK_CUDA(cudaMemcpyAsync(cdev, cl.data(), a * sizeof(int), cudaMemcpyHostToDevice, s));
         // conj(w) w: the basis pointer is w itself at "j = 0" with R = 0 stride
-        mvh_kernel<<<dim3(kMB, a), kMT, 0, s>>>(n, 0, 1, cdev, wr, wi, wr, wi, partial);
+        mvh_kernel<<<dim3(nb, a), kMT, 0, s>>>(n, 0, 1, cdev, wr, wi, wr, wi, partial);
         HZ_CHECK_LAUNCH();
-        mvh_reduce_kernel<<<a, kMaxM, 0, s>>>(1, partial, hdev, hsum, 0);
+        mvh_reduce_kernel<<<dim3(1, a), 128, 0, s>>>(1, nb, partial, hdev, hsum, 0);
         HZ_CHECK_LAUNCH();
         HZ_CHECK_CUDA(cudaMemcpyAsync(hn_host.data(), hdev, (size_t)a * kMaxM * 2 * sizeof(double),
                                       cudaMemcpyDeviceToHost, s));
@@ -307,9 +333,9 @@ int gmres_multi_solve(MultiOp &A, int64_t n, int R, int m, const double *b_re, c
             const int a = (int)cyc.size();
             HZ_CHECK_CUDA(cudaMemcpyAsync(cdev, cyc.data(), a * sizeof(int), cudaMemcpyHostToDevice, s));
             for (int pass = 0; pass < 2; pass++) {
-                mvh_kernel<<<dim3(kMB, a), kMT, 0, s>>>(n, R, k + 1, cdev, vr, vi, wr, wi, partial);
+                mvh_kernel<<<dim3(nb, a), kMT, 0, s>>>(n, R, k + 1, cdev, vr, vi, wr, wi, partial);
                 HZ_CHECK_LAUNCH();
-                mvh_reduce_kernel<<<a, kMaxM, 0, s>>>(k + 1, partial, hdev, hsum, pass);
+                mvh_reduce_kernel<<<dim3((k + 4) / 4, a), 128, 0, s>>>(k + 1, nb, partial, hdev, hsum, pass);
                 HZ_CHECK_LAUNCH();
                 mvupdate_kernel<<<dim3(gx, a), kMT, 0, s>>>(n, R, k + 1, cdev, vr, vi, hdev, wr, wi);
                 HZ_CHECK_LAUNCH();
