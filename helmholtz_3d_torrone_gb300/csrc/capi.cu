@@ -639,7 +639,9 @@ int hz_build(hz_operator *op, int64_t *n_out)
                      op->w.as<double>(), op->pos64.as<double4_32a>(), op->nrm64.as<double4_32a>(), op->err.as<unsigned>(), s,
                      op->dreg.as<double>()));
     HZ_TRY(check_device_error(op, "hz_build"));
-    if (op->p.wave >= 1.0) {
+    const SweepConst sc = sweep_const(op);
+    op->use_split = split_serves(n, sc.wave, op->H, sc.extent);
+    if (op->p.wave >= 1.0 && !op->use_split) {  // records of the scaled sweep in FP64 instructions
         HZ_TRY(op->posk64.ensure(nn * sizeof(double4_32a)));
         HZ_TRY(scale_records64(n, op->p.wave, op->pos64.as<double4_32a>(), op->posk64.as<double4_32a>(), s));
     } else {
@@ -647,8 +649,6 @@ int hz_build(hz_operator *op, int64_t *n_out)
     }
     const double lambda = lambda32(op->p.wave);
     HZ_TRY(build_records32(op, lambda, sweep32_reg_scale(op->p.interior, lambda)));
-    const SweepConst sc = sweep_const(op);
-    op->use_split = split_serves(n, sc.wave, op->H, sc.extent);
     if (op->use_split) {
         HZ_TRY(op->split64.ensure(split_record_bytes(op->r32.npad)));
         op->split = split_record_views(op->split64.ptr, op->r32);

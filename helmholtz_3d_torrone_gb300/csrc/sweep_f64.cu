@@ -1,4 +1,5 @@
-// sweep_f64.cu -- FP64 matrix-free pair sweep: q = A p, qt = A^H pt.
+// sweep_f64.cu -- FP64 matrix-free pair sweep in FP64 instructions: q = A p,
+// qt = A^H pt, for the operators that sweep_split.cu does not serve.
 //
 // The operator is the reference's omp_get_Ccomp entry (large3Dexample2.c:
 // 4463-4564) applied on the fly:
