@@ -32,6 +32,7 @@ constexpr int SPLIT_DK = 8;
 
 struct ArgsSplit {
     int64_t npad, units;
+    int part;                   // sources per unit: 128 or 64 (launch_split)
     int64_t nctas;
     float tau2, ktau;
     double wave, tau;
@@ -356,12 +357,12 @@ __device__ __forceinline__ void split_pair(const ArgsSplit &a, const float4 (*st
 }
 
 template <int MODE, bool DIR, bool CLOSE>
-__device__ __forceinline__ void split_half(const ArgsSplit &a, const float4 (*st)[kHalf], const float2 *tab,
+__device__ __forceinline__ void split_part(const ArgsSplit &a, const float4 (*st)[kHalf], const float2 *tab,
                                            const Offsets &t, const TargetNormal &tn, FF treg, const TileUnits &u,
                                            int64_t tslot, int64_t sslot0, double (&dA)[2], double (&dH)[2])
 {
 #pragma unroll 1
-    for (int j0 = 0; j0 < kHalf; j0 += kRun) {
+    for (int j0 = 0; j0 < a.part; j0 += kRun) {
         FF accA[2] = {{0.f, 0.f}, {0.f, 0.f}}, accH[2] = {{0.f, 0.f}, {0.f, 0.f}};
 #pragma unroll 1
         for (int j = j0; j < j0 + kRun; j++)
@@ -501,7 +502,8 @@ __global__ void __launch_bounds__(kTile32, 2) sweep_split_kernel(ArgsSplit a)
     __shared__ alignas(8) uint64_t bar[2];
     float2 *tab = reinterpret_cast<float2 *>(smem);
     float4(*stage)[kHalf] = reinterpret_cast<float4(*)[kHalf]>(smem + kSplitTable * sizeof(float2));
-    const int64_t halves = a.npad / kHalf;
+    const int64_t parts = a.npad / a.part;
+    const int last = kTile32 / a.part - 1;  // parts of a tile less one: 1 or 3
     const int64_t u_begin = (int64_t)blockIdx.x * a.units / a.nctas;
     const int64_t u_end = ((int64_t)blockIdx.x + 1) * a.units / a.nctas;
     if (threadIdx.x == 0) {
@@ -514,8 +516,8 @@ __global__ void __launch_bounds__(kTile32, 2) sweep_split_kernel(ArgsSplit a)
     __syncthreads();
     if (u_begin >= u_end) return;
     auto issue = [&](int64_t u, int buf) {
-        const int64_t base = (u % halves) * kHalf;
-        const uint32_t bytes = kHalf * sizeof(float4);
+        const int64_t base = (u % parts) * a.part;
+        const uint32_t bytes = a.part * (uint32_t)sizeof(float4);
         mbar_arrive_expect_tx(&bar[buf], NA * bytes);
 #pragma unroll
         for (int r = 0; r < kRecs; r++) bulk_g2s(&stage[buf * NA + r][0], a.rec + r * a.npad + base, bytes, &bar[buf]);
@@ -525,9 +527,9 @@ __global__ void __launch_bounds__(kTile32, 2) sweep_split_kernel(ArgsSplit a)
     if (threadIdx.x == 0) issue(u_begin, 0);
     int seg = 0;
     for (int64_t u = u_begin; u < u_end;) {
-        const int64_t blk = u / halves;
-        const int64_t seg_end = (u_end < (blk + 1) * halves) ? u_end : (blk + 1) * halves;
-        const bool whole = (u == blk * halves) && (seg_end == (blk + 1) * halves);
+        const int64_t blk = u / parts;
+        const int64_t seg_end = (u_end < (blk + 1) * parts) ? u_end : (blk + 1) * parts;
+        const bool whole = (u == blk * parts) && (seg_end == (blk + 1) * parts);
         const int64_t slot = blk * kTile32 + threadIdx.x;
         const double4_32a to = a.tile[blk];
         double X, Y, Z, nx, ny, nz;
@@ -544,8 +546,8 @@ __global__ void __launch_bounds__(kTile32, 2) sweep_split_kernel(ArgsSplit a)
             const int64_t it = u - u_begin;
             const int buf = (int)(it & 1);
             if (threadIdx.x == 0 && u + 1 < u_end) issue(u + 1, buf ^ 1);
-            const int64_t half = u - blk * halves, tile = half >> 1;
-            if (fresh || !(half & 1)) {
+            const int64_t part = u - blk * parts, tile = part >> (last == 1 ? 1 : 2);
+            if (fresh || (part & last) == 0) {
                 fresh = false;
                 set_tile<TGT>(a, tile, to, X, Y, Z, nx, ny, nz, tab, t, un, close, phr, phi);
             }
@@ -559,10 +561,10 @@ __global__ void __launch_bounds__(kTile32, 2) sweep_split_kernel(ArgsSplit a)
                 return;
             }
             if (close)
-                split_half<MODE, DIR, true>(a, stage + buf * NA, tab, t, tn, treg, un, slot, half * kHalf, dA, dH);
+                split_part<MODE, DIR, true>(a, stage + buf * NA, tab, t, tn, treg, un, slot, part * a.part, dA, dH);
             else
-                split_half<MODE, DIR, false>(a, stage + buf * NA, tab, t, tn, treg, un, slot, half * kHalf, dA, dH);
-            if ((half & 1) || u + 1 == seg_end) {
+                split_part<MODE, DIR, false>(a, stage + buf * NA, tab, t, tn, treg, un, slot, part * a.part, dA, dH);
+            if ((part & last) == last || u + 1 == seg_end) {
                 if (close) {
                     q[0] += dA[0];
                     q[1] += dA[1];
@@ -601,13 +603,13 @@ template <int MODE>
 __global__ void __launch_bounds__(4 * kFixSlots) split_fixup_kernel(ArgsSplit a)
 {
     __shared__ double4_32a part[3][kFixSlots];
-    const int64_t blk = blockIdx.x, halves = a.npad / kHalf;
+    const int64_t blk = blockIdx.x, parts = a.npad / a.part;
     auto cta_of = [&](int64_t u) { return ((u + 1) * a.nctas - 1) / a.units; };
-    const int64_t c_lo = cta_of(blk * halves), c_hi = cta_of((blk + 1) * halves - 1);
+    const int64_t c_lo = cta_of(blk * parts), c_hi = cta_of((blk + 1) * parts - 1);
     if (c_lo == c_hi) return;
     const int g = threadIdx.x / kFixSlots, s = threadIdx.x % kFixSlots, slot = blockIdx.y * kFixSlots + s;
     // only the first CTA can have begun in an earlier tile (its slot 1)
-    const int first = (c_lo * a.units / a.nctas) / halves == blk ? 0 : 1;
+    const int first = (c_lo * a.units / a.nctas) / parts == blk ? 0 : 1;
     double q[4] = {0, 0, 0, 0};
 #pragma unroll 4
     for (int64_t c = c_lo + g; c <= c_hi; c += 4) {
@@ -919,10 +921,15 @@ int launch_split(ArgsSplit a, size_t partial_bytes, cudaStream_t s)
     HZ_CHECK_CUDA(cudaFuncSetAttribute(sweep_split_kernel<MODE, DIR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem));
     const int64_t tiles = a.npad / kTile32;
-    a.units = tiles * (a.npad / kHalf);
     int64_t p = 2 * (int64_t)sm_count();
     const int64_t room = (int64_t)(partial_bytes / (2 * kTile32 * sizeof(double4_32a)));
     if (p > room) p = room;
+    // Units of 128 sources, or of 64 where that takes a tenth off the fullest
+    // CTA's share (n = 3,168: 392 units on 304 CTAs, 0.171 -> 0.138 ms; a unit's
+    // end costs 2 % of 64 sources, so elsewhere 128).
+    auto share = [&](int64_t part) { return (tiles * (a.npad / part) + p - 1) / p * part; };
+    a.part = p > 0 && 11 * share(64) < 10 * share(kHalf) ? 64 : kHalf;
+    a.units = tiles * (a.npad / a.part);
     if (p > a.units) p = a.units;
     if (p < 1) {
         set_error("split FP64 sweep: partial buffer too small");
