@@ -8,10 +8,9 @@ R=0.6, r=0.25 sampled as its analytic signed distance on a 256^3 grid over
 
 The headline ``value`` is the wall time of one complete solve of that
 system to an FP64 relative residual below 1e-6: FP32 inner GMRES(120)
-solves (one FP32 pair sweep per iteration, tile-local origins, phase k rho
-reduced with a split k/(2 pi) before the SFU sin/cos) inside FP64
-iterative refinement whose residual b - A x comes from the FP64 pair
-sweep.  It replaces the reference's
+solves (one FP32 pair sweep per iteration, tile-local origins, the phase
+k rho taken about the source tile) inside FP64 iterative refinement whose
+residual b - A x comes from the FP64 pair sweep (split FP32 arithmetic).  It replaces the reference's
 parallel_BiCGcomplex (large3Dexample2.c:2954-3514).  ``e2e`` is the same
 solve through the public C ABI with host buffers (H2D of b, D2H of x inside
 the timed region).
@@ -19,9 +18,8 @@ the timed region).
 Beside it: the plain FP64 GPU solve with the same method (measured seconds
 of one FP64 product x the product count of a complete FP64 GMRES(120)
 solve of this workload, measured once with ``--solve --fp64-full`` and
-recorded in FP64_SOLVE_ITERS), the roofline of the FP64 sweep (the kernel
-that takes most of the solve's time: two FP64 residual products), and the
-FP32 sweep's rate and roofline over ``--steps`` timed inner iterations (L2
+recorded in FP64_SOLVE_ITERS), the roofline of the sweep that takes most of
+the solve's time and of the other one, and the FP32 sweep's rate over ``--steps`` timed inner iterations (L2
 flushed between them).
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl gb300|reference]
@@ -78,7 +76,9 @@ SWEEP32_TRAFFIC = 22.36e6 * 581420 / 145272
 # the 128^3 torus, scaled by n.
 SWEEP32_TRAFFIC_A = 15.19e6 * 581420 / 145272
 SWEEP64_TRAFFIC = 16.5e6 * 581420 / 145272  # ncu DRAM read of the FP64 sweep at 128^3, scaled by n
-FP64_OPS_PER_PAIR = 38.5  # FP64 instructions per pair of the A-mode FP64 sweep (ncu, 128^3 torus, scaled records)
+# FP32-pipe slots per pair of the A-mode FP64 sweep, which works in pairs of
+# FP32 numbers and 64-bit integers (counted in the source)
+FP64_SLOTS_PER_PAIR = 215
 
 
 def parse():
@@ -109,7 +109,7 @@ def parse():
                     help="--solve: inner Krylov method(s) of the refined solves")
     ap.add_argument("--restart", type=int, default=40, help="--solve: GMRES restart length")
     ap.add_argument("--phase", choices=["direct", "split"], default="split",
-                    help="--solve: phase mode of the FP32 sweeps (hz_set_phase_mode; split is the library default)")
+                    help="--solve: hz_set_phase_mode (both settings run the same sweep)")
     ap.add_argument("--inner-tol", type=float, default=INNER_TOL,
                     help="--solve: tightest inner FP32 tolerance of the refined solves")
     ap.add_argument("--save", default="",
@@ -184,7 +184,7 @@ def workload_desc(N, wave, n):
 
 def solve_desc():
     return {"tol": SOLVE_TOL, "inner_tol_floor": INNER_TOL, "method": "gmres(%d)" % RESTART,
-            "fp32_phase": "k rho reduced with a split k/(2 pi) (the library default)",
+            "fp32_phase": "k rho about the source tile's origin",
             "value": "seconds of one complete solve to FP64 relative residual < tol: FP32 inner GMRES (one FP32 "
                      "sweep A p per iteration) inside FP64 iterative refinement (residual b - A x from the FP64 "
                      "sweep); b resident in HBM, CUDA events on the operator's stream, run once after the step loop",
@@ -443,7 +443,7 @@ def run_gb300(a, rank, world, local):
                "solve_products": fp64_solve_products(N, wave),
                "solve_s_extrapolated": (per_prod * fp64_solve_products(N, wave)
                                         if fp64_solve_products(N, wave) else None),
-               "how": "measured seconds of one FP64 product (sweep64_kernel, CUDA events) x the product count of "
+               "how": "measured seconds of one FP64 product (sweep_split_kernel, CUDA events) x the product count of "
                       "a complete FP64 GMRES(%d) solve of this workload to the same tol, measured once (bench.py "
                       "--solve --fp64-full); GMRES adds only FP64 Gram-Schmidt (milliseconds) per product" % RESTART}
         if f64["solve_s_extrapolated"]:
@@ -465,16 +465,16 @@ def run_gb300(a, rank, world, local):
     roof64 = None
     if f64:
         a64 = float(n) * n * FLOPS_PER_PAIR / f64["seconds_per_product"] / 1e12
-        roof64 = {"bound": "fp64", "kernel": "sweep64_kernel (A x, the FP64 refinement residual)",
-                  "achieved": a64, "peak": fp64_peak, "unit": "TFLOP/s", "frac": a64 / fp64_peak,
-                  "fp64_ops_per_pair": FP64_OPS_PER_PAIR,
-                  "pipe_frac": float(n) * n * FP64_OPS_PER_PAIR / f64["seconds_per_product"] / (fp64_peak * 0.5e12),
-                  "note": "frac counts the reference formula's 40 flops per pair against the DFMA peak (2 flops per "
-                          "instruction); pipe_frac counts the FP64 instructions the kernel executes (ncu) against "
-                          "the pipe's instruction rate (peak / 2)",
+        roof64 = {"bound": "fp32", "kernel": "sweep_split_kernel (A x, the FP64 refinement residual)",
+                  "achieved": a64, "peak": fp32_peak, "unit": "TFLOP/s", "frac": a64 / fp32_peak,
+                  "fp64_peak": fp64_peak, "fp32_slots_per_pair": FP64_SLOTS_PER_PAIR,
+                  "pipe_frac": float(n) * n * FP64_SLOTS_PER_PAIR / f64["seconds_per_product"] / (fp32_peak * 0.5e12),
+                  "note": "FP64 products in split FP32 arithmetic: frac counts the reference formula's 40 flops per "
+                          "pair against the FP32 FFMA peak (2 flops per instruction); pipe_frac counts the FP32-pipe "
+                          "slots the kernel takes against the pipe's instruction rate (peak / 2)",
                   "traffic": SWEEP64_TRAFFIC, "flops_per_pair": FLOPS_PER_PAIR, "pairs_per_launch": n * n,
                   "avg_launch_ms": f64["seconds_per_product"] * 1e3, "launches_timed": a.fp64_iters,
-                  "peak_source": "FP64 DFMA chains measured live on this GPU (hz_measure_fma_peaks)",
+                  "peak_source": "FP32 FFMA chains measured live on this GPU (hz_measure_fma_peaks)",
                   "share_of_solve": sinfo["outer"] * f64["seconds_per_product"] / solve_s}
     # the roofline of the kernel that takes most of the timed solve
     if roof64 and (roof64["share_of_solve"] or 0) > (roof32["share_of_solve"] or 0):
