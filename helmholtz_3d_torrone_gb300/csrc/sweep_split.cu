@@ -5,10 +5,10 @@
 // FP64 instructions (about 2,600 slots) of sweep64_kernel.
 //
 // One thread owns one target of the blocked sweep order (Rec32::perm); a CTA
-// of 256 threads walks a contiguous range of (target tile, half source tile)
-// units, as sweep32_kernel does, so the chip is full from a few thousand
-// points on.  Half tiles of 128 sources (96 bytes of fixed record and 16 of
-// density each) come by TMA bulk copies, double-buffered on mbarriers with
+// of 256 threads walks a contiguous range of (target tile, half or quarter
+// source tile) units, as sweep32_kernel does, so the chip is full from a few
+// thousand points on.  Units of 128 or 64 sources (96 bytes of fixed record
+// and 16 of density each) come by TMA bulk copies, double-buffered on mbarriers with
 // bounded waits; the cosine table takes 64 KB of shared memory, which leaves
 // room for two CTAs an SM.  Per target and source tile about 50 FP64
 // instructions set up the offsets and the phase of the tile's origin; they and
