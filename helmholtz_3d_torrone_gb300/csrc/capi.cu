@@ -640,7 +640,7 @@ int hz_build(hz_operator *op, int64_t *n_out)
                      op->dreg.as<double>()));
     HZ_TRY(check_device_error(op, "hz_build"));
     const SweepConst sc = sweep_const(op);
-    op->use_split = split_serves(n, sc.wave, op->H, sc.extent);
+    op->use_split = split_serves(n, sc.wave, op->H, op->tau, sc.extent);
     if (op->p.wave >= 1.0 && !op->use_split) {  // records of the scaled sweep in FP64 instructions
         HZ_TRY(op->posk64.ensure(nn * sizeof(double4_32a)));
         HZ_TRY(scale_records64(n, op->p.wave, op->pos64.as<double4_32a>(), op->posk64.as<double4_32a>(), s));

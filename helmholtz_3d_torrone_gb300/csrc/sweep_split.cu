@@ -230,6 +230,7 @@ struct TileUnits {
     int x;               // close tiles: extra shift that keeps r^2 below 2^62
     float w32, w8;       // 2^32 and 2^8 units of W
     float r32, r8;       // the same after the extra shift
+    float lo, hi;        // close tiles: r^2 in [lo, hi] is formed again from the FP64 coordinates
     float n32, n8;       // 2^32 and 2^8 units of A.n
 };
 
@@ -260,11 +261,13 @@ __device__ __forceinline__ void split_entry(const ArgsSplit &a, const float4 (*s
     if (CLOSE) {
         r2 = ff_of_int((W >> u.x) + t.a2i, u.r32, u.r8, e);
         far = r2.h > a.tau2;
-        if (fabsf(fsub(r2.h, a.tau2)) <= 1e-6f * a.tau2) {
+        if (r2.h >= u.lo && r2.h <= u.hi) {
             // decided as the reference does: rho^2 without fused operations
             const double4_32a p = a.tpos[tslot], q = a.tpos[sslot];
             const double dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-            far = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz))) > a.tau;
+            const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+            far = __dsqrt_rn(d2) > a.tau;
+            r2 = ff_of_double(a.wave * (a.wave * d2));
         }
     } else {
         w = ff_of_int(W, u.w32, u.w8, e);
@@ -426,6 +429,15 @@ __device__ __forceinline__ void set_tile(const ArgsSplit &a, int64_t tile, const
     const double a2 = 0.25 * fma(az, az, fma(ay, ay, ax * ax));
     if (close) {
         t.a2i = __double2ll_rn(a2 * pow2d(60 - eL - eS - un.x));
+        // r^2 is off by less than 2^-52 of 2^(eL + eS + x) (typically a quarter of
+        // that), whatever its size.  Below 2^-9 of that (rho below 1/8 to 1/16
+        // of the tile's radius) it would be off by more than 2^-43 of itself and
+        // is formed again, as it is next to tau^2: on the 64^3 sphere (tiles of
+        // 10 h, tau = 2 h) a lane in 0.02 % of a warp's steps.  (From 2^-8 on,
+        // 0.6 % of the steps: 3 to 9 % more time.)
+        const float off = pow2f(eL + eS + un.x - 52);
+        un.lo = a.tau2 - fmaxf(1e-6f * a.tau2, off);
+        un.hi = fmaxf(a.tau2 + 1e-6f * a.tau2, pow2f(eL + eS + un.x - 9));
     } else {
         const double y0 = (double)rsqrt_seed((float)a2);
         const double e = fma(-(a2 * y0), y0, 1.0);
@@ -973,10 +985,14 @@ RecSplit split_record_views(void *mem, const Rec32 &r)
 // wavelength) keeps the phases within a tile small, so the error stays at or
 // below the FP64 sweep's (at k h = 1, 4.5e-15 against 4.2e-15); k >= 1/64
 // keeps 1/(k rho)^3 far inside the FP32 range; below 2048 points the FP64
-// sweep's error (2e-15 and less) is the smaller one.
-bool split_serves(int64_t n, double wave, double H, double extent)
+// sweep's error (2e-15 and less) is the smaller one.  tau >= h: the projection
+// (x_t - x_s).n carries an error of 2^-51 of the tile's radius (10 to 30 h),
+// which is 2^-46 of the nearest far pairs' entries at rho = h and would grow as
+// 1 / rho below (the FP64 sweep keeps that at k below 1, where it subtracts the
+// unscaled coordinates).
+bool split_serves(int64_t n, double wave, double H, double tau, double extent)
 {
-    return n >= 2048 && wave >= 1.0 / 64 && wave * H <= 0.8 && wave * extent < 4000.0;
+    return n >= 2048 && wave >= 1.0 / 64 && wave * H <= 0.8 && tau >= H && wave * extent < 4000.0;
 }
 
 int build_split_records(const SweepConst &c, const RecSplit &v, const Rec32 &r, const double4_32a *pos,
