@@ -160,16 +160,18 @@ __global__ void __launch_bounds__(256) split_max_kernel(int64_t n, const double4
 }
 
 // Densities scaled to at most 1 and split: -k^2 sg/(8 pi) w p for A (the
-// entries carry -2 (x_t - x_s).n), +k^2 sg/(8 pi) pt for A^H; the scale's
-// exponents go to expo.
+// entries carry -2 (x_t - x_s).n), +k^2 sg/(8 pi) pt for A^H.  The exponents
+// taken out, the densities' and k^2's (k^2 sg/(8 pi) = scale 2^scale_exp), go to
+// expo: what is left lies in the FP32 range whatever the unit of length.
 __global__ void __launch_bounds__(256) split_dens_kernel(int64_t npad, const int *__restrict__ perm,
                                                          const double4_32a *__restrict__ tpos,
                                                          const double *__restrict__ p_re,
                                                          const double *__restrict__ p_im,
                                                          const double *__restrict__ pt_re,
                                                          const double *__restrict__ pt_im, double scale,
-                                                         const int *__restrict__ part, int *__restrict__ expo,
-                                                         float4 *__restrict__ densA, float4 *__restrict__ densH)
+                                                         int scale_exp, const int *__restrict__ part,
+                                                         int *__restrict__ expo, float4 *__restrict__ densA,
+                                                         float4 *__restrict__ densH)
 {
     __shared__ int ex[2];
     if (threadIdx.x < 64) {
@@ -182,7 +184,7 @@ __global__ void __launch_bounds__(256) split_dens_kernel(int64_t npad, const int
         e = max(-1000, min(1000, e));
         if ((threadIdx.x & 31) == 0) {
             ex[m] = e;
-            if (blockIdx.x == 0) expo[m] = e;
+            if (blockIdx.x == 0) expo[m] = e + scale_exp;
         }
     }
     __syncthreads();
@@ -488,13 +490,13 @@ __device__ __forceinline__ void split_write(const ArgsSplit &a, int64_t s, doubl
     const int c = a.perm[s];
     if (c < 0) return;
     if (MODE & SWEEP_A) {
-        const double f = pow2d(a.expo[0]), r = f * ar, i = f * ai;
+        const double r = ldexp(ar, a.expo[0]), i = ldexp(ai, a.expo[0]);
         if (!(MODE & SPLIT_DK) && (!isfinite(r) || !isfinite(i))) atomicOr(a.err, DEV_ERR_NONFINITE);
         a.q_re[c] = (MODE & SPLIT_DK) ? r : r + 0.5 * a.p_re[c];
         a.q_im[c] = (MODE & SPLIT_DK) ? i : i + 0.5 * a.p_im[c];
     }
     if (MODE & SWEEP_AH) {
-        const double f = pow2d(a.expo[1]), w = a.tpos[s].w, r = f * (w * hr), i = f * (w * hi);
+        const double w = a.tpos[s].w, r = ldexp(w * hr, a.expo[1]), i = ldexp(w * hi, a.expo[1]);
         if (!isfinite(r) || !isfinite(i)) atomicOr(a.err, DEV_ERR_NONFINITE);
         a.qt_re[c] = r + 0.5 * a.pt_re[c];
         a.qt_im[c] = i + 0.5 * a.pt_im[c];
@@ -690,8 +692,8 @@ __global__ void __launch_bounds__(256) cols_dens_kernel(int64_t n, int64_t npad,
                                                         const double4_32a *__restrict__ tpos,
                                                         const double *__restrict__ p_re,
                                                         const double *__restrict__ p_im, double scale,
-                                                        const int *__restrict__ part, int *__restrict__ expo,
-                                                        float4 *__restrict__ dens)
+                                                        int scale_exp, const int *__restrict__ part,
+                                                        int *__restrict__ expo, float4 *__restrict__ dens)
 {
     const int r = blockIdx.y;
     __shared__ int ex;
@@ -702,7 +704,7 @@ __global__ void __launch_bounds__(256) cols_dens_kernel(int64_t n, int64_t npad,
         v = __reduce_max_sync(0xffffffffu, v);
         if (threadIdx.x == 0) {
             ex = max(-1000, min(1000, (v >> 20) - 1022));
-            if (blockIdx.x == 0) expo[r] = ex;
+            if (blockIdx.x == 0) expo[r] = ex + scale_exp;
         }
     }
     __syncthreads();
@@ -837,7 +839,7 @@ __global__ void __launch_bounds__(kTile32, kColsCtas<RB>) cols_kernel(ArgsSplit 
 #pragma unroll
     for (int r = 0; r < RB; r++) {
         if (r >= m.nr) break;
-        const double f = pow2d(a.expo[r]), x = f * q[2 * r * STEP], y = f * q[(2 * r + 1) * STEP];
+        const double x = ldexp(q[2 * r * STEP], a.expo[r]), y = ldexp(q[(2 * r + 1) * STEP], a.expo[r]);
         if (!isfinite(x) || !isfinite(y)) atomicOr(a.err, DEV_ERR_NONFINITE);
         m.q_re[r * m.n + c] = x + 0.5 * m.p_re[r * m.n + c];
         m.q_im[r * m.n + c] = y + 0.5 * m.p_im[r * m.n + c];
@@ -858,9 +860,8 @@ __global__ void __launch_bounds__(256) cols_reduce_kernel(ArgsSplit a, ColsArgs 
         x += v.x;
         y += v.y;
     }
-    const double f = pow2d(a.expo[r]);
-    x *= f;
-    y *= f;
+    x = ldexp(x, a.expo[r]);
+    y = ldexp(y, a.expo[r]);
     if (!isfinite(x) || !isfinite(y)) atomicOr(a.err, DEV_ERR_NONFINITE);
     m.q_re[r * m.n + c] = x + 0.5 * m.p_re[r * m.n + c];
     m.q_im[r * m.n + c] = y + 0.5 * m.p_im[r * m.n + c];
@@ -909,8 +910,10 @@ int launch_cols(const SweepConst &c, const RecSplit &v, const double4_32a *nrm, 
     int64_t b = (v.npad + 255) / 256;
     if (b > 2 * sms) b = 2 * sms;
     const double sg = (c.interior == 1) ? -1.0 : 1.0;
-    cols_dens_kernel<<<dim3((unsigned)b, RB), 256, 0, s>>>(c.n, v.npad, nr, v.perm, v.tpos, p_re, p_im,
-                                                           sg * c.wave * c.wave / (8.0 * kPiS), part, expo, dens);
+    int es;
+    const double scale = frexp(sg * c.wave * c.wave / (8.0 * kPiS), &es);
+    cols_dens_kernel<<<dim3((unsigned)b, RB), 256, 0, s>>>(c.n, v.npad, nr, v.perm, v.tpos, p_re, p_im, scale, es,
+                                                           part, expo, dens);
     HZ_CHECK_LAUNCH();
     ArgsSplit a = split_args(c, v, nrm);
     a.densA = dens;
@@ -983,8 +986,9 @@ RecSplit split_record_views(void *mem, const Rec32 &r)
 // Where the split sweep serves: the table reduction of the origin phases ends
 // at k rho = 4000 (as the FP64 sweep's); k h <= 0.8 (eight points a
 // wavelength) keeps the phases within a tile small, so the error stays at or
-// below the FP64 sweep's (at k h = 1, 4.5e-15 against 4.2e-15); k >= 1/64
-// keeps 1/(k rho)^3 far inside the FP32 range; below 2048 points the FP64
+// below the FP64 sweep's (at k h = 1, 4.5e-15 against 4.2e-15); k tau >= 2^-28
+// keeps 1/(k rho)^2 below 2^56 and the units of a close tile's r^2, 2^-53 of
+// (k tau)^2, inside the FP32 range; below 2048 points the FP64
 // sweep's error (2e-15 and less) is the smaller one.  tau >= h: the projection
 // (x_t - x_s).n carries an error of 2^-51 of the tile's radius (10 to 30 h),
 // which is 2^-46 of the nearest far pairs' entries at rho = h and would grow as
@@ -992,7 +996,8 @@ RecSplit split_record_views(void *mem, const Rec32 &r)
 // unscaled coordinates).
 bool split_serves(int64_t n, double wave, double H, double tau, double extent)
 {
-    return n >= 2048 && wave >= 1.0 / 64 && wave * H <= 0.8 && tau >= H && wave * extent < 4000.0;
+    return n >= 2048 && wave > 1e-100 && wave < 1e100 && wave * tau >= 0x1p-28 && wave * H <= 0.8 && tau >= H &&
+           wave * extent < 4000.0;
 }
 
 int build_split_records(const SweepConst &c, const RecSplit &v, const Rec32 &r, const double4_32a *pos,
@@ -1022,8 +1027,10 @@ int split_densities(const SweepConst &c, const RecSplit &v, const double4_32a *n
     int64_t b = (v.npad + 255) / 256;
     const int64_t cap = 8 * (int64_t)sm_count();
     if (b > cap) b = cap;
-    split_dens_kernel<<<(unsigned)b, 256, 0, s>>>(v.npad, v.perm, v.tpos, pr, pi, tr, ti, scale, part, v.expo, v.dens,
-                                                  v.dens + v.npad);
+    int es;
+    scale = frexp(scale, &es);
+    split_dens_kernel<<<(unsigned)b, 256, 0, s>>>(v.npad, v.perm, v.tpos, pr, pi, tr, ti, scale, es, part, v.expo,
+                                                  v.dens, v.dens + v.npad);
     HZ_CHECK_LAUNCH();
     return HZ_OK;
 }

@@ -76,3 +76,26 @@ def test_wide_tiles(hz, oracle, tau_factor):
     p = hz.params(48, 9.0, int_l=-1.0, int_u=1.0, factor=3.0, tau_factor=tau_factor, dirichlet=1)
     worst, n = columns(hz, oracle, p, two_spheres(48), 40, np.random.default_rng(2))
     assert n >= 2048 and worst <= 1.0
+
+
+@pytest.mark.parametrize("half,k,dirichlet", [
+    (1e-9, 1 / 64, 1), (3e-10, 1 / 64, 0), (1e-10, 1 / 64, 1),            # k tau far below 2^-28
+    (1.0, 2.0 ** -28 * 6.0 * 0.999, 1), (1.0, 2.0 ** -28 * 6.0 * 1.001, 0),  # tau = 1/6: on both sides of it
+    (1e-7, 5e7, 1), (1e7, 5e-7, 0), (1e20, 5e-20, 1), (1e-15, 5e15, 0),   # other units of length
+    (100.0, 0.01, 1)])
+def test_units_of_length(hz, oracle, half, k, dirichlet):
+    """k times the box decides, not k."""
+    from helmholtz_3d_torrone_gb300 import geometry as G
+    d = G.sphere(24, radius=0.5, center=(0.011, 0.017, 0.005)) * half
+    p = hz.params(24, k, int_l=-half, int_u=half, factor=3.0, dirichlet=dirichlet)
+    worst, n = columns(hz, oracle, p, d, 8, np.random.default_rng(3))
+    assert n >= 2048 and worst <= 1.0
+    with hz.Operator(p) as op:
+        op.set_distance(d)
+        n = op.build()
+        V = np.exp(1j * np.outer([1, 2, 3], np.arange(n) / n))
+        one = np.array([op.matvec(v) for v in V])
+        assert np.max(np.abs(op.matvec_multi(V, precision=hz.PREC_F64) - one)) <= 2.0 ** -42 * 4
+        pq, pt = op.matvec_pair(V[0], V[1])
+        assert np.max(np.abs(pq - one[0])) <= 2.0 ** -42 * 4
+        assert np.max(np.abs(pt - op.matvec(V[1], adjoint=True))) <= 2.0 ** -42 * 4
