@@ -38,9 +38,10 @@ __device__ __noinline__ bool field_pair(double x, double y, double z, double nx,
 // Pairs with r <= tau are skipped, as in the reference.
 //
 // Bound by the FP64 pipe (1.65 lanes a clock an SM): sincos, sqrt and the
-// division are 67 FP64 instructions a pair; far_factor64 on coordinates scaled
-// by k is 38, and 5 a source for the scaling and w sigma are shared by the R
-// receivers.  The 32 KB phase table is filled once a block, so the blocks stay
+// division are 67 FP64 instructions a pair; far_factor64 on (k r)^2 is 39, and
+// two a source for w sigma are shared by the R receivers.  Coordinates are
+// subtracted unscaled, so neither the factor nor the test r <= tau depends on
+// how far from the origin the box lies.  The 32 KB phase table is filled once a block, so the blocks stay
 // and take receivers in turn.  The table serves k r < 4000; pairs beyond,
 // within 1e-12 of tau, and NaN go through field_pair.
 // The split FP32 arithmetic of the products would be 8 times as fast, but
@@ -51,8 +52,8 @@ template <bool SINGLE, int R>
 __global__ void __launch_bounds__(kEvalThreads, 2)
     eval_kernel(int64_t n, const double4_32a *__restrict__ pos, const double4_32a *__restrict__ nrm,
                 const double *__restrict__ s_re, const double *__restrict__ s_im, int64_t m,
-                const double *__restrict__ rx, double wave, double tau, double near_lo, double near_hi, double plain,
-                double scale, double *u_re, double *u_im)
+                const double *__restrict__ rx, double wave, double k2, double tau, double near_lo, double near_hi,
+                double plain, double scale, double *u_re, double *u_im)
 {
     const float kscale = (float)(kPhaseTable / (2 * 3.14159265358979323846));
     __shared__ alignas(16) double2 tab[kPhaseTable];
@@ -64,27 +65,26 @@ __global__ void __launch_bounds__(kEvalThreads, 2)
 #pragma unroll
         for (int g = 0; g < R; g++) {
             const int64_t r = min(r0 + g, m - 1);
-            for (int a = 0; a < 3; a++) X[g][a] = wave * rx[3 * r + a];
+            for (int a = 0; a < 3; a++) X[g][a] = rx[3 * r + a];
             ur[g] = ui[g] = 0.0;
         }
         for (int64_t c = threadIdx.x; c < n; c += kEvalThreads) {
             const double4_32a p = pos[c], q = nrm[c];
-            const double px = wave * p.x, py = wave * p.y, pz = wave * p.z;
             const double d0 = q.w * s_re[c], d1 = q.w * s_im[c];
 #pragma unroll
             for (int g = 0; g < R; g++) {
-                const double x = X[g][0] - px, y = X[g][1] - py, z = X[g][2] - pz;
-                const double r2 = fma(z, z, fma(y, y, x * x));
+                const double x = X[g][0] - p.x, y = X[g][1] - p.y, z = X[g][2] - p.z;
+                const double r2 = fma(z, z, fma(y, y, x * x)), kr2 = k2 * r2;
                 double vr, vi;
-                if (r2 > near_hi && r2 < 1.6e7) {
+                if (r2 > near_hi && kr2 < 1.6e7) {
                     if (SINGLE) {
                         double y;
-                        far_wave64(r2, kscale, tab, vr, vi, y);
+                        far_wave64(kr2, kscale, tab, vr, vi, y);
                         vr *= y;
                         vi *= y;
                     } else {
                         double y2;
-                        far_factor64<true>(r2, 1.0, kscale, tab, vr, vi, y2);
+                        far_factor64<true>(kr2, 1.0, kscale, tab, vr, vi, y2);
                         const double f = fma(z, q.z, fma(y, q.y, x * q.x)) * y2;
                         vr *= f;
                         vi *= f;
@@ -92,10 +92,7 @@ __global__ void __launch_bounds__(kEvalThreads, 2)
                 } else if (r2 <= near_lo) {
                     continue;
                 } else {
-                    const int64_t r = min(r0 + g, m - 1);
-                    if (!field_pair<SINGLE>(rx[3 * r] - p.x, rx[3 * r + 1] - p.y, rx[3 * r + 2] - p.z, q.x, q.y, q.z,
-                                            wave, tau, vr, vi))
-                        continue;
+                    if (!field_pair<SINGLE>(x, y, z, q.x, q.y, q.z, wave, tau, vr, vi)) continue;
                     vr *= plain;
                     vi *= plain;
                 }
@@ -133,14 +130,14 @@ int eval_blocks(int64_t n, const double4_32a *pos, const double4_32a *nrm, const
 {
     const double kt = wave * tau, inf = std::numeric_limits<double>::infinity();
     const bool table = wave > 0.0 && kt * kt > 1e-30 && kt < 4000.0;
-    // the table's pairs are the fields' over k (single layer) and k^2
-    const double f = !table ? 1.0 : SINGLE ? wave : wave * wave, c = (SINGLE ? -1.0 : sg) / (4.0 * 3.14159265358979323846264338328);
+    // the table's pairs are the fields' over k (single layer) and k^3
+    const double f = !table ? 1.0 : SINGLE ? wave : wave * wave * wave, c = (SINGLE ? -1.0 : sg) / (4.0 * 3.14159265358979323846264338328);
     int64_t b = (m + R - 1) / R;
     const int64_t cap = 2 * (int64_t)sm_count();
     if (b > cap) b = cap;
     eval_kernel<SINGLE, R><<<(unsigned)b, kEvalThreads, 0, s>>>(
-        n, pos, nrm, s_re, s_im, m, rx, wave, tau, table ? kt * kt * (1 - 1e-12) : -1.0,
-        table ? kt * kt * (1 + 1e-12) : inf, 1.0 / f, c * f, u_re, u_im);
+        n, pos, nrm, s_re, s_im, m, rx, wave, wave * wave, tau, table ? tau * tau * (1 - 1e-12) : -1.0,
+        table ? tau * tau * (1 + 1e-12) : inf, 1.0 / f, c * f, u_re, u_im);
     HZ_CHECK_LAUNCH();
     return HZ_OK;
 }

@@ -54,3 +54,40 @@ def test_fields_against_the_oracle(hz, oracle, case, m):
             bad[5] = np.inf
             with np.errstate(invalid="ignore"):
                 assert not np.all(np.isfinite(op.evaluate(rx, bad, layer)))
+
+
+@pytest.mark.parametrize("dirichlet", [0, 1])
+def test_fields_far_from_the_origin(hz, oracle, dirichlet):
+    """A box at 10^6: the coordinates' own rounding (10^-10) is all that is
+    lost, and receivers within 3e-9 of tau of a point fall on the side of tau
+    that their stored coordinates say."""
+    import oracle as O
+    from helmholtz_3d_torrone_gb300 import geometry as G
+    N, k, lo = 24, 6.3, 1e6
+    d = G.sphere(N, radius=0.5, center=(lo + 1.011, lo + 1.017, lo + 1.005), int_l=lo, int_u=lo + 2)
+    p = hz.params(N, k, int_l=lo, int_u=lo + 2, factor=3.0, dirichlet=dirichlet)
+    po = O.make_params(N, k, int_l=lo, int_u=lo + 2, factor=3.0, dirichlet=dirichlet)
+    tp = oracle.pipeline(po, d)
+    rng = np.random.default_rng(7)
+    xs, w = np.asarray(tp["xs"]).reshape(-1, 3), np.asarray(tp["w"])
+    m = 400
+    u = rng.standard_normal((m, 3))
+    u /= np.linalg.norm(u, axis=1)[:, None]
+    tau = po.tau_factor * 2.0 / N
+    rx = xs[rng.integers(0, len(xs), m)] + tau * (1 + 3e-9 * rng.uniform(-1, 1, (m, 1))) * u
+    rx[::4] = lo + 1 + 0.3 * u[::4]
+    with hz.Operator(p) as op:
+        op.set_distance(d)
+        n = op.build()
+        assert np.array_equal(op.tube()["xs"].reshape(-1, 3), xs)
+        sigma = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+        for layer in (hz.SINGLE_LAYER, hz.DOUBLE_LAYER):
+            got = op.evaluate(rx, sigma, layer)
+            want = oracle.evaluate(po, tp, sigma, rx, layer == hz.DOUBLE_LAYER)
+            for i in range(m):
+                rho = np.linalg.norm(xs - rx[i], axis=1)
+                far = rho > 0.1 * tau
+                size = np.abs(w * sigma)[far] / rho[far] / (4 * np.pi)
+                if layer == hz.DOUBLE_LAYER:
+                    size = size * (k + 1 / rho[far])
+                assert abs(got[i] - want[i]) <= (BOUND + 2.0 ** -49 * k * rho.max()) * size.sum()
