@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(kEvalThreads, 2)
     const float kscale = (float)(kPhaseTable / (2 * 3.14159265358979323846));
     __shared__ alignas(16) double2 tab[kPhaseTable];
     __shared__ double sh[2 * R][kEvalThreads / 32];
-    fill_phase_table(tab);
+    fill_phase_table_folded(tab);
     for (int64_t r0 = blockIdx.x * (int64_t)R; r0 < m; r0 += gridDim.x * (int64_t)R) {
         __syncthreads();
         double X[R][3], ur[R], ui[R];
