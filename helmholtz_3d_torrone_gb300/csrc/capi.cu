@@ -647,7 +647,7 @@ int hz_build(hz_operator *op, int64_t *n_out)
     } else {
         op->posk64.release();
     }
-    const double lambda = lambda32(op->p.wave);
+    const double lambda = lambda32(op->p.wave, op->tau);
     HZ_TRY(build_records32(op, lambda, sweep32_reg_scale(op->p.interior, lambda)));
     if (op->use_split) {
         HZ_TRY(op->split64.ensure(split_record_bytes(op->r32.npad)));

@@ -263,9 +263,9 @@ int sweep_f32(const SweepConst &c, const Rec32 &r, const double4_32a *pos64, int
               const double *p_re, const double *p_im, const double *pt_re, const double *pt_im,
               double *q_re, double *q_im, double *qt_re, double *qt_im, float *dens,
               cudaStream_t s, cudaEvent_t ev0 = nullptr, cudaEvent_t ev1 = nullptr, int cfg = 0);
-// The factor of the FP32 coordinates for wave number k, and the factor of the
+// The factor of the FP32 coordinates for wave number k and near-field radius tau, and the factor of the
 // regularisation factors in pos32.w (the inverse of the densities').
-double lambda32(double wave);
+double lambda32(double wave, double tau);
 struct Const32 {
     int scaled;
     float k, kh, kl, tau2, guard_lo, guard_hi;

@@ -13,8 +13,8 @@
 // three SFU ones a pair, against 29 and three with the phase k rho reduced
 // per pair, which the other tiles keep.
 //
-// Records with lambda = 1 (k below 2^-14, where 1/(k rho)^3 could leave the
-// FP32 range, and negative k) reduce k rho in revolutions with k/(2 pi) split
+// Records with lambda = 1 (k below 2^-14, negative k, k tau below 2^-40:
+// lambda32 in sweep_f32.cu) reduce k rho in revolutions with k/(2 pi) split
 // into an FP32 head and tail.
 #pragma once
 

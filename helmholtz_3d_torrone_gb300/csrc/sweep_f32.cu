@@ -1040,9 +1040,11 @@ Const32 constants32(const SweepConst &c, double lambda)
     return r;
 }
 
-// Below k = 2^-14 (and for k <= 0) the coordinates stay unscaled: 1/(k rho)^3
-// must stay inside the FP32 range.
-double lambda32(double wave) { return wave >= 1.0 / 16384 ? wave : 1.0; }
+// Below k = 2^-14 (and for k <= 0) the coordinates stay unscaled, so that k^2 on
+// the densities costs no more than 2^-28 of the FP32 range; below k tau = 2^-40 as
+// well, so that (k rho)^2 and its inverse stay inside it whatever the unit of
+// length.
+double lambda32(double wave, double tau) { return wave >= 1.0 / 16384 && wave * tau >= 0x1p-40 ? wave : 1.0; }
 
 double sweep32_reg_scale(int interior, double lambda)
 {
