@@ -182,39 +182,53 @@ __device__ __forceinline__ bool is_near(const Args32 &a, float r2, int64_t tslot
     return r2 <= a.tau2;
 }
 
-// One source against TG targets, scalar (records with lambda = 1).
-template <int MODE, bool DIR, int NT, int TG>
-__device__ __forceinline__ void pair_scalar(const Args32 &a, const float *st, int j, bool maybe_near,
+// A unit of a tile against TG targets, scalar (records with lambda = 1).  Four
+// sources' values come by one 128-bit load a row (a load a value: 13 to 21 %
+// more time at n = 19,532).
+template <int MODE, bool DIR, int NT, int TG, bool NEAR>
+__device__ __forceinline__ void unit_scalar(const Args32 &a, const float *st, int j0, int j1,
                                             const float3 (&rel)[TG], const Targets<TG> &t, int64_t tslot0,
-                                            int64_t src_slot, float (&fAr)[TG], float (&fAi)[TG], float (&fHr)[TG],
+                                            int64_t sslot0, float (&fAr)[TG], float (&fAi)[TG], float (&fHr)[TG],
                                             float (&fHi)[TG])
 {
-    constexpr int T = kTile32;
-    const float sx = st[j], sy = st[T + j], sz = st[2 * T + j];
-    const float nx = st[3 * T + j], ny = st[4 * T + j], nz = st[5 * T + j], sreg = st[6 * T + j];
-    const float *d = st + kFixed * T + j;
+    constexpr int ROWS = kFixed + kDens<MODE>, H0 = ROWS - 3;  // the last three rows: the densities of A^H
 #pragma unroll
-    for (int g = 0; g < TG; g++) {
-        const float dx = rel[g].x + sx, dy = rel[g].y + sy, dz = rel[g].z + sz;
-        const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-        const bool near = maybe_near && is_near(a, r2, tslot0 + (int64_t)g * NT, src_slot);
-        float u1, u2, rr;
-        kernel32<false, true>(a.wave, r2, 0.f, u1, u2, rr);
-        const float ps = fmaf(dx, nx, fmaf(dy, ny, dz * nz));                          // (x_t - x_s).n_s
-        const float pt = fmaf(dx, t.tn[g].x, fmaf(dy, t.tn[g].y, dz * t.tn[g].z));    // (x_t - x_s).n_t
-        if (MODE & SWEEP_A) {
-            const float q = rr * (DIR ? ps : pt);
-            const float vr = near ? (DIR ? sreg : t.reg[g]) : -u1 * q, vi = near ? 0.f : u2 * q;
-            fAr[g] = fmaf(vr, d[0], fmaf(-vi, d[T], fAr[g]));
-            fAi[g] = fmaf(vr, d[T], fmaf(vi, d[0], fAi[g]));
+    for (int g = 0; g < TG; g++) fAr[g] = fAi[g] = fHr[g] = fHi[g] = 0.f;
+#pragma unroll 1
+    for (int j = j0; j < j1; j += 4) {
+        float v[ROWS][4];
+#pragma unroll
+        for (int r = 0; r < ROWS; r++) {
+            const float4 x = *reinterpret_cast<const float4 *>(st + r * kTile32 + j);
+            v[r][0] = x.x;
+            v[r][1] = x.y;
+            v[r][2] = x.z;
+            v[r][3] = x.w;
         }
-        if (MODE & SWEEP_AH) {
-            const float *e = d + (kDens<MODE> - 3) * T;
-            const float q = rr * (DIR ? pt : ps);
-            const float vr = near ? (DIR ? t.reg[g] : sreg) : u1 * q, vi = near ? 0.f : u2 * q;
-            fHr[g] = fmaf(vr, e[0], fmaf(-vi, e[T], fHr[g]));
-            fHi[g] = fmaf(vr, e[T], fmaf(vi, e[0], fHi[g]));
-        }
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+#pragma unroll
+            for (int g = 0; g < TG; g++) {
+                const float dx = rel[g].x + v[0][q], dy = rel[g].y + v[1][q], dz = rel[g].z + v[2][q];
+                const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                const bool near = NEAR && is_near(a, r2, tslot0 + (int64_t)g * NT, sslot0 + j + q);
+                float u1, u2, rr;
+                kernel32<false, true>(a.wave, r2, 0.f, u1, u2, rr);
+                const float ps = fmaf(dx, v[3][q], fmaf(dy, v[4][q], dz * v[5][q]));        // (x_t - x_s).n_s
+                const float pt = fmaf(dx, t.tn[g].x, fmaf(dy, t.tn[g].y, dz * t.tn[g].z));  // (x_t - x_s).n_t
+                if (MODE & SWEEP_A) {
+                    const float f = rr * (DIR ? ps : pt), dr = v[kFixed][q], di = v[kFixed + 1][q];
+                    const float vr = near ? (DIR ? v[6][q] : t.reg[g]) : -u1 * f, vi = near ? 0.f : u2 * f;
+                    fAr[g] = fmaf(vr, dr, fmaf(-vi, di, fAr[g]));
+                    fAi[g] = fmaf(vr, di, fmaf(vi, dr, fAi[g]));
+                }
+                if (MODE & SWEEP_AH) {
+                    const float f = rr * (DIR ? pt : ps), dr = v[H0][q], di = v[H0 + 1][q];
+                    const float vr = near ? (DIR ? t.reg[g] : v[6][q]) : u1 * f, vi = near ? 0.f : u2 * f;
+                    fHr[g] = fmaf(vr, dr, fmaf(-vi, di, fHr[g]));
+                    fHi[g] = fmaf(vr, di, fmaf(vi, dr, fHi[g]));
+                }
+            }
     }
 }
 
@@ -428,10 +442,10 @@ __device__ __forceinline__ void tile_pairs(const Args32 &a, const float *st, int
     };
     if (!(MODE & SWEEP_SCALED)) {
         units([&](int j0, int j1, float (&fAr)[TG], float (&fAi)[TG], float (&fHr)[TG], float (&fHi)[TG]) {
-#pragma unroll
-            for (int g = 0; g < TG; g++) fAr[g] = fAi[g] = fHr[g] = fHi[g] = 0.f;
-            for (int j = j0; j < j1; j++)
-                pair_scalar<MODE, DIR, NT, TG>(a, st, j, near, rel, t, slot0, sslot0 + j, fAr, fAi, fHr, fHi);
+            if (near)
+                unit_scalar<MODE, DIR, NT, TG, true>(a, st, j0, j1, rel, t, slot0, sslot0, fAr, fAi, fHr, fHi);
+            else
+                unit_scalar<MODE, DIR, NT, TG, false>(a, st, j0, j1, rel, t, slot0, sslot0, fAr, fAi, fHr, fHi);
         });
     } else if (!centred) {
         units([&](int j0, int j1, float (&fAr)[TG], float (&fAi)[TG], float (&fHr)[TG], float (&fHi)[TG]) {
