@@ -32,8 +32,9 @@ struct hz_batch {
     int64_t nmax = 0, max_npad = 0;
     int device = 0;
     cudaStream_t stream = nullptr;
-    int shape = 0;  // FP32 batch sweep shape (hz_batch_autotune); 256 threads of one target: the packed loop
-                    // holds 122 registers, and two targets in 128 spill (n = 19,532: 0.38 against 0.47 ms)
+    int shape = 0;  // FP32 batch sweep shape (hz_batch_autotune).  256 threads of one target: at 128 registers
+                    // the kernel spills 100 bytes, two targets in 128 threads 108 to 500, 80 registers 504
+                    // (n = 11,088, 4,978 and 2,938 together: 0.184 ms a product, the others 0.194 to 0.23)
     DevBuf desc;    // kBatchShapes descriptor arrays
     int64_t units[kBatchShapes] = {};
     std::vector<Batch32Item> items;

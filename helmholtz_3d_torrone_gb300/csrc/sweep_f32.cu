@@ -768,11 +768,28 @@ struct BatchVec {
     const double *p_re, *p_im;
     double *q_re, *q_im;
     int64_t stride;
+    int64_t *begins;  // [nctas + 1] partition of the launch
 };
 
-// dens of every operator from its column of P (blockIdx.y = operator)
-__global__ void batch_prep_kernel(const BatchOp *__restrict__ ops, BatchVec v)
+// First unit of CTA c: the operators' cuts laid end to end by their costs.
+__device__ __forceinline__ int64_t batch_begin(const BatchOp *ops, int nops, int nctas, int c)
 {
+    const int64_t total = ops[nops - 1].cost0 + ops[nops - 1].cost;
+    const int64_t x = total / nctas * c + total % nctas * c / nctas;
+    int o = 0;
+    while (o + 1 < nops && x >= ops[o + 1].cost0) o++;
+    const int64_t y = x - ops[o].cost0, n = ops[o].cost;
+    return ops[o].unit0 + __ldg(ops[o].a.cuts + (y / n * kCuts + y % n * kCuts / n));
+}
+
+// dens of every operator from its column of P (blockIdx.y = operator), and the
+// partition (found anew for every piece of a split block, six 64-bit divisions
+// a time, it took 10 us of a batch of one and 40 of eight operators of six tiles)
+__global__ void batch_prep_kernel(const BatchOp *__restrict__ ops, int nops, int64_t units, int nctas, BatchVec v)
+{
+    if (blockIdx.x == gridDim.x - 1 && blockIdx.y == 0)
+        for (int c = threadIdx.x; c <= nctas; c += blockDim.x)
+            v.begins[c] = c == nctas ? units : batch_begin(ops, nops, nctas, c);
     const BatchOp &o = ops[blockIdx.y];
     const double *pr = v.p_re + (int64_t)o.col * v.stride, *pi = v.p_im + (int64_t)o.col * v.stride;
     if (blockIdx.x == 0)
@@ -803,17 +820,6 @@ __global__ void batch_cost_kernel(BatchOp *ops, int nops)
     }
 }
 
-// First unit of CTA c: the operators' cuts laid end to end by their costs.
-__device__ __forceinline__ int64_t batch_begin(const BatchOp *ops, int nops, int nctas, int c)
-{
-    const int64_t total = ops[nops - 1].cost0 + ops[nops - 1].cost;
-    const int64_t x = total / nctas * c + total % nctas * c / nctas;
-    int o = 0;
-    while (o + 1 < nops && x >= ops[o + 1].cost0) o++;
-    const int64_t y = x - ops[o].cost0, n = ops[o].cost;
-    return ops[o].unit0 + __ldg(ops[o].a.cuts + (y / n * kCuts + y % n * kCuts / n));
-}
-
 __device__ __forceinline__ void batch_write(const Args32 &a, int64_t s, double ar, double ai, const double *p_re,
                                             const double *p_im, double *q_re, double *q_im)
 {
@@ -833,14 +839,16 @@ __device__ __forceinline__ bool batch_tiles(const Args32 &a, const BatchOp *ops,
                                             float (*stage)[kStage<SWEEP_A>], uint64_t *bar)
 {
     const uint32_t *mrow = a.nearmask + blk * a.mwords;
+    const int shift = a.sub >> 1;  // log2 of 1, 2 or 4
     for (; u < seg_end; it++) {
         const int buf = (int)(it & 1);
-        const int64_t tile = (u - u0) / a.sub;
-        const int q0 = (int)((u - u0) % a.sub), q1 = (int)min((int64_t)a.sub, q0 + seg_end - u);
+        const int64_t tile = (u - u0) >> shift;
+        const int q0 = (int)(u - u0) & (a.sub - 1), q1 = (int)min((int64_t)a.sub, q0 + seg_end - u);
         u += q1 - q0;
-        if (threadIdx.x == 0 && u < u_end) {
-            const int o2 = batch_op_of_unit(ops, nops, u, o);
-            issue_tile<SWEEP_A>(ops[o2].a, (u - ops[o2].unit0) / ops[o2].a.sub % ops[o2].ntiles, stage[buf ^ 1], &bar[buf ^ 1]);
+        if (threadIdx.x == 0 && u < u_end) {  // the next tile: of this block, else the first of the next one
+            const bool same = tile + 1 < ops[o].ntiles;
+            const int o2 = same ? o : batch_op_of_unit(ops, nops, u, o);
+            issue_tile<SWEEP_A>(same ? a : ops[o2].a, same ? tile + 1 : 0, stage[buf ^ 1], &bar[buf ^ 1]);
         }
         const bool near = (__ldg(mrow + (tile >> 5)) >> (tile & 31)) & 1u;
         float3 rel[TG];
@@ -865,13 +873,12 @@ __device__ __forceinline__ bool batch_tiles(const Args32 &a, const BatchOp *ops,
 // operators of different sizes share the GPU without a tail per operator.
 template <int NT, int TG, int MINB>
 __global__ void __launch_bounds__(NT, MINB) sweep32_batch_kernel(const BatchOp *__restrict__ ops, int nops,
-                                                                 int64_t units, int nctas, double4_32a *partial,
-                                                                 BatchVec v)
+                                                                 int nctas, double4_32a *partial, BatchVec v)
 {
     constexpr int SLOTS = NT * TG;
     __shared__ alignas(128) float stage[2][kStage<SWEEP_A>];
     __shared__ alignas(8) uint64_t bar[2];
-    auto begin = [&](int c) { return c >= nctas ? units : batch_begin(ops, nops, nctas, c); };
+    auto begin = [&](int c) { return __ldg(v.begins + c); };
     const int64_t u_begin = begin(blockIdx.x), u_end = begin(blockIdx.x + 1);
     if (threadIdx.x == 0) {
         mbar_init(&bar[0], 1);
@@ -947,17 +954,25 @@ int64_t batch_resident_ctas()
 
 template <int NT, int TG, int MINB>
 int launch_batch(const BatchOp *ops_dev, int nops, int64_t units, double4_32a *partial, size_t partial_bytes,
-                 const BatchVec &v, cudaStream_t s)
+                 BatchVec v, int64_t max_npad, cudaStream_t s, cudaEvent_t ev0)
 {
     constexpr int SLOTS = NT * TG;
+    constexpr size_t piece = 2 * SLOTS * sizeof(double4_32a);
     int64_t p = batch_resident_ctas<NT, TG, MINB>();
     if (p > units) p = units;
-    if ((size_t)p * 2 * SLOTS * sizeof(double4_32a) > partial_bytes) p = partial_bytes / (2 * SLOTS * sizeof(double4_32a));
+    if (p * (piece + sizeof(int64_t)) + sizeof(int64_t) > partial_bytes)
+        p = partial_bytes / (piece + sizeof(int64_t)) - 1;
     if (p < 1) {
         set_error("batched FP32 sweep: partial buffer too small");
         return HZ_ERR_STATE;
     }
-    sweep32_batch_kernel<NT, TG, MINB><<<(unsigned)p, NT, 0, s>>>(ops_dev, nops, units, (int)p, partial, v);
+    v.begins = reinterpret_cast<int64_t *>(partial + p * 2 * SLOTS);
+    long long bx = (max_npad + 255) / 256;
+    if (bx > 256) bx = 256;
+    batch_prep_kernel<<<dim3((unsigned)bx, (unsigned)nops), 256, 0, s>>>(ops_dev, nops, units, (int)p, v);
+    HZ_CHECK_LAUNCH();
+    if (ev0) HZ_CHECK_CUDA(record_timing_event(ev0, s));
+    sweep32_batch_kernel<NT, TG, MINB><<<(unsigned)p, NT, 0, s>>>(ops_dev, nops, (int)p, partial, v);
     HZ_CHECK_LAUNCH();
     return HZ_OK;
 }
@@ -1188,14 +1203,12 @@ int batch32_describe(const Batch32Item *items, int R, int cfg, void *desc_dev, i
 
 size_t batch32_partial_bytes()
 {
-    const size_t v[kShapes] = {
-        (size_t)batch_resident_ctas<256, 1, 2>() * 2 * 256 * sizeof(double4_32a),
-        (size_t)batch_resident_ctas<128, 2, 4>() * 2 * 256 * sizeof(double4_32a),
-        (size_t)batch_resident_ctas<256, 1, 3>() * 2 * 256 * sizeof(double4_32a),
-        (size_t)batch_resident_ctas<128, 2, 3>() * 2 * 256 * sizeof(double4_32a)};
-    size_t m = 0;
-    for (size_t x : v) m = x > m ? x : m;
-    return m;
+    const int64_t v[kShapes] = {batch_resident_ctas<256, 1, 2>(), batch_resident_ctas<128, 2, 4>(),
+                                batch_resident_ctas<256, 1, 3>(), batch_resident_ctas<128, 2, 3>()};
+    int64_t m = 0;
+    for (int64_t x : v) m = x > m ? x : m;
+    // the pieces of split blocks, and the partition
+    return (size_t)m * (2 * 256 * sizeof(double4_32a) + sizeof(int64_t)) + sizeof(int64_t);
 }
 
 int sweep_f32_batch(int cfg, const void *desc_dev, int R, int ncols, int64_t units, double4_32a *partial, size_t partial_bytes, const double *p_re, const double *p_im,
@@ -1207,17 +1220,13 @@ int sweep_f32_batch(int cfg, const void *desc_dev, int R, int ncols, int64_t uni
     HZ_CHECK_CUDA(cudaMemsetAsync(q_im, 0, (size_t)ncols * stride * sizeof(double), s));
     if (R <= 0 || units <= 0) return HZ_OK;
     const BatchOp *ops = static_cast<const BatchOp *>(desc_dev);
-    BatchVec v{p_re, p_im, q_re, q_im, stride};
-    long long bx = (max_npad + 255) / 256;
-    if (bx > 256) bx = 256;
-    batch_prep_kernel<<<dim3((unsigned)bx, (unsigned)R), 256, 0, s>>>(ops, v);
-    HZ_CHECK_LAUNCH();
-    if (ev0) HZ_CHECK_CUDA(record_timing_event(ev0, s));
+    BatchVec v{p_re, p_im, q_re, q_im, stride, nullptr};
+    const size_t pb = partial_bytes;
     switch (cfg % kShapes) {
-    case 1: HZ_TRY((launch_batch<128, 2, 4>(ops, R, units, partial, partial_bytes, v, s))); break;
-    case 2: HZ_TRY((launch_batch<256, 1, 3>(ops, R, units, partial, partial_bytes, v, s))); break;
-    case 3: HZ_TRY((launch_batch<128, 2, 3>(ops, R, units, partial, partial_bytes, v, s))); break;
-    default: HZ_TRY((launch_batch<256, 1, 2>(ops, R, units, partial, partial_bytes, v, s))); break;
+    case 1: HZ_TRY((launch_batch<128, 2, 4>(ops, R, units, partial, pb, v, max_npad, s, ev0))); break;
+    case 2: HZ_TRY((launch_batch<256, 1, 3>(ops, R, units, partial, pb, v, max_npad, s, ev0))); break;
+    case 3: HZ_TRY((launch_batch<128, 2, 3>(ops, R, units, partial, pb, v, max_npad, s, ev0))); break;
+    default: HZ_TRY((launch_batch<256, 1, 2>(ops, R, units, partial, pb, v, max_npad, s, ev0))); break;
     }
     if (ev1) HZ_CHECK_CUDA(record_timing_event(ev1, s));
     return HZ_OK;
