@@ -1026,13 +1026,17 @@ int launch_streamk(Args32 a, bool persistent, size_t partial_bytes, cudaStream_t
 
 // Compiled variants: (block size, targets per thread, minimum resident
 // blocks) x (persistent stream-K grid, or one CTA per target block).  Every
-// shape covers the 256 slots of one target tile.
+// shape covers the 256 slots of one target tile.  Below 24 tiles the persistent
+// variants all run the first shape: a CTA has one or two units of 64 sources
+// there, and two targets a thread or 80 registers only make it longer (n = 2,938:
+// 39 us, the others 48 to 75).
 constexpr int kShapes = 4;
 template <int MODE, bool DIR>
 int launch_cfg(int cfg, const Args32 &a, size_t pb, cudaStream_t s)
 {
     const bool persistent = cfg < kShapes;
-    switch (cfg % kShapes) {
+    const int shape = a.sub == 4 && persistent ? 0 : cfg % kShapes;
+    switch (shape) {
     case 1: return launch_streamk<MODE, DIR, 128, 2, 4>(a, persistent, pb, s);
     case 2: return launch_streamk<MODE, DIR, 256, 1, 3>(a, persistent, pb, s);
     case 3: return launch_streamk<MODE, DIR, 128, 2, 3>(a, persistent, pb, s);
