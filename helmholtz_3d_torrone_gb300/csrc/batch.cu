@@ -38,6 +38,8 @@ struct hz_batch {
     DevBuf desc;    // kBatchShapes descriptor arrays
     int64_t units[kBatchShapes] = {};
     std::vector<Batch32Item> items;
+    std::vector<uint64_t> builds;  // of the operators, when they were described
+    uint64_t described = 0;        // descriptions so far
     // the FP32 launch over a subset of the operators (sub_n > 0)
     DevBuf desc_sub;
     int sub_n = 0, sub_shape = -1;
@@ -79,7 +81,8 @@ struct BatchF32 final : MultiOp {
     uint64_t key() const override
     {
         const uint64_t g = sub ? b->sub_gen : 0;
-        return ((uint64_t)(uintptr_t)b << 4) ^ (uint64_t)(b->shape + 1) ^ (g << 40);
+        return ((uint64_t)(uintptr_t)b << 4) ^ (uint64_t)(b->shape + 1) ^ (g << 40) ^
+               b->described * 0x9e3779b97f4a7c15ull;
     }
     int restrict_to(const std::vector<int> &cols, cudaStream_t s) override
     {
@@ -157,18 +160,56 @@ struct BatchF64 final : MultiOp {
     }
 };
 
+// The operators' sizes and FP32 descriptors, as they are built now.
+int describe(hz_batch *b, int bad)
+{
+    b->nmax = b->max_npad = 0;
+    b->items.resize(b->R);
+    b->builds.resize(b->R);
+    b->sub_n = 0;
+    b->sub_shape = -1;
+    b->described++;
+    for (int r = 0; r < b->R; r++) {
+        hz_operator *op = b->ops[r];
+        if (!op || !op->built || op->combo || op->r32.npad <= 0 || op->device != b->ops[0]->device) {
+            set_error("hz_batch: operator %d is missing, not built, Combo, empty or on another device", r);
+            return bad;
+        }
+        b->nmax = op->n > b->nmax ? op->n : b->nmax;
+        b->max_npad = op->r32.npad > b->max_npad ? op->r32.npad : b->max_npad;
+        b->items[r].c = sweep_const(op);
+        b->items[r].r = op->r32;
+        b->items[r].pos64 = op->pos64.as<double4_32a>();
+        b->items[r].dens = op->dens32.as<float>();
+        b->builds[r] = 0;  // until it is described
+    }
+    HZ_CHECK_CUDA(cudaSetDevice(b->ops[0]->device));
+    const size_t db = batch32_desc_bytes(b->R);
+    HZ_TRY(b->desc.ensure(kBatchShapes * db));
+    HZ_TRY(b->desc_sub.ensure(db));
+    for (int k = 0; k < kBatchShapes; k++)
+        HZ_TRY(batch32_describe(b->items.data(), b->R, k, b->desc.as<char>() + (size_t)k * db, b->units[k], b->stream));
+    for (int r = 0; r < b->R; r++) b->builds[r] = b->ops[r]->builds;
+    return HZ_OK;
+}
+
+// A batch goes on with operators that were built again: their sizes, records and
+// counters may lie elsewhere, so they are described anew.
 int check_batch(hz_batch *b)
 {
     if (!b || b->R < 1) {
         set_error("batch is NULL or empty");
         return HZ_ERR_ARG;
     }
-    for (hz_operator *op : b->ops)
-        if (!op->built) {
-            set_error("an operator of the batch was rebuilt or invalidated; create the batch again");
+    bool same = true;
+    for (int r = 0; r < b->R; r++) {
+        if (!b->ops[r]->built) {
+            set_error("operator %d of the batch is not built", r);
             return HZ_ERR_STATE;
         }
-    return HZ_OK;
+        same = same && b->builds[r] == b->ops[r]->builds;
+    }
+    return same ? HZ_OK : describe(b, HZ_ERR_STATE);
 }
 
 int clear_errors(hz_batch *b, cudaStream_t s)
@@ -214,36 +255,16 @@ int hz_batch_create(hz_operator *const *ops, int count, hz_batch **out)
         set_error("hz_batch_create: bad arguments");
         return HZ_ERR_ARG;
     }
+    if (!ops[0]) {
+        set_error("hz_batch_create: operator 0 is missing");
+        return HZ_ERR_ARG;
+    }
     hz_batch *b = new hz_batch;
     b->R = count;
-    for (int r = 0; r < count; r++) {
-        hz_operator *op = ops[r];
-        if (!op || !op->built || op->combo || op->r32.npad <= 0 || (r > 0 && op->device != ops[0]->device)) {
-            delete b;
-            set_error("hz_batch_create: operator %d is missing, not built, Combo, empty or on another device", r);
-            return HZ_ERR_ARG;
-        }
-        b->ops.push_back(op);
-        b->nmax = op->n > b->nmax ? op->n : b->nmax;
-        b->max_npad = op->r32.npad > b->max_npad ? op->r32.npad : b->max_npad;
-    }
+    b->ops.assign(ops, ops + count);
     b->device = ops[0]->device;
     b->stream = ops[0]->stream;
-    int rc = cudaSetDevice(b->device) == cudaSuccess ? HZ_OK : HZ_ERR_CUDA;
-    const size_t db = batch32_desc_bytes(count);
-    if (rc == HZ_OK) rc = b->desc.ensure(kBatchShapes * db);
-    if (rc == HZ_OK) rc = b->desc_sub.ensure(db);
-    std::vector<Batch32Item> &items = b->items;
-    items.resize(count);
-    for (int r = 0; r < count && rc == HZ_OK; r++) {
-        hz_operator *op = ops[r];
-        items[r].c = sweep_const(op);
-        items[r].r = op->r32;
-        items[r].pos64 = op->pos64.as<double4_32a>();
-        items[r].dens = op->dens32.as<float>();
-    }
-    for (int k = 0; k < kBatchShapes && rc == HZ_OK; k++)
-        rc = batch32_describe(items.data(), count, k, b->desc.as<char>() + (size_t)k * db, b->units[k], b->stream);
+    int rc = describe(b, HZ_ERR_ARG);
     if (rc == HZ_OK) {
         b->partial_bytes = batch32_partial_bytes();
         rc = b->partial.ensure(b->partial_bytes);

@@ -616,6 +616,7 @@ int hz_build(hz_operator *op, int64_t *n_out)
         return HZ_ERR_STATE;
     }
     HZ_CHECK_CUDA(cudaSetDevice(op->device));
+    op->builds++;
     cudaStream_t s = op->stream;
     const int N = op->p.N;
     const size_t S = (size_t)N + 1, nodes = S * S * S;

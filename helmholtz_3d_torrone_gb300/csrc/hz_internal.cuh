@@ -322,6 +322,7 @@ struct hz_operator {
     // grids
     hz::DevBuf d, gx, gy, gz, mc, gc;
     bool have_distance = false, built = false;
+    uint64_t builds = 0;  // calls of hz_build: what describes this operator elsewhere (batches) compares it
     // tube
     int64_t n = 0;
     hz::DevBuf idx, xs, nrm, delta, jac, reg, w, dreg;

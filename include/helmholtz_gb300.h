@@ -376,7 +376,8 @@ HZ_API int hz_dense_assemble(int kind, const hz_params *p, const hz_dense_opts *
  * graph.  Vectors are passed per operator: arrays of `count` pointers, the
  * r-th of length hz_tube_size(ops[r]).  The operators must be built, use
  * the classic formulation and live on the same device; the batch keeps
- * pointers to them (destroy the batch first). */
+ * pointers to them (destroy the batch first).  An operator that is built again
+ * takes part with its new tube. */
 typedef struct hz_batch hz_batch;
 HZ_API int hz_batch_create(hz_operator *const *ops, int count, hz_batch **out);
 HZ_API void hz_batch_destroy(hz_batch *b);

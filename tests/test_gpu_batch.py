@@ -94,3 +94,43 @@ def test_batch_columns_leave_when_converged(hz, batch, precision):
             continue
         x64, _ = op.solve(rhs, method=hz.BICGSTAB, precision=hz.PREC_F64, tol=1e-12)
         assert rel_err(x, x64) < 1e-8
+
+
+def test_operators_built_again(hz):
+    """A batch follows operators that are built again, with more, fewer or as
+    many points: their records, costs and counters have moved."""
+    from helmholtz_3d_torrone_gb300 import geometry as G
+    N, k = 24, 4.0
+
+    def sphere(r):
+        return G.sphere(N, radius=r, center=(0.011, 0.017, 0.005))
+
+    ops = []
+    for r in (0.5, 0.45, 0.4):
+        op = hz.Operator(hz.params(N, k, int_l=-1.0, int_u=1.0, factor=3.0, dirichlet=1))
+        op.set_distance(sphere(r))
+        op.build()
+        ops.append(op)
+
+    def check(batch):
+        vs = [np.exp(1j * np.arange(o.n) / o.n) for o in ops]
+        for o, v, q32, q64 in zip(ops, vs, batch.matvec(vs), batch.matvec(vs, precision=hz.PREC_F64)):
+            want = o.matvec(v)
+            assert np.max(np.abs(q64 - want)) <= 1e-13 * np.max(np.abs(want))
+            assert np.max(np.abs(q32 - want)) <= 1e-5 * np.max(np.abs(want))
+            assert np.max(np.abs(o.matvec(v, precision=hz.PREC_F32) - want)) <= 1e-5 * np.max(np.abs(want))
+        xs, info, res = batch.solve(vs, precision=hz.PREC_F32_REFINED, tol=1e-10)
+        for o, v, x in zip(ops, vs, xs):
+            assert np.linalg.norm(o.matvec(x) - v) <= 1e-9 * np.linalg.norm(v)
+
+    with hz.Batch(ops) as batch:
+        check(batch)
+        for which, r in ((1, 0.7), (0, 0.3), (2, 0.4), (1, 0.45)):
+            ops[which].set_distance(sphere(r))
+            with pytest.raises(hz.HzError) as e:
+                batch.matvec([np.ones(o.n, dtype=complex) for o in ops])
+            assert e.value.code == hz.HZ_ERR_STATE
+            ops[which].build()
+            check(batch)
+    for op in ops:
+        op.close()
