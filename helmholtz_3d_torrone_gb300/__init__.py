@@ -25,6 +25,7 @@ PREC_F64, PREC_F32, PREC_F32_REFINED = 0, 1, 2
 BICG, BICGSTAB, GMRES = 0, 1, 2
 SINGLE_LAYER, DOUBLE_LAYER, COMBO_LAYER = 0, 1, 2
 PHASE_DIRECT, PHASE_SPLIT = 0, 1
+F64_SPLIT, F64_PLAIN = 0, 1
 RHS_POINT_DIRICHLET, RHS_POINT_NEUMANN, RHS_MONOPOLE_NEUMANN, RHS_MONOPOLE_DIRICHLET = 0, 1, 2, 3
 NOALLOC_MAX_POINTS = 32768  # HZ_NOALLOC_MAX_POINTS
 
@@ -136,6 +137,7 @@ SIGNATURES = {
     "hz_autotune": ([_vp, C.POINTER(C.c_int), _dp], C.c_int),
     "hz_set_sweep_config": ([_vp, C.c_int], C.c_int),
     "hz_set_phase_mode": ([_vp, C.c_int], C.c_int),
+    "hz_set_f64_mode": ([_vp, C.c_int], C.c_int),
     "hz_get_grids": ([_vp, _vp, _vp, _vp, _vp, _vp, C.c_int], C.c_int),
     "hz_get_tube": ([_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, C.c_int], C.c_int),
     "hz_matvec": ([_vp, C.c_int, C.c_int, _vp, _vp, _vp, _vp, C.c_int], C.c_int),
@@ -333,6 +335,11 @@ class Operator:
         """PHASE_SPLIT (default) or PHASE_DIRECT; the FP32 sweeps take the
         phase about the source tile in both."""
         _check(load().hz_set_phase_mode(self.h, mode))
+
+    def set_f64_mode(self, mode):
+        """F64_SPLIT (default: FP64 products in split arithmetic where that
+        serves) or F64_PLAIN (FP64 instructions everywhere)."""
+        _check(load().hz_set_f64_mode(self.h, mode))
 
     def sweep_timing(self, enable=-1):
         """Enable (1) / disable (0) per-sweep CUDA-event timing, or read (-1):

@@ -103,7 +103,7 @@ Rec64 rec64(hz_operator *op)
     r.pos = op->pos64.as<double4_32a>();
     r.nrm = op->nrm64.as<double4_32a>();
     r.posk = op->posk64.ptr ? op->posk64.as<double4_32a>() : nullptr;
-    r.split = op->use_split ? &op->split : nullptr;
+    r.split = op->use_split && !op->f64_plain ? &op->split : nullptr;
     return r;
 }
 
@@ -348,6 +348,17 @@ int need_built(hz_operator *op)
 
 }  // namespace
 
+// Records of the scaled sweep in FP64 instructions, where that may run.
+static int build_records64(hz_operator *op)
+{
+    if (!(op->p.wave >= 1.0) || (op->use_split && !op->f64_plain)) {
+        op->posk64.release();
+        return HZ_OK;
+    }
+    HZ_TRY(op->posk64.ensure((size_t)(op->n > 0 ? op->n : 1) * sizeof(double4_32a)));
+    return scale_records64(op->n, op->p.wave, op->pos64.as<double4_32a>(), op->posk64.as<double4_32a>(), op->stream);
+}
+
 // FP32 sweep records of the tube (or annulus) points in blocked order.
 static int build_records32(hz_operator *op, double lambda, double reg_scale)
 {
@@ -463,6 +474,20 @@ int hz_set_phase_mode(hz_operator *op, int mode)
         return HZ_ERR_ARG;
     }
     return HZ_OK;  // both modes run the phase centred on the source tile (pair32.cuh)
+}
+
+int hz_set_f64_mode(hz_operator *op, int mode)
+{
+    if (!op || (mode != HZ_F64_SPLIT && mode != HZ_F64_PLAIN)) {
+        set_error("hz_set_f64_mode: need an operator and HZ_F64_SPLIT or HZ_F64_PLAIN");
+        return HZ_ERR_ARG;
+    }
+    if (op->f64_plain == (mode == HZ_F64_PLAIN)) return HZ_OK;
+    HZ_CHECK_CUDA(cudaSetDevice(op->device));
+    op->f64_plain = mode == HZ_F64_PLAIN;
+    op->solver->outer.invalidate_graph();  // they hold the other sweep's launches
+    op->solver->inner.invalidate_graph();
+    return op->built && !op->combo ? build_records64(op) : HZ_OK;
 }
 
 int hz_set_combo(hz_operator *op, const hz_dense_opts *o)
@@ -642,12 +667,7 @@ int hz_build(hz_operator *op, int64_t *n_out)
     HZ_TRY(check_device_error(op, "hz_build"));
     const SweepConst sc = sweep_const(op);
     op->use_split = split_serves(n, sc.wave, op->H, op->tau, sc.extent);
-    if (op->p.wave >= 1.0 && !op->use_split) {  // records of the scaled sweep in FP64 instructions
-        HZ_TRY(op->posk64.ensure(nn * sizeof(double4_32a)));
-        HZ_TRY(scale_records64(n, op->p.wave, op->pos64.as<double4_32a>(), op->posk64.as<double4_32a>(), s));
-    } else {
-        op->posk64.release();
-    }
+    HZ_TRY(build_records64(op));
     const double lambda = lambda32(op->p.wave, op->tau);
     HZ_TRY(build_records32(op, lambda, sweep32_reg_scale(op->p.interior, lambda)));
     if (op->use_split) {
@@ -1395,7 +1415,7 @@ int hz_misfit_gradient(hz_operator *op, const hz_solve_opts *opts_in, const doub
     // k-derivatives: (dE/dk) sigma at the receivers, (dA/dk) sigma over the tube
     HZ_TRY(launch_eval_dk(n, op->pos64.as<double4_32a>(), op->nrm64.as<double4_32a>(), sg0, sg1, m, R, op->p.wave,
                           op->tau, op->p.interior, layer, Q0, Q1, s));
-    if (op->use_split)
+    if (op->use_split && !op->f64_plain)
         HZ_TRY(sweep_split_dk(sweep_const(op), op->split, op->nrm64.as<double4_32a>(), op->dreg.as<double>(), sg0, sg1,
                               d0, d1, s));
     else

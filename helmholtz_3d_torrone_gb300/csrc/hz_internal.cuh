@@ -330,7 +330,8 @@ struct hz_operator {
     hz::DevBuf posk64;  // pos64 with the coordinates scaled by k (FP64 sweep)
     hz::DevBuf split64;  // records of the split FP64 sweep
     hz::RecSplit split{};
-    bool use_split = false;
+    bool use_split = false;  // the split sweep serves this tube
+    bool f64_plain = false;  // hz_set_f64_mode: it is not to be used all the same
     // FP32 sweep records
     hz::Rec32 r32{};
     hz::DevBuf perm, pos32, nrm32, soa32, origin32, tpos32, split32, nearmask32, partial32;

@@ -52,7 +52,8 @@ extern "C" {
 #define HZ_DEVICE 1
 
 /* Arithmetic of a matvec or solve. */
-#define HZ_PREC_F64 0         /* plain FP64 everywhere                                  */
+#define HZ_PREC_F64 0         /* FP64 coordinates, densities and results; the entries in
+                                 FP64 instructions or in split arithmetic (hz_set_f64_mode) */
 #define HZ_PREC_F32 1         /* FP32 pair sweep (tile-local origins and phases), FP64
                                  inner products                                          */
 #define HZ_PREC_F32_REFINED 2 /* FP32 inner solves inside FP64 iterative refinement whose
@@ -179,6 +180,19 @@ HZ_API int hz_set_sweep_config(hz_operator *op, int cfg);
 #define HZ_PHASE_SPLIT 1
 HZ_API int hz_set_phase_mode(hz_operator *op, int mode);
 
+/* Arithmetic of the FP64 products (hz_matvec*, FP64 solves, refinement
+ * residuals, dA/dk).  HZ_F64_SPLIT (default): pairs of FP32 numbers and 64-bit
+ * integers, ten times as fast, where that serves (2,048 points or more,
+ * k h <= 0.8, tau >= h, k tau >= 2^-28, k times the domain's diagonal below
+ * 4000), else FP64 instructions.  An entry is off by about 2^-46.5 of itself,
+ * so a product of a smooth density by as much as in FP64 instructions or less
+ * (their long sums lose more), one of a random or concentrated density by up to
+ * five times as much (1.1e-15 against 2e-16 at n = 2,938).  HZ_F64_PLAIN: FP64
+ * instructions (entries to about 2^-50) everywhere. */
+#define HZ_F64_SPLIT 0
+#define HZ_F64_PLAIN 1
+HZ_API int hz_set_f64_mode(hz_operator *op, int mode);
+
 /* Per-kernel timing of the pair sweeps: CUDA events recorded on the launch
  * stream around every sweep kernel (also inside the solver's iteration
  * graphs).  enable = 1 / 0 switches it on / off and clears the totals,
@@ -205,7 +219,8 @@ HZ_API int hz_matvec_pair(hz_operator *op, int precision, const double *p_re, co
 /* Multi right-hand side: Q = A P for nrhs column vectors stored one after
  * the other (vector r at offset r*n), one kernel evaluation per pair and
  * kernel pass; a pass takes a block of 8, 16 or 32 right-hand sides (FP64:
- * 8 or 16), the smallest block that holds the remaining columns. */
+ * 8 or 16, in split arithmetic 4, 8 or 16), the smallest block that holds the
+ * remaining columns (FP32, 17 to 24: a block of 16 and one of 8). */
 HZ_API int hz_matvec_multi(hz_operator *op, int precision, int nrhs, const double *p_re,
                     const double *p_im, double *q_re, double *q_im, int where);
 

@@ -15,10 +15,11 @@ def two_spheres(N):
     return np.maximum(*f)
 
 
-def columns(hz, oracle, p, d, count, rng, scale=1.0):
-    """(largest error of a column's entries over their bound, n): sources with
-    the closest far neighbours and `count` others.  The bound's scale is the
-    entry with |x_t - x_s| for the projection (w (k + 1/rho) / (4 pi rho))."""
+def column_errors(hz, oracle, p, d, count, rng, mode=0):
+    """Errors of columns of A and A^H over their entries' size, with max(rho,
+    tau) and max |x|: sources with the closest far neighbours and `count`
+    others.  An entry's size has |x_t - x_s| for the projection
+    (w (k + 1/rho) / (4 pi rho))."""
     import oracle as O
     po = O.make_params(p.N, p.wave, int_l=p.int_l, int_u=p.int_u, factor=p.factor, tau_factor=p.tau_factor,
                        dirichlet=p.dirichlet, interior=p.interior)
@@ -28,6 +29,7 @@ def columns(hz, oracle, p, d, count, rng, scale=1.0):
     tau = p.tau_factor * (p.int_u - p.int_l) / p.N
     with hz.Operator(p) as op:
         op.set_distance(d)
+        op.set_f64_mode(mode)
         n = op.build()
         assert n == len(w)
         near = np.full(n, np.inf)
@@ -35,7 +37,6 @@ def columns(hz, oracle, p, d, count, rng, scale=1.0):
             r = np.linalg.norm(xs[i:i + 512, None] - xs[None], axis=2)
             near[i:i + 512] = np.where(r > tau, r, np.inf).min(axis=1)
         pick = np.concatenate([np.argsort(near)[:count], rng.integers(0, n, count)])
-        worst = 0.0
         for adjoint in (False, True):
             for s in pick:
                 v = np.zeros(n, dtype=complex)
@@ -47,14 +48,19 @@ def columns(hz, oracle, p, d, count, rng, scale=1.0):
                 size = np.abs(np.where(p.dirichlet ^ adjoint, reg[s], reg))
                 size[far] = (p.wave + 1 / rho[far]) / (4 * np.pi * rho[far])
                 size *= w if adjoint else w[s]
-                # r^2 off by 2^-43, three halves of it in the entry, the rest of
-                # the split arithmetic 2^-44; coordinates times k 2^-53 of |x|
-                # each, seven times that over rho
-                tol = 2.0 ** -42 + 2.0 ** -50 * np.abs(xs).max() / np.maximum(rho, tau)
                 err = np.abs(q - A * v[s]) / abs(v[s])
-                err[s] -= 2.0 ** -52
-                worst = max(worst, float(np.max(err / np.where(size > 0, tol * size, np.inf))))
-        return worst, n
+                err[s] = max(0.0, err[s] - 2.0 ** -52)  # beside the diagonal's 1/2
+                yield err[size > 0] / size[size > 0], np.maximum(rho, tau)[size > 0], np.abs(xs).max()
+
+
+def columns(hz, oracle, p, d, count, rng):
+    """Largest error of an entry over its bound: r^2 off by 2^-43, three halves
+    of it in the entry, the rest of the split arithmetic 2^-44; coordinates times
+    k 2^-53 of |x| each, seven times that over rho."""
+    worst, n = 0.0, 0
+    for err, rho, x in column_errors(hz, oracle, p, d, count, rng):
+        worst, n = max(worst, float(np.max(err / (2.0 ** -42 + 2.0 ** -50 * x / rho)))), len(err)
+    return worst, n
 
 
 @pytest.mark.parametrize("tau_factor", [2.0, 1.0, 0.999, 0.25, 0.02, 1e-3, 1e-6])
@@ -99,3 +105,58 @@ def test_units_of_length(hz, oracle, half, k, dirichlet):
         pq, pt = op.matvec_pair(V[0], V[1])
         assert np.max(np.abs(pq - one[0])) <= 2.0 ** -42 * 4
         assert np.max(np.abs(pt - op.matvec(V[1], adjoint=True))) <= 2.0 ** -42 * 4
+
+
+@pytest.mark.parametrize("k,dirichlet", [(5.0, 1), (8.4, 0)])
+def test_entries_in_both_arithmetics(hz, oracle, k, dirichlet):
+    """Split arithmetic: entries off by 2^-46.5 of themselves, root mean square
+    (and by no more than the other tests' bound); FP64 instructions by less than
+    a quarter of that."""
+    from helmholtz_3d_torrone_gb300 import geometry as G
+    p = hz.params(24, k, int_l=-1.0, int_u=1.0, factor=3.0, dirichlet=dirichlet)
+    d = G.sphere(24, radius=0.5, center=(0.011, 0.017, 0.005))
+
+    def rms(mode):
+        e = [e for e, _, _ in column_errors(hz, oracle, p, d, 20, np.random.default_rng(5), mode=mode)]
+        return float(np.sqrt(np.mean(np.concatenate(e) ** 2)))
+
+    split, plain = rms(hz.F64_SPLIT), rms(hz.F64_PLAIN)
+    assert split <= 2.0 ** -46 and plain <= split / 4
+
+
+def test_switching_the_arithmetic(hz):
+    """hz_set_f64_mode before and after the build, in products, columns, solves
+    (whose graphs hold the sweep's launches), gradients and batches."""
+    from helmholtz_3d_torrone_gb300 import geometry as G
+    p = hz.params(24, 5.0, int_l=-1.0, int_u=1.0, factor=3.0, dirichlet=1)
+    d = G.sphere(24, radius=0.5, center=(0.011, 0.017, 0.005))
+    rx = G.random_sphere_points(5, 0.9, seed=6)
+    with hz.Operator(p) as op, hz.Operator(p) as first:
+        first.set_f64_mode(hz.F64_PLAIN)
+        for o in (op, first):
+            o.set_distance(d)
+            n = o.build()
+        v = np.exp(1j * np.arange(n) / n)
+
+        def outputs(o):
+            q, qt = o.matvec_pair(v, v)
+            x, info = o.solve(v, method=hz.BICG, precision=hz.PREC_F64, tol=1e-9)
+            g = o.misfit_gradient(v, rx, np.ones(5, dtype=complex), method=hz.GMRES, precision=hz.PREC_F64, tol=1e-9)
+            with hz.Batch([o]) as b:
+                bq = b.matvec([v], precision=hz.PREC_F64)[0]
+            return [o.matvec(v), o.matvec(v, adjoint=True), q, qt, o.matvec_multi([v, 2 * v], precision=hz.PREC_F64),
+                    x, g[1], np.array([g[0], g[2]]), bq]
+
+        split, plain = outputs(op), outputs(first)
+        for a, b in zip(split, plain):
+            assert not np.array_equal(a, b) and np.max(np.abs(a - b)) <= 1e-7 * np.max(np.abs(b))
+        for mode, want in ((hz.F64_PLAIN, plain), (hz.F64_SPLIT, split)):
+            op.set_f64_mode(mode)
+            for a, b in zip(outputs(op), want):
+                assert np.array_equal(a, b)
+            op.build()
+            for a, b in zip(outputs(op), want):
+                assert np.array_equal(a, b)
+        with pytest.raises(hz.HzError) as e:
+            op.set_f64_mode(2)
+        assert e.value.code == hz.HZ_ERR_ARG
