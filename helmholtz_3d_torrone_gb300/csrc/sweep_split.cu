@@ -983,21 +983,29 @@ RecSplit split_record_views(void *mem, const Rec32 &r)
     return v;
 }
 
-// Where the split sweep serves: the table reduction of the origin phases ends
-// at k rho = 4000 (as the FP64 sweep's); k h <= 0.8 (eight points a
-// wavelength) keeps the phases within a tile small, so the error stays at or
-// below the FP64 sweep's (at k h = 1, 4.5e-15 against 4.2e-15); k tau >= 2^-28
-// keeps 1/(k rho)^2 below 2^56 and the units of a close tile's r^2, 2^-53 of
-// (k tau)^2, inside the FP32 range; below 2048 points the FP64
-// sweep's error (2e-15 and less) is the smaller one.  tau >= h: the projection
-// (x_t - x_s).n carries an error of 2^-51 of the tile's radius (10 to 30 h),
-// which is 2^-46 of the nearest far pairs' entries at rho = h and would grow as
-// 1 / rho below (the FP64 sweep keeps that at k below 1, where it subtracts the
-// unscaled coordinates).
+// Where the split sweep serves.
+// * k rho < 4000: there the table reduction of the origin phases ends (as the
+//   FP64 sweep's).
+// * (k h)^2 <= sqrt(n) / 308 (k h <= 0.42 at n = 2,938, 0.56 at 9,352, 0.79 at
+//   36,212) and k h <= 0.8: the phases, and with them the entries' error, grow
+//   with k h, the FP64 sweep's error with its sequential sum over n.  Error of
+//   smooth densities, root mean square over A and A^H of both problems, as a
+//   part of the FP64 sweep's: n = 2,308 at k h = 0.4 0.94, 2,938 at 0.42 0.81 (at
+//   0.5 1.23), 5,675 at 0.5 0.75, 9,352 at 0.5 0.82 (0.6 1.01), 13,952 at 0.6 0.84,
+//   19,532 at 0.7 0.93 (0.8 1.18), 36,212 at 0.78 0.68.
+// * n >= 2048: towards that size the two errors meet (n = 2,308, k h 0.2 to 0.4:
+//   0.82 to 1.07).  The FP64 sweep takes milliseconds there, the split one 0.1.
+// * k tau >= 2^-28 keeps 1/(k rho)^2 below 2^56 and the units of a close tile's
+//   r^2, 2^-53 of (k tau)^2, inside the FP32 range.
+// * tau >= h: the projection (x_t - x_s).n carries an error of 2^-51 of the
+//   tile's radius (10 to 30 h), which is 2^-46 of the nearest far pairs' entries
+//   at rho = h and would grow as 1 / rho below (the FP64 sweep keeps that at k
+//   below 1, where it subtracts the unscaled coordinates).
 bool split_serves(int64_t n, double wave, double H, double tau, double extent)
 {
-    return n >= 2048 && wave > 1e-100 && wave < 1e100 && wave * tau >= 0x1p-28 && wave * H <= 0.8 && tau >= H &&
-           wave * extent < 4000.0;
+    const double kh = wave * H;
+    return n >= 2048 && wave > 1e-100 && wave < 1e100 && wave * tau >= 0x1p-28 && kh <= 0.8 &&
+           308.0 * kh * kh <= sqrt((double)n) && tau >= H && wave * extent < 4000.0;
 }
 
 int build_split_records(const SweepConst &c, const RecSplit &v, const Rec32 &r, const double4_32a *pos,

@@ -107,7 +107,7 @@ def test_units_of_length(hz, oracle, half, k, dirichlet):
         assert np.max(np.abs(pt - op.matvec(V[1], adjoint=True))) <= 2.0 ** -42 * 4
 
 
-@pytest.mark.parametrize("k,dirichlet", [(5.0, 1), (8.4, 0)])
+@pytest.mark.parametrize("k,dirichlet", [(5.0, 1), (4.0, 0)])
 def test_entries_in_both_arithmetics(hz, oracle, k, dirichlet):
     """Split arithmetic: entries off by 2^-46.5 of themselves, root mean square
     (and by no more than the other tests' bound); FP64 instructions by less than
@@ -160,3 +160,45 @@ def test_switching_the_arithmetic(hz):
         with pytest.raises(hz.HzError) as e:
             op.set_f64_mode(2)
         assert e.value.code == hz.HZ_ERR_ARG
+
+
+@pytest.mark.parametrize("N,kh", [(24, 0.41), (24, 0.43), (24, 0.5), (24, 0.79), (34, 0.49), (34, 0.7), (44, 0.79)])
+def test_smooth_densities_lose_nothing(hz, N, kh):
+    """Products of plane-wave densities, A and A^H of both problems, against rows
+    in long double: what runs by default is off by no more than the FP64
+    instructions (5 % for the sample of rows)."""
+    from helmholtz_3d_torrone_gb300 import geometry as G
+    LD, k = np.longdouble, kh * N / 2
+    err = np.zeros(2)
+    for dirichlet in (1, 0):
+        rng = np.random.default_rng(N)
+        with hz.Operator(hz.params(N, k, int_l=-1.0, int_u=1.0, factor=3.0, dirichlet=dirichlet)) as op:
+            op.set_distance(G.sphere(N, radius=0.5, center=(0.011, 0.017, 0.005)))
+            n = op.build()
+            t = op.tube()
+            x, nrm, w, reg = t["xs"].reshape(-1, 3), t["nrm"].reshape(-1, 3).astype(LD), t["w"], t["reg"].astype(LD)
+            V = []
+            for _ in range(4):
+                u = rng.standard_normal((4, 3))
+                a = rng.standard_normal(4) + 1j * rng.standard_normal(4)
+                V.append(np.exp(1j * k * (x @ (u / np.linalg.norm(u, axis=1)[:, None]).T)) @ a)
+            rows = rng.choice(n, 32, replace=False)
+            for adjoint in (False, True):
+                src = bool(dirichlet) != adjoint  # whose normal the entry has
+                want = np.empty((len(V), len(rows)), dtype=np.clongdouble)
+                for i, r in enumerate(rows):
+                    D = x[r].astype(LD) - x.astype(LD)
+                    rho = np.sqrt((D * D).sum(axis=1))
+                    far = np.sqrt(((x[r] - x) ** 2).sum(axis=1)) > op.p.tau_factor * 2.0 / N
+                    rho[~far] = 1
+                    c, s = np.cos(LD(k) * rho), np.sin(LD(k) * rho)
+                    f = (D * (nrm if src else nrm[r])).sum(axis=1) / (4 * np.arctan(LD(1)) * 4 * rho * rho)
+                    e = (-(c / rho + LD(k) * s) + 1j * (LD(k) * c - s / rho)) * f
+                    e = np.where(far, -e.conj() if adjoint else e, (reg if src else reg[r]) + 0j)
+                    e = e * (w[r] if adjoint else w).astype(LD)
+                    want[:, i] = [(e * v).sum() + v[r] / 2 for v in V]
+                for m, mode in enumerate((hz.F64_SPLIT, hz.F64_PLAIN)):
+                    op.set_f64_mode(mode)
+                    got = np.array([op.matvec(v, adjoint=adjoint)[rows] for v in V])
+                    err[m] += float((np.abs(got - want) ** 2).sum() / (np.abs(want) ** 2).sum())
+    assert err[0] <= 1.05 ** 2 * err[1]
