@@ -13,6 +13,7 @@ central differences of the reference's own solve.
 """
 import multiprocessing as mp
 import os
+import unittest
 
 import numpy as np
 
@@ -40,6 +41,11 @@ def _serve(conn, variant, N, wave, d, want_matrix, threads, chunk):
     conn.close()
 
 
+class ReferenceNotBuilt(unittest.SkipTest):
+    """The reference build is not on this machine: a test that asks for it is
+    skipped, anything else sees an exception."""
+
+
 class RefWorker:
     """One reference configuration in a child process: .tube has the
     reference's tube (idx, xs, nrm, delta, jac, reg, w, and the dense matrix
@@ -47,6 +53,10 @@ class RefWorker:
     that OpenMP chunk when omp_chunk > 0)."""
 
     def __init__(self, variant, N, wave, d, matrix=False, timeout=900, threads=None, omp_chunk=0):
+        from oracle import REF_DIR
+        lib = os.path.join(REF_DIR, "libref_%s.so" % variant)
+        if not os.path.exists(lib):
+            raise ReferenceNotBuilt("no reference build: " + lib)
         ctx = mp.get_context("spawn")
         self.timeout = timeout
         threads = threads or (os.cpu_count() or 1)
