@@ -41,13 +41,13 @@ __device__ __noinline__ bool field_pair(double x, double y, double z, double nx,
 // division are 67 FP64 instructions a pair; far_factor64 on (k r)^2 is 39, and
 // two a source for w sigma are shared by the R receivers.  Coordinates are
 // subtracted unscaled, so neither the factor nor the test r <= tau depends on
-// how far from the origin the box lies.  The 32 KB phase table is filled once a block, so the blocks stay
-// and take receivers in turn.  The table serves k r < 4000; pairs beyond,
-// within 1e-12 of tau, and NaN go through field_pair.
+// how far from the origin the box lies.  The 32 KB phase table is filled once a
+// block, so the blocks stay and take receivers in turn.  The table serves
+// k r < 4000; pairs beyond, within 1e-12 of tau, and NaN go through field_pair.
 // The split FP32 arithmetic of the products would be 8 times as fast, but
 // its entries carry 2^-46.5 where these carry 2^-52: a field was off by
 // 2.2e-15 instead of 5e-16.  9,216 receivers of a sphere's tube at 48^3:
-// 13.3 -> 8.2 ms.
+// 13.3 -> 8.3 ms.
 template <bool SINGLE, int R>
 __global__ void __launch_bounds__(kEvalThreads, 2)
     eval_kernel(int64_t n, const double4_32a *__restrict__ pos, const double4_32a *__restrict__ nrm,
@@ -121,15 +121,16 @@ __global__ void __launch_bounds__(kEvalThreads, 2)
     }
 }
 
-// The phase table holds for receivers in general position; k = 0, a negative k
-// and one so small that (k tau)^2 leaves the FP32 range take field_pair alone.
+// The phase table holds for receivers in general position; k = 0, a negative k,
+// one so small that (k tau)^2 leaves the FP32 range and one whose cube leaves the
+// FP64 range take field_pair alone.
 template <bool SINGLE, int R>
 int eval_blocks(int64_t n, const double4_32a *pos, const double4_32a *nrm, const double *s_re, const double *s_im,
                 int64_t m, const double *rx, double wave, double tau, double sg, double *u_re, double *u_im,
                 cudaStream_t s)
 {
     const double kt = wave * tau, inf = std::numeric_limits<double>::infinity();
-    const bool table = wave > 0.0 && kt * kt > 1e-30 && kt < 4000.0;
+    const bool table = wave > 1e-100 && wave < 1e100 && kt * kt > 1e-30 && kt < 4000.0;
     // the table's pairs are the fields' over k (single layer) and k^3
     const double f = !table ? 1.0 : SINGLE ? wave : wave * wave * wave, c = (SINGLE ? -1.0 : sg) / (4.0 * 3.14159265358979323846264338328);
     int64_t b = (m + R - 1) / R;

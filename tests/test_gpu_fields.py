@@ -91,3 +91,34 @@ def test_fields_far_from_the_origin(hz, oracle, dirichlet):
                 if layer == hz.DOUBLE_LAYER:
                     size = size * (k + 1 / rho[far])
                 assert abs(got[i] - want[i]) <= (BOUND + 2.0 ** -49 * k * rho.max()) * size.sum()
+
+
+@pytest.mark.parametrize("half,k", [(1e102, 1e-104), (1e101, 1e-101), (1e-9, 5e9), (1e9, 5e-9)])
+@pytest.mark.parametrize("dirichlet", [0, 1])
+def test_fields_in_other_units_of_length(hz, oracle, half, k, dirichlet):
+    """Boxes whose k^3 leaves the FP64 range, and ones whose k^3 does not (boxes
+    below 1e-18 are out of reach: the interpolation adds 1e-19 to a coordinate)."""
+    import oracle as O
+    from helmholtz_3d_torrone_gb300 import geometry as G
+    N = 16
+    d = G.sphere(N, radius=0.5, center=(0.011, 0.017, 0.005)) * half
+    p = hz.params(N, k, int_l=-half, int_u=half, factor=3.0, dirichlet=dirichlet)
+    po = O.make_params(N, k, int_l=-half, int_u=half, factor=3.0, dirichlet=dirichlet)
+    tp = oracle.pipeline(po, d)
+    rng = np.random.default_rng(8)
+    xs, w = np.asarray(tp["xs"]).reshape(-1, 3), np.asarray(tp["w"])
+    rx = half * rng.uniform(-1, 1, (40, 3))
+    with hz.Operator(p) as op:
+        op.set_distance(d)
+        n = op.build()
+        sigma = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+        for layer in (hz.SINGLE_LAYER, hz.DOUBLE_LAYER):
+            got = op.evaluate(rx, sigma, layer)
+            want = oracle.evaluate(po, tp, sigma, rx, layer == hz.DOUBLE_LAYER)
+            for i in range(len(rx)):
+                rho = np.sqrt((((xs - rx[i]) / half) ** 2).sum(axis=1)) * half
+                far = rho > 0.1 * po.tau_factor * 2 * half / N
+                size = np.abs(w * sigma)[far] / rho[far] / (4 * np.pi)
+                if layer == hz.DOUBLE_LAYER:
+                    size = size * (k + 1 / rho[far])
+                assert abs(got[i] - want[i]) <= (BOUND + 2.0 ** -49 * k * rho.max()) * size.sum()
