@@ -38,3 +38,26 @@ def test_grids_bitexact_vs_oracle(hz, oracle, N, step):
         if step == "box":
             for g, w in zip(hz.assign_gradient(d, N, H, weno_order=3), oracle.gradient(N, H, d, order=3)):
                 assert np.array_equal(np.asarray(g).ravel().view(np.uint64), np.asarray(w).ravel().view(np.uint64))
+
+
+@pytest.mark.parametrize("N", [8, 31])
+@pytest.mark.parametrize("step", ["box", "tiny"])
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+def test_nonfinite_nodes(hz, oracle, N, step, value):
+    """NaN and infinities at a few nodes, corners and neighbours among them: the
+    same nodes become NaN or infinite as in the oracle, the others keep their bits."""
+    H = {"box": 2.0 / N, "tiny": 2.0 ** -400}[step]
+    rng = np.random.default_rng(N)
+    for d in list(fields(N, 2.0 / N, N))[:3]:
+        d = np.array(np.broadcast_to(d, (N + 1,) * 3))
+        at = rng.integers(0, N + 1, (4, 3))
+        at[0] = 0
+        at[1] = (N, N, N // 2)
+        at[3] = np.minimum(at[2] + (0, 1, 2), N)
+        d[tuple(at.T)] = value * np.array([1, 1, 1, -1])
+        got = list(hz.assign_gradient(d, N, H)) + list(hz.assign_curvatures(d, N, H))
+        with np.errstate(all="ignore"):
+            want = list(oracle.gradient(N, H, d)) + list(oracle.curvatures(N, H, d))
+        for g, w in zip(got, want):
+            g, w = np.asarray(g).ravel(), np.asarray(w).ravel()
+            assert np.all((g.view(np.uint64) == w.view(np.uint64)) | (np.isnan(g) & np.isnan(w)))
