@@ -71,3 +71,20 @@ def test_fp32_products(hz, shape, N, k, half, dirichlet, interior):
             for v in range(4):
                 batch.set_variant(v)
                 assert close(batch.matvec([V[0]])[0], Q[0], sums)
+
+
+def test_phase_modes_give_one_product(hz):
+    """hz_set_phase_mode takes both settings, and both run the same sweep."""
+    op, n = operator(hz, "sphere", 24, 9.0, 1)
+    v = np.exp(1j * np.arange(n))
+    with op:
+        out = []
+        for mode in (hz.PHASE_DIRECT, hz.PHASE_SPLIT):
+            op.set_phase_mode(mode)
+            out.append([op.matvec(v, precision=hz.PREC_F32), *op.matvec_pair(v, v, precision=hz.PREC_F32)])
+        for a, b in zip(*out):
+            assert np.array_equal(a, b)
+        for mode in (-1, 2):
+            with pytest.raises(hz.HzError) as e:
+                op.set_phase_mode(mode)
+            assert e.value.code == hz.HZ_ERR_ARG
