@@ -4,14 +4,16 @@
 // SCALED records hold the coordinates times k (Rec32::lambda = k), so that
 // rho below is k rho and the entry's factor is
 //   e^{i rho} (-1/rho + i) / rho^2 (x_t - x_s).n   (k^2 on the densities).
-// In a tile without near pairs whose radius is at most kCentreRadius the phase
-// is taken about the tile: theta = rho - rc with rc = |x_t - o|, the FP32
+// In a tile whose radius is at most kCentreRadius the phase is taken about the
+// tile (tiles with near pairs too, in the single and batched sweeps, whose
+// regularised pairs have sums of their own; not in the multi right-hand-side
+// sweep, which has one sum for both): theta = rho - rc with rc = |x_t - o|, the FP32
 // distance to the tile's origin, so |theta| is at most the radius, needs no
 // range reduction before the SFU's sin and cos, and the tile's sum is turned
 // once by e^{i rc} (Turn).  Any FP32 value near |x_t - o| serves as rc, as
 // long as the turn belongs to that very value.  22 FP32 instructions and
 // three SFU ones a pair, against 29 and three with the phase k rho reduced
-// per pair, which the other tiles keep.
+// per pair, which wider tiles and the multi sweep's near tiles keep.
 //
 // Records with lambda = 1 (k below 2^-14, negative k, k tau below 2^-40:
 // lambda32 in sweep_f32.cu) reduce k rho in revolutions with k/(2 pi) split

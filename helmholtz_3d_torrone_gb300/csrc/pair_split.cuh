@@ -4,8 +4,7 @@
 //
 // GB300 issues one FP64 instruction for about 70 FP32 ones, so a pair
 // evaluated here (about 215 FP32-pipe slots) costs a tenth of the 38.5 FP64
-// instructions of pair64.cuh.  What keeps the result as accurate as the FP64
-// sweep's:
+// instructions of pair64.cuh.  What keeps the error small:
 //
 // * Coordinates are scaled by k and taken about the source tile's origin o:
 //   s = x_s - o, a = x_t - o, A = -2a, all formed in FP64 and split into a
@@ -30,10 +29,12 @@
 //   entries r^2/2 < 7.4e-8 and its FP32 rounding stays below 2^-47.
 // * Products drop only tail times tail; sums use TwoSum (Knuth) or, where
 //   the order of magnitude is known, Fast2Sum (Dekker).
-// Entries carry a relative error of about 2^-46.5, of random sign: a product
-// of a smooth density on n points is off by 1.9e-15 (n = 2,938) to 3e-15
-// (n = 36,212), against 2.4e-15 to 9.7e-15 for the FP64 sweep, whose
-// sequential FP64 sum grows like sqrt(n).
+// Entries carry a relative error of about 2^-46.5, of random sign, against
+// 2^-50 in pair64.cuh, whose sums of n entries one after another add an error
+// that grows like sqrt(n): which of the two is the smaller in a product of a
+// smooth density depends on n and k h (split_serves has the figures and the
+// line).  A random or concentrated density gets the entries' own error: at
+// n = 2,938 1.2e-15 against 2.4e-16.
 #pragma once
 
 #include <cstdint>

@@ -10,9 +10,9 @@
 //    x_t - o = (t_hi - o_hi) + (t_lo - o_lo): the head difference is rounded
 //    to half an ulp of itself, so the offset of close pairs keeps FP32
 //    relative precision with no FP64 instruction in the tile loop.
-//  * Coordinates are stored times k, and away from near tiles the phase is
-//    taken about the source tile's origin (pair32.cuh): |k rho - k rho_c| is
-//    small, goes to the SFU's sin/cos without a range reduction, and the
+//  * Coordinates are stored times k, and the phase is taken about the source
+//    tile's origin (pair32.cuh), except where a tile's radius is above 6 / k:
+//    |k rho - k rho_c| is small, goes to the SFU's sin/cos without a range reduction, and the
 //    tile's sum is turned by e^{i k rho_c} once.  Against the phase reduced per
 //    pair the error to the FP64 product fell, 3.2e-7 -> 2.6e-7 of |K p| on the
 //    64^3 torus (k = 15) and 3.4e-7 -> 3.1e-7 at 128^3 (k = 20).
@@ -93,8 +93,9 @@ template <int MODE>
 constexpr int kStage = (kFixed + kDens<MODE>) * kTile32;  // floats of a staged tile
 
 // A tile counts `sub` units, and the FP32 sums over a unit are added to the
-// cross-tile sums one by one: a product does not depend on where the units are
-// cut.  Whole tiles are the cheapest (a unit's end costs 2 % of a half), but
+// cross-tile sums one by one, so products agree to the rounding of those sums
+// (about 2^-48) wherever the units are cut: variants and grid sizes change
+// their last bits.  Whole tiles are the cheapest (a unit's end costs 2 % of a half), but
 // small tubes need parts for every CTA to have its share: n = 2,938 0.042 ms
 // with tiles, 0.039 with halves, 0.037 with quarters; n = 9,765 0.123 and
 // 0.120 with halves; n = 145,272 17.5 with tiles, 17.9 with halves.
@@ -104,7 +105,7 @@ int sub_of(int64_t ntiles) { return ntiles < 24 ? 4 : ntiles < 80 ? 2 : 1; }
 // Relative cost of a tile: far, near tile (near-field test, its branch
 // taken now and then), the target tile itself (taken for most sources).
 constexpr int kCostFar = 16, kCostNear = 19, kCostSelf = 30;
-constexpr int kCuts = 16384;  // equal-cost cuts kept per tube: 27 or more a CTA
+constexpr int kCuts = 16384;  // equal-cost cuts kept per tube: 26 or more a CTA (608 CTAs)
 
 // First unit of CTA c of P.  Cut by count, the CTAs with the near tiles set
 // the time: 0.149 ms at n = 9,765 and 1.30 at n = 36,212, of which 0.03 and

@@ -173,9 +173,10 @@ HZ_API int64_t hz_tube_size(const hz_operator *op);
 HZ_API int hz_autotune(hz_operator *op, int *chosen, double *ms_per_sweep);
 HZ_API int hz_set_sweep_config(hz_operator *op, int cfg);
 
-/* Phase of the FP32 pair sweep.  Every FP32 sweep takes the phase about the
- * source tile's origin, which needs no reduction per pair; both settings are
- * accepted and run it. */
+/* Phase of the FP32 pair sweeps.  They take it about the source tile's origin,
+ * where it needs no reduction per pair (tiles wider than 6 / k, and the multi
+ * right-hand-side sweep's near tiles, reduce it per pair; the Combo sweep passes
+ * it to the SFU as one FP32 product).  Both settings are accepted and run this. */
 #define HZ_PHASE_DIRECT 0
 #define HZ_PHASE_SPLIT 1
 HZ_API int hz_set_phase_mode(hz_operator *op, int mode);
