@@ -16,7 +16,7 @@ solve through the public C ABI with host buffers (H2D of b, D2H of x inside
 the timed region).
 
 Beside it: the plain FP64 GPU solve with the same method (measured seconds
-of one FP64 product x the product count of a complete FP64 GMRES(120)
+of one FP64 product, in split arithmetic too, x the product count of a complete FP64 GMRES(120)
 solve of this workload, measured once with ``--solve --fp64-full`` and
 recorded in FP64_SOLVE_ITERS), the roofline of the sweep that takes most of
 the solve's time and of the other one, and the FP32 sweep's rate over ``--steps`` timed inner iterations (L2
@@ -67,18 +67,13 @@ def fp64_solve_products(N, wave):
     return FP64_SOLVE_ITERS if (N, float(wave)) == FP64_SOLVE_ITERS_WORKLOAD else None
 
 
-# DRAM bytes (read + write) per launch of the fused FP32 sweep at 256^3:
-# 22.36 MB measured by ncu on the 128^3 torus (n = 145,272), scaled by n to
-# n = 581,420.  The sweep reads every record once from DRAM and the tiles
-# from L2, so traffic grows in proportion to n.
-SWEEP32_TRAFFIC = 22.36e6 * 581420 / 145272
-# The same for one A p launch of the FP32 sweep: 15.19 MB measured by ncu on
-# the 128^3 torus, scaled by n.
-SWEEP32_TRAFFIC_A = 15.19e6 * 581420 / 145272
-SWEEP64_TRAFFIC = 16.5e6 * 581420 / 145272  # ncu DRAM read of the FP64 sweep at 128^3, scaled by n
-# FP32-pipe slots per pair of the A-mode FP64 sweep, which works in pairs of
-# FP32 numbers and 64-bit integers (counted in the source)
-FP64_SLOTS_PER_PAIR = 215
+# DRAM bytes (read + write) of one A p launch, measured by ncu on the 128^3
+# torus (n = 145,272) and scaled by n: the sweeps read their records once from
+# DRAM and the tiles from L2, so traffic grows in proportion to n.
+SWEEP32_TRAFFIC_A = 14.42e6 * 581420 / 145272  # sweep32_kernel
+SWEEP64_TRAFFIC = 23.85e6 * 581420 / 145272    # sweep_split_kernel
+# Instructions issued per pair by the A-mode split FP64 sweep (ncu, same torus)
+FP64_INSTRUCTIONS_PER_PAIR = 232
 
 
 def parse():
@@ -464,14 +459,16 @@ def run_gb300(a, rank, world, local):
               "share_of_solve": (sinfo["iterations"] * avg_sweep_s / solve_s) if avg_sweep_s else None}
     roof64 = None
     if f64:
+        issue_peak = torch.cuda.get_device_properties(dev).multi_processor_count * 128 * clk["sm_mhz"] * 1e6 if clk else None
         a64 = float(n) * n * FLOPS_PER_PAIR / f64["seconds_per_product"] / 1e12
         roof64 = {"bound": "fp32", "kernel": "sweep_split_kernel (A x, the FP64 refinement residual)",
                   "achieved": a64, "peak": fp32_peak, "unit": "TFLOP/s", "frac": a64 / fp32_peak,
-                  "fp64_peak": fp64_peak, "fp32_slots_per_pair": FP64_SLOTS_PER_PAIR,
-                  "pipe_frac": float(n) * n * FP64_SLOTS_PER_PAIR / f64["seconds_per_product"] / (fp32_peak * 0.5e12),
+                  "fp64_peak": fp64_peak, "instructions_per_pair": FP64_INSTRUCTIONS_PER_PAIR,
+                  "issue_frac": (float(n) * n * FP64_INSTRUCTIONS_PER_PAIR / f64["seconds_per_product"] / issue_peak
+                                 if issue_peak else None),
                   "note": "FP64 products in split FP32 arithmetic: frac counts the reference formula's 40 flops per "
-                          "pair against the FP32 FFMA peak (2 flops per instruction); pipe_frac counts the FP32-pipe "
-                          "slots the kernel takes against the pipe's instruction rate (peak / 2)",
+                          "pair against the FP32 FFMA peak (2 flops per instruction); issue_frac counts the "
+                          "instructions issued per pair (ncu) against four warp instructions a clock an SM",
                   "traffic": SWEEP64_TRAFFIC, "flops_per_pair": FLOPS_PER_PAIR, "pairs_per_launch": n * n,
                   "avg_launch_ms": f64["seconds_per_product"] * 1e3, "launches_timed": a.fp64_iters,
                   "peak_source": "FP32 FFMA chains measured live on this GPU (hz_measure_fma_peaks)",
