@@ -666,7 +666,7 @@ int hz_build(hz_operator *op, int64_t *n_out)
                      op->dreg.as<double>()));
     HZ_TRY(check_device_error(op, "hz_build"));
     const SweepConst sc = sweep_const(op);
-    op->use_split = split_serves(n, sc.wave, op->H, op->tau, sc.extent);
+    op->use_split = split_serves(n, sc.wave, op->H, op->tau, sc.extent, sc.dirichlet != 0);
     HZ_TRY(build_records64(op));
     const double lambda = lambda32(op->p.wave, op->tau);
     HZ_TRY(build_records32(op, lambda, sweep32_reg_scale(op->p.interior, lambda)));

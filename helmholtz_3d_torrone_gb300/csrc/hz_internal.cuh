@@ -236,7 +236,7 @@ int sweep_f64(const SweepConst &c, const Rec64 &r, int mode, const double *p_re,
 // sweep_split.cu
 size_t split_record_bytes(int64_t npad);
 RecSplit split_record_views(void *mem, const Rec32 &r);
-bool split_serves(int64_t n, double wave, double H, double tau, double extent);
+bool split_serves(int64_t n, double wave, double H, double tau, double extent, bool dirichlet);
 int build_split_records(const SweepConst &c, const RecSplit &v, const Rec32 &r, const double4_32a *pos,
                         const double4_32a *nrm, cudaStream_t s);
 int sweep_split(const SweepConst &c, const RecSplit &v, const double4_32a *nrm, int mode, const double *p_re,

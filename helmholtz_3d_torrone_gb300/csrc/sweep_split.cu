@@ -986,26 +986,35 @@ RecSplit split_record_views(void *mem, const Rec32 &r)
 // Where the split sweep serves.
 // * k rho < 4000: there the table reduction of the origin phases ends (as the
 //   FP64 sweep's).
-// * (k h)^2 <= sqrt(n) / 308 (k h <= 0.42 at n = 2,938, 0.56 at 9,352, 0.79 at
-//   36,212) and k h <= 0.8: the phases, and with them the entries' error, grow
-//   with k h, the FP64 sweep's error with its sequential sum over n.  Error of
-//   smooth densities, root mean square over A and A^H of both problems, as a
-//   part of the FP64 sweep's: n = 2,308 at k h = 0.4 0.94, 2,938 at 0.42 0.81 (at
-//   0.5 1.23), 5,675 at 0.5 0.75, 9,352 at 0.5 0.82 (0.6 1.01), 13,952 at 0.6 0.84,
-//   19,532 at 0.7 0.93 (0.8 1.18), 36,212 at 0.78 0.68.
-// * n >= 2048: towards that size the two errors meet (n = 2,308, k h 0.2 to 0.4:
-//   0.82 to 1.07).  The FP64 sweep takes milliseconds there, the split one 0.1.
+// * (k h)^2 <= n^(1/2) / 308 (Dirichlet; k h <= 0.42 at n = 2,938, 0.56 at 9,352, 0.79
+//   at 36,212) or n^(3/4) / 3480 (Neumann; 0.34, 0.52, 0.8), and k h <= 0.8: the
+//   phases, and with them the entries' error, grow with k h, the FP64 sweep's error
+//   with its sequential sum over n.  Error of smooth densities, root mean square,
+//   as a part of the FP64 sweep's, Dirichlet / Neumann: n = 2,938 at k h = 0.30
+//   0.71 / 0.83, 0.42 0.91 / 1.03; 3,427 at 0.23 0.73 / 0.81, 0.43 0.91 / 1.35; 3,906 at 0.17
+//   0.66 / 0.83, 0.41 0.92 / 1.12; 4,465 at 0.27 0.64 / 0.77, 0.46 0.95 / 0.98; 6,338 at 0.46
+//   0.70 / 0.70; 9,352 at 0.51 0.85 / 0.90, 0.56 0.90 / 1.16; 24,643 at 0.71 0.90 / 0.91; 36,212
+//   at 0.78 0.76 / 0.80.
+// * n >= 2800 and k h n^2 >= 2.4e6 (k h >= 0.28 at n = 2,938, 0.12 at 4,465, 0.03 at
+//   9,352): at low k the near pairs' projections, off by 2^-51 of the tile's
+//   radius, are the error, and a sum over few points costs FP64 instructions
+//   little.  The same part for the worse of A and A^H, Neumann: n = 2,511 at
+//   k h = 0.05 2.18, 0.36 1.21; 2,938 at 0.05 1.99, 0.11 1.28, 0.22 0.91; 3,427 at 0.10 1.18,
+//   0.16 1.16, 0.23 0.84; 4,465 at 0.04 1.28, 0.10 1.08, 0.17 0.86; 6,338 at 0.03 0.89; 9,352
+//   at 0.03 0.84; 57,290 at 0.01 0.35.  The FP64 sweep takes milliseconds there, the
+//   split one 0.1.
 // * k tau >= 2^-28 keeps 1/(k rho)^2 below 2^56 and the units of a close tile's
 //   r^2, 2^-53 of (k tau)^2, inside the FP32 range.
 // * tau >= h: the projection (x_t - x_s).n carries an error of 2^-51 of the
 //   tile's radius (10 to 30 h), which is 2^-46 of the nearest far pairs' entries
 //   at rho = h and would grow as 1 / rho below (the FP64 sweep keeps that at k
 //   below 1, where it subtracts the unscaled coordinates).
-bool split_serves(int64_t n, double wave, double H, double tau, double extent)
+bool split_serves(int64_t n, double wave, double H, double tau, double extent, bool dirichlet)
 {
-    const double kh = wave * H;
-    return n >= 2048 && wave > 1e-100 && wave < 1e100 && wave * tau >= 0x1p-28 && kh <= 0.8 &&
-           308.0 * kh * kh <= sqrt((double)n) && tau >= H && wave * extent < 4000.0;
+    const double kh = wave * H, m = (double)n;
+    const double most = dirichlet ? sqrt(m) / 308.0 : sqrt(m * sqrt(m)) / 3480.0;
+    return n >= 2800 && kh * m * m >= 2.4e6 && kh <= 0.8 && kh * kh <= most && wave > 1e-100 && wave < 1e100 &&
+           wave * tau >= 0x1p-28 && tau >= H && wave * extent < 4000.0;
 }
 
 int build_split_records(const SweepConst &c, const RecSplit &v, const Rec32 &r, const double4_32a *pos,

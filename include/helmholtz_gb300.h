@@ -183,9 +183,10 @@ HZ_API int hz_set_phase_mode(hz_operator *op, int mode);
 
 /* Arithmetic of the FP64 products (hz_matvec*, FP64 solves, refinement
  * residuals, dA/dk).  HZ_F64_SPLIT (default): pairs of FP32 numbers and 64-bit
- * integers, ten times as fast, where that serves (n >= 2,048 points,
- * (k h)^2 <= sqrt(n) / 308 and k h <= 0.8, tau >= h, k tau >= 2^-28, k times the
- * domain's diagonal below 4000), else FP64 instructions.  An entry is off by about 2^-46.5 of itself,
+ * integers, ten times as fast, where that serves (n >= 2,800 points,
+ * k h n^2 >= 2.4e6, (k h)^2 <= n^(1/2) / 308 (Neumann: n^(3/4) / 3480), k h <= 0.8,
+ * tau >= h, k tau >= 2^-28, k times the domain's diagonal below 4000), else FP64
+ * instructions.  An entry is off by about 2^-46.5 of itself,
  * so a product of a smooth density by as much as in FP64 instructions or less
  * (their long sums lose more), one of a random or concentrated density by up to
  * five times as much (1.1e-15 against 2e-16 at n = 2,938).  HZ_F64_PLAIN: FP64
