@@ -3,7 +3,7 @@
 // bits), or a 64-bit integer where cancellation would eat those bits.
 //
 // GB300 issues one FP64 instruction for about 70 FP32 ones, so a pair
-// evaluated here (about 215 FP32-pipe slots) costs a tenth of the 38.5 FP64
+// evaluated here (232 instructions) costs a tenth of the 38.5 FP64
 // instructions of pair64.cuh.  What keeps the error small:
 //
 // * Coordinates are scaled by k and taken about the source tile's origin o:

@@ -1,8 +1,9 @@
 // sweep_split.cu -- the FP64 products q = A p, qt = A^H pt (sweep_f64.cu) with
 // every pair evaluated as pairs of FP32 numbers (pair_split.cuh).
 //
-// Bound by the FP32 pipe: about 215 of its slots a pair (A p), against the 38.5
-// FP64 instructions (about 2,600 slots) of sweep64_kernel.
+// Bound by issue slots: 232 instructions a pair (A p; 326 for the fused pass) on
+// 77 % of the cycles, the FMA pipe 63 % busy (n = 145,272: 159 ms, 132 Gpair/s),
+// against the 38.5 FP64 instructions (about 2,600 FP32 slots) of sweep64_kernel.
 //
 // One thread owns one target of the blocked sweep order (Rec32::perm); a CTA
 // of 256 threads walks a contiguous range of (target tile, half or quarter
